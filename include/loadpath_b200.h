@@ -259,6 +259,8 @@ int lpb_dinv_mask_f64(double* av, const double* dinv, const uint8_t* m, int nx, 
 /* ---- SIMP loop (loadpath/simp.py:1143-1228, :1861, :1901-1904, :2001;
  * loadpath/benchmarks/reference.py:48-110; loadpath/femops.py:51-78, loadpath/mg.py:975-988) */
 int lpb_filter(double* out, const double* v, const int* toff, const double* tw, int ntaps, const double* hs_in, const double* hs_out, double* e_out, double penal, double emin, int nx, int ny, int nz, int pz, int cpz, void* stream);
+/* lpb_filter with the taps' reach (the largest |offset|) named by the caller */
+int lpb_filter_reach(double* out, const double* v, const int* toff, const double* tw, int ntaps, int reach, const double* hs_in, const double* hs_out, double* e_out, double penal, double emin, int nx, int ny, int nz, int pz, int cpz, void* stream);
 int lpb_simp_law(double* e, const double* x, double penal, double emin, int nx, int ny, int nz, int pz, int cpz, void* stream);
 int lpb_element_energy_f64(double* ce, const double* u, const double* v, const double* ke, int nx, int ny, int nz, int pz, int cpz, void* stream);
 /* femops.element_energy (loadpath/femops.py:236-242) on a general mesh: ce[e] = u_e^T ke v_e with
@@ -289,6 +291,12 @@ int lpb_project(double* xp, double* dxp, const double* xt, double beta, double e
 /* xn = clip(x sqrt(-dc / dv) / sqrt(lm), max(0, x - move), min(1, x + move)), held cells 1 / 0
  * (loadpath/simp.py:2314-2318, the optimality-criteria step at one volume multiplier) */
 int lpb_oc_stepped(double* xn, const double* x, const double* dc, const double* dv, double lm, double move, const uint8_t* flags, int nx, int ny, int nz, int pz, int cpz, void* stream);
+/* The same step, the filter and the projection of one trial in one pass: ts = x sqrt(-dc / dv), formed
+ * once per step (lpb_oc_step_base); then per multiplier lm xn = the clipped step, xt = H xn / hs, xp
+ * its projection, *vol = sum xp w. xn, xt, xp: all given, or all NULL when only the volume is wanted.
+ * part: 592 doubles (loadpath/simp.py:2320-2376, the volume multiplier's trials) */
+int lpb_oc_step_base(double* ts, const double* x, const double* dc, const double* dv, int nx, int ny, int nz, int pz, int cpz, void* stream);
+int lpb_oc_trial(double* xn, double* xt, double* xp, const double* ts, const double* x, double lm, double move, const uint8_t* flags, const int* toff, const double* tw, int ntaps, int reach, const double* hs, double beta, double eta, const double* w, double* part, double* vol, int nx, int ny, int nz, int pz, int cpz, void* stream);
 /* out = a * b (b NULL: a), 0 on held cells, then min(out, 0) (clip0 1) or max(out, 1e-12) (clip0 2):
  * the products the filter chain rule feeds to H^T and its clips (loadpath/simp.py:2001, :2077, :2191,
  * :2204) */

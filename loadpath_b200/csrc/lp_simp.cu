@@ -1,6 +1,5 @@
-// SIMP-loop kernels: the cone density filter and its transpose (loadpath/simp.py:1143-1228,
-// loadpath/benchmarks/reference.py:48-71), the SIMP law (loadpath/simp.py:1861), element
-// strain energy u_e^T Ke v_e (loadpath/femops.py:51-78, loadpath/mg.py:975-988), sensitivities
+// SIMP-loop kernels: the SIMP law (loadpath/simp.py:1861), element strain energy u_e^T Ke v_e
+// (loadpath/femops.py:51-78, loadpath/mg.py:975-988), sensitivities
 // (loadpath/benchmarks/reference.py:89-99) and the OC volume pass (reference.py:100-110).
 // All in float64.
 #include <algorithm>
@@ -8,122 +7,9 @@
 #include "lp_common.cuh"
 #include "lp_modal.cuh"
 
-#define LP_MAX_TAPS 1024
 #define LP_MAX_LAMBDA 64
 
 namespace {
-
-// out[c] = sum_t w_t v[c + d_t] (zeros outside the grid); optional pre-division of v by hs
-// and post-division of out by hs2; optional SIMP law on the result.
-//   mode 0: out = H v
-//   mode 1: out = H (v / hs_in)
-//   mode 2: out = (H v) / hs_out ; e_out = emin + out^p (1 - emin) if e_out != null
-// A block takes a tile of 32 x 8 cell columns times one z chunk (4 cells): it stages the tile with
-// its halo of reach R (the largest |offset| of the taps, up to LP_FT_R) in shared memory, v / hs_in
-// formed once per staged cell and zeros outside the grid, and each thread sums the taps for the 4
-// cells of its column in the taps' order, so the sums are those of a gather cell by cell. The
-// staging reads whole rows of chunks (32-byte sectors, contiguous along x). Taps reaching further
-// than LP_FT_R are gathered from global memory instead, cell by cell.
-#define LP_FT_X 32
-#define LP_FT_Y 8
-#define LP_FT_R 2
-__global__ void __launch_bounds__(256) k_filter(double* __restrict__ out, const double* __restrict__ v,
-                                                const int* __restrict__ toff, const double* __restrict__ tw,
-                                                int ntaps, const double* __restrict__ hs_in,
-                                                const double* __restrict__ hs_out, double* __restrict__ e_out,
-                                                double penal, double emin, LpGrid g) {
-  extern __shared__ unsigned char smem_raw[];
-  __shared__ double tile[(4 + 2 * LP_FT_R) * (LP_FT_Y + 2 * LP_FT_R) * (LP_FT_X + 2 * LP_FT_R)];
-  __shared__ int s_reach;
-  int* so = reinterpret_cast<int*>(smem_raw);
-  double* sw = reinterpret_cast<double*>(smem_raw + ((3 * ntaps * sizeof(int) + 15) & ~15));
-  if (threadIdx.x == 0) s_reach = 0;
-  __syncthreads();
-  int reach = 0;
-  for (int i = threadIdx.x; i < ntaps; i += blockDim.x) {
-    const int dx = toff[3 * i], dy = toff[3 * i + 1], dz = toff[3 * i + 2];
-    so[3 * i] = dx;
-    so[3 * i + 1] = dy;
-    so[3 * i + 2] = dz;
-    sw[i] = tw[i];
-    reach = max(reach, max(abs(dx), max(abs(dy), abs(dz))));
-  }
-  if (reach) atomicMax(&s_reach, reach);
-  __syncthreads();
-  const int R = s_reach;
-  const int nbx = (g.nx + LP_FT_X - 1) / LP_FT_X, nby = (g.ny + LP_FT_Y - 1) / LP_FT_Y;
-  const int bx = (int)(blockIdx.x % nbx), rest = (int)(blockIdx.x / nbx);
-  const int by = rest % nby, cz = rest / nby;
-  const int x0 = bx * LP_FT_X, y0 = by * LP_FT_Y;
-  const int x = x0 + (int)(threadIdx.x & 31), y = y0 + (int)(threadIdx.x >> 5);
-  const bool own = x < g.nx && y < g.ny;
-  if (R > LP_FT_R) {
-    if (!own) return;
-    for (int zq = 0; zq < 4; ++zq) {
-      const int z = 4 * cz + zq;
-      if (z >= g.nz) break;
-      double acc = 0.0;
-      for (int i = 0; i < ntaps; ++i) {
-        const int xx = x + so[3 * i], yy = y + so[3 * i + 1], zz = z + so[3 * i + 2];
-        if (xx < 0 || yy < 0 || zz < 0 || xx >= g.nx || yy >= g.ny || zz >= g.nz) continue;
-        const long long c = g.cell(xx, yy, zz);
-        double vi = v[c];
-        if (hs_in) vi = vi / hs_in[c];
-        acc += sw[i] * vi;
-      }
-      const long long c = g.cell(x, y, z);
-      if (hs_out) acc = acc / hs_out[c];
-      out[c] = acc;
-      if (e_out) e_out[c] = emin + pow(acc, penal) * (1.0 - emin);
-    }
-    return;
-  }
-  const int XH = LP_FT_X + 2 * R, YH = LP_FT_Y + 2 * R, ZH = 4 + 2 * R, P = XH * YH;
-  const int CR = (R + 3) / 4;  // halo chunks on each side
-  // the taps' offsets in the staged tile, written over their first coordinate
-  for (int i = threadIdx.x; i < ntaps; i += blockDim.x) so[3 * i] += (so[3 * i + 2] * YH + so[3 * i + 1]) * XH;
-  // a warp stages a (chunk, y) row at a time: 4 XH doubles contiguous in memory, lanes along it
-  const int rowlen = 4 * XH, nrows = (2 * CR + 1) * YH;
-  const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5), nwarps = (int)(blockDim.x >> 5);
-  for (int row = warp; row < nrows; row += nwarps) {
-    const int cr = row / YH, yl = row - cr * YH;
-    const int gy = y0 - R + yl, zbase = 4 * (cz - CR + cr);
-    const bool yok = gy >= 0 && gy < g.ny;
-    for (int j = lane; j < rowlen; j += 32) {
-      const int xl = j >> 2, gz = zbase + (j & 3);
-      const int zl = gz - (4 * cz - R);
-      if (zl < 0 || zl >= ZH) continue;
-      const int gx = x0 - R + xl;
-      double val = 0.0;
-      if (yok && gx >= 0 && gx < g.nx && gz >= 0 && gz < g.nz) {
-        const long long c = g.cell(gx, gy, gz);
-        val = v[c];
-        if (hs_in) val = val / hs_in[c];
-      }
-      tile[(zl * YH + yl) * XH + xl] = val;
-    }
-  }
-  __syncthreads();
-  if (!own) return;
-  const int ctr = (R * YH + R + (int)(threadIdx.x >> 5)) * XH + R + (int)(threadIdx.x & 31);
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int i = 0; i < ntaps; ++i) {
-    const int o = ctr + so[3 * i];
-    const double w = sw[i];
-#pragma unroll
-    for (int zq = 0; zq < 4; ++zq) acc[zq] += w * tile[o + zq * P];
-  }
-#pragma unroll
-  for (int zq = 0; zq < 4; ++zq) {
-    const int z = 4 * cz + zq;
-    if (z >= g.nz) break;
-    const long long c = g.cell(x, y, z);
-    double r = acc[zq];
-    if (hs_out) r = r / hs_out[c];
-    out[c] = r;
-    if (e_out) e_out[c] = emin + pow(r, penal) * (1.0 - emin);
-  }
-}
 
 // e = emin + x^p (1 - emin) on the grid's cells (padding untouched)
 __global__ void k_simp_law(double* __restrict__ e, const double* __restrict__ x, double penal, double emin, LpGrid g) {
@@ -572,20 +458,6 @@ __global__ void k_energy_edof(double* __restrict__ ce, const double* __restrict_
 #define LP_ENERGY_BLOCKS 592  // 148 SMs x 4 resident blocks of 128 (128 registers)
 
 extern "C" {
-
-int lpb_filter(double* out, const double* v, const int* toff, const double* tw, int ntaps, const double* hs_in,
-               const double* hs_out, double* e_out, double penal, double emin, LP_GRID_ARGS, void* stream) {
-  LpGrid g = LP_GRID;
-  if (!lp_grid_ok(g) || !out || !v || !toff || !tw || ntaps < 1 || ntaps > LP_MAX_TAPS) return LP_ERR_ARG;
-  if (out == v) return LP_ERR_ARG;
-  size_t smem = ((3 * ntaps * sizeof(int) + 15) & ~(size_t)15) + ntaps * sizeof(double);
-  const long long tiles = (long long)((g.nx + LP_FT_X - 1) / LP_FT_X) * ((g.ny + LP_FT_Y - 1) / LP_FT_Y) *
-                          ((g.nz + 3) / 4);
-  if (tiles > 2147483647LL) return LP_ERR_ARG;
-  k_filter<<<(unsigned)tiles, 256, smem, LP_ST>>>(out, v, toff, tw, ntaps, hs_in, hs_out, e_out, penal, emin, g);
-  LP_LAUNCH_CHECK();
-  return LP_OK;
-}
 
 int lpb_simp_law(double* e, const double* x, double penal, double emin, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;

@@ -49,6 +49,7 @@ class DeviceFilter:
         self.grid = grid
         taps = filter_taps(radius, pitch)
         self.ntaps = len(taps)
+        self.reach = max(max(abs(v) for v in d) for d, _ in taps)
         self.toff = torch.tensor([list(d) for d, _ in taps], dtype=torch.int32, device=grid.device).reshape(-1)
         self.tw = torch.tensor([w for _, w in taps], dtype=torch.float64, device=grid.device)
         self.full = float(sum(w for _, w in taps))
@@ -63,9 +64,9 @@ class DeviceFilter:
 
     def apply(self, out, v, hs_in=None, hs_out=None, e_out=None, penal=3.0, emin=1e-9):
         """out = H (v / hs_in) / hs_out; with e_out also e_out = emin + out^p (1 - emin)."""
-        lib().lpb_filter(out.data_ptr(), v.data_ptr(), self.toff.data_ptr(), self.tw.data_ptr(), self.ntaps,
-                         ptr(hs_in), ptr(hs_out), ptr(e_out), float(penal), float(emin), *self.grid.args,
-                         stream_handle())
+        lib().lpb_filter_reach(out.data_ptr(), v.data_ptr(), self.toff.data_ptr(), self.tw.data_ptr(), self.ntaps,
+                               self.reach, ptr(hs_in), ptr(hs_out), ptr(e_out), float(penal), float(emin),
+                               *self.grid.args, stream_handle())
         return out
 
 
@@ -274,6 +275,7 @@ class LiveCells:
             self._cache = None
 
 
+FUSED_REACH = 3       # largest reach of the filter that a volume trial runs in its own pass (lp_filter.cu)
 VOLUME_RTOL = 1e-13   # the volume multiplier's stopping tolerance (loadpath/simp.py:1234)
 
 
@@ -304,6 +306,7 @@ class ProjectedDesign:
         self._tmp = g.cell_field(torch.float64)
         self._part = torch.zeros(592, dtype=torch.float64, device=g.device)
         self._vol = torch.zeros(1, dtype=torch.float64, device=g.device)
+        self._ts = None          # x sqrt(-dc / dv) of an OC step
         self.lam_last = None
         self.n_eval = 0
 
@@ -338,8 +341,28 @@ class ProjectedDesign:
         st = stream_handle()
         n_eval = [0]
 
+        # A trial needs only its volume: one pass over ts = x sqrt(-dc / dv) and x forms the step, the
+        # filter and the projection as it goes (lpb_oc_trial) and the last trial's design is written
+        # once, after the search. Mirror planes average each trial's design before it is filtered,
+        # and taps past the fused pass's staged reach are cheaper through the filter alone.
+        fused = not self.mirror and self.flt.reach <= FUSED_REACH and x.data_ptr() != self.xn.data_ptr()
+        if fused:
+            if self._ts is None:
+                self._ts = g.cell_field(torch.float64)
+            L.lpb_oc_step_base(self._ts.data_ptr(), x.data_ptr(), dc.data_ptr(), dv.data_ptr(), *g.args, st)
+
+        def trial(lm_, out):
+            xn, xt, xp = (self.xn, self.xt, self.xp) if out else (None, None, None)
+            L.lpb_oc_trial(ptr(xn), ptr(xt), ptr(xp), self._ts.data_ptr(), x.data_ptr(), float(lm_), float(move),
+                           ptr(self.flags), self.flt.toff.data_ptr(), self.flt.tw.data_ptr(), self.flt.ntaps,
+                           self.flt.reach, self.flt.hs.data_ptr(), float(beta), float(eta), self.w.data_ptr(), self._part.data_ptr(),
+                           self._vol.data_ptr(), *g.args, st)
+
         def stepped(lm_):
             n_eval[0] += 1
+            if fused:
+                trial(lm_, False)
+                return float(self._vol.item()) - target
             L.lpb_oc_stepped(self.xn.data_ptr(), x.data_ptr(), dc.data_ptr(), dv.data_ptr(), float(lm_), float(move),
                              ptr(self.flags), *g.args, st)
             for ax in self.mirror:
@@ -397,6 +420,8 @@ class ProjectedDesign:
                     if side == -1:
                         f1 *= 0.5
                     side = -1
+        if fused:
+            trial(lm, True)
         self.lam_last = lm
         self.n_eval = n_eval[0]
         return self.xn, lm, f1 is not None and f2 is not None
