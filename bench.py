@@ -749,6 +749,7 @@ def run_micro_band(args):
     torch.cuda.synchronize()
     lv = ge.levels[-1]
     gr = lv.grid
+    ge._coarse["ainv"]   # the band's buffers (a hierarchy that inverts the level as a chain has none)
     w = ge._work
     t, linv, sgn, info, bar, ainv = (w[k] for k in ("band_t", "band_linv", "band_sgn", "band_info", "band_bar",
                                                     "band_ainv"))

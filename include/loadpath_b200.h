@@ -188,6 +188,21 @@ int lpb_band_solve_f64(double* f_out, const double* f_in, const double* ainv, do
 int lpb_band_solve_cols_f32(float* f_out, const float* f_in, long long cstride, int ncol, const double* ainv, double* v, int nx, int ny, int nz, int pz, int cpz, void* stream);
 int lpb_band_solve_cols_f64(double* f_out, const double* f_in, long long cstride, int ncol, const double* ainv, double* v, int nx, int ny, int nz, int pz, int cpz, void* stream);
 
+/* ---- the same level as a chain of node planes: separator planes cut the band into segments, which
+ * are inverted side by side, then the separators' Schur complement; a solve is three matrix-vector
+ * passes. lpb_chain_dims: doubles of workspace, 0 where the band form is the one to use; out (may be
+ * NULL) = {segments, dofs per plane, padded segment size, separator dofs, kernels of a factorisation}.
+ * lpb_chain_factor: from the band t (left as it is) into ws (16-byte aligned); *info: 0, or nonzero when
+ * a pivot lost its digits or its sign (singular and roundoff-indefinite levels among them): factor the
+ * band instead. lpb_chain_solve_*: f_out = A^-1 f_in; ws also holds their scratch, so solves of one ws
+ * do not overlap. Replaces the SuperLU call of loadpath/mg.py:708-754. */
+long long lpb_chain_dims(int nx, int ny, int nz, long long* out);
+int lpb_chain_factor(double* ws, const double* t, int* info, int nx, int ny, int nz, int pz, int cpz, void* stream);
+int lpb_chain_solve_f32(float* f_out, const float* f_in, double* ws, int nx, int ny, int nz, int pz, int cpz, void* stream);
+int lpb_chain_solve_f64(double* f_out, const double* f_in, double* ws, int nx, int ny, int nz, int pz, int cpz, void* stream);
+int lpb_chain_solve_cols_f32(float* f_out, const float* f_in, long long cstride, int ncol, double* ws, int nx, int ny, int nz, int pz, int cpz, void* stream);
+int lpb_chain_solve_cols_f64(double* f_out, const double* f_in, long long cstride, int ncol, double* ws, int nx, int ny, int nz, int pz, int cpz, void* stream);
+
 /* ---- Chebyshev smoother (loadpath/mg.py:771-821, loadpath/mgops.py:312-343) with its
  * coefficients in device memory: lpb_cheb_coef turns the power iteration's dots (vv[k] = |v|^2
  * before step k, vav[k] = v.D^-1 A v after it) into coef[0] = lmax (safety * max(vav[its-1],

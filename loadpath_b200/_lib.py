@@ -27,7 +27,7 @@ _STATUS = {-1: "bad arguments", -2: "kernel launch failed", -3: "size beyond the
 # kernels each entry point launches (1 when not listed; 0 for host-only entries)
 _KERNELS = {"lpb_modal_ke": 0, "lpb_modal_g1": 0, "lpb_reduce_blocks": 0, "lpb_max_f64": 2, "lpb_max_abs_diff_f64": 2, "lpb_dot_f64": 2,
             "lpb_dot_f32": 2, "lpb_dot_f64_f32": 2, "lpb_cg_step": 2, "lpb_cg_step_r": 2, "lpb_apply_fine_dot_f64": 2, "lpb_oc_volumes": 2, "lpb_oc_apply": 2, "lpb_oc_apply_at": 2, "lpb_oc_walk_init": 2,
-            "lpb_band_dims": 0, "lpb_band_inverse": 2, "lpb_band_solve_f32": 2, "lpb_band_solve_f64": 2,
+            "lpb_band_dims": 0, "lpb_chain_dims": 0, "lpb_chain_solve_f32": 3, "lpb_chain_solve_f64": 3, "lpb_band_inverse": 2, "lpb_band_solve_f32": 2, "lpb_band_solve_f64": 2,
             "lpb_count_positive_f64": 2, "lpb_count_active_weights_f32": 2, "lpb_count_active_weights_f64": 2,
             "lpb_count_active_explicit_f32": 2, "lpb_count_active_explicit_f64": 2, "lpb_count_ne_u8": 2,
             "lpb_memcpy_async": 0, "lpb_memset_async": 0, "lpb_event_record": 0, "lpb_capture_begin": 0,
@@ -42,8 +42,17 @@ _KERNELS = {"lpb_modal_ke": 0, "lpb_modal_g1": 0, "lpb_reduce_blocks": 0, "lpb_m
             "lpb_mg_destroy": 0,
             # the handle's entries launch on its own stream; their kernels are not counted here
             "lpb_mg_create": 0, "lpb_mg_set_moduli": 0, "lpb_mg_solve": 0}
+def _chain_kernels(nx, ny, nz):
+    out = (ctypes.c_longlong * 5)()
+    lib().fns["lpb_chain_dims"](nx, ny, nz, out)
+    return out[4]
+
+
 # entries whose kernel count depends on their arguments
 _VARIABLE = {"lpb_sensitivity": lambda a: 1 + (a[9] is not None), "lpb_stress_pass": lambda a: 1 + (a[0] < 2),
+             "lpb_chain_factor": lambda a: _chain_kernels(*a[3:6]),
+             "lpb_chain_solve_cols_f32": lambda a: 3 * ((a[3] + 3) // 4 + (a[3] % 4 == 3)),
+             "lpb_chain_solve_cols_f64": lambda a: 3 * ((a[3] + 3) // 4 + (a[3] % 4 == 3)),
              "lpb_band_solve_cols_f32": lambda a: a[3] + (a[3] + 7) // 8,
              "lpb_band_solve_cols_f64": lambda a: a[3] + (a[3] + 7) // 8}
 _COUNT = [0]

@@ -17,6 +17,7 @@
 // The factorisation costs O(n bw^2) instead of the dense O(n^3): at the 17 x 9 x 9-node coarsest
 // level of a 256 x 128 x 128 grid, n = 4131 and bw = 275.
 #include "lp_common.cuh"
+#include "lp_dmma.cuh"
 #include "lp_tma.cuh"
 
 #define LP_BAR_LIMIT (1u << 22)   // polls before a progress wait gives up and flags an error
@@ -77,14 +78,6 @@ __device__ __forceinline__ void publish_row(unsigned* prog, int row, unsigned v)
 }
 
 // Tiles another block wrote are read with ld.global.cg (L2, not a possibly stale L1 line).
-
-// FP64 tensor-core MMA, m8n8k4 (row-major A 8 x 4, column-major B 4 x 8, C/D 8 x 8). Lane l holds
-// A[l >> 2][l & 3], B[l & 3][l >> 2] and D[l >> 2][2 (l & 3) + i], i = 0, 1.
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
 
 // ---- 32 x 32 tiles in registers and shared memory ----
 // NW warps (of a group starting at some warp) hold a tile 32 / NW entries per thread in the

@@ -313,6 +313,8 @@ struct Mg {
   // coarsest level
   bool has_coarse = false;
   double* ainv = nullptr;
+  double* band_t = nullptr;
+  double* chain = nullptr;   // the chain's workspace, null when the band's inverse is in use
   double* cv = nullptr;
   int* info = nullptr;
   double* e0 = nullptr;     // the moduli of the last set_moduli (own copy)
@@ -512,7 +514,23 @@ Level coarsen(Mg& m, Level& fine, int depth) {
   return lv;
 }
 
-// the coarsest level's band factor and dense inverse (loadpath/mg.py:708-754)
+// the band's signed Cholesky and dense inverse (grids too short for the chain, or a chain whose pivot
+// test failed)
+void band_inverse(Mg& m, const HGrid& g) {
+  long long dims[4];
+  lpb_band_dims(g.nx, g.ny, g.nz, dims);
+  const long long nt = dims[1], npad = 32 * nt;
+  double* linv = (double*)m.buf("band_linv", 8 * 1024 * (size_t)nt);
+  unsigned* bar = (unsigned*)m.buf("band_bar", 8 * (size_t)std::max(64LL, nt));
+  m.ainv = (double*)m.buf("band_ainv", 8 * (size_t)npad * npad);
+  double* sgn = (double*)m.buf("band_sgn", 8 * (size_t)npad);
+  m.chain = nullptr;
+  cudaMemsetAsync(m.info, 0, 8, m.st);
+  m.ok(lpb_band_factor(m.band_t, linv, sgn, m.info, bar, m.info + 1, HG(g), m.st));
+  m.ok(lpb_band_inverse(m.ainv, m.band_t, linv, sgn, HG(g), m.st));
+}
+
+// the coarsest level's direct solve (loadpath/mg.py:708-754): the chain of planes, or the band
 void build_coarse(Mg& m, Level& lv) {
   m.has_coarse = false;
   if (m.levels.size() < 2) return;
@@ -532,15 +550,18 @@ void build_coarse(Mg& m, Level& lv) {
     m.ok(m.f32 ? lpb_coarse_band_f32(t, 2, nullptr, nullptr, nullptr, nullptr, (const float*)lv.k, lv.mask, HG(g), m.st)
                : lpb_coarse_band_f64(t, 2, nullptr, nullptr, nullptr, nullptr, (const double*)lv.k, lv.mask, HG(g),
                                      m.st));
-  double* linv = (double*)m.buf("band_linv", 8 * 1024 * (size_t)nt);
   m.info = (int*)m.buf("band_info", 8);
-  unsigned* bar = (unsigned*)m.buf("band_bar", 8 * (size_t)std::max(64LL, nt));
-  m.ainv = (double*)m.buf("band_ainv", 8 * (size_t)npad * npad);
-  double* sgn = (double*)m.buf("band_sgn", 8 * (size_t)npad);
   m.cv = (double*)m.buf("coarse_v", 8 * (size_t)npad);
+  m.band_t = t;
+  m.chain = nullptr;
   cudaMemsetAsync(m.info, 0, 8, m.st);
-  m.ok(lpb_band_factor(t, linv, sgn, m.info, bar, m.info + 1, HG(g), m.st));
-  m.ok(lpb_band_inverse(m.ainv, t, linv, sgn, HG(g), m.st));
+  const long long words = lpb_chain_dims(g.nx, g.ny, g.nz, nullptr);
+  if (words) {
+    m.chain = (double*)m.buf("chain_ws", 8 * (size_t)words);
+    m.ok(lpb_chain_factor(m.chain, t, m.info, HG(g), m.st));
+  } else {
+    band_inverse(m, g);
+  }
   m.has_coarse = true;
 }
 
@@ -667,6 +688,11 @@ bool build(Mg& m) {
     int st2[2] = {0, 0};
     cudaMemcpyAsync(st2, m.info, 8, cudaMemcpyDeviceToHost, m.st);
     cudaStreamSynchronize(m.st);
+    if (st2[0] && m.chain) {
+      band_inverse(m, m.levels.back().g);
+      cudaMemcpyAsync(st2, m.info, 8, cudaMemcpyDeviceToHost, m.st);
+      cudaStreamSynchronize(m.st);
+    }
     if (st2[1]) {
       m.status = LP_ERR_LAUNCH;   // a wait of the factorisation gave up
       return true;
@@ -760,8 +786,12 @@ void* vcycle(Mg& m, int i, const void* b, const double* r64 = nullptr, double* d
   void* x = m.field("x" + s, g, f);
   if (i == (int)m.levels.size() - 1) {
     if (m.has_coarse) {
-      m.ok(f ? lpb_band_solve_f32((float*)x, (const float*)b, m.ainv, m.cv, HG(g), m.st)
-             : lpb_band_solve_f64((double*)x, (const double*)b, m.ainv, m.cv, HG(g), m.st));
+      if (m.chain)
+        m.ok(f ? lpb_chain_solve_f32((float*)x, (const float*)b, m.chain, HG(g), m.st)
+               : lpb_chain_solve_f64((double*)x, (const double*)b, m.chain, HG(g), m.st));
+      else
+        m.ok(f ? lpb_band_solve_f32((float*)x, (const float*)b, m.ainv, m.cv, HG(g), m.st)
+               : lpb_band_solve_f64((double*)x, (const double*)b, m.ainv, m.cv, HG(g), m.st));
     } else {
       smooth(m, i, b, x, true);
       smooth(m, i, b, x, false);

@@ -12,9 +12,10 @@ Hierarchy (built on the device at every set_moduli, as the reference builds it):
   level 1   "weights"  the eight child moduli per coarse cell with the eight fixed Galerkin
                        matrices M_k = P_k^T Ke P_k; cells touching held dofs as explicit patches
   level >=2 "explicit" Galerkin 24 x 24 per coarse cell, P^T K P over the eight children
-  coarsest  dense D K D + (I - D), Cholesky-factored once per hierarchy and applied as a
-            dense inverse (the reference factors the same operator with SuperLU on the host
-            and round-trips every V-cycle; here it stays on the device)
+  coarsest  D K D + (I - D) inverted once per hierarchy, as a chain of node planes (lp_chain.cu) or,
+            where a pivot loses its digits, by a band Cholesky and its dense inverse (lp_band.cu)
+            (the reference factors the same operator with SuperLU on the host and round-trips
+            every V-cycle; here it stays on the device)
 Smoother: Chebyshev of `degree` on D^-1 A over [lmax/30, lmax] with lmax from 12 power
 iterations x 1.3 (the reference's), or damped Jacobi (smoother="jacobi", omega).
 Precision: the V-cycle in `dtype` (float32 = mixed, float64 = the plain FP64 path); the
@@ -24,6 +25,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import weakref
 
 import numpy as np
 import torch
@@ -258,6 +260,25 @@ class DevLevel:
         else:
             getattr(L, f"lpb_diag_explicit_{sfx}")(d.data_ptr(), self.k.data_ptr(), *g.args, st)
         return d
+
+
+class _CoarseSolve(dict):
+    """The coarsest level's direct solve: chain (the workspace of lp_chain.cu's blocks, or None), or the
+    band's dense inverse ainv with its scratch v; n dofs on grid. With the chain in use, ainv is
+    formed from the same band when it is first asked for."""
+
+    def __init__(self, ge, **kw):
+        super().__init__(**kw)
+        self._ge = weakref.ref(ge)
+
+    def __missing__(self, key):
+        if key != "ainv":
+            raise KeyError(key)
+        ge = self._ge()
+        ge._join_coarse()
+        ge._band_buffers(self["v"].numel() // 32)
+        ge._band_inverse()
+        return self[key]
 
 
 class GridElasticity:
@@ -542,18 +563,22 @@ class GridElasticity:
                 self._lmax_fine_early(plan["depth"] + 1)
         self.levels = levels
         self._l0s = l0s
-        info = self._build_coarse(levels[-1])
+        info = self._build_coarse(levels[-1], plan)
         self._all_lmax(len(levels))
         self._join_coarse()
         if plan is None:
             if info is not None:
                 st_pivot, st_barrier = (int(v) for v in info.cpu().numpy())
+                if st_pivot and self._coarse["chain"] is not None:
+                    self._coarse_to_band()
+                    st_pivot, st_barrier = (int(v) for v in info.cpu().numpy())
                 if st_barrier:
                     raise RuntimeError("coarsest-level factorisation: a grid-barrier wait gave up")
                 if st_pivot:
                     return self._singular()
             self._plan = {"strict": self.strict, "shape": tuple(e_dev.shape), "depth": depth,
-                          "counts": counts, "patch": self._patch_plan}
+                          "counts": counts, "patch": self._patch_plan,
+                          "band": info is not None and self._coarse["chain"] is None}
             return True
         # one copy back: every count the plan's decisions rest on, the patch-flag mismatches
         # and the coarse factor's status
@@ -572,6 +597,10 @@ class GridElasticity:
         if depth >= 1 and int(hc[31]) != 0:
             return False
         if info is not None:
+            if int(self._info_host[0]) != 0 and self._coarse["chain"] is not None:
+                self._coarse_to_band()
+                plan["band"] = True
+                self._info_host.copy_(info)
             if int(self._info_host[1]) != 0:
                 raise RuntimeError("coarsest-level factorisation: a grid-barrier wait gave up")
             if int(self._info_host[0]) != 0:
@@ -692,12 +721,14 @@ class GridElasticity:
                                  lv.k.data_ptr(), ncp, MODAL_TOL, st)
         return lv
 
-    def _build_coarse(self, lv: DevLevel):
-        """Direct solve of the coarsest level (loadpath/mg.py:708-754): its operator as a band,
-        a tiled band Cholesky and the dense inverse from it, all on the device, once per
-        hierarchy; the V-cycle then applies the inverse with one GEMV. Returns the device status
-        pair (0 0 when fine; [0]: a non-positive pivot, the operator is singular; [1]: a
-        grid-barrier wait of the factorisation gave up), or None when there is no coarse solve."""
+    def _build_coarse(self, lv: DevLevel, plan):
+        """Direct solve of the coarsest level (loadpath/mg.py:708-754), all on the device, once per
+        hierarchy: its operator as a band, inverted as a chain of node planes (lp_chain.cu; grids too
+        short to cut, and plans whose chain lost a pivot's digits, take the tiled band Cholesky
+        and its dense inverse); the V-cycle then applies the inverse's blocks. Returns the device
+        status pair (0 0 when fine; [0]: the chain's pivot test failed, or the band's operator is
+        singular; [1]: a grid-barrier wait of the band's factorisation gave up), or None when there is
+        no coarse solve."""
         self._coarse = None
         if lv is self.levels[0]:
             return None
@@ -721,26 +752,61 @@ class GridElasticity:
         else:
             getattr(L, f"lpb_coarse_band_{sfx}")(t.data_ptr(), 2, None, None, None, None, lv.k.data_ptr(),
                                                  lv.mask.data_ptr(), *g.args, st)
-        linv = self._tbuf("band_linv", (nt * 1024,), torch.float64)
         info = self._tbuf("band_info", (2,), torch.int32)
-        bar = self._tbuf("band_bar", (2 * max(64, nt),), torch.int32)
-        ainv = self._tbuf("band_ainv", (npad, npad), torch.float64)
-        sgn = self._tbuf("band_sgn", (npad,), torch.float64)
-        self._coarse = {"ainv": ainv, "v": self._tbuf("coarse_v", (npad,), torch.float64), "n": n}
-        # The factorisation and the inverse are latency-bound chains on a fraction of the SMs;
-        # they run on a high-priority side stream, overlapped with the power iterations the
-        # caller issues next on the main stream, which joins before anything reads them.
-        main = torch.cuda.current_stream()
-        self._ev_fork.record(main)
-        self._side.wait_event(self._ev_fork)
-        ss = self._side.cuda_stream
-        L.lpb_memset_async(info.data_ptr(), 0, 8, ss)
-        L.lpb_band_factor(t.data_ptr(), linv.data_ptr(), sgn.data_ptr(), info.data_ptr(), bar.data_ptr(),
-                          info[1:].data_ptr(), *g.args, ss)
-        L.lpb_band_inverse(ainv.data_ptr(), t.data_ptr(), linv.data_ptr(), sgn.data_ptr(), *g.args, ss)
-        self._ev_join.record(self._side)
+        self._coarse = _CoarseSolve(self, n=n, grid=g, chain=None, v=self._tbuf("coarse_v", (npad,), torch.float64))
+        words = 0 if plan is not None and plan["band"] else int(L.lpb_chain_dims(g.nx, g.ny, g.nz, None))
+        if words:
+            self._coarse["chain"] = ws = self._tbuf("chain_ws", (words,), torch.float64)
+
+            def factor():
+                L.lpb_memset_async(info.data_ptr(), 0, 8, stream_handle())
+                L.lpb_chain_factor(ws.data_ptr(), t.data_ptr(), info.data_ptr(), *g.args, stream_handle())
+        else:
+            self._band_buffers(nt)
+            factor = self._band_inverse
+        # The factorisation is a latency-bound chain of launches; it runs on a high-priority side
+        # stream, overlapped with the power iterations the caller issues next on the main stream,
+        # which joins before anything reads its result.
+        graph = self._graph(("chain",), factor) if words and plan is not None and self.use_graphs else None
+        self._ev_fork.record()
+        with torch.cuda.stream(self._side):
+            self._side.wait_event(self._ev_fork)
+            if graph is not None:
+                self._replay(graph)
+            else:
+                factor()
+            self._ev_join.record()
         self._joined = False
         return info
+
+    def _band_buffers(self, nt):
+        """The band factor's buffers (the band itself and the status pair exist)."""
+        self._tbuf("band_linv", (nt * 1024,), torch.float64)
+        self._tbuf("band_bar", (2 * max(64, nt),), torch.int32)
+        self._tbuf("band_sgn", (32 * nt,), torch.float64)
+        self._coarse["ainv"] = self._tbuf("band_ainv", (32 * nt, 32 * nt), torch.float64)
+
+    def _band_inverse(self):
+        """The tiled band Cholesky (in place of the band) and the dense inverse from it, on the current
+        stream."""
+        L = lib()
+        st = stream_handle()
+        w, args = self._work, self._coarse["grid"].args
+        info = w["band_info"]
+        L.lpb_memset_async(info.data_ptr(), 0, 8, st)
+        L.lpb_band_factor(w["band_t"].data_ptr(), w["band_linv"].data_ptr(), w["band_sgn"].data_ptr(), info.data_ptr(),
+                          w["band_bar"].data_ptr(), info[1:].data_ptr(), *args, st)
+        L.lpb_band_inverse(w["band_ainv"].data_ptr(), w["band_t"].data_ptr(), w["band_linv"].data_ptr(),
+                           w["band_sgn"].data_ptr(), *args, st)
+
+    def _coarse_to_band(self):
+        """The chain's pivot test failed: the same band (the chain's build leaves it as it is) by
+        the signed Cholesky, on the working stream."""
+        self._join_coarse()
+        self._coarse["chain"] = None
+        self._band_buffers(self._coarse["v"].numel() // 32)
+        self._band_inverse()
+        self._gen += 1               # captured V-cycles name the chain's workspace
 
     def _join_coarse(self):
         """The main stream waits for the side stream's factorisation and inverse."""
@@ -946,8 +1012,11 @@ class GridElasticity:
         if i == len(self.levels) - 1:
             if self._coarse is not None:
                 c = self._coarse
-                getattr(L, f"lpb_band_solve_{sfx}")(x.data_ptr(), b.data_ptr(), c["ainv"].data_ptr(),
-                                                    c["v"].data_ptr(), *g.args, st)
+                if c["chain"] is not None:
+                    getattr(L, f"lpb_chain_solve_{sfx}")(x.data_ptr(), b.data_ptr(), c["chain"].data_ptr(), *g.args, st)
+                else:
+                    getattr(L, f"lpb_band_solve_{sfx}")(x.data_ptr(), b.data_ptr(), c["ainv"].data_ptr(),
+                                                        c["v"].data_ptr(), *g.args, st)
             else:
                 self._smooth(i, b, x, True)
                 self._smooth(i, b, x, False)
@@ -1314,7 +1383,7 @@ class GridElasticity:
             self._blk(f"bb{i}", k, lv.grid, self.tdtype)
             for key in ("r", "d", "t"):
                 self._buf(f"{key}{i}", lv.grid, self.tdtype)
-        if self._coarse is not None:
+        if self._coarse is not None and self._coarse["chain"] is None:
             self._flat_buf("band_vcols", k * self._coarse["v"].numel(), torch.float64)
         bufs["sc"] = self._tbuf("bcg_sc", (k, 8), torch.float64)
         if getattr(self, "_bhost", None) is None or self._bhost.shape[0] != k:
@@ -1336,9 +1405,13 @@ class GridElasticity:
         if i == len(self.levels) - 1:
             if self._coarse is not None:
                 c = self._coarse
-                v = self._flat_buf("band_vcols", k * c["v"].numel(), torch.float64)
-                getattr(L, f"lpb_band_solve_cols_{sfx}")(xb.data_ptr(), bb.data_ptr(), xb[0].numel(), k,
-                                                         c["ainv"].data_ptr(), v.data_ptr(), *g.args, st)
+                if c["chain"] is not None:
+                    getattr(L, f"lpb_chain_solve_cols_{sfx}")(xb.data_ptr(), bb.data_ptr(), xb[0].numel(), k,
+                                                              c["chain"].data_ptr(), *g.args, st)
+                else:
+                    v = self._flat_buf("band_vcols", k * c["v"].numel(), torch.float64)
+                    getattr(L, f"lpb_band_solve_cols_{sfx}")(xb.data_ptr(), bb.data_ptr(), xb[0].numel(), k,
+                                                             c["ainv"].data_ptr(), v.data_ptr(), *g.args, st)
             else:
                 for j in range(k):
                     self._smooth(i, bb[j], xb[j], True)
