@@ -8,8 +8,8 @@
 // The kernel marches z like the fine kernel (four cells per step, x neighbours by shuffles, y
 // neighbours through shared memory) and forms each cell's product in that basis: ~450 flops
 // against the 4608 of the dense sum. Cells touching held dofs ("patch" cells: weights zero,
-// an explicit masked matrix instead) are added by a second, node-centric pass over the box of
-// nodes they touch.
+// an explicit masked matrix instead) are taken in the same march, a warp's lanes sharing a cell's
+// dense product.
 //
 // Levels >= 2 ("explicit"): K_c stored per cell, symmetric, as the 300 upper-triangle entries
 // in entry-major order (entry p of consecutive cells contiguous, so a warp's loads coalesce).
@@ -18,13 +18,12 @@
 #include <cstring>
 
 #include "lp_common.cuh"
+#include "lp_modal.cuh"
 #include "lp_tma.cuh"
 
 #include <mutex>
 
 namespace {
-
-constexpr int TXC = 16, TYC = 16;
 
 template <typename T>
 struct G1 {
@@ -427,57 +426,85 @@ __global__ void k_walsh_chunks(T* __restrict__ wc, const T* __restrict__ w, LpGr
   }
 }
 
-constexpr int WSTAGE = 3;
-constexpr int WBOX = TXC + 1;
+constexpr int LX = 16, LY = 8;          // cell columns per block: 15 x 7 owned node columns
+constexpr int LBX = LX + 1, LBY = LY + 1;
+constexpr int LCOL = LX * LY;
+constexpr int LST = 2;                  // TMA ring depth
+constexpr int L1_MAX_BLOCKS = 296;
+constexpr int L1_PATCH = 64;            // patch cells of a tile's chunk taken together
 
 template <typename T, int N>
 struct alignas(128) WSlot {
   T v[(N * sizeof(T) + 127) / 128 * 128 / sizeof(T)];
 };
 
-// float32: the Walsh coefficients of the block's 16 x 16 cell columns arrive by TMA with the
+// float32: the Walsh coefficients of the block's 16 x 8 cell columns arrive by TMA with the
 // node values, one 128-byte row per column in the 128-byte swizzle (a warp's 16-byte reads of
 // eight consecutive rows then meet no bank twice); float64 reads them from global memory
 template <typename T>
 struct WCoef {
-  static constexpr int N = sizeof(T) == 4 ? 32 * TXC * TYC : 32;
+  static constexpr int N = sizeof(T) == 4 ? 32 * LCOL : 32;
 };
 
 template <typename T>
-struct WSmem {
-  alignas(1024) T w[WSTAGE][WCoef<T>::N];            // Walsh coefficients [y][x][cell][t] (float32)
-  WSlot<T, 3 * WBOX * WBOX * 4> u[WSTAGE];            // node values [comp][y][x][z]
-  WSlot<T, 3 * (TXC - 1) * (TYC - 1) * 4> o[2];       // outputs staged for the TMA store [comp][y][x][z]
-  T red[3][4][TXC * TYC];                             // corners 01 + 11 (to y + 1)
-  T own[3][4][TXC * TYC];                             // corners 00 + 10 with the -x neighbour's
-  alignas(8) uint64_t full[WSTAGE];
+struct L1Smem {
+  alignas(1024) T w[LST][WCoef<T>::N];                // Walsh coefficients [y][x][cell][t] (float32)
+  WSlot<T, 3 * LBX * LBY * 4> u[LST];                 // node values [comp][y][x][z]
+  // by chunk parity, component and plane: corners 00 + 10 with the -x neighbour's, and corners 01 + 11
+  // (to y + 1)
+  T own[2][3][4][LCOL];
+  T red[2][3][4][LCOL];
+  // the chunk's patch cells: their modes, products, matrices and cells (thread, z)
+  T pv[L1_PATCH][24];
+  T pf[L1_PATCH][24];
+  int pmat[L1_PATCH], pcell[L1_PATCH], npatch;
+  alignas(8) uint64_t full[LST];
+};
+
+struct L1Maps {
+  CUtensorMap u;    // (4 NX, NY, pz / 4, 3), box (4 * 17, 9, 1, 3)
+  CUtensorMap w;    // float32 Walsh coefficients (32, nx, ny, cpz / 4), box (32, 16, 8, 1), 128-byte swizzle
+};
+
+// block b takes units [u0[b], u0[b + 1]) of (tile, chunk), tile-major
+struct L1Split {
+  int u0[L1_MAX_BLOCKS + 1];
+};
+
+// cell columns [x, hx) x [y, hy) that hold the patch cells
+struct L1Box {
+  int x, hx, y, hy;
 };
 
 template <typename T>
-struct WMaps {
-  CUtensorMap u;    // (4 NX, NY, pz / 4, 3), box (4 * 17, 17, 1, 3)
-  CUtensorMap out;  // (4 NX, NY, pz / 4, 3), box (4 * 15, 15, 1, 3)
-  CUtensorMap w;    // float32 Walsh coefficients (32, nx, ny, cpz / 4), box (32, 16, 16, 1), 128-byte swizzle
+struct L1Cheb {
+  T* x;
+  T* r;
+  T* d;
+  const T* b;
+  const T* dinv;
+  const double* coef;
 };
 
 // node-plane forces of one cell: rows (3q + cc, 3(q + 4) + cc) of the modal product give the
 // lower face (f0 - f1) and upper face (f0 + f1) of mode (q, cc); fp = carry + lower face and the
 // upper face becomes the next carry, row pair by row pair
 template <int Q, int CC, typename T>
-__device__ __forceinline__ void fold_pair(const G1<T>& g, const T (&c)[8], const T (&v)[24], T (&fp)[4][3],
-                                          T (&up)[4][3]) {
+__device__ __forceinline__ void fold_pair(const G1<T>& g, const T (&c)[8], const T (&v)[24], T& fp, T& up) {
   const T f0 = g1_row<3 * Q + CC, T>(g, c, v), f1 = g1_row<3 * (Q + 4) + CC, T>(g, c, v);
-  fp[Q][CC] = up[Q][CC] + (f0 - f1);
-  up[Q][CC] = f0 + f1;
+  fp = up + (f0 - f1);
+  up = f0 + f1;
 }
 
 template <typename T>
 __device__ __forceinline__ void fold_rows(const G1<T>& g, const T (&c)[8], const T (&v)[24], T (&fp)[4][3],
                                           T (&up)[4][3]) {
-  fold_pair<0, 0>(g, c, v, fp, up); fold_pair<0, 1>(g, c, v, fp, up); fold_pair<0, 2>(g, c, v, fp, up);
-  fold_pair<1, 0>(g, c, v, fp, up); fold_pair<1, 1>(g, c, v, fp, up); fold_pair<1, 2>(g, c, v, fp, up);
-  fold_pair<2, 0>(g, c, v, fp, up); fold_pair<2, 1>(g, c, v, fp, up); fold_pair<2, 2>(g, c, v, fp, up);
-  fold_pair<3, 0>(g, c, v, fp, up); fold_pair<3, 1>(g, c, v, fp, up); fold_pair<3, 2>(g, c, v, fp, up);
+  fold_pair<0, 0>(g, c, v, fp[0][0], up[0][0]); fold_pair<0, 1>(g, c, v, fp[0][1], up[0][1]);
+  fold_pair<0, 2>(g, c, v, fp[0][2], up[0][2]); fold_pair<1, 0>(g, c, v, fp[1][0], up[1][0]);
+  fold_pair<1, 1>(g, c, v, fp[1][1], up[1][1]); fold_pair<1, 2>(g, c, v, fp[1][2], up[1][2]);
+  fold_pair<2, 0>(g, c, v, fp[2][0], up[2][0]); fold_pair<2, 1>(g, c, v, fp[2][1], up[2][1]);
+  fold_pair<2, 2>(g, c, v, fp[2][2], up[2][2]); fold_pair<3, 0>(g, c, v, fp[3][0], up[3][0]);
+  fold_pair<3, 1>(g, c, v, fp[3][1], up[3][1]); fold_pair<3, 2>(g, c, v, fp[3][2], up[3][2]);
 }
 
 // x-y modes of plane zz of this thread's four node columns, from a staged slot
@@ -485,195 +512,390 @@ template <typename T>
 __device__ __forceinline__ void slot_modes(const T* __restrict__ slot, int i, int j, int zz, T (&a)[4][3]) {
 #pragma unroll
   for (int cc = 0; cc < 3; ++cc) {
-    const T* b = slot + cc * WBOX * WBOX * 4 + zz;
+    const T* b = slot + cc * LBX * LBY * 4 + zz;
     T m[4];
-    xy4(b[(j * WBOX + i) * 4], b[(j * WBOX + i + 1) * 4], b[((j + 1) * WBOX + i) * 4],
-        b[((j + 1) * WBOX + i + 1) * 4], m);
+    xy4(b[(j * LBX + i) * 4], b[(j * LBX + i + 1) * 4], b[((j + 1) * LBX + i) * 4],
+        b[((j + 1) * LBX + i + 1) * 4], m);
 #pragma unroll
     for (int q = 0; q < 4; ++q) a[q][cc] = m[q];
   }
 }
 
-// level-1 operator, u zero on masked dofs: out = m K u (the patch cells' rows are added by
-// k_patch_add). One block per SM: the modal product keeps ~230 registers busy, and capping it at
-// 168 or 128 (two blocks) spills and runs slower (65 us against 47 us at 128 x 64 x 64 cells).
-// A block owns 15 x 15 node columns over a z segment and runs 16 x 16 threads,
-// one per cell column plus a one-cell halo; u arrives by TMA into a 3-stage mbarrier ring
-// (one chunk of 17 x 17 node columns x 3 components), the Walsh coefficients by 128-byte loads
-// per cell column and chunk,
-// the outputs leave by TMA stores. Waits are bounded and a block that gives up sets *err.
+// The patch cells of a chunk in one go: f^ = K^ v with each cell's dense corner-parity matrix (patch_m,
+// row by row), the block's threads sharing the modes (a thread per cell and component) and the
+// rows (a thread per row), so their loads of the matrices are in flight together.
 template <typename T>
-__global__ void __launch_bounds__(TXC * TYC, 1)
-k_weights_tma(const __grid_constant__ WMaps<T> maps, const T* __restrict__ wc, const uint8_t* __restrict__ mask,
-              const G1<T> gc, LpGrid g, int zch, int nchunks, int* __restrict__ err) {
+__device__ __forceinline__ void patch_products(L1Smem<T>& sm, const T* us, const T* un, const T* __restrict__ pm) {
+  const int n = min(sm.npatch, L1_PATCH);
+  constexpr int H = sizeof(T) == 4 ? 3 : 1;   // rows a thread has in flight
+  T k[H][24];
+  // the first rows' loads are issued before the modes are formed
+  auto load = [&](int e0) {
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int e = min(e0 + h * LCOL, 24 * n - 1), q = e / 24, r = e - 24 * q;
+      const T* row = pm + (long long)sm.pmat[q] * 576 + 24 * r;
+#pragma unroll
+      for (int c = 0; c < 24; c += 4) lp_ldg4(row + c, &k[h][c]);
+    }
+  };
+  if (n > 0) load(threadIdx.x);
+  for (int e = threadIdx.x; e < 3 * n; e += LCOL) {
+    const int q = e / 3, cc = e - 3 * q, th = sm.pcell[q] >> 2, t = sm.pcell[q] & 3;
+    const int at = (cc * LBY + th / LX) * LBX + th % LX;
+    T a[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int col = 4 * (at + cx_(i) + LBX * cy_(i)), z = t + cz_(i);
+      a[i] = z < 4 ? us[col + z] : (un ? un[col] : T(0));
+    }
+    lp_walsh8(a);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) sm.pv[q][3 * m + cc] = a[m];
+  }
+  __syncthreads();
+  for (int e0 = threadIdx.x; e0 < 24 * n; e0 += H * LCOL) {
+    if (e0 >= H * LCOL) load(e0);
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int e = e0 + h * LCOL;
+      if (e < 24 * n) {
+        const T* v = sm.pv[e / 24];
+        T f0 = T(0), f1 = T(0);
+#pragma unroll
+        for (int c = 0; c < 24; c += 2) {
+          f0 += k[h][c] * v[c];
+          f1 += k[h][c + 1] * v[c + 1];
+        }
+        sm.pf[e / 24][e % 24] = f0 + f1;
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// The dense product of a patch cell that found no place among those (more than L1_PATCH in a chunk),
+// by its own thread: the same sums in the same order, so which cells are placed changes no bit.
+template <typename T>
+__device__ __noinline__ void patch_alone(const T* __restrict__ pm, int patch, const T* v, T* f) {
+#pragma unroll 1
+  for (int r = 0; r < 24; ++r) {
+    T f0 = T(0), f1 = T(0);
+#pragma unroll 1
+    for (int c = 0; c < 24; c += 2) {
+      f0 += __ldg(pm + (long long)patch * 576 + 24 * r + c) * v[c];
+      f1 += __ldg(pm + (long long)patch * 576 + 24 * r + c + 1) * v[c + 1];
+    }
+    f[r] = f0 + f1;
+  }
+}
+
+// Level-1 operator, u zero on masked dofs: out = m K u (MODE 0), or a degree-2 Chebyshev update formed
+// where K u is stored (modes 1..3 as lpb_apply_fine_cheb_f32's, the vector kernels' expressions).
+//
+// What bounds it: instruction issue. A cell's product is 279 products in rows of 8 to 19 (about 560
+// floating-point instructions with the modes and the corner sums) and keeps 230 registers busy, so two
+// warps per scheduler issue them; what can be cut is the waiting and the rest: two blocks of four
+// warps per SM, whose barriers do not meet, instead of one of eight; one barrier per chunk; masks and
+// patch indices loaded a chunk ahead of their use; the patch cells (dense products) shared by a
+// warp's lanes in the same launch; units split evenly over the SMs instead of whole z segments. Sharing a
+// cell's rows between two warps (half the registers, twice the warps) ran 1.2x slower: the modes and
+// indices formed twice cost more issue slots than the extra warps filled.
+//
+// A block runs 16 x 8 cell columns (15 x 7 owned node columns; halo on the low sides) in persistent
+// segments of (tile, chunk) units, split evenly by weight (a tile with patch cells weighs more);
+// a segment recomputes the top cell of the chunk below it. u and the Walsh coefficients arrive by
+// TMA into a two-stage ring; the next chunk's first plane is waited for only when the last cell of a
+// chunk needs it. Waits are bounded and a block that gives up sets *err.
+template <typename T, int MODE>
+__global__ void __launch_bounds__(LCOL, 2)
+k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split split, T* __restrict__ out,
+         const T* __restrict__ wc, const int* __restrict__ pid, const T* __restrict__ pm,
+         const uint8_t* __restrict__ mask, const __grid_constant__ G1<T> gc, LpGrid g, int nchunks, int* __restrict__ err,
+         const L1Cheb<T> ch, const L1Box pbox) {
   extern __shared__ unsigned char wsm_raw[];
   const uint32_t raw_off = lp_smem_addr(wsm_raw);
-  WSmem<T>& sm = *reinterpret_cast<WSmem<T>*>(wsm_raw + ((1024u - (raw_off & 1023u)) & 1023u));
+  L1Smem<T>& sm = *reinterpret_cast<L1Smem<T>*>(wsm_raw + ((1024u - (raw_off & 1023u)) & 1023u));
   constexpr bool staged_w = sizeof(T) == 4;
   const int tid = threadIdx.x;
-  const int i = tid % TXC, j = tid / TXC;
-  const int x0 = blockIdx.x * (TXC - 1), y0 = blockIdx.y * (TYC - 1);
-  const int c_begin = blockIdx.z * zch;
-  const int c_end = min(c_begin + zch, nchunks);
-  if (c_begin >= c_end) return;
-  const int cstart = c_begin > 0 ? c_begin - 1 : 0;
-  const int nload = min(c_end + 1, nchunks) - cstart;
-  const int nproc = c_end - cstart;
-  const bool own = i >= 1 && j >= 1;
-  const int cx = x0 - 1 + i, cy = y0 - 1 + j;
-  const bool cell_ok = cx >= 0 && cx < g.nx && cy >= 0 && cy < g.ny;
-  const long long wstride = 32LL * g.nx * g.ny;   // one chunk of Walsh runs to the next
-  const T* wcol = wc + (cell_ok ? ((long long)cy * g.nx + cx) * 32 : 0);
-  constexpr uint32_t UBYTES = 3 * WBOX * WBOX * 4 * sizeof(T);
-  constexpr uint32_t WBYTES = staged_w ? 32 * TXC * TYC * sizeof(T) : 0;
+  const int i = tid % LX, j = tid / LX;
+  const int gx = (g.NX() + LX - 2) / (LX - 1);
+  const long long u0 = split.u0[blockIdx.x], u1 = split.u0[blockIdx.x + 1];
+  constexpr uint32_t UBYTES = 3 * LBX * LBY * 4 * sizeof(T);
+  constexpr uint32_t WBYTES = staged_w ? 32 * LCOL * sizeof(T) : 0;
+  if (u0 >= u1) return;
   __shared__ int bad;
   if (tid == 0) {
     int code = 0;
     uint32_t so = 0, sw = 0;
-    for (int s = 0; s < WSTAGE; ++s) {
+    for (int s = 0; s < LST; ++s) {
       so |= lp_smem_addr(sm.u[s].v);
       sw |= lp_smem_addr(sm.w[s]);
     }
-    so |= lp_smem_addr(sm.o[0].v) | lp_smem_addr(sm.o[1].v);
     if ((so & 127) || (staged_w && (sw & 1023))) code = 20;
     else if (staged_w && (reinterpret_cast<uintptr_t>(&maps.w) & 63)) code = 26;
     else if (reinterpret_cast<uintptr_t>(&maps.u) & 63) code = 21;
-    else if (reinterpret_cast<uintptr_t>(&maps.out) & 63) code = 22;
+    else if (MODE == 0 && (reinterpret_cast<uintptr_t>(out) & 15)) code = 22;
+    else if (MODE != 0 && ((reinterpret_cast<uintptr_t>(ch.x) | reinterpret_cast<uintptr_t>(ch.r) |
+                            reinterpret_cast<uintptr_t>(ch.d) | reinterpret_cast<uintptr_t>(ch.b) |
+                            reinterpret_cast<uintptr_t>(ch.dinv)) & 15)) code = 27;
     else if (lp_smem_addr(&sm.full[0]) & 7) code = 23;
     else if (reinterpret_cast<uintptr_t>(mask) & 3) code = 24;
-    else if (reinterpret_cast<uintptr_t>(wc) & 15) code = 25;
+    else if ((reinterpret_cast<uintptr_t>(wc) & 15) || (reinterpret_cast<uintptr_t>(pid) & 15)) code = 25;
     bad = code;
     if (code) atomicExch(err, code);
   }
   __syncthreads();
   if (bad) return;
+  T cs_s = T(0), cs_c1 = T(0), cs_c2 = T(0);
+  if constexpr (MODE != 0) {
+    cs_s = (T)ch.coef[1];
+    cs_c1 = (T)ch.coef[2];
+    cs_c2 = (T)ch.coef[3];
+  }
+  // thread 0 issues the block's loads in order: its segment, the loads issued in it and in all
+  int total = 0, issued = 0, pk = 0;
+  long long pu = u0;
+  LpSeg ps = lp_seg(u0, u1, nchunks);
   if (tid == 0) {
-    for (int s = 0; s < WSTAGE; ++s) lp_mbar_init(&sm.full[s], 1);
+    for (long long u = u0; u < u1;) {
+      const LpSeg q = lp_seg(u, u1, nchunks);
+      total += q.nload;
+      u += q.ce - q.cb;
+    }
+    for (int s = 0; s < LST; ++s) lp_mbar_init(&sm.full[s], 1);
     lp_fence_barrier_init();
   }
   __syncthreads();
-  auto issue = [&](int k) {
-    const int s = k % WSTAGE;
+  auto issue_next = [&]() {
+    if (pk == ps.nload) {
+      pu += ps.ce - ps.cb;
+      ps = lp_seg(pu, u1, nchunks);
+      pk = 0;
+    }
+    const int s = issued % LST;
+    const int x0 = (ps.tile % gx) * (LX - 1), y0 = (ps.tile / gx) * (LY - 1);
     lp_mbar_expect_tx(&sm.full[s], UBYTES + WBYTES);
-    lp_tma_load_4d(sm.u[s].v, &maps.u, 4 * (x0 - 1), y0 - 1, cstart + k, 0, &sm.full[s]);
-    if constexpr (staged_w) lp_tma_load_4d(sm.w[s], &maps.w, 0, x0 - 1, y0 - 1, cstart + k, &sm.full[s]);
+    lp_tma_load_4d(sm.u[s].v, &maps.u, 4 * (x0 - 1), y0 - 1, ps.cstart + pk, 0, &sm.full[s]);
+    if constexpr (staged_w) lp_tma_load_4d(sm.w[s], &maps.w, 0, x0 - 1, y0 - 1, ps.cstart + pk, &sm.full[s]);
+    ++pk;
+    ++issued;
   };
-  if (tid == 0) {
-    issue(0);
-    if (nload > 1) issue(1);
-  }
-  T up_carry[4][3], a_lo[4][3];
+  if (tid == 0)
+    while (issued < LST && issued < total) issue_next();
+  const long long wstride = 32LL * g.nx * g.ny, cs = g.comp_stride(), zcs = g.node_zc_stride();
+  bool ok = true, failed = false;
+  int n = 0, it = 0;   // the load in hand, chunks processed
+  for (long long u = u0; u < u1 && !failed;) {
+    const LpSeg sg = lp_seg(u, u1, nchunks);
+    u += sg.ce - sg.cb;
+    const int x0 = (sg.tile % gx) * (LX - 1), y0 = (sg.tile / gx) * (LY - 1);
+    const int cx = x0 - 1 + i, cy = y0 - 1 + j;
+    const bool cell_ok = cx >= 0 && cx < g.nx && cy >= 0 && cy < g.ny;
+    const T* wcol = wc + (cell_ok ? ((long long)cy * g.nx + cx) * 32 : 0);
+    // the tile's cells reach into the box of the patch cells
+    const bool tile_patches = pid && x0 - 1 < pbox.hx && x0 - 1 + LX > pbox.x && y0 - 1 < pbox.hy && y0 - 1 + LY > pbox.y;
+    const bool writer = i >= 1 && j >= 1 && cx < g.NX() && cy < g.NY();   // owns the node column (cx, cy)
+    const long long obase = writer ? g.node(cx, cy, 0) : 0;               // chunk c at obase + c * zcs
+    const long long pstride = g.cell_zc_stride();
+    const int* pcol = pid + (cell_ok ? g.cell(cx, cy, 0) : 0);
+    int4 p_next = make_int4(-1, -1, -1, -1);   // the next chunk's patch cells of this column
+    if (tile_patches && cell_ok) p_next = __ldg(reinterpret_cast<const int4*>(pcol + sg.cstart * pstride));
+    T up[4][3], a_lo[4][3];
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
+    for (int q = 0; q < 4; ++q)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) up_carry[q][c] = a_lo[q][c] = T(0);
-
-  for (int k = 0; k < nproc; ++k) {
-    const int c = cstart + k;
-    const bool halo = c < c_begin;
-    const int s = k % WSTAGE;
-    if (tid == 0) {
-      if (k + 2 < nload) issue(k + 2);
-      lp_bulk_wait_read<1>();
-    }
-    bool ok = lp_mbar_wait(&sm.full[s], (k / WSTAGE) & 1);
-    const bool has_next = k + 1 < nload;
-    if (has_next) ok = ok && lp_mbar_wait(&sm.full[(k + 1) % WSTAGE], ((k + 1) / WSTAGE) & 1);
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) {
-        atomicExch(err, 1);
-        for (int kk = k; kk < min(k + 3, nload); ++kk) lp_mbar_wait(&sm.full[kk % WSTAGE], (kk / WSTAGE) & 1);
+      for (int c = 0; c < 3; ++c) up[q][c] = T(0);
+    ok = ok && lp_mbar_wait(&sm.full[n % LST], (n / LST) & 1);
+    slot_modes(sm.u[n % LST].v, i, j, sg.cb > sg.cstart ? 3 : 0, a_lo);
+    for (int k = 0; k < sg.nproc; ++k, ++n, ++it) {
+      const int c = sg.cstart + k;
+      const bool halo = c < sg.cb, has_next = k + 1 < sg.nload;
+      const int s = n % LST, s1 = (n + 1) % LST;
+      const uint32_t mb = writer && !halo ? __ldg(reinterpret_cast<const uint32_t*>(mask + obase + c * zcs)) : 0u;
+      const int4 p4 = p_next;   // the column's patch cells
+      int4 sl = make_int4(-1, -1, -1, -1);   // and their places in pf
+      if (tile_patches && cell_ok && k + 1 < sg.nproc) p_next = __ldg(reinterpret_cast<const int4*>(pcol + (c + 1) * pstride));
+      ok = ok && lp_mbar_wait(&sm.full[s], (n / LST) & 1);
+      if (tile_patches) {   // uniform across the block
+        if (tid == 0) sm.npatch = 0;
+        __syncthreads();
+        auto place = [&](int p, int t) {
+          if (p < 0 || (halo && t < 3)) return -1;
+          const int q = atomicAdd(&sm.npatch, 1);   // (the order of the places changes no bit)
+          if (q < L1_PATCH) {
+            sm.pmat[q] = p;
+            sm.pcell[q] = 4 * tid + t;
+          }
+          return q;
+        };
+        sl = make_int4(place(p4.x, 0), place(p4.y, 1), place(p4.z, 2), place(p4.w, 3));
+        if (has_next) ok = ok && lp_mbar_wait(&sm.full[s1], ((n + 1) / LST) & 1);
+        __syncthreads();
+        patch_products<T>(sm, sm.u[s].v, has_next ? sm.u[s1].v : nullptr, pm);
       }
-      break;
-    }
-    const T* us = sm.u[s].v;
-    const T* un = sm.u[(k + 1) % WSTAGE].v;
-    if (k == 0) slot_modes(us, i, j, halo ? 3 : 0, a_lo);
-    const T* wch = wcol + (long long)c * wstride;   // this chunk's Walsh run (128 bytes in float32)
+      const T* us = sm.u[s].v;
+      const T* wch = wcol + (long long)c * wstride;   // this chunk's Walsh run
 #pragma unroll 1
-    for (int t = halo ? 3 : 0; t < 4; ++t) {
-      T a_hi[4][3];
-      if (t < 3) {
-        slot_modes(us, i, j, t + 1, a_hi);
-      } else if (has_next) {
-        slot_modes(un, i, j, 0, a_hi);
-      } else {
+      for (int t = halo ? 3 : 0; t < 4; ++t) {
+        T cw[8];
+        if constexpr (staged_w) {
+          // this cell's eight coefficients: two 16-byte reads of the column's swizzled row
+          const unsigned char* wb = reinterpret_cast<const unsigned char*>(sm.w[s]);
+          const float4 c0 = *reinterpret_cast<const float4*>(wb + lp_swz128((uint32_t)tid * 128u + (uint32_t)t * 32u));
+          const float4 c1 = *reinterpret_cast<const float4*>(wb + lp_swz128((uint32_t)tid * 128u + (uint32_t)t * 32u + 16u));
+          cw[0] = c0.x; cw[1] = c0.y; cw[2] = c0.z; cw[3] = c0.w;
+          cw[4] = c1.x; cw[5] = c1.y; cw[6] = c1.z; cw[7] = c1.w;
+        } else {
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) cw[kk] = __ldg(wch + t * 8 + kk);
+        }
+        T a_hi[4][3];
+        if (t < 3) {
+          slot_modes(us, i, j, t + 1, a_hi);
+        } else if (has_next) {
+          ok = ok && lp_mbar_wait(&sm.full[s1], ((n + 1) / LST) & 1);
+          slot_modes(sm.u[s1].v, i, j, 0, a_hi);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int cc = 0; cc < 3; ++cc) a_hi[q][cc] = T(0);
+        }
+        T v[24];
 #pragma unroll
         for (int q = 0; q < 4; ++q)
 #pragma unroll
-          for (int cc = 0; cc < 3; ++cc) a_hi[q][cc] = T(0);
-      }
-      T v[24], cw[8];
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int cc = 0; cc < 3; ++cc) {
-          const T lo = a_lo[q][cc], hi = a_hi[q][cc];
-          v[3 * q + cc] = lo + hi;
-          v[3 * (q + 4) + cc] = hi - lo;
-          a_lo[q][cc] = hi;
-        }
-      if constexpr (staged_w) {
-        // this cell's eight coefficients: two 16-byte reads of the column's swizzled row
-        const uint32_t row = (uint32_t)(j * TXC + i);
-        const unsigned char* wb = reinterpret_cast<const unsigned char*>(sm.w[s]);
-        const float4 c0 = *reinterpret_cast<const float4*>(wb + lp_swz128(row * 128u + (uint32_t)t * 32u));
-        const float4 c1 = *reinterpret_cast<const float4*>(wb + lp_swz128(row * 128u + (uint32_t)t * 32u + 16u));
-        cw[0] = c0.x; cw[1] = c0.y; cw[2] = c0.z; cw[3] = c0.w;
-        cw[4] = c1.x; cw[5] = c1.y; cw[6] = c1.z; cw[7] = c1.w;
+          for (int cc = 0; cc < 3; ++cc) {
+            const T lo = a_lo[q][cc], hi = a_hi[q][cc];
+            v[3 * q + cc] = lo + hi;
+            v[3 * (q + 4) + cc] = hi - lo;
+            a_lo[q][cc] = hi;
+          }
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) cw[kk] = cell_ok ? cw[kk] : T(0);
-      } else {
+        T fp[4][3];
+        fold_rows<T>(gc, cw, v, fp, up);
+        if (tile_patches) {
+          const int slot = t == 0 ? sl.x : t == 1 ? sl.y : t == 2 ? sl.z : sl.w;
+          if (slot >= 0) {
+            if (slot < L1_PATCH) {
+              const T* f = sm.pf[slot];
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) cw[kk] = cell_ok ? __ldg(wch + t * 8 + kk) : T(0);
-      }
-      T fp[4][3];
-      fold_rows<T>(gc, cw, v, fp, up_carry);
-      if (!halo) {
+              for (int q = 0; q < 12; ++q) {
+                fp[q / 3][q % 3] += f[q] - f[12 + q];
+                up[q / 3][q % 3] += f[q] + f[12 + q];
+              }
+            } else {
+              const int patch = t == 0 ? p4.x : t == 1 ? p4.y : t == 2 ? p4.z : p4.w;
+              T vv[24], f[24];
 #pragma unroll
-        for (int cc = 0; cc < 3; ++cc) {
-          const T t0 = fp[0][cc] - fp[2][cc], t1 = fp[1][cc] - fp[3][cc];
-          const T t2 = fp[0][cc] + fp[2][cc], t3 = fp[1][cc] + fp[3][cc];
-          const T c10 = __shfl_up_sync(0xffffffffu, t0 + t1, 1, TXC);
-          const T c11 = __shfl_up_sync(0xffffffffu, t2 + t3, 1, TXC);
-          sm.own[cc][t][tid] = (t0 - t1) + c10;
-          sm.red[cc][t][tid] = (t2 - t3) + c11;
+              for (int q = 0; q < 24; ++q) vv[q] = v[q];
+              patch_alone<T>(pm, patch, vv, f);
+#pragma unroll
+              for (int q = 0; q < 12; ++q) {
+                fp[q / 3][q % 3] += f[q] - f[12 + q];
+                up[q / 3][q % 3] += f[q] + f[12 + q];
+              }
+            }
+          }
+        }
+        if (!halo) {
+#pragma unroll
+          for (int cc = 0; cc < 3; ++cc) {
+            const T t0 = fp[0][cc] - fp[2][cc], t1 = fp[1][cc] - fp[3][cc];
+            const T t2 = fp[0][cc] + fp[2][cc], t3 = fp[1][cc] + fp[3][cc];
+            const T c10 = __shfl_up_sync(0xffffffffu, t0 + t1, 1, LX);
+            const T c11 = __shfl_up_sync(0xffffffffu, t2 + t3, 1, LX);
+            sm.own[it & 1][cc][t][tid] = (t0 - t1) + c10;
+            sm.red[it & 1][cc][t][tid] = (t2 - t3) + c11;
+          }
         }
       }
-    }
-    if (halo) {
-      __syncthreads();
-      continue;
-    }
-    __syncthreads();
-    if (own) {
-      const bool inside = cx < g.NX() && cy < g.NY();
-      uint8_t mbs[4] = {0, 0, 0, 0};
-      if (inside) {
-        const uchar4 mb = *reinterpret_cast<const uchar4*>(mask + g.node(cx, cy, 4 * c));
-        mbs[0] = mb.x; mbs[1] = mb.y; mbs[2] = mb.z; mbs[3] = mb.w;
+      if (__syncthreads_or(!ok)) {
+        if (tid == 0) {
+          atomicExch(err, 1);
+          // let the loads already issued land before the block exits (bounded as well)
+          for (int kk = n; kk < issued; ++kk) lp_mbar_wait(&sm.full[kk % LST], (kk / LST) & 1);
+        }
+        failed = true;
+        break;
       }
+      // this chunk's stage is read (its last plane's modes are in registers): the load after the next
+      if (tid == 0 && issued < total && issued < n + 1 + LST) issue_next();
+      if (halo) continue;   // uniform across the block
+      if (!writer) continue;
 #pragma unroll
       for (int cc = 0; cc < 3; ++cc) {
         T o[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-          const T v = sm.own[cc][t][tid] + sm.red[cc][t][tid - TXC];
-          o[t] = ((mbs[t] >> cc) & 1) ? v : T(0);
+          const T val = sm.own[it & 1][cc][t][tid] + sm.red[it & 1][cc][t][tid - LX];
+          o[t] = ((mb >> (8 * t + cc)) & 1u) ? val : T(0);
         }
-        T* dst = &sm.o[k & 1].v[((cc * (TYC - 1) + (j - 1)) * (TXC - 1) + (i - 1)) * 4];
+        const long long idx = cc * cs + obase + c * zcs;
+        if constexpr (MODE == 0) {
+          lp_st4(out + idx, o);
+        } else {
+          T dv[4], d[4];
+          lp_ld4(ch.dinv + idx, dv);
+          if constexpr (MODE == 1) {
+            T b[4], x[4];
+            lp_ld4(ch.d + idx, d);
+            lp_ld4(ch.b + idx, b);
 #pragma unroll
-        for (int t = 0; t < 4; ++t) dst[t] = o[t];
+            for (int t = 0; t < 4; ++t) x[t] = lp_cheb2_zero_v(d[t], b[t], o[t], dv[t], cs_c1, cs_c2);
+            lp_st4(ch.x + idx, x);
+          } else if constexpr (MODE == 2) {
+            T b[4], r[4];
+            lp_ld4(ch.b + idx, b);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) lp_residual_scaled_v(b[t], o[t], dv[t], cs_s, r[t], d[t]);
+            lp_st4(ch.r + idx, r);
+            lp_st4(ch.d + idx, d);
+          } else {
+            T x[4], r[4], y[4];
+            lp_ld4(ch.x + idx, x);   // read, then written, by this thread
+            lp_ld4(ch.d + idx, d);
+            lp_ld4(ch.r + idx, r);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) y[t] = lp_cheb2_v(x[t], d[t], r[t], o[t], dv[t], cs_c1, cs_c2);
+            lp_st4(ch.x + idx, y);
+          }
+        }
       }
     }
-    lp_fence_proxy_async();
-    __syncthreads();
-    if (tid == 0) {
-      lp_tma_store_4d(&maps.out, 4 * x0, y0, c, 0, sm.o[k & 1].v);
-      lp_bulk_commit();
+    // the segment's last load (the chunk above) was only read as the next chunk's first plane
+    if (!failed && sg.nload > sg.nproc) {
+      ++n;
+      __syncthreads();
+      if (tid == 0 && issued < total && issued < n + LST) issue_next();
     }
   }
-  if (tid == 0) lp_bulk_wait_all();
+}
+
+// a patch cell's matrix in the corner-parity basis, K^ = T K T^T / 64 with T = kron(H, I3); one block per
+// cell, float64 inside
+template <typename T>
+__global__ void __launch_bounds__(192) k_patch_modal(T* __restrict__ pm, const T* __restrict__ pk) {
+  __shared__ double a[24][25], b[24][25];
+  const long long p = blockIdx.x;
+  for (int e = threadIdx.x; e < 576; e += 192) a[e / 24][e % 24] = (double)pk[p * 576 + e];
+  __syncthreads();
+  // rows, then columns: b[3 m + c][.] = sum_k H[m][k] a[3 k + c][.]
+  for (int e = threadIdx.x; e < 576; e += 192) {
+    const int r = e / 24, c = e % 24, m = r / 3, cc = r % 3;
+    double s = 0.0;
+    for (int k = 0; k < 8; ++k) s += lp_walsh_h(m, k) * a[3 * k + cc][c];
+    b[r][c] = s;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 576; e += 192) {
+    const int c = e / 24, r = e % 24, m = c / 3, cc = c % 3;
+    double s = 0.0;
+    for (int k = 0; k < 8; ++k) s += lp_walsh_h(m, k) * b[r][3 * k + cc];
+    pm[p * 576 + r * 24 + c] = (T)(s / 64.0);
+  }
 }
 
 // patch cells (weights zero, an explicit masked matrix): out += m * sum of their rows times
@@ -1085,56 +1307,106 @@ static const int G1_ROWS[279] = {3, 3, 3, 3, 3, 3, 3, 3, 3, 3, 3, 3, 4, 4, 4, 4,
 static const int G1_TS[279] = {0, 0, 0, 1, 1, 2, 2, 3, 4, 4, 5, 6, 0, 0, 1, 2, 4, 4, 5, 6, 0, 0, 1, 2, 2, 3, 4, 6, 0, 0, 1, 2, 4, 4, 5, 6, 0, 0, 0, 1, 1, 2, 2, 3, 4, 4, 5, 6, 0, 0, 1, 1, 2, 3, 4, 5, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 4, 5, 5, 6, 6, 7, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 4, 5, 5, 6, 6, 7, 0, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 4, 5, 6, 0, 0, 1, 2, 2, 3, 4, 6, 0, 0, 1, 1, 2, 3, 4, 5, 0, 0, 0, 1, 1, 2, 2, 3, 4, 4, 5, 6, 0, 0, 1, 1, 1, 2, 3, 3, 4, 4, 4, 5, 5, 6, 6, 7, 0, 0, 0, 1, 1, 1, 2, 3, 4, 4, 4, 5, 5, 6, 0, 0, 1, 1, 1, 2, 3, 3, 4, 4, 4, 5, 5, 6, 6, 7, 0, 0, 0, 1, 2, 2, 2, 3, 4, 4, 4, 5, 6, 6, 0, 0, 1, 2, 2, 2, 3, 3, 4, 4, 4, 5, 5, 6, 6, 7, 0, 0, 1, 2, 2, 2, 3, 3, 4, 4, 4, 5, 5, 6, 6, 7, 0, 1, 1, 1, 2, 2, 3, 3, 3, 4, 4, 5, 5, 5, 6, 6, 6, 7, 7, 0, 1, 1, 2, 2, 2, 3, 3, 3, 4, 4, 5, 5, 5, 6, 6, 6, 7, 7, 0, 1, 1, 2, 2, 3, 3, 3, 4, 4, 4, 5, 5, 5, 6, 6, 6, 7, 7};
 static const int G1_COLS[279] = {3, 7, 14, 10, 17, 9, 20, 23, 15, 19, 22, 21, 4, 6, 9, 10, 16, 18, 21, 22, 5, 12, 15, 11, 18, 21, 17, 23, 4, 6, 9, 10, 16, 18, 21, 22, 3, 7, 14, 10, 17, 9, 20, 23, 15, 19, 22, 21, 8, 13, 11, 16, 19, 22, 20, 23, 9, 20, 4, 6, 23, 3, 7, 14, 10, 17, 21, 16, 18, 15, 19, 22, 10, 17, 3, 7, 14, 4, 6, 23, 9, 20, 22, 15, 19, 16, 18, 21, 11, 16, 18, 8, 13, 21, 5, 12, 22, 15, 19, 23, 20, 17, 5, 12, 15, 11, 18, 21, 17, 23, 8, 13, 11, 16, 19, 22, 20, 23, 3, 7, 14, 10, 17, 9, 20, 23, 15, 19, 22, 21, 15, 19, 5, 12, 22, 21, 11, 18, 3, 7, 14, 10, 17, 9, 20, 23, 11, 16, 18, 8, 13, 21, 22, 19, 4, 6, 23, 9, 20, 10, 10, 17, 3, 7, 14, 23, 9, 20, 5, 12, 22, 15, 19, 11, 18, 21, 11, 16, 18, 21, 5, 12, 22, 15, 4, 6, 23, 9, 10, 17, 15, 19, 22, 8, 13, 21, 11, 16, 3, 7, 14, 10, 17, 9, 20, 23, 9, 20, 23, 3, 7, 14, 10, 17, 8, 13, 21, 11, 16, 15, 19, 22, 21, 11, 16, 18, 15, 19, 5, 12, 22, 9, 20, 4, 6, 23, 3, 7, 14, 10, 17, 22, 15, 19, 11, 16, 18, 8, 13, 21, 10, 17, 3, 7, 14, 4, 6, 23, 9, 20, 23, 9, 20, 10, 17, 3, 7, 14, 11, 16, 18, 8, 13, 21, 5, 12, 22, 15, 19};
 
-template <typename T>
-static int launch_weights_tma(T* out, const T* u, const T* wc, const int* pid, const T* pk, const uint8_t* mask,
-                              const double* g1_host, const int* pbox, int* err, LpGrid g, cudaStream_t st) {
-  if (!lp_grid_ok(g) || g.pz % 4 || g.cpz != g.pz || !out || !u || !wc || !mask || !g1_host || !err || out == u)
+// pbox: the node box of the patch cells (host, 6 ints), which the split weighs
+template <typename T, int MODE>
+static int launch_level1(T* out, const T* u, const T* wc, const int* pid, const T* pm, const uint8_t* mask,
+                         const double* g1_host, const int* pbox, int* err, LpGrid g, cudaStream_t st,
+                         const L1Cheb<T>& ch) {
+  if (!lp_grid_ok(g) || g.pz % 4 || g.cpz != g.pz || !out || !u || !wc || !mask || !g1_host || !err)
     return LP_ERR_ARG;
   G1<T> gc;
   for (int i = 0; i < 279; ++i) gc.c[i] = (T)g1_host[i];
-  WMaps<T> maps;
+  L1Maps maps;
   const uint64_t nd[4] = {4 * (uint64_t)g.NX(), (uint64_t)g.NY(), (uint64_t)g.pz / 4, 3};
-  const uint32_t bin[4] = {4 * WBOX, WBOX, 1, 3};
-  const uint32_t bout[4] = {4 * (TXC - 1), TYC - 1, 1, 3};
-  if (!lp_make_map(&maps.u, u, 4, nd, bin, sizeof(T)) || !lp_make_map(&maps.out, out, 4, nd, bout, sizeof(T)))
-    return LP_ERR_ARG;
+  const uint32_t bin[4] = {4 * LBX, LBY, 1, 3};
+  if (!lp_make_map(&maps.u, u, 4, nd, bin, sizeof(T))) return LP_ERR_ARG;
   memset(&maps.w, 0, sizeof(maps.w));
   if (sizeof(T) == 4) {
     const uint64_t wd[4] = {32, (uint64_t)g.nx, (uint64_t)g.ny, (uint64_t)g.cpz / 4};
-    const uint32_t wb[4] = {32, TXC, TYC, 1};
+    const uint32_t wb[4] = {32, LX, LY, 1};
     if (!lp_make_map(&maps.w, wc, 4, wd, wb, sizeof(T), 128)) return LP_ERR_ARG;
   }
-  const int smem = (int)sizeof(WSmem<T>) + 1024;
+  const int smem = (int)sizeof(L1Smem<T>) + 1024;
   static long long slots = 0;   // resident blocks on the device (queried once per process)
+  int dev = 0, nsm = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (!slots) {
-    if (cudaFuncSetAttribute(k_weights_tma<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(k_level1<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return LP_ERR_LAUNCH;
-    int per_sm = 1, dev = 0, nsm = 148;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_weights_tma<T>, TXC * TYC, smem);
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    int per_sm = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_level1<T, MODE>, LCOL, smem);
     slots = (long long)(per_sm > 0 ? per_sm : 1) * nsm;
   }
-  const int gx = (g.NX() + TXC - 2) / (TXC - 1), gy = (g.NY() + TYC - 2) / (TYC - 1);
-  const int nchunks = g.pz / 4;
-  int best = nchunks;
-  double bc = 1e30;
-  for (int zch = 1; zch <= nchunks; ++zch) {
-    const long long nseg = (nchunks + zch - 1) / zch, units = (long long)gx * gy * nseg;
-    const double cost = (double)((units + slots - 1) / slots) * (zch + (nseg > 1 ? 0.3 : 0.0));
-    if (cost < bc - 1e-9) { bc = cost; best = zch; }
-  }
+  const int gx = (g.NX() + LX - 2) / (LX - 1), gy = (g.NY() + LY - 2) / (LY - 1), nchunks = g.pz / 4;
+  // persistent blocks: all resident ones (or the tuned number per SM)
+  long long nb = slots < L1_MAX_BLOCKS ? slots : L1_MAX_BLOCKS;
   const int tuned = lp_tune_lookup(sizeof(T) == 4 ? LP_KNOB_L1_F32 : LP_KNOB_L1_F64, g.nx, g.ny, g.nz);
-  if (tuned >= 1 && tuned <= nchunks) best = tuned;
-  dim3 grid(gx, gy, (nchunks + best - 1) / best);
-  k_weights_tma<T><<<grid, TXC * TYC, smem, st>>>(maps, wc, mask, gc, g, best, nchunks, err);
+  if (tuned >= 1 && (long long)tuned * nsm < nb) nb = (long long)tuned * nsm;
+  const long long units = (long long)gx * gy * nchunks;
+  if (units > 2147483647LL) return LP_ERR_SIZE;
+  if (nb > units) nb = units;
+  // block b starts where b / nb of the total weight is reached: a chunk weighs 4, 8 in a tile that holds
+  // patch cells (measured: with equal weights the support face's blocks ran 1.8x as long as the mean,
+  // 47 us against 36 at 128 x 64 x 64)
+  const bool patches = pid && pm && pbox && pbox[3] > 0 && pbox[4] > 0 && pbox[5] > 0;
+  const L1Box box = patches ? L1Box{pbox[0], pbox[0] + pbox[3] - 1, pbox[1], pbox[1] + pbox[4] - 1} : L1Box{};
+  auto weight = [&](int tile) {
+    const int x0 = (tile % gx) * (LX - 1) - 1, y0 = (tile / gx) * (LY - 1) - 1;
+    return patches && x0 < box.hx && x0 + LX > box.x && y0 < box.hy && y0 + LY > box.y ? 8 : 4;
+  };
+  L1Split split;
+  long long sum = 0;
+  for (int t = 0; t < gx * gy; ++t) sum += weight(t);
+  sum *= nchunks;
+  int b = 0;
+  long long done = 0;
+  for (int t = 0; t < gx * gy; ++t) {
+    const int w = weight(t);
+    for (; b < nb && sum * b < (done + (long long)w * nchunks) * nb; ++b) {
+      const long long into = (sum * b - done * nb + (long long)w * nb - 1) / ((long long)w * nb);
+      split.u0[b] = (int)((long long)t * nchunks + into);
+    }
+    done += (long long)w * nchunks;
+  }
+  for (; b <= nb; ++b) split.u0[b] = (int)units;
+  k_level1<T, MODE><<<(unsigned)nb, LCOL, smem, st>>>(maps, split, out, wc, patches ? pid : nullptr, pm, mask, gc, g,
+                                                      nchunks, err, ch, box);
+  LP_LAUNCH_CHECK();
+  return LP_OK;
+}
+
+// lpb_apply_weights_tma_*: the march without the patch cells, then their node-basis matrices node by node
+template <typename T>
+static int apply_weights_tma(T* out, const T* u, const T* wc, const int* pid, const T* pk, const uint8_t* mask,
+                             const double* g1, const int* pbox, int* err, LpGrid g, cudaStream_t st) {
+  if (out == u) return LP_ERR_ARG;
+  const int rc = launch_level1<T, 0>(out, u, wc, nullptr, nullptr, mask, g1, nullptr, err, g, st, L1Cheb<T>{});
+  if (rc != LP_OK) return rc;
   if (pid && pk && pbox && pbox[3] > 0 && pbox[4] > 0 && pbox[5] > 0) {
     const long long nb = (long long)pbox[3] * pbox[4] * pbox[5];
     k_patch_add<T><<<lp_blocks(nb * 32, 256), 256, 0, st>>>(out, u, pid, pk, mask, g, pbox[0], pbox[1], pbox[2],
                                                             pbox[3], pbox[4], pbox[5]);
+    LP_LAUNCH_CHECK();
   }
-  LP_LAUNCH_CHECK();
   return LP_OK;
+}
+
+template <typename T>
+static int apply_level1(int mode, T* out, T* x, T* r, T* d, const T* u, const T* b, const T* dinv, const double* coef,
+                        const T* wc, const int* pid, const T* pm, const uint8_t* mask, const double* g1, const int* pbox,
+                        int* err, LpGrid g, cudaStream_t st) {
+  if (!u || mode < 0 || mode > 3 || (mode && (!dinv || !coef))) return LP_ERR_ARG;
+  const L1Cheb<T> ch{x, r, d, b, dinv, coef};
+  if (mode == 0 && out && out != u)
+    return launch_level1<T, 0>(out, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch);
+  if (mode == 1 && x && d && b && u == d && x != d)
+    return launch_level1<T, 1>(x, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch);
+  if (mode == 2 && r && d && b && u == x && r != u && d != u && r != d)
+    return launch_level1<T, 2>(r, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch);
+  if (mode == 3 && x && d && r && u == d && x != d && r != d && r != x)
+    return launch_level1<T, 3>(x, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch);
+  return LP_ERR_ARG;
 }
 
 template <typename T>
@@ -1250,19 +1522,53 @@ int lpb_walsh_chunks_f64(double* wc, const double* w, LP_GRID_ARGS, void* stream
   return LP_OK;
 }
 
-// level-1 apply, TMA-staged (same result as lpb_apply_weights_march_*): wc from
+// level-1 apply, its patch cells from their node-basis matrices in a second launch: wc from
 // lpb_walsh_chunks_*; g1 and pbox are HOST arrays; err: a device int set when a wait gave up
-// (or to an alignment code, 20..25)
+// (or to an alignment code, 20..27)
 int lpb_apply_weights_tma_f32(float* out, const float* u, const float* wc, const int* patch_id, const float* patch_k,
                               const uint8_t* mask, const double* g1, const int* pbox, int* err, LP_GRID_ARGS,
                               void* stream) {
-  return launch_weights_tma<float>(out, u, wc, patch_id, patch_k, mask, g1, pbox, err, LP_GRID, LP_ST);
+  return apply_weights_tma<float>(out, u, wc, patch_id, patch_k, mask, g1, pbox, err, LP_GRID, LP_ST);
 }
 
 int lpb_apply_weights_tma_f64(double* out, const double* u, const double* wc, const int* patch_id,
                               const double* patch_k, const uint8_t* mask, const double* g1, const int* pbox, int* err,
                               LP_GRID_ARGS, void* stream) {
-  return launch_weights_tma<double>(out, u, wc, patch_id, patch_k, mask, g1, pbox, err, LP_GRID, LP_ST);
+  return apply_weights_tma<double>(out, u, wc, patch_id, patch_k, mask, g1, pbox, err, LP_GRID, LP_ST);
+}
+
+// the patch cells' matrices (npatch, 24, 24) in the corner-parity basis
+int lpb_patch_modal_f32(float* pm, const float* pk, long long npatch, void* stream) {
+  if (!pm || !pk || npatch < 1 || npatch > 2147483647LL) return LP_ERR_ARG;
+  k_patch_modal<float><<<(unsigned)npatch, 192, 0, LP_ST>>>(pm, pk);
+  LP_LAUNCH_CHECK();
+  return LP_OK;
+}
+
+int lpb_patch_modal_f64(double* pm, const double* pk, long long npatch, void* stream) {
+  if (!pm || !pk || npatch < 1 || npatch > 2147483647LL) return LP_ERR_ARG;
+  k_patch_modal<double><<<(unsigned)npatch, 192, 0, LP_ST>>>(pm, pk);
+  LP_LAUNCH_CHECK();
+  return LP_OK;
+}
+
+// the level-1 apply with its patch cells (patch_m from lpb_patch_modal_*) in one launch: mode 0 out = m K u;
+// modes 1..3 the Chebyshev updates of lpb_apply_fine_cheb_f32 (out not used; the fields a mode does
+// not name may be NULL)
+int lpb_apply_level1_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b,
+                         const float* dinv, const double* coef, const float* wc, const int* patch_id,
+                         const float* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err,
+                         LP_GRID_ARGS, void* stream) {
+  return apply_level1<float>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, mask, g1, pbox, err, LP_GRID,
+                             LP_ST);
+}
+
+int lpb_apply_level1_f64(int mode, double* out, double* x, double* r, double* d, const double* u, const double* b,
+                         const double* dinv, const double* coef, const double* wc, const int* patch_id,
+                         const double* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err,
+                         LP_GRID_ARGS, void* stream) {
+  return apply_level1<double>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, mask, g1, pbox, err, LP_GRID,
+                              LP_ST);
 }
 
 int lpb_apply_explicit_sym_f32(float* out, const float* u, const float* kp, float* ft, const uint8_t* mask,

@@ -72,8 +72,8 @@ static inline bool lp_grid_ok(const LpGrid& g) {
 }
 
 // Launch-geometry tuning table (lp_graph.cu): a value set for (knob, grid) by lpb_tune_set, or 0
-// when none is (the launcher's own cost model then decides). Knobs: the z-segment length in
-// chunks of the fine float32 / float64 apply and of the level-1 float32 / float64 apply.
+// when none is (the launcher's own cost model then decides). Knobs: persistent blocks
+// per SM of the fine float32 / float64 apply and of the level-1 float32 / float64 apply.
 enum { LP_KNOB_FINE_F32 = 1, LP_KNOB_FINE_F64 = 2, LP_KNOB_L1_F32 = 3, LP_KNOB_L1_F64 = 4, LP_KNOB_MAX = 4 };
 int lp_tune_lookup(int knob, int nx, int ny, int nz);
 
@@ -175,6 +175,32 @@ __host__ __device__ __forceinline__ int cz_(int k) { return (k >> 2) & 1; }
 
 template <typename T>
 __device__ __forceinline__ T lp_ldg(const T* p) { return __ldg(p); }
+
+// four consecutive values (16-byte aligned)
+__device__ __forceinline__ void lp_ld4(const float* p, float (&v)[4]) {
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+__device__ __forceinline__ void lp_ld4(const double* p, double (&v)[4]) {
+  const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void lp_st4(float* p, const float (&v)[4]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void lp_st4(double* p, const double (&v)[4]) {
+  *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+  *reinterpret_cast<double2*>(p + 2) = make_double2(v[2], v[3]);
+}
+
+__device__ __forceinline__ void lp_ldg4(const float* p, float* v) {
+  const float4 a = __ldg(reinterpret_cast<const float4*>(p));
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+__device__ __forceinline__ void lp_ldg4(const double* p, double* v) {
+  const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p + 2));
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
 
 // Block-wide sum of a double; every thread gets the result. blockDim.x <= 1024.
 __device__ __forceinline__ double lp_block_sum(double v, double* sh) {

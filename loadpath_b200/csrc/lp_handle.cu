@@ -269,6 +269,7 @@ struct Level {
   const void* mcat = nullptr;
   int* patch_id = nullptr;
   void* patch_k = nullptr;
+  void* patch_m = nullptr;   // patch_k in the corner-parity basis
   int npatch = 0;
   int pbox[6] = {0, 0, 0, 0, 0, 0};
   void* wc = nullptr;
@@ -365,6 +366,22 @@ int dot_v(bool f32, const void* a, const void* b, long long n, double* part, dou
              : lpb_dot_f64((const double*)a, (const double*)b, n, part, out, st);
 }
 
+// the weights level's march (mode 0 out = m K u, 1..3 a Chebyshev update; lpb_apply_level1_*)
+void level1(Mg& m, Level& lv, int mode, void* out, const void* u, void* x = nullptr, void* r = nullptr,
+            void* d = nullptr, const void* b = nullptr) {
+  const HGrid& g = lv.g;
+  int* pid = lv.npatch ? lv.patch_id : nullptr;
+  const void* pm = lv.npatch ? lv.patch_m : nullptr;
+  const double* coef = mode ? lv.coef : nullptr;
+  const void* dinv = mode ? lv.dinv : nullptr;
+  m.ok(lv.f32 ? lpb_apply_level1_f32(mode, (float*)out, (float*)x, (float*)r, (float*)d, (const float*)u, (const float*)b,
+                                     (const float*)dinv, coef, (const float*)lv.wc, pid, (const float*)pm, lv.mask, m.g1,
+                                     lv.pbox, m.err, HG(g), m.st)
+              : lpb_apply_level1_f64(mode, (double*)out, (double*)x, (double*)r, (double*)d, (const double*)u,
+                                     (const double*)b, (const double*)dinv, coef, (const double*)lv.wc, pid,
+                                     (const double*)pm, lv.mask, m.g1, lv.pbox, m.err, HG(g), m.st));
+}
+
 void apply(Mg& m, Level& lv, void* out, const void* u) {
   const HGrid& g = lv.g;
   if (lv.kind == K_SCALED) {
@@ -372,13 +389,7 @@ void apply(Mg& m, Level& lv, void* out, const void* u) {
                 : lpb_apply_fine_f64((double*)out, (const double*)u, (const double*)lv.e, lv.mask, m.kmodal, m.err, HG(g),
                                      m.st));
   } else if (lv.kind == K_WEIGHTS) {
-    int* pid = lv.npatch ? lv.patch_id : nullptr;
-    m.ok(lv.f32 ? lpb_apply_weights_tma_f32((float*)out, (const float*)u, (const float*)lv.wc, pid,
-                                            (const float*)(lv.npatch ? lv.patch_k : nullptr), lv.mask, m.g1, lv.pbox,
-                                            m.err, HG(g), m.st)
-                : lpb_apply_weights_tma_f64((double*)out, (const double*)u, (const double*)lv.wc, pid,
-                                            (const double*)(lv.npatch ? lv.patch_k : nullptr), lv.mask, m.g1, lv.pbox,
-                                            m.err, HG(g), m.st));
+    level1(m, lv, 0, out, u);
   } else if (lv.km) {
     m.ok(lpb_apply_explicit_modal_f32((float*)out, (const float*)u, (const float*)lv.km, (const float*)lv.kpc,
                                       lv.glist, lv.gcount, (float*)lv.ft, lv.mask, HG(g), m.st));
@@ -468,6 +479,9 @@ Level coarsen(Mg& m, Level& fine, int depth) {
                                           (const double*)fine.e, m.ke64, fine.mask, HG(gf), HG(gc), m.st)
                  : lpb_patch_matrices_f64((double*)lv.patch_k, (double*)lv.w, lv.patch_id, pc, lv.npatch,
                                           (const double*)fine.e, m.ke64, fine.mask, HG(gf), HG(gc), m.st));
+      lv.patch_m = m.buf("patch_m", vb * 576 * (size_t)lv.npatch);
+      m.ok(m.f32 ? lpb_patch_modal_f32((float*)lv.patch_m, (const float*)lv.patch_k, lv.npatch, m.st)
+                 : lpb_patch_modal_f64((double*)lv.patch_m, (const double*)lv.patch_k, lv.npatch, m.st));
       cudaStreamSynchronize(m.st);   // pcells' host copy is released below
     }
     lv.wc = m.buf("wc1", vb * 8 * ncp);
@@ -737,6 +751,17 @@ void smooth(Mg& m, int i, const void* b, void* x, bool from_zero) {
     } else {
       fused(2, x);
       fused(3, d);
+    }
+    return;
+  }
+  if (lv.kind == K_WEIGHTS) {
+    if (from_zero) {
+      m.ok(f ? lpb_cheb_d_start_f32((const float*)b, (const float*)lv.dinv, coef, (float*)d, n, m.st)
+             : lpb_cheb_d_start_f64((const double*)b, (const double*)lv.dinv, coef, (double*)d, n, m.st));
+      level1(m, lv, 1, nullptr, d, x, nullptr, d, b);
+    } else {
+      level1(m, lv, 2, nullptr, x, x, r, d, b);
+      level1(m, lv, 3, nullptr, d, x, r, d);
     }
     return;
   }

@@ -154,6 +154,7 @@ class DevLevel:
         self.g1 = None           # weights: 279 corner-parity coefficients (host)
         self.wc = None           # weights: Walsh coefficients (cpz/4, ny, nx, 4, 8)
         self.pbox = None         # weights: node box of the patch cells (host, 6 ints)
+        self.patch_m = None      # weights: the patch cells' matrices in the corner-parity basis
         self.mask = None
         self.dinv = None
         self.coef = None         # device: lmax and the Chebyshev coefficients (lpb_cheb_coef)
@@ -203,11 +204,7 @@ class DevLevel:
                                                        int(mask_in), 1, st)
         elif self.kind == "weights":
             if fine_kernel and not mask_in:
-                getattr(L, f"lpb_apply_weights_tma_{sfx}")(out.data_ptr(), u.data_ptr(), self.wc.data_ptr(),
-                                                            ptr(self.patch_id) if self.npatch else None,
-                                                            ptr(self.patch_k) if self.npatch else None,
-                                                            self.mask.data_ptr(), self.g1.ctypes.data,
-                                                            self.pbox.ctypes.data, self.err.data_ptr(), *g.args, st)
+                self.level1(0, out, u)
             else:
                 getattr(L, f"lpb_apply_weights_{sfx}")(out.data_ptr(), u.data_ptr(), self.w.data_ptr(),
                                                         self.mcat.data_ptr(), ptr(self.patch_id),
@@ -225,6 +222,16 @@ class DevLevel:
                 getattr(L, f"lpb_apply_explicit_{sfx}")(out.data_ptr(), u.data_ptr(), self.k.data_ptr(),
                                                          self.mask.data_ptr(), *g.args, int(mask_in), 1, st)
         return out
+
+    def level1(self, mode, out, u, x=None, r=None, d=None, b=None, coef=None):
+        """The weights level's march: mode 0 out = m K u (u zero on masked dofs), modes 1..3 a Chebyshev
+        update formed where K u is stored (lpb_apply_level1_*)."""
+        sfx = self._sfx()
+        getattr(lib(), f"lpb_apply_level1_{sfx}")(mode, ptr(out), ptr(x), ptr(r), ptr(d), u.data_ptr(), ptr(b),
+                                                  self.dinv.data_ptr() if mode else None, coef, self.wc.data_ptr(),
+                                                  ptr(self.patch_id) if self.npatch else None, ptr(self.patch_m),
+                                                  self.mask.data_ptr(), self.g1.ctypes.data, self.pbox.ctypes.data,
+                                                  self.err.data_ptr(), *self.grid.args, stream_handle())
 
     def apply_dot(self, out, u, part, dot):
         """out = m K u on the float64 fine level (u zero on masked dofs) and *dot = u . out, in one
@@ -679,6 +686,8 @@ class GridElasticity:
                                                         pcells.data_ptr(), lv.npatch, fine.e.data_ptr(),
                                                         self.ke64.data_ptr(), fine.mask.data_ptr(), *gf.args,
                                                         *gc.args, st)
+                lv.patch_m = self._tbuf("patch_m", (lv.npatch, 576), dt)
+                getattr(L, f"lpb_patch_modal_{sfx}")(lv.patch_m.data_ptr(), lv.patch_k.data_ptr(), lv.npatch, st)
             else:
                 lv.patch_k = None
             lv.patch_cells = pcells
@@ -968,6 +977,15 @@ class GridElasticity:
             else:
                 fused(2, x)
                 fused(3, d)
+            return x
+        if self.degree == 2 and lv.kind == "weights":
+            # the first coarse level too, where its march stores A u
+            if from_zero:
+                getattr(L, f"lpb_cheb_d_start_{sfx}")(b.data_ptr(), lv.dinv.data_ptr(), coef, d.data_ptr(), n, st)
+                lv.level1(1, None, d, x=x, d=d, b=b, coef=coef)
+            else:
+                lv.level1(2, None, x, x=x, r=r, d=d, b=b, coef=coef)
+                lv.level1(3, None, d, x=x, r=r, d=d, coef=coef)
             return x
         if self.degree == 2:
             # the two Chebyshev steps in two passes (same bits as the step-by-step form)

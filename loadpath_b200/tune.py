@@ -1,11 +1,9 @@
 """Launch-geometry autotuner for the stencil applies.
 
-The level-1 apply marches along z in segments of chunks (four node planes); a segment recomputes
-one halo cell, so short segments fill the GPU's resident blocks at the cost of more halo work, long
-ones the other way round. The fine-level applies run persistent blocks that share the (tile,
-chunk) units out evenly; their knob is the number of blocks per SM (0: all that fit). The
-launchers pick a geometry by a cost model; `autotune(ge)` instead times the applies of a built
-hierarchy at a set of candidates (CUDA events on the working stream, after a warm-up launch) and
+The fine-level and level-1 applies run persistent blocks that share the (tile, chunk) units out
+evenly; a block recomputes one halo cell per segment, so fewer blocks do less work and more hide
+more latency. The knob is the number of blocks per SM (0: all that fit). `autotune(ge)` times the
+applies of a built hierarchy at a set of candidates (CUDA events on the working stream, after a warm-up launch) and
 records the fastest in the library's tuning table (`lpb_tune_set`), per grid and precision. Only
 launch geometry is tuned: the smoothing schedule (Chebyshev degree 2, as the reference's V-cycle)
 is part of the algorithm the CG iteration counts are checked against, and stays fixed.
@@ -29,15 +27,14 @@ KNOBS = {"fine_f32": 1, "fine_f64": 2, "level1_f32": 3, "level1_f64": 4}
 _RESULTS = {}        # (knob name, nx, ny, nz) -> {"best": value, "us": {value: time}}
 
 
-def candidates(nchunks, lo):
-    """Segment lengths to time: a geometric spread up to the whole column (and 0, the cost
-    model's own choice)."""
-    c = {0, nchunks}
+def candidates(most, lo):
+    """Knob values to time: a geometric spread from lo up to most (and 0, the launcher's own choice)."""
+    c = {0, most}
     v = lo
-    while v < nchunks:
+    while v < most:
         c.add(v)
         v = v + 1 if v < 4 else int(v * 1.5)
-    return sorted(x for x in c if x == 0 or lo <= x <= nchunks)
+    return sorted(x for x in c if x == 0 or lo <= x <= most)
 
 
 def _time(fn, reps):
@@ -51,10 +48,10 @@ def _time(fn, reps):
     return a.elapsed_time(b) * 1e3 / reps
 
 
-FINE_CANDIDATES = (0, 1, 2)   # persistent fine-apply blocks per SM (0: all that fit)
+BLOCKS_PER_SM = 2        # the most any of the applies keeps resident
 
 
-def _tune_one(name, grid, fn, lo, reps):
+def _tune_one(name, grid, fn, reps):
     L = lib()
     knob = KNOBS[name]
     key = (name, grid.nx, grid.ny, grid.nz)
@@ -62,8 +59,7 @@ def _tune_one(name, grid, fn, lo, reps):
         L.lpb_tune_set(knob, grid.nx, grid.ny, grid.nz, _RESULTS[key]["best"])
         return _RESULTS[key]
     times = {}
-    cands = FINE_CANDIDATES if name.startswith("fine") else candidates(grid.pz // 4, lo)
-    for z in cands:
+    for z in candidates(BLOCKS_PER_SM, 1):
         L.lpb_tune_set(knob, grid.nx, grid.ny, grid.nz, z)
         times[z] = _time(fn, reps)
     best = min(times, key=times.get)
@@ -86,11 +82,11 @@ def autotune(ge, reps=5):
     raw = g.node_field(torch.float64).normal_()
     u64, o64 = g.node_field(torch.float64), g.node_field(torch.float64)
     L.lpb_mask_field_f64(u64.data_ptr(), raw.data_ptr(), l0.mask.data_ptr(), *g.args, 0, st)
-    out["fine_f64"] = _tune_one("fine_f64", g, lambda: l0.apply(o64, u64), 2, reps)
+    out["fine_f64"] = _tune_one("fine_f64", g, lambda: l0.apply(o64, u64), reps)
     if ge._l0s is not l0:
         s = ge._l0s
         u32, o32 = u64.float(), g.node_field(torch.float32)
-        out["fine_f32"] = _tune_one("fine_f32", g, lambda: s.apply(o32, u32), 2, reps)
+        out["fine_f32"] = _tune_one("fine_f32", g, lambda: s.apply(o32, u32), reps)
     if len(ge.levels) > 1 and ge.levels[1].kind == "weights" and getattr(ge.levels[1], "wc", None) is not None:
         l1 = ge.levels[1]
         g1 = l1.grid
@@ -99,7 +95,7 @@ def autotune(ge, reps=5):
         raw1 = g1.node_field(dt).normal_()
         u1, o1 = g1.node_field(dt), g1.node_field(dt)
         getattr(L, f"lpb_mask_field_{sfx}")(u1.data_ptr(), raw1.data_ptr(), l1.mask.data_ptr(), *g1.args, 0, st)
-        out[f"level1_{sfx}"] = _tune_one(f"level1_{sfx}", g1, lambda: l1.apply(o1, u1), 1, reps)
+        out[f"level1_{sfx}"] = _tune_one(f"level1_{sfx}", g1, lambda: l1.apply(o1, u1), reps)
     torch.cuda.synchronize()
     ge._gen += 1          # graphs captured before hold the old launch geometry: capture again
     return out
