@@ -291,6 +291,7 @@ __global__ void __launch_bounds__(TXC * TYC, (sizeof(T) == 4 ? 2 : 1))
 k_apply_fine(const __grid_constant__ FineMaps maps, T* __restrict__ out, const uint8_t* __restrict__ mask,
              const KSym<T> ks, LpGrid g, int nchunks, int* __restrict__ err, const FineCheb ch,
              double* __restrict__ dotp) {
+  lp_after_launch();
   typedef PairOps<T> O;
   typedef Pair<T> P;
   extern __shared__ unsigned char smem_raw[];
@@ -515,6 +516,7 @@ k_apply_fine(const __grid_constant__ FineMaps maps, T* __restrict__ out, const u
 
 // ordered sum of the per-block partials (the same bits every run)
 __global__ void k_fine_dot_final(const double* __restrict__ part, long long n, double* __restrict__ out) {
+  lp_after_launch();
   __shared__ double sh[32];
   double s = 0.0;
   for (long long i = threadIdx.x; i < n; i += blockDim.x) s += part[i];
@@ -662,17 +664,17 @@ static int launch_fine(T* out, const T* u, const T* e, const uint8_t* mask, cons
   const dim3 grid((unsigned)nb);
   if constexpr (sizeof(T) == 4) {
     if (mode == 1)
-      k_apply_fine<float, 1><<<grid, TXC * TYC, smem, st>>>(maps, out, mask, ks, g, nchunks, err, c, nullptr);
+      lp_launch(k_apply_fine<float, 1>, grid, TXC * TYC, smem, st, maps, out, mask, ks, g, nchunks, err, c, nullptr);
     else if (mode == 2)
-      k_apply_fine<float, 2><<<grid, TXC * TYC, smem, st>>>(maps, out, mask, ks, g, nchunks, err, c, nullptr);
+      lp_launch(k_apply_fine<float, 2>, grid, TXC * TYC, smem, st, maps, out, mask, ks, g, nchunks, err, c, nullptr);
     else if (mode == 3)
-      k_apply_fine<float, 3><<<grid, TXC * TYC, smem, st>>>(maps, out, mask, ks, g, nchunks, err, c, nullptr);
+      lp_launch(k_apply_fine<float, 3>, grid, TXC * TYC, smem, st, maps, out, mask, ks, g, nchunks, err, c, nullptr);
     else
-      k_apply_fine<float, 0><<<grid, TXC * TYC, smem, st>>>(maps, out, mask, ks, g, nchunks, err, c, nullptr);
+      lp_launch(k_apply_fine<float, 0>, grid, TXC * TYC, smem, st, maps, out, mask, ks, g, nchunks, err, c, nullptr);
   } else {
-    k_apply_fine<double, 0><<<grid, TXC * TYC, smem, st>>>(maps, out, mask, ks, g, nchunks, err, c, dp);
+    lp_launch(k_apply_fine<double, 0>, grid, TXC * TYC, smem, st, maps, out, mask, ks, g, nchunks, err, c, dp);
   }
-  if (dp) k_fine_dot_final<<<1, 1024, 0, st>>>(dp, nb, dot_out);
+  if (dp) lp_launch(k_fine_dot_final, 1, 1024, 0, st, dp, nb, dot_out);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }

@@ -502,6 +502,7 @@ __device__ void critical_rows(double* __restrict__ t, double* __restrict__ sg, c
 __global__ void __launch_bounds__(256, 1) k_band_factor(double* __restrict__ t, double* __restrict__ sg, LpBand bd,
                                                         int* __restrict__ info, unsigned* __restrict__ prog,
                                                         unsigned* __restrict__ pdone, int* __restrict__ err) {
+  lp_after_launch();
   extern __shared__ __align__(16) unsigned char band_smem_raw[];
   BandSmem& smu = *reinterpret_cast<BandSmem*>(band_smem_raw);
   if (blockIdx.x == 0) {
@@ -633,6 +634,7 @@ constexpr int INV_TILE = 32 * INV_LD;   // doubles per staged 32 x 32 block
 __global__ void __launch_bounds__(512, 1) k_band_inverse(double* __restrict__ ainv, const double* __restrict__ t,
                                                          const double* __restrict__ linv, const double* __restrict__ sg,
                                                          LpBand bd, int chunk) {
+  lp_after_launch();
   extern __shared__ __align__(16) double sm_inv[];
   double* tiles = sm_inv;                           // chunk band tiles
   double* blks = sm_inv + (long long)chunk * INV_TILE;  // chunk result blocks
@@ -745,6 +747,7 @@ template <int CB>
 __global__ void __launch_bounds__(32 * InvRing<CB>::NW, 1)
 k_band_inverse_ring(double* __restrict__ ainv, const double* __restrict__ t, const double* __restrict__ linv,
                     const double* __restrict__ sg, LpBand bd) {
+  lp_after_launch();
   typedef InvRing<CB> IR;
   extern __shared__ __align__(16) double sm_inv[];
   const int D = bd.D, RS = D + 1, R1 = D + 1;
@@ -847,6 +850,7 @@ k_band_inverse_ring(double* __restrict__ ainv, const double* __restrict__ t, con
 // a[i][j] = a[j][i] for i < j (copy the lower triangle onto the upper), 32 x 32 tiles via
 // shared memory; block (bi, bj) with bi <= bj writes tile (bi, bj)
 __global__ void k_sym_lower(double* __restrict__ a, long long np) {
+  lp_after_launch();
   __shared__ double s[32][33];
   const int bi = blockIdx.y, bj = blockIdx.x;
   if (bi > bj) return;
@@ -862,6 +866,7 @@ __global__ void k_sym_lower(double* __restrict__ a, long long np) {
 // v[i] = field at band dof i (0 past n)
 template <typename T>
 __global__ void k_field_to_band(double* __restrict__ v, const T* __restrict__ f, LpGrid g, LpBand bd) {
+  lp_after_launch();
   const long long np = 32LL * bd.nt;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < np; i += (long long)gridDim.x * blockDim.x) {
     double x = 0.0;
@@ -878,6 +883,7 @@ __global__ void k_field_to_band(double* __restrict__ v, const T* __restrict__ f,
 template <typename T>
 __global__ void k_band_gemv_to_field(T* __restrict__ f, const double* __restrict__ a, const double* __restrict__ v,
                                      LpGrid g, LpBand bd) {
+  lp_after_launch();
   const long long np = 32LL * bd.nt;
   const int lane = threadIdx.x & 31;
   const long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
@@ -899,6 +905,7 @@ __global__ void k_band_gemv_to_field(T* __restrict__ f, const double* __restrict
 template <typename T, int K>
 __global__ void k_band_gemm_to_field(T* __restrict__ f, long long cstride, const double* __restrict__ a,
                                      const double* __restrict__ v, LpGrid g, LpBand bd) {
+  lp_after_launch();
   const long long np = 32LL * bd.nt;
   const int lane = threadIdx.x & 31;
   const long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
@@ -927,7 +934,7 @@ __global__ void k_band_gemm_to_field(T* __restrict__ f, long long cstride, const
 template <typename T, int K>
 void band_gemm_launch(T* f_out, long long cstride, const double* ainv, const double* v, LpGrid g, LpBand bd,
                       cudaStream_t st) {
-  k_band_gemm_to_field<T, K><<<lp_blocks(bd.n * 32, 256), 256, 0, st>>>(f_out, cstride, ainv, v, g, bd);
+  lp_launch(k_band_gemm_to_field<T, K>, lp_blocks(bd.n * 32, 256), 256, 0, st, f_out, cstride, ainv, v, g, bd);
 }
 
 template <typename T>
@@ -937,7 +944,7 @@ int band_solve_cols(T* f_out, const T* f_in, long long cstride, int ncol, const 
   const LpBand bd = lp_band(g.NX(), g.NY(), g.NZ());
   const long long np = 32LL * bd.nt;
   for (int c = 0; c < ncol; ++c)
-    k_field_to_band<T><<<lp_blocks(np, 256), 256, 0, st>>>(v + c * np, f_in + c * cstride, g, bd);
+    lp_launch(k_field_to_band<T>, lp_blocks(np, 256), 256, 0, st, v + c * np, f_in + c * cstride, g, bd);
   for (int c0 = 0; c0 < ncol; c0 += 8) {
     const int k = ncol - c0 < 8 ? ncol - c0 : 8;
     T* fo = f_out + c0 * cstride;
@@ -962,8 +969,8 @@ int band_solve(T* f_out, const T* f_in, const double* ainv, double* v, LpGrid g,
   if (!lp_grid_ok(g) || !f_out || !f_in || !ainv || !v) return LP_ERR_ARG;
   const LpBand bd = lp_band(g.NX(), g.NY(), g.NZ());
   const long long np = 32LL * bd.nt;
-  k_field_to_band<T><<<lp_blocks(np, 256), 256, 0, st>>>(v, f_in, g, bd);
-  k_band_gemv_to_field<T><<<lp_blocks(bd.n * 32, 256), 256, 0, st>>>(f_out, ainv, v, g, bd);
+  lp_launch(k_field_to_band<T>, lp_blocks(np, 256), 256, 0, st, v, f_in, g, bd);
+  lp_launch(k_band_gemv_to_field<T>, lp_blocks(bd.n * 32, 256), 256, 0, st, f_out, ainv, v, g, bd);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -971,6 +978,7 @@ int band_solve(T* f_out, const T* f_in, const double* ainv, double* v, LpGrid g,
 // linv + 1024 R = the inverse of diagonal factor tile R (for k_band_inverse), one warp per tile:
 // lane c forms column c, right-looking (the 32 row updates of a step are independent)
 __global__ void k_diag_inverses(double* __restrict__ linv, const double* __restrict__ t, LpBand bd) {
+  lp_after_launch();
   __shared__ double sm[32][33];
   const int R = blockIdx.x;
   const double* d = tile_at(const_cast<double*>(t), bd, R, 0);
@@ -1048,7 +1056,7 @@ int lpb_band_factor(double* t, double* linv, double* sgn, int* info, unsigned* b
   if (cudaLaunchCooperativeKernel((const void*)k_band_factor, dim3((unsigned)nblocks), dim3(256), args, (size_t)smem,
                                   LP_ST) != cudaSuccess)
     return LP_ERR_LAUNCH;
-  k_diag_inverses<<<bd.nt, 32, 0, LP_ST>>>(linv, t, bd);
+  lp_launch(k_diag_inverses, bd.nt, 32, 0, LP_ST, linv, t, bd);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -1066,9 +1074,8 @@ int lpb_band_inverse(double* ainv, const double* t, const double* linv, const do
     if (cudaFuncSetAttribute(k_band_inverse_ring<INV_RING_CB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem) != cudaSuccess)
       return LP_ERR_SIZE;
-    k_band_inverse_ring<INV_RING_CB>
-        <<<(unsigned)(np / INV_RING_CB), 32 * IR::NW, smem, LP_ST>>>(ainv, t, linv, sgn, bd);
-    k_sym_lower<<<dim3(bd.nt, bd.nt), 256, 0, LP_ST>>>(ainv, np);
+    lp_launch(k_band_inverse_ring<INV_RING_CB>, (unsigned)(np / INV_RING_CB), 32 * IR::NW, smem, LP_ST, ainv, t, linv, sgn, bd);
+    lp_launch(k_sym_lower, dim3(bd.nt, bd.nt), 256, 0, LP_ST, ainv, np);
     LP_LAUNCH_CHECK();
     return LP_OK;
   }
@@ -1079,8 +1086,8 @@ int lpb_band_inverse(double* ainv, const double* t, const double* linv, const do
   const long long smem = (2LL * chunk + 2) * INV_TILE * sizeof(double);
   if (cudaFuncSetAttribute(k_band_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return LP_ERR_SIZE;
-  k_band_inverse<<<(unsigned)(np / INV_COLS), 512, (size_t)smem, LP_ST>>>(ainv, t, linv, sgn, bd, chunk);
-  k_sym_lower<<<dim3(bd.nt, bd.nt), 256, 0, LP_ST>>>(ainv, np);
+  lp_launch(k_band_inverse, (unsigned)(np / INV_COLS), 512, (size_t)smem, LP_ST, ainv, t, linv, sgn, bd, chunk);
+  lp_launch(k_sym_lower, dim3(bd.nt, bd.nt), 256, 0, LP_ST, ainv, np);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }

@@ -128,6 +128,7 @@ __device__ __forceinline__ int couple_dof(const LpBand& bd, int r, int q) {
 // the segments' matrices (tiles on and below the diagonal; identity past a segment's dofs), the
 // separators' couplings, the original diagonals and the dofs' places in a field
 __global__ void k_chain_gather(double* __restrict__ ws, const double* __restrict__ t, Chain c, LpGrid g) {
+  lp_after_launch();
   const long long M = c.M, na = c.P * M * M, ne = 2LL * (c.P - 1) * 27 * c.b, nd = c.P * M + c.MS;
   const long long total = na + ne + nd + c.bd.n;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
@@ -241,6 +242,7 @@ struct SweepJob {
 
 // the first panel and pivot of every matrix
 __global__ void __launch_bounds__(256) k_sweep_first(SweepJob job) {
+  lp_after_launch();
   __shared__ double s[32][CLD];
   __shared__ PivotCols col;
   const int j = blockIdx.y;
@@ -297,6 +299,7 @@ struct alignas(16) SweepSmem {
 // Step K of a batch's sweeps. Block 0 of a matrix: the next pivot; the others: 64 x 64 tiles (I, J),
 // I >= J, eight warps of 16 x 32 entries each (a warp lies in one 32 x 32 tile).
 __global__ void __launch_bounds__(256, 2) k_sweep_step(SweepJob job, int K) {
+  lp_after_launch();
   extern __shared__ __align__(16) unsigned char sw_raw[];
   SweepSmem& sm = *reinterpret_cast<SweepSmem*>(sw_raw);
   __shared__ PivotCols col;
@@ -432,6 +435,7 @@ __global__ void __launch_bounds__(256, 2) k_sweep_step(SweepJob job, int K) {
 
 // a <- -a, the lower triangle copied onto the upper, 32 x 32 tiles
 __global__ void k_sweep_finish(double* __restrict__ a, long long astride, int ld) {
+  lp_after_launch();
   __shared__ double s[32][33];
   const int bi = blockIdx.y, bj = blockIdx.x;
   if (bi < bj) return;
@@ -450,6 +454,7 @@ __global__ void k_sweep_finish(double* __restrict__ a, long long astride, int ld
 // W^T (2b x M per segment: the left separator's dofs, then the right one's) and W: a 32 x 32 tile of
 // separator dofs and segment dofs per block
 __global__ void __launch_bounds__(256) k_chain_w(double* __restrict__ ws, Chain c) {
+  lp_after_launch();
   __shared__ double s[32][33];
   __shared__ double ec[32][27];
   __shared__ int dc[32][27];
@@ -490,6 +495,7 @@ __global__ void __launch_bounds__(256) k_chain_w(double* __restrict__ ws, Chain 
 
 // S = A_s - B^T W, tiles on and below the diagonal (identity past its dofs)
 __global__ void __launch_bounds__(256) k_chain_schur(double* __restrict__ ws, const double* __restrict__ t, Chain c) {
+  lp_after_launch();
   const int bi = blockIdx.y, bj = blockIdx.x;
   if (bi < bj) return;
   // the couplings of the tile's rows with the planes left and right of their separator
@@ -589,6 +595,7 @@ constexpr int SEG_ROWS = 16;    // rows of a segment's inverse per block, two pe
 template <typename T, int NC>
 __global__ void __launch_bounds__(256) k_chain_y(double* __restrict__ ws, const T* __restrict__ f, long long cstride,
                                                  Chain c) {
+  lp_after_launch();
   extern __shared__ __align__(16) unsigned char sv_raw[];
   double* v = reinterpret_cast<double*>(sv_raw);   // [2][NC][M]
   const int* idx = reinterpret_cast<const int*>(ws + c.idx);
@@ -655,6 +662,7 @@ __global__ void __launch_bounds__(256) k_chain_y(double* __restrict__ ws, const 
 // x_s = S^-1 g
 template <typename T, int NC>
 __global__ void __launch_bounds__(256) k_chain_s(double* __restrict__ ws, T* __restrict__ f, long long cstride, Chain c) {
+  lp_after_launch();
   extern __shared__ __align__(16) unsigned char sv_raw[];
   double* v = reinterpret_cast<double*>(sv_raw);   // [NC][MS]
   const int* idx = reinterpret_cast<const int*>(ws + c.idx);
@@ -682,6 +690,7 @@ __global__ void __launch_bounds__(256) k_chain_s(double* __restrict__ ws, T* __r
 // x_I = y - W x_s
 template <typename T, int NC>
 __global__ void __launch_bounds__(256) k_chain_x(double* __restrict__ ws, T* __restrict__ f, long long cstride, Chain c) {
+  lp_after_launch();
   extern __shared__ __align__(16) unsigned char sv_raw[];
   double* v = reinterpret_cast<double*>(sv_raw);   // [NC][2b]: the segment's left and right separator
   const int* idx = reinterpret_cast<const int*>(ws + c.idx);
@@ -720,12 +729,12 @@ int sweep_all(SweepJob job, cudaStream_t st) {
   const int smem = (int)sizeof(SweepSmem);
   if (cudaFuncSetAttribute(k_sweep_step, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return LP_ERR_LAUNCH;
-  k_sweep_first<<<dim3((unsigned)(job.ld / 32), (unsigned)job.n), 256, 0, st>>>(job);
+  lp_launch(k_sweep_first, dim3((unsigned)(job.ld / 32), (unsigned)job.n), 256, 0, st, job);
   const int T = (steps + 1) / 2;
   for (int K = 0; K < steps; ++K)
-    k_sweep_step<<<dim3((unsigned)(1 + T * (T + 1) / 2), (unsigned)job.n), 256, smem, st>>>(job, K);
+    lp_launch(k_sweep_step, dim3((unsigned)(1 + T * (T + 1) / 2), (unsigned)job.n), 256, smem, st, job, K);
   const unsigned nt = (unsigned)(job.ld / 32);
-  k_sweep_finish<<<dim3(nt, nt, (unsigned)job.n), 256, 0, st>>>(job.a, job.astride, job.ld);
+  lp_launch(k_sweep_finish, dim3(nt, nt, (unsigned)job.n), 256, 0, st, job.a, job.astride, job.ld);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -743,9 +752,9 @@ int chain_pass(double* ws, const T* fi, T* fo, long long cstride, const Chain& c
       cudaFuncSetAttribute(k_chain_s<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, s2) != cudaSuccess ||
       cudaFuncSetAttribute(k_chain_x<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, s3) != cudaSuccess)
     return LP_ERR_SIZE;
-  k_chain_y<T, NC><<<pairs + gb, 256, s1, st>>>(ws, fi, cstride, c);
-  k_chain_s<T, NC><<<(c.nS + SOLVE_ROWS - 1) / SOLVE_ROWS, 256, s2, st>>>(ws, fo, cstride, c);
-  k_chain_x<T, NC><<<rows, 256, s3, st>>>(ws, fo, cstride, c);
+  lp_launch(k_chain_y<T, NC>, pairs + gb, 256, s1, st, ws, fi, cstride, c);
+  lp_launch(k_chain_s<T, NC>, (c.nS + SOLVE_ROWS - 1) / SOLVE_ROWS, 256, s2, st, ws, fo, cstride, c);
+  lp_launch(k_chain_x<T, NC>, rows, 256, s3, st, ws, fo, cstride, c);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -809,7 +818,7 @@ int lpb_chain_factor(double* ws, const double* t, int* info, LP_GRID_ARGS, void*
       !chain_plan(nx, ny, nz, c))
     return LP_ERR_ARG;
   if (cudaMemsetAsync(info, 0, sizeof(int), LP_ST) != cudaSuccess) return LP_ERR_LAUNCH;
-  k_chain_gather<<<148 * 8, 256, 0, LP_ST>>>(ws, t, c, g);
+  lp_launch(k_chain_gather, 148 * 8, 256, 0, LP_ST, ws, t, c, g);
   SweepJob job{};
   job.a = ws + c.ai;
   job.astride = (long long)c.M * c.M;
@@ -822,8 +831,8 @@ int lpb_chain_factor(double* ws, const double* t, int* info, LP_GRID_ARGS, void*
   for (int j = 0; j < c.P; ++j) job.steps[j] = (short)((c.size(j) + 31) / 32);
   int rc = sweep_all(job, LP_ST);
   if (rc != LP_OK) return rc;
-  k_chain_w<<<dim3((unsigned)(c.M / 32), (unsigned)((c.b + 31) / 32), (unsigned)(2 * c.P)), 256, 0, LP_ST>>>(ws, c);
-  k_chain_schur<<<dim3((unsigned)(c.MS / 32), (unsigned)(c.MS / 32)), 256, 0, LP_ST>>>(ws, t, c);
+  lp_launch(k_chain_w, dim3((unsigned)(c.M / 32), (unsigned)((c.b + 31) / 32), (unsigned)(2 * c.P)), 256, 0, LP_ST, ws, c);
+  lp_launch(k_chain_schur, dim3((unsigned)(c.MS / 32), (unsigned)(c.MS / 32)), 256, 0, LP_ST, ws, t, c);
   job.a = ws + c.s;
   job.astride = 0;
   job.ld = c.MS;

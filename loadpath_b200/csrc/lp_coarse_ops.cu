@@ -414,6 +414,7 @@ __device__ __forceinline__ void xy4(T u00, T u10, T u01, T u11, T (&a)[4]) {
 // Formed once per hierarchy (after the patch cells' weights are zeroed).
 template <typename T>
 __global__ void k_walsh_chunks(T* __restrict__ wc, const T* __restrict__ w, LpGrid g) {
+  lp_after_launch();
   const long long ncp = g.cells_padded();
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < ncp; c += (long long)gridDim.x * blockDim.x) {
     T wk[8], cw[8];
@@ -613,6 +614,7 @@ k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split sp
          const T* __restrict__ wc, const int* __restrict__ pid, const T* __restrict__ pm,
          const uint8_t* __restrict__ mask, const __grid_constant__ G1<T> gc, LpGrid g, int nchunks, int* __restrict__ err,
          const L1Cheb<T> ch, const L1Box pbox) {
+  lp_after_launch();
   extern __shared__ unsigned char wsm_raw[];
   const uint32_t raw_off = lp_smem_addr(wsm_raw);
   L1Smem<T>& sm = *reinterpret_cast<L1Smem<T>*>(wsm_raw + ((1024u - (raw_off & 1023u)) & 1023u));
@@ -878,6 +880,7 @@ k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split sp
 // cell, float64 inside
 template <typename T>
 __global__ void __launch_bounds__(192) k_patch_modal(T* __restrict__ pm, const T* __restrict__ pk) {
+  lp_after_launch();
   __shared__ double a[24][25], b[24][25];
   const long long p = blockIdx.x;
   for (int e = threadIdx.x; e < 576; e += 192) a[e / 24][e % 24] = (double)pk[p * 576 + e];
@@ -905,6 +908,7 @@ template <typename T>
 __global__ void k_patch_add(T* __restrict__ out, const T* __restrict__ u, const int* __restrict__ pid,
                             const T* __restrict__ pk, const uint8_t* __restrict__ mask, LpGrid g, int bx0, int by0,
                             int bz0, int bnx, int bny, int bnz) {
+  lp_after_launch();
   const long long total = (long long)bnx * bny * bnz;
   const long long cs = g.comp_stride();
   const int lane = threadIdx.x & 31;
@@ -1001,6 +1005,7 @@ __global__ void __launch_bounds__(32 * EX_WARPS)
 k_explicit_cells(T* __restrict__ ft, const T* __restrict__ u, const T* __restrict__ kp, LpGrid g) {
   extern __shared__ __align__(16) unsigned char ex_raw[];
   ExCells<T>& sm = *reinterpret_cast<ExCells<T>*>(ex_raw);
+  lp_after_launch();
   const long long ncp = g.cells_padded(), cs = g.comp_stride();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long c = blockIdx.x * 32LL + lane;
@@ -1064,6 +1069,7 @@ template <typename Ti>
 __global__ void __launch_bounds__(128) k_pack_modal(float* __restrict__ km, int* __restrict__ glist,
                                                     int* __restrict__ gcount, float* __restrict__ kpc,
                                                     const Ti* __restrict__ k, long long ncp, double tol) {
+  lp_after_launch();
   __shared__ double sk[4][576];
   __shared__ double sa[4][576];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1234,6 +1240,7 @@ __global__ void __launch_bounds__(128, 4) k_explicit_modal_cells(float* __restri
                                                                 const int* __restrict__ glist,
                                                                 const int* __restrict__ gcount, LpGrid g,
                                                                 int modal_blocks) {
+  lp_after_launch();
   __shared__ float sk[4][300];
   __shared__ float su[4][24];
   if ((int)blockIdx.x < modal_blocks) {
@@ -1246,6 +1253,7 @@ __global__ void __launch_bounds__(128, 4) k_explicit_modal_cells(float* __restri
 template <typename T>
 __global__ void k_explicit_gather(T* __restrict__ out, const T* __restrict__ ft, const uint8_t* __restrict__ mask,
                                   LpGrid g) {
+  lp_after_launch();
   const long long total = g.nodes_padded();
   const long long ncp = g.cells_padded(), cs = g.comp_stride();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -1270,25 +1278,27 @@ __global__ void k_explicit_gather(T* __restrict__ out, const T* __restrict__ ft,
 // The explicit gather with a degree-2 Chebyshev update applied to each node's A u as it is formed
 // (the standalone kernels' expressions): mode 1 x = d + (c1 d + c2 dinv (b - A d)); mode 2 r = b - A x,
 // d = s dinv r; mode 3 x = (x + d) + (c1 d + c2 dinv (r - A d)). Padding is left as it is (zero).
+template <typename T>
 struct ChebArgs {
-  float* x;
-  float* r;
-  float* d;
-  const float* b;
-  const float* dinv;
+  T* x;
+  T* r;
+  T* d;
+  const T* b;
+  const T* dinv;
   const double* coef;
 };
 
-template <int MODE>
-__global__ void k_explicit_gather_cheb(const float* __restrict__ ft, const uint8_t* __restrict__ mask, LpGrid g,
-                                       ChebArgs a) {
+template <typename T, int MODE>
+__global__ void k_explicit_gather_cheb(const T* __restrict__ ft, const uint8_t* __restrict__ mask, LpGrid g,
+                                       ChebArgs<T> a) {
+  lp_after_launch();
   const long long total = g.nodes_padded();
   const long long ncp = g.cells_padded(), cs = g.comp_stride();
-  const float s = (float)a.coef[1], c1 = (float)a.coef[2], c2 = (float)a.coef[3];
+  const T s = (T)a.coef[1], c1 = (T)a.coef[2], c2 = (T)a.coef[3];
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int x, y, z;
     if (!g.node_at(t, x, y, z)) continue;
-    float acc[3] = {0.0f, 0.0f, 0.0f};
+    T acc[3] = {T(0), T(0), T(0)};
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int cx = x - cx_(k), cy = y - cy_(k), cz = z - cz_(k);
@@ -1302,11 +1312,11 @@ __global__ void k_explicit_gather_cheb(const float* __restrict__ ft, const uint8
 #pragma unroll
     for (int cc = 0; cc < 3; ++cc) {
       const long long i = cc * cs + n;
-      const float adi = ((mb >> cc) & 1) ? acc[cc] : 0.0f;
+      const T adi = ((mb >> cc) & 1) ? acc[cc] : T(0);
       if (MODE == 1) {
         a.x[i] = lp_cheb2_zero_v(a.d[i], a.b[i], adi, a.dinv[i], c1, c2);
       } else if (MODE == 2) {
-        float ri, di;
+        T ri, di;
         lp_residual_scaled_v(a.b[i], adi, a.dinv[i], s, ri, di);
         a.r[i] = ri;
         a.d[i] = di;
@@ -1320,6 +1330,7 @@ __global__ void k_explicit_gather_cheb(const float* __restrict__ ft, const uint8
 // full (cells, 576) matrices -> packed symmetric entry-major (the average of K and K^T)
 template <typename Ti, typename To>
 __global__ void k_pack_sym(To* __restrict__ kp, const Ti* __restrict__ k, long long ncp) {
+  lp_after_launch();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < 300 * ncp; t += (long long)gridDim.x * blockDim.x) {
     const int p = (int)(t / ncp);
     const long long c = t % ncp;
@@ -1413,7 +1424,7 @@ static int launch_level1(T* out, const T* u, const T* wc, const int* pid, const 
     done += (long long)w * nchunks;
   }
   for (; b <= nb; ++b) split.u0[b] = (int)units;
-  k_level1<T, MODE><<<(unsigned)nb, LCOL, smem, st>>>(maps, split, out, wc, patches ? pid : nullptr, pm, mask, gc, g,
+  lp_launch(k_level1<T, MODE>, (unsigned)nb, LCOL, smem, st, maps, split, out, wc, patches ? pid : nullptr, pm, mask, gc, g,
                                                       nchunks, err, ch, box);
   LP_LAUNCH_CHECK();
   return LP_OK;
@@ -1428,7 +1439,7 @@ static int apply_weights_tma(T* out, const T* u, const T* wc, const int* pid, co
   if (rc != LP_OK) return rc;
   if (pid && pk && pbox && pbox[3] > 0 && pbox[4] > 0 && pbox[5] > 0) {
     const long long nb = (long long)pbox[3] * pbox[4] * pbox[5];
-    k_patch_add<T><<<lp_blocks(nb * 32, 256), 256, 0, st>>>(out, u, pid, pk, mask, g, pbox[0], pbox[1], pbox[2],
+    lp_launch(k_patch_add<T>, lp_blocks(nb * 32, 256), 256, 0, st, out, u, pid, pk, mask, g, pbox[0], pbox[1], pbox[2],
                                                             pbox[3], pbox[4], pbox[5]);
     LP_LAUNCH_CHECK();
   }
@@ -1458,8 +1469,8 @@ static int launch_explicit(T* out, const T* u, const T* kp, T* ft, const uint8_t
   constexpr int smem = (int)sizeof(ExCells<T>);   // above the 48 KB default in float64
   if (cudaFuncSetAttribute(k_explicit_cells<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return LP_ERR_LAUNCH;
-  k_explicit_cells<T><<<lp_blocks(g.cells_padded(), 32), 32 * EX_WARPS, smem, st>>>(ft, u, kp, g);
-  k_explicit_gather<T><<<lp_blocks(g.nodes_padded(), 256), 256, 0, st>>>(out, ft, mask, g);
+  lp_launch(k_explicit_cells<T>, lp_blocks(g.cells_padded(), 32), 32 * EX_WARPS, smem, st, ft, u, kp, g);
+  lp_launch(k_explicit_gather<T>, lp_blocks(g.nodes_padded(), 256), 256, 0, st, out, ft, mask, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -1555,7 +1566,7 @@ int lpb_modal_g1(const double* ke, double* g1_out) {
 int lpb_walsh_chunks_f32(float* wc, const float* w, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || g.cpz % 4 || !wc || !w) return LP_ERR_ARG;
-  k_walsh_chunks<float><<<lp_blocks(g.cells_padded(), 256), 256, 0, LP_ST>>>(wc, w, g);
+  lp_launch(k_walsh_chunks<float>, lp_blocks(g.cells_padded(), 256), 256, 0, LP_ST, wc, w, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -1563,7 +1574,7 @@ int lpb_walsh_chunks_f32(float* wc, const float* w, LP_GRID_ARGS, void* stream) 
 int lpb_walsh_chunks_f64(double* wc, const double* w, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || g.cpz % 4 || !wc || !w) return LP_ERR_ARG;
-  k_walsh_chunks<double><<<lp_blocks(g.cells_padded(), 256), 256, 0, LP_ST>>>(wc, w, g);
+  lp_launch(k_walsh_chunks<double>, lp_blocks(g.cells_padded(), 256), 256, 0, LP_ST, wc, w, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -1586,14 +1597,14 @@ int lpb_apply_weights_tma_f64(double* out, const double* u, const double* wc, co
 // the patch cells' matrices (npatch, 24, 24) in the corner-parity basis
 int lpb_patch_modal_f32(float* pm, const float* pk, long long npatch, void* stream) {
   if (!pm || !pk || npatch < 1 || npatch > 2147483647LL) return LP_ERR_ARG;
-  k_patch_modal<float><<<(unsigned)npatch, 192, 0, LP_ST>>>(pm, pk);
+  lp_launch(k_patch_modal<float>, (unsigned)npatch, 192, 0, LP_ST, pm, pk);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_patch_modal_f64(double* pm, const double* pk, long long npatch, void* stream) {
   if (!pm || !pk || npatch < 1 || npatch > 2147483647LL) return LP_ERR_ARG;
-  k_patch_modal<double><<<(unsigned)npatch, 192, 0, LP_ST>>>(pm, pk);
+  lp_launch(k_patch_modal<double>, (unsigned)npatch, 192, 0, LP_ST, pm, pk);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -1652,7 +1663,7 @@ int lpb_pack_modal_f32(float* km, int* glist, int* gcount, float* kpc, const flo
   if (!km || !glist || !gcount || !kpc || !k || ncells < 1) return LP_ERR_ARG;
   if (cudaMemsetAsync(gcount, 0, sizeof(int), LP_ST) != cudaSuccess) return LP_ERR_LAUNCH;
   const long long blocks = (ncells + 3) / 4;
-  k_pack_modal<float><<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 128, 0, LP_ST>>>(km, glist, gcount, kpc,
+  lp_launch(k_pack_modal<float>, (unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 128, 0, LP_ST, km, glist, gcount, kpc,
                                                                                           k, ncells, tol);
   LP_LAUNCH_CHECK();
   return LP_OK;
@@ -1665,8 +1676,8 @@ int lpb_apply_explicit_modal_f32(float* out, const float* u, const float* km, co
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !out || !u || !km || !kpc || !glist || !gcount || !ft || !mask || out == u) return LP_ERR_ARG;
   const int modal_blocks = lp_blocks(g.cells_padded(), 128);
-  k_explicit_modal_cells<<<modal_blocks + 148, 128, 0, LP_ST>>>(ft, u, km, kpc, glist, gcount, g, modal_blocks);
-  k_explicit_gather<float><<<lp_blocks(g.nodes_padded(), 256), 256, 0, LP_ST>>>(out, ft, mask, g);
+  lp_launch(k_explicit_modal_cells, modal_blocks + 148, 128, 0, LP_ST, ft, u, km, kpc, glist, gcount, g, modal_blocks);
+  lp_launch(k_explicit_gather<float>, lp_blocks(g.nodes_padded(), 256), 256, 0, LP_ST, out, ft, mask, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -1686,26 +1697,26 @@ int lpb_apply_explicit_modal_cheb_f32(int mode, float* x, float* r, float* d, co
   if (mode == 3 && (!x || !d || !r || u != d || x == d)) return LP_ERR_ARG;
   if (mode < 1 || mode > 3) return LP_ERR_ARG;
   const int modal_blocks = lp_blocks(g.cells_padded(), 128);
-  k_explicit_modal_cells<<<modal_blocks + 148, 128, 0, LP_ST>>>(ft, u, km, kpc, glist, gcount, g, modal_blocks);
-  const ChebArgs a{x, r, d, b, dinv, coef};
+  lp_launch(k_explicit_modal_cells, modal_blocks + 148, 128, 0, LP_ST, ft, u, km, kpc, glist, gcount, g, modal_blocks);
+  const ChebArgs<float> a{x, r, d, b, dinv, coef};
   const int nb = lp_blocks(g.nodes_padded(), 256);
-  if (mode == 1) k_explicit_gather_cheb<1><<<nb, 256, 0, LP_ST>>>(ft, mask, g, a);
-  else if (mode == 2) k_explicit_gather_cheb<2><<<nb, 256, 0, LP_ST>>>(ft, mask, g, a);
-  else k_explicit_gather_cheb<3><<<nb, 256, 0, LP_ST>>>(ft, mask, g, a);
+  if (mode == 1) lp_launch(k_explicit_gather_cheb<float, 1>, nb, 256, 0, LP_ST, ft, mask, g, a);
+  else if (mode == 2) lp_launch(k_explicit_gather_cheb<float, 2>, nb, 256, 0, LP_ST, ft, mask, g, a);
+  else lp_launch(k_explicit_gather_cheb<float, 3>, nb, 256, 0, LP_ST, ft, mask, g, a);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_pack_sym_f32(float* kp, const float* k, long long ncells, void* stream) {
   if (!kp || !k || ncells < 0) return LP_ERR_ARG;
-  k_pack_sym<float, float><<<lp_blocks(300 * ncells, 256), 256, 0, LP_ST>>>(kp, k, ncells);
+  lp_launch(k_pack_sym<float, float>, lp_blocks(300 * ncells, 256), 256, 0, LP_ST, kp, k, ncells);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_pack_sym_f64(double* kp, const double* k, long long ncells, void* stream) {
   if (!kp || !k || ncells < 0) return LP_ERR_ARG;
-  k_pack_sym<double, double><<<lp_blocks(300 * ncells, 256), 256, 0, LP_ST>>>(kp, k, ncells);
+  lp_launch(k_pack_sym<double, double>, lp_blocks(300 * ncells, 256), 256, 0, LP_ST, kp, k, ncells);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }

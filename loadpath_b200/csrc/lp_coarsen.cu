@@ -24,6 +24,7 @@ __device__ __forceinline__ double pw(int k, int q, int r) {
 // w[k, C] = e[2C + CORNERS[k]] for C inside the fine grid's half, else 0 (loadpath/mg.py:617-620)
 template <typename Te, typename Tw>
 __global__ void k_weights_from_e(Tw* __restrict__ w, const Te* __restrict__ e, LpGrid gf, LpGrid gc) {
+  lp_after_launch();
   const long long total = gc.cells_padded();
   const int hx = gf.nx / 2, hy = gf.ny / 2, hz = gf.nz / 2;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -44,6 +45,7 @@ __global__ void k_weights_from_e(Tw* __restrict__ w, const Te* __restrict__ e, L
 template <typename Te>
 __global__ void k_patch_flags(uint8_t* __restrict__ flag, const Te* __restrict__ e, const uint8_t* __restrict__ mf,
                               LpGrid gf, LpGrid gc) {
+  lp_after_launch();
   const long long total = gc.cells_padded();
   const int hx = gf.nx / 2, hy = gf.ny / 2, hz = gf.nz / 2;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -71,6 +73,7 @@ __global__ void k_patch_matrices(Tw* __restrict__ pk, Tw* __restrict__ w, int* _
                                  const long long* __restrict__ pcells, int npatch, const Te* __restrict__ e,
                                  const double* __restrict__ ke, const uint8_t* __restrict__ mf, LpGrid gf,
                                  LpGrid gc) {
+  lp_after_launch();
   __shared__ double kc[576];
   __shared__ double tt[576];
   __shared__ double dm[24];
@@ -126,6 +129,7 @@ __global__ void k_galerkin_explicit(Tw* __restrict__ kout, int fine_kind, const 
                                     const Tw* __restrict__ mcat, const int* __restrict__ patch_id,
                                     const Tw* __restrict__ patch_k, const Tw* __restrict__ fk,
                                     const uint8_t* __restrict__ mf, int strict, LpGrid gf, LpGrid gc) {
+  lp_after_launch();
   __shared__ double kf[576];
   __shared__ double tt[576];
   __shared__ double dm[24];
@@ -196,6 +200,7 @@ __global__ void k_galerkin_explicit(Tw* __restrict__ kout, int fine_kind, const 
 __global__ void k_strict_held_kept(uint8_t* __restrict__ held_c, float* __restrict__ kept,
                                    const uint8_t* __restrict__ held_f, const uint8_t* __restrict__ mf, LpGrid gf,
                                    LpGrid gc) {
+  lp_after_launch();
   const int FX = gf.NX(), FY = gf.NY(), FZ = gf.NZ();
   const long long total = gc.nodes_padded();
   const long long ccs = gc.comp_stride();
@@ -232,6 +237,7 @@ __global__ void k_strict_held_kept(uint8_t* __restrict__ held_c, float* __restri
 // level-0 held bits: alive and fixed
 __global__ void k_held0(uint8_t* __restrict__ held, const uint8_t* __restrict__ mask0,
                         const uint8_t* __restrict__ fixed_bits, long long n) {
+  lp_after_launch();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     held[i] = (uint8_t)(((mask0[i] >> 3) & fixed_bits[i]) & 7);
 }
@@ -289,6 +295,7 @@ __global__ void k_coarse_dense(double* __restrict__ a, int kind, const Tw* __res
                                const Tw* __restrict__ mcat, const int* __restrict__ patch_id,
                                const Tw* __restrict__ patch_k, const Tw* __restrict__ k,
                                const uint8_t* __restrict__ mask, LpGrid g) {
+  lp_after_launch();
   const int NX = g.NX(), NY = g.NY(), NZ = g.NZ();
   const long long NN = (long long)NX * NY * NZ;
   const long long n = 3 * NN;
@@ -313,6 +320,7 @@ template <typename Tw>
 __global__ void k_coarse_band(double* __restrict__ t, int kind, const Tw* __restrict__ w, const Tw* __restrict__ mcat,
                               const int* __restrict__ patch_id, const Tw* __restrict__ patch_k,
                               const Tw* __restrict__ k, const uint8_t* __restrict__ mask, LpGrid g, LpBand bd) {
+  lp_after_launch();
   const long long total = (long long)bd.nt * (bd.D + 1) * 1024;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
@@ -346,6 +354,7 @@ __global__ void k_coarse_band(double* __restrict__ t, int kind, const Tw* __rest
 template <typename Tw>
 __global__ void __launch_bounds__(288, 1) k_galerkin_w2(Tw* __restrict__ kout, const Tw* __restrict__ w1,
                                                         const Tw* __restrict__ nkq, LpGrid gf, LpGrid gc) {
+  lp_after_launch();
   constexpr int CB = 4;
   __shared__ __align__(16) double ws[CB][64];   // float64 here: the inner loop converts nothing
   const int e = blockIdx.y * 288 + threadIdx.x;
@@ -396,6 +405,7 @@ __global__ void __launch_bounds__(288, 1) k_galerkin_w2(Tw* __restrict__ kout, c
 template <typename Tw>
 __global__ void k_galerkin_patch_add(Tw* __restrict__ kout, const int* __restrict__ patch_id,
                                      const Tw* __restrict__ patch_k, LpGrid gf, LpGrid gc) {
+  lp_after_launch();
   __shared__ double kf[576];
   __shared__ double tt[576];
   __shared__ int pids[8];
@@ -461,7 +471,7 @@ int lpb_weights_from_e_f64_f32(float* w, const double* e, LP_FC_ARGS, void* stre
   LpGrid gf = LP_GF, gc = LP_GC;
   if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || !w || !e) return LP_ERR_ARG;
   long long total = gc.cells_padded();
-  k_weights_from_e<double, float><<<lp_blocks(total, 256), 256, 0, LP_ST>>>(w, e, gf, gc);
+  lp_launch(k_weights_from_e<double, float>, lp_blocks(total, 256), 256, 0, LP_ST, w, e, gf, gc);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -470,7 +480,7 @@ int lpb_weights_from_e_f64_f64(double* w, const double* e, LP_FC_ARGS, void* str
   LpGrid gf = LP_GF, gc = LP_GC;
   if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || !w || !e) return LP_ERR_ARG;
   long long total = gc.cells_padded();
-  k_weights_from_e<double, double><<<lp_blocks(total, 256), 256, 0, LP_ST>>>(w, e, gf, gc);
+  lp_launch(k_weights_from_e<double, double>, lp_blocks(total, 256), 256, 0, LP_ST, w, e, gf, gc);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -479,7 +489,7 @@ int lpb_patch_flags(uint8_t* flag, const double* e, const uint8_t* mf, LP_FC_ARG
   LpGrid gf = LP_GF, gc = LP_GC;
   if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || !flag || !e || !mf) return LP_ERR_ARG;
   long long total = gc.cells_padded();
-  k_patch_flags<double><<<lp_blocks(total, 256), 256, 0, LP_ST>>>(flag, e, mf, gf, gc);
+  lp_launch(k_patch_flags<double>, lp_blocks(total, 256), 256, 0, LP_ST, flag, e, mf, gf, gc);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -489,7 +499,7 @@ int lpb_patch_matrices_f32(float* pk, float* w, int* patch_id, const long long* 
   LpGrid gf = LP_GF, gc = LP_GC;
   if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || npatch < 0) return LP_ERR_ARG;
   if (npatch == 0) return LP_OK;
-  k_patch_matrices<double, float><<<npatch, 256, 0, LP_ST>>>(pk, w, patch_id, pcells, npatch, e, ke, mf, gf, gc);
+  lp_launch(k_patch_matrices<double, float>, npatch, 256, 0, LP_ST, pk, w, patch_id, pcells, npatch, e, ke, mf, gf, gc);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -499,7 +509,7 @@ int lpb_patch_matrices_f64(double* pk, double* w, int* patch_id, const long long
   LpGrid gf = LP_GF, gc = LP_GC;
   if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || npatch < 0) return LP_ERR_ARG;
   if (npatch == 0) return LP_OK;
-  k_patch_matrices<double, double><<<npatch, 256, 0, LP_ST>>>(pk, w, patch_id, pcells, npatch, e, ke, mf, gf, gc);
+  lp_launch(k_patch_matrices<double, double>, npatch, 256, 0, LP_ST, pk, w, patch_id, pcells, npatch, e, ke, mf, gf, gc);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -514,9 +524,9 @@ int lpb_patch_matrices_f64(double* pk, double* w, int* patch_id, const long long
     const long long ncell = (long long)gc.nx * gc.ny * gc.nz;                                               \
     long long nb = (ncell + 3) / 4;                                                                         \
     if (nb > 148 * 8) nb = 148 * 8;                                                                         \
-    k_galerkin_w2<T><<<dim3((unsigned)nb, 2), 288, 0, LP_ST>>>(kout, w1, nkq, gf, gc);                      \
+    lp_launch(k_galerkin_w2<T>, dim3((unsigned)nb, 2), 288, 0, LP_ST, kout, w1, nkq, gf, gc);                      \
     if (patch_id && patch_k)                                                                                \
-      k_galerkin_patch_add<T><<<(unsigned)ncell, 256, 0, LP_ST>>>(kout, patch_id, patch_k, gf, gc);          \
+      lp_launch(k_galerkin_patch_add<T>, (unsigned)ncell, 256, 0, LP_ST, kout, patch_id, patch_k, gf, gc);          \
     LP_LAUNCH_CHECK();                                                                                      \
     return LP_OK;                                                                                           \
   }
@@ -531,7 +541,7 @@ int lpb_galerkin_explicit_f32(float* kout, int fine_kind, const float* fw, const
   if (fine_kind == 1 && (!fw || !mcat)) return LP_ERR_ARG;
   if (fine_kind == 2 && !fk) return LP_ERR_ARG;
   long long ncell = (long long)gc.nx * gc.ny * gc.nz;
-  k_galerkin_explicit<float><<<(unsigned)ncell, 256, 0, LP_ST>>>(kout, fine_kind, fw, mcat, patch_id, patch_k, fk, mf,
+  lp_launch(k_galerkin_explicit<float>, (unsigned)ncell, 256, 0, LP_ST, kout, fine_kind, fw, mcat, patch_id, patch_k, fk, mf,
                                                                  strict, gf, gc);
   LP_LAUNCH_CHECK();
   return LP_OK;
@@ -545,7 +555,7 @@ int lpb_galerkin_explicit_f64(double* kout, int fine_kind, const double* fw, con
   if (fine_kind == 1 && (!fw || !mcat)) return LP_ERR_ARG;
   if (fine_kind == 2 && !fk) return LP_ERR_ARG;
   long long ncell = (long long)gc.nx * gc.ny * gc.nz;
-  k_galerkin_explicit<double><<<(unsigned)ncell, 256, 0, LP_ST>>>(kout, fine_kind, fw, mcat, patch_id, patch_k, fk,
+  lp_launch(k_galerkin_explicit<double>, (unsigned)ncell, 256, 0, LP_ST, kout, fine_kind, fw, mcat, patch_id, patch_k, fk,
                                                                   mf, strict, gf, gc);
   LP_LAUNCH_CHECK();
   return LP_OK;
@@ -556,14 +566,14 @@ int lpb_strict_held_kept(uint8_t* held_c, float* kept, const uint8_t* held_f, co
   LpGrid gf = LP_GF, gc = LP_GC;
   if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || !held_c || !kept || !held_f || !mf) return LP_ERR_ARG;
   long long total = gc.nodes_padded();
-  k_strict_held_kept<<<lp_blocks(total, 256), 256, 0, LP_ST>>>(held_c, kept, held_f, mf, gf, gc);
+  lp_launch(k_strict_held_kept, lp_blocks(total, 256), 256, 0, LP_ST, held_c, kept, held_f, mf, gf, gc);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_held0(uint8_t* held, const uint8_t* mask0, const uint8_t* fixed_bits, long long n, void* stream) {
   if (!held || !mask0 || !fixed_bits) return LP_ERR_ARG;
-  k_held0<<<lp_blocks(n, 256), 256, 0, LP_ST>>>(held, mask0, fixed_bits, n);
+  lp_launch(k_held0, lp_blocks(n, 256), 256, 0, LP_ST, held, mask0, fixed_bits, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -574,7 +584,7 @@ int lpb_coarse_dense_f32(double* a, int kind, const float* w, const float* mcat,
   if (!lp_grid_ok(g) || !a || !mask) return LP_ERR_ARG;
   long long n = 3LL * g.NX() * g.NY() * g.NZ();
   if (n > 40000) return LP_ERR_SIZE;
-  k_coarse_dense<float><<<lp_blocks(n * n, 256), 256, 0, LP_ST>>>(a, kind, w, mcat, patch_id, patch_k, k, mask, g);
+  lp_launch(k_coarse_dense<float>, lp_blocks(n * n, 256), 256, 0, LP_ST, a, kind, w, mcat, patch_id, patch_k, k, mask, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -585,7 +595,7 @@ int lpb_coarse_dense_f64(double* a, int kind, const double* w, const double* mca
   if (!lp_grid_ok(g) || !a || !mask) return LP_ERR_ARG;
   long long n = 3LL * g.NX() * g.NY() * g.NZ();
   if (n > 40000) return LP_ERR_SIZE;
-  k_coarse_dense<double><<<lp_blocks(n * n, 256), 256, 0, LP_ST>>>(a, kind, w, mcat, patch_id, patch_k, k, mask, g);
+  lp_launch(k_coarse_dense<double>, lp_blocks(n * n, 256), 256, 0, LP_ST, a, kind, w, mcat, patch_id, patch_k, k, mask, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -598,7 +608,7 @@ int lpb_coarse_band_f32(double* t, int kind, const float* w, const float* mcat, 
   if (!lp_grid_ok(g) || !t || !mask || (kind == 1 && (!w || !mcat)) || (kind == 2 && !k)) return LP_ERR_ARG;
   const LpBand bd = lp_band(g.NX(), g.NY(), g.NZ());
   const long long total = (long long)bd.nt * (bd.D + 1) * 1024;
-  k_coarse_band<float><<<lp_blocks(total, 256), 256, 0, LP_ST>>>(t, kind, w, mcat, patch_id, patch_k, k, mask, g, bd);
+  lp_launch(k_coarse_band<float>, lp_blocks(total, 256), 256, 0, LP_ST, t, kind, w, mcat, patch_id, patch_k, k, mask, g, bd);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -609,7 +619,7 @@ int lpb_coarse_band_f64(double* t, int kind, const double* w, const double* mcat
   if (!lp_grid_ok(g) || !t || !mask || (kind == 1 && (!w || !mcat)) || (kind == 2 && !k)) return LP_ERR_ARG;
   const LpBand bd = lp_band(g.NX(), g.NY(), g.NZ());
   const long long total = (long long)bd.nt * (bd.D + 1) * 1024;
-  k_coarse_band<double><<<lp_blocks(total, 256), 256, 0, LP_ST>>>(t, kind, w, mcat, patch_id, patch_k, k, mask, g,
+  lp_launch(k_coarse_band<double>, lp_blocks(total, 256), 256, 0, LP_ST, t, kind, w, mcat, patch_id, patch_k, k, mask, g,
                                                                   bd);
   LP_LAUNCH_CHECK();
   return LP_OK;

@@ -176,6 +176,30 @@ __host__ __device__ __forceinline__ int cz_(int k) { return (k >> 2) & 1; }
 template <typename T>
 __device__ __forceinline__ T lp_ldg(const T* p) { return __ldg(p); }
 
+// Launches overlap their start with the kernel before them (programmatic dependent launch): every kernel
+// of the library begins with lp_after_launch, which waits until the kernel before it has finished and
+// its writes are visible, then lets the one after it start; lp_launch is the launch that allows
+// it. A kernel's blocks are so already in place (parameters fetched, barriers set up) when their
+// turn comes, which is most of the time of the many launches of a coarse level.
+__device__ __forceinline__ void lp_after_launch() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+static inline void lp_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // a failure is left for LP_LAUNCH_CHECK
+}
+
 // four consecutive values (16-byte aligned)
 __device__ __forceinline__ void lp_ld4(const float* p, float (&v)[4]) {
   const float4 a = *reinterpret_cast<const float4*>(p);

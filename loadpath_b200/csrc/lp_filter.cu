@@ -288,6 +288,7 @@ template <int R, class In, class Out>
 __global__ void __launch_bounds__(FT_THREADS, (R < 3 ? 2 : 1))
 k_filter_march(const __grid_constant__ FilterMaps maps, const In in, const Out o, const int* __restrict__ toff,
                const double* __restrict__ tw, int ntaps, LpGrid g, int seg, int tma, int vec, double* __restrict__ part) {
+  lp_after_launch();
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw_off = lp_smem_addr(smem_raw);
   unsigned char* slabs = smem_raw + ((1024u - (raw_off & 1023u)) & 1023u);   // a: stages 0, 1, then b: 0, 1
@@ -432,6 +433,7 @@ k_filter_march(const __grid_constant__ FilterMaps maps, const In in, const Out o
 
 // ordered sum of the blocks' volumes
 __global__ void k_filter_volume(const double* __restrict__ part, int n, double* __restrict__ out) {
+  lp_after_launch();
   __shared__ double sh[32];
   double s = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += part[i];
@@ -442,6 +444,7 @@ __global__ void k_filter_volume(const double* __restrict__ part, int n, double* 
 // ts = x sqrt(-dc / dv)
 __global__ void k_oc_step_base(double* __restrict__ ts, const double* __restrict__ x, const double* __restrict__ dc,
                                const double* __restrict__ dv, LpGrid g) {
+  lp_after_launch();
   const long long total = g.cells_padded();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int x_, y_, z;
@@ -479,7 +482,7 @@ int launch_reach(const In& in, const Out& o, const int* toff, const double* tw, 
   if (cudaFuncSetAttribute(k_filter_march<R, In, Out>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            4 * Slab<R>::BYTES + 1024) != cudaSuccess)
     return LP_ERR_LAUNCH;
-  k_filter_march<R, In, Out><<<nb, FT_THREADS, smem, st>>>(maps, in, o, toff, tw, ntaps, g, best, tma ? 1 : 0, vec ? 1 : 0,
+  lp_launch(k_filter_march<R, In, Out>, nb, FT_THREADS, smem, st, maps, in, o, toff, tw, ntaps, g, best, tma ? 1 : 0, vec ? 1 : 0,
                                                            part);
   if (nblocks) *nblocks = nb;
   LP_LAUNCH_CHECK();
@@ -529,7 +532,7 @@ int lpb_filter(double* out, const double* v, const int* toff, const double* tw, 
 int lpb_oc_step_base(double* ts, const double* x, const double* dc, const double* dv, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !ts || !x || !dc || !dv) return LP_ERR_ARG;
-  k_oc_step_base<<<lp_blocks(g.cells_padded(), 256), 256, 0, LP_ST>>>(ts, x, dc, dv, g);
+  lp_launch(k_oc_step_base, lp_blocks(g.cells_padded(), 256), 256, 0, LP_ST, ts, x, dc, dv, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -559,7 +562,7 @@ int lpb_oc_trial(double* xn, double* xt, double* xp, const double* ts, const dou
     rc = launch_march(in, o, toff, tw, ntaps, reach, g, vec, part, &nb, LP_ST);
   }
   if (rc != LP_OK) return rc;
-  k_filter_volume<<<1, 512, 0, LP_ST>>>(part, nb, vol);
+  lp_launch(k_filter_volume, 1, 512, 0, LP_ST, part, nb, vol);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }

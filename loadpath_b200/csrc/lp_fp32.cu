@@ -20,6 +20,7 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
 __global__ void __launch_bounds__(128) k_rf_cells(float* __restrict__ ft, const float* __restrict__ h,
                                                   const float* __restrict__ l, const uint8_t* __restrict__ mask,
                                                   const float* __restrict__ e, const float* __restrict__ ke, LpGrid g) {
+  lp_after_launch();
   __shared__ float sk[576];
   for (int i = threadIdx.x; i < 576; i += blockDim.x) sk[i] = ke[i];
   __syncthreads();
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(128) k_rf_cells(float* __restrict__ ft, const 
 // out = m * (sum of the node's cells' rows) + (1 - m) * h
 __global__ void k_rf_gather(float* __restrict__ out, const float* __restrict__ ft, const float* __restrict__ h,
                             const uint8_t* __restrict__ mask, LpGrid g) {
+  lp_after_launch();
   const long long total = g.nodes_padded();
   const long long ncp = g.cells_padded(), cs = g.comp_stride();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -114,12 +116,14 @@ __global__ void k_rf_gather(float* __restrict__ out, const float* __restrict__ f
 // r = (bh - ax) + bl
 __global__ void k_pair_residual(float* __restrict__ r, const float* __restrict__ bh, const float* __restrict__ ax,
                                 const float* __restrict__ bl, long long n) {
+  lp_after_launch();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     r[i] = __fadd_rn(__fsub_rn(bh[i], ax[i]), bl[i]);
 }
 
 // (xh, xl) += d in pair arithmetic: xh, e = two_sum(xh, d); xl += e; xh, xl = two_sum(xh, xl)
 __global__ void k_pair_add(float* __restrict__ xh, float* __restrict__ xl, const float* __restrict__ d, long long n) {
+  lp_after_launch();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     float s, e;
     two_sum(xh[i], d[i], s, e);
@@ -146,22 +150,22 @@ int lpb_apply_rf_f32(float* out, const float* h, const float* l, const uint8_t* 
                      const float* ke, float* ft, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !out || !h || !mask || !e || !ke || !ft || out == h || out == l) return LP_ERR_ARG;
-  k_rf_cells<<<lp_blocks(g.cells_padded(), 128), 128, 0, LP_ST>>>(ft, h, l, mask, e, ke, g);
-  k_rf_gather<<<lp_blocks(g.nodes_padded(), 256), 256, 0, LP_ST>>>(out, ft, h, mask, g);
+  lp_launch(k_rf_cells, lp_blocks(g.cells_padded(), 128), 128, 0, LP_ST, ft, h, l, mask, e, ke, g);
+  lp_launch(k_rf_gather, lp_blocks(g.nodes_padded(), 256), 256, 0, LP_ST, out, ft, h, mask, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_pair_residual_f32(float* r, const float* bh, const float* ax, const float* bl, long long n, void* stream) {
   if (!r || !bh || !ax || !bl || n < 0) return LP_ERR_ARG;
-  k_pair_residual<<<lp_blocks(n, 256), 256, 0, LP_ST>>>(r, bh, ax, bl, n);
+  lp_launch(k_pair_residual, lp_blocks(n, 256), 256, 0, LP_ST, r, bh, ax, bl, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_pair_add_f32(float* xh, float* xl, const float* d, long long n, void* stream) {
   if (!xh || !xl || !d || n < 0) return LP_ERR_ARG;
-  k_pair_add<<<lp_blocks(n, 256), 256, 0, LP_ST>>>(xh, xl, d, n);
+  lp_launch(k_pair_add, lp_blocks(n, 256), 256, 0, LP_ST, xh, xl, d, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }

@@ -16,6 +16,7 @@ namespace {
 // otherwise. The loop continues while the test fails and fewer than maxiter iterations ran.
 __global__ void k_cg_continue(cudaGraphConditionalHandle handle, const double* __restrict__ sc,
                               long long* __restrict__ state, double rtol, long long maxiter) {
+  lp_after_launch();
   const long long it = state[0] + 1;
   state[0] = it;
   const double bb = sc[0], pap = sc[3], rr = sc[4];
@@ -32,6 +33,7 @@ __global__ void k_cg_continue(cudaGraphConditionalHandle handle, const double* _
 // iteration count. The loop continues while a column runs and fewer than maxiter iterations ran.
 __global__ void k_cg_continue_cols(cudaGraphConditionalHandle handle, const double* __restrict__ sc,
                                    long long* __restrict__ state, int k, double rtol, long long maxiter) {
+  lp_after_launch();
   const long long it = state[2 * k] + 1;
   state[2 * k] = it;
   bool running = false;
@@ -57,6 +59,7 @@ __global__ void k_cg_continue_cols(cudaGraphConditionalHandle handle, const doub
 __global__ void k_snapshot_converged(double* __restrict__ out, const double* __restrict__ x,
                                      const uint8_t* __restrict__ m, const long long* __restrict__ state, int col,
                                      int k, LpGrid g) {
+  lp_after_launch();
   if (state[2 * col + 1] != 1 || state[2 * col] != state[2 * k]) return;
   const long long nn = g.nodes_padded();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < 3 * nn; t += (long long)gridDim.x * blockDim.x) {
@@ -163,7 +166,7 @@ int lpb_while_end(void* stream, void* graph, void** exec) {
 int lpb_cg_continue(long long handle, const double* sc, long long* state, double rtol, long long maxiter,
                     void* stream) {
   if (!sc || !state || maxiter < 1) return LP_ERR_ARG;
-  k_cg_continue<<<1, 1, 0, LP_ST>>>((cudaGraphConditionalHandle)handle, sc, state, rtol, maxiter);
+  lp_launch(k_cg_continue, 1, 1, 0, LP_ST, (cudaGraphConditionalHandle)handle, sc, state, rtol, maxiter);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -211,7 +214,7 @@ int lpb_graph_free(void* exec) {
 int lpb_cg_continue_cols(long long handle, const double* sc, long long* state, int k, double rtol, long long maxiter,
                          void* stream) {
   if (!sc || !state || k < 1 || maxiter < 1) return LP_ERR_ARG;
-  k_cg_continue_cols<<<1, 1, 0, LP_ST>>>((cudaGraphConditionalHandle)handle, sc, state, k, rtol, maxiter);
+  lp_launch(k_cg_continue_cols, 1, 1, 0, LP_ST, (cudaGraphConditionalHandle)handle, sc, state, k, rtol, maxiter);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -221,7 +224,7 @@ int lpb_snapshot_converged(double* out, const double* x, const uint8_t* mask, co
                            LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !out || !x || !mask || !state || col < 0 || col >= k || out == x) return LP_ERR_ARG;
-  k_snapshot_converged<<<lp_blocks(3 * g.nodes_padded(), 256), 256, 0, LP_ST>>>(out, x, mask, state, col, k, g);
+  lp_launch(k_snapshot_converged, lp_blocks(3 * g.nodes_padded(), 256), 256, 0, LP_ST, out, x, mask, state, col, k, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }

@@ -21,6 +21,7 @@ constexpr int LH = LT + 2;       // with the halo
 // partial counts of alive cells
 __global__ void k_live_seed(uint8_t* __restrict__ state, const double* __restrict__ xp,
                             const uint8_t* __restrict__ flags, double thr, LpGrid g, double* __restrict__ part) {
+  lp_after_launch();
   __shared__ double sh[32];
   const long long total = g.cells_padded();
   double cnt = 0.0;
@@ -44,6 +45,7 @@ __global__ void k_live_seed(uint8_t* __restrict__ state, const double* __restric
 // partial counts of the cells alive in state (seeded: nonzero) but not kept in keep (a flooded state: 2)
 __global__ void k_live_outside(const uint8_t* __restrict__ state, const uint8_t* __restrict__ keep, LpGrid g,
                                double* __restrict__ part) {
+  lp_after_launch();
   __shared__ double sh[32];
   const long long total = g.cells_padded();
   double cnt = 0.0;
@@ -54,6 +56,7 @@ __global__ void k_live_outside(const uint8_t* __restrict__ state, const uint8_t*
 }
 
 __global__ void k_live_count_final(const double* __restrict__ part, int n, double* __restrict__ out) {
+  lp_after_launch();
   __shared__ double sh[32];
   double s = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += part[i];
@@ -63,6 +66,7 @@ __global__ void k_live_count_final(const double* __restrict__ part, int n, doubl
 
 __global__ void __launch_bounds__(LT * LT * LT) k_live_flood(uint8_t* __restrict__ state, LpGrid g,
                                                             int* __restrict__ changed) {
+  lp_after_launch();
   __shared__ uint8_t s[LH][LH][LH];
   const int tid = threadIdx.x;
   const int x0 = blockIdx.x * LT - 1, y0 = blockIdx.y * LT - 1, z0 = blockIdx.z * LT - 1;
@@ -101,6 +105,7 @@ __global__ void __launch_bounds__(LT * LT * LT) k_live_flood(uint8_t* __restrict
 // e_out = e on reached cells, 0 elsewhere
 __global__ void k_live_moduli(double* __restrict__ e_out, const double* __restrict__ e,
                               const uint8_t* __restrict__ state, long long n) {
+  lp_after_launch();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
     e_out[t] = state[t] == 2 ? e[t] : 0.0;
 }
@@ -108,6 +113,7 @@ __global__ void k_live_moduli(double* __restrict__ e_out, const double* __restri
 // dofs that carry a load but no stiffness (the level-0 mask's alive bits clear)
 __global__ void k_dead_loads(const double* __restrict__ f, const uint8_t* __restrict__ mask, LpGrid g,
                              double* __restrict__ part) {
+  lp_after_launch();
   __shared__ double sh[32];
   const long long nn = g.nodes_padded();
   double cnt = 0.0;
@@ -135,8 +141,8 @@ int lpb_live_seed(uint8_t* state, const double* xp, const uint8_t* flags, double
                   double* n_alive, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !state || !xp || !part || !n_alive) return LP_ERR_ARG;
-  k_live_seed<<<LP_LIVE_BLOCKS, 256, 0, LP_ST>>>(state, xp, flags, alive_thr, g, part);
-  k_live_count_final<<<1, 1024, 0, LP_ST>>>(part, LP_LIVE_BLOCKS, n_alive);
+  lp_launch(k_live_seed, LP_LIVE_BLOCKS, 256, 0, LP_ST, state, xp, flags, alive_thr, g, part);
+  lp_launch(k_live_count_final, 1, 1024, 0, LP_ST, part, LP_LIVE_BLOCKS, n_alive);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -146,7 +152,7 @@ int lpb_live_flood(uint8_t* state, int* changed, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !state || !changed) return LP_ERR_ARG;
   const dim3 grid((g.nx + LT - 1) / LT, (g.ny + LT - 1) / LT, (g.nz + LT - 1) / LT);
-  k_live_flood<<<grid, LT * LT * LT, 0, LP_ST>>>(state, g, changed);
+  lp_launch(k_live_flood, grid, LT * LT * LT, 0, LP_ST, state, g, changed);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -155,7 +161,7 @@ int lpb_live_moduli(double* e_out, const double* e, const uint8_t* state, LP_GRI
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !e_out || !e || !state) return LP_ERR_ARG;
   const long long n = g.cells_padded();
-  k_live_moduli<<<lp_blocks(n, 256), 256, 0, LP_ST>>>(e_out, e, state, n);
+  lp_launch(k_live_moduli, lp_blocks(n, 256), 256, 0, LP_ST, e_out, e, state, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -167,8 +173,8 @@ int lpb_live_outside(const uint8_t* state, const uint8_t* keep, double* part, do
                      void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !state || !keep || !part || !count) return LP_ERR_ARG;
-  k_live_outside<<<LP_LIVE_BLOCKS, 256, 0, LP_ST>>>(state, keep, g, part);
-  k_live_count_final<<<1, 1024, 0, LP_ST>>>(part, LP_LIVE_BLOCKS, count);
+  lp_launch(k_live_outside, LP_LIVE_BLOCKS, 256, 0, LP_ST, state, keep, g, part);
+  lp_launch(k_live_count_final, 1, 1024, 0, LP_ST, part, LP_LIVE_BLOCKS, count);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -177,8 +183,8 @@ int lpb_live_outside(const uint8_t* state, const uint8_t* keep, double* part, do
 int lpb_dead_loads(const double* f, const uint8_t* mask, double* part, double* count, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !f || !mask || !part || !count) return LP_ERR_ARG;
-  k_dead_loads<<<LP_LIVE_BLOCKS, 256, 0, LP_ST>>>(f, mask, g, part);
-  k_live_count_final<<<1, 1024, 0, LP_ST>>>(part, LP_LIVE_BLOCKS, count);
+  lp_launch(k_dead_loads, LP_LIVE_BLOCKS, 256, 0, LP_ST, f, mask, g, part);
+  lp_launch(k_live_count_final, 1, 1024, 0, LP_ST, part, LP_LIVE_BLOCKS, count);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }

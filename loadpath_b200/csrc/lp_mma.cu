@@ -58,6 +58,7 @@ __device__ __forceinline__ void block_reduce(double (&v)[K], const bool (&is_max
 
 __global__ void k_mma_final(const double* __restrict__ part, int nblocks, int K, const int* __restrict__ maxmask,
                             double* __restrict__ out) {
+  lp_after_launch();
   // one warp per value, blocks summed in a fixed order
   const int k = blockIdx.x;
   if (k >= K) return;
@@ -80,6 +81,7 @@ __global__ void __launch_bounds__(LP_MMA_THREADS) k_mma_prepare(
     double* __restrict__ df0, double* __restrict__ df, double* __restrict__ alfa, double* __restrict__ beta,
     double* __restrict__ p0, double* __restrict__ q0, double* __restrict__ P, double* __restrict__ Q,
     double* __restrict__ part) {
+  lp_after_launch();
   double acc[M];
   bool is_max[M];
 #pragma unroll
@@ -136,6 +138,7 @@ __global__ void __launch_bounds__(LP_MMA_THREADS) k_mma_prepare(
 // ---- subsolver -------------------------------------------------------------------------------
 __global__ void k_mma_sub_init(long long n, const double* __restrict__ alfa, const double* __restrict__ beta,
                                double* __restrict__ xs, double* __restrict__ xsi, double* __restrict__ eta) {
+  lp_after_launch();
   for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x) {
     const double a = alfa[j], b = beta[j], x = 0.5 * (a + b);
     xs[j] = x;
@@ -158,6 +161,7 @@ __global__ void __launch_bounds__(LP_MMA_THREADS) k_mma_newton_a(long long n, in
                                                                  double epsi, double* __restrict__ delx,
                                                                  double* __restrict__ diagx,
                                                                  double* __restrict__ part) {
+  lp_after_launch();
   constexpr int K = 2 * M + M * (M + 1) / 2;
   double acc[K];
   bool is_max[K];
@@ -211,6 +215,7 @@ __global__ void __launch_bounds__(LP_MMA_THREADS) k_mma_newton_b(long long n, in
                                                                  double epsi, double* __restrict__ dx,
                                                                  double* __restrict__ dxsi, double* __restrict__ deta,
                                                                  double* __restrict__ part) {
+  lp_after_launch();
   double acc[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
   const bool is_max[4] = {true, true, true, true};
   for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x) {
@@ -251,6 +256,7 @@ __global__ void __launch_bounds__(LP_MMA_THREADS) k_mma_trial(long long n, int m
                                                               double epsi, double* __restrict__ xs,
                                                               double* __restrict__ xsi, double* __restrict__ eta,
                                                               double* __restrict__ part) {
+  lp_after_launch();
   constexpr int K = 2 + M;
   double acc[K];
   bool is_max[K];
@@ -291,6 +297,7 @@ __global__ void __launch_bounds__(LP_MMA_THREADS) k_mma_trial(long long n, int m
 __global__ void k_mma_finish(long long n, const double* __restrict__ xs, const double* __restrict__ x,
                              const double* __restrict__ alfa, const double* __restrict__ beta,
                              double* __restrict__ xnew) {
+  lp_after_launch();
   for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x) {
     double v = xs[j];
     if (!isfinite(v)) v = x[j];
@@ -304,7 +311,7 @@ __device__ int g_mask_max4[4] = {1, 1, 1, 1};
 __device__ int g_mask_trial[2 + LP_MMA_MAXM] = {0, 1};   // [1]: the largest magnitude
 
 static int final_reduce(const double* part, int K, const int* mask_dev, double* out, cudaStream_t st) {
-  k_mma_final<<<K, 32, 0, st>>>(part, LP_MMA_BLOCKS, K, mask_dev, out);
+  lp_launch(k_mma_final, K, 32, 0, st, part, LP_MMA_BLOCKS, K, mask_dev, out);
   return LP_OK;
 }
 
@@ -334,10 +341,10 @@ static MVec mvec(const double* h, int m) {
 #define MMA_GRID LP_MMA_BLOCKS, LP_MMA_THREADS, 0, LP_ST
 #define MMA_DISPATCH(KERNEL, ...)                                              \
   switch (mma_m_template(m)) {                                                  \
-    case 1: KERNEL<1><<<MMA_GRID>>>(__VA_ARGS__); break;                        \
-    case 2: KERNEL<2><<<MMA_GRID>>>(__VA_ARGS__); break;                        \
-    case 4: KERNEL<4><<<MMA_GRID>>>(__VA_ARGS__); break;                        \
-    default: KERNEL<8><<<MMA_GRID>>>(__VA_ARGS__); break;                       \
+    case 1: lp_launch(KERNEL<1>, MMA_GRID, __VA_ARGS__); break;                        \
+    case 2: lp_launch(KERNEL<2>, MMA_GRID, __VA_ARGS__); break;                        \
+    case 4: lp_launch(KERNEL<4>, MMA_GRID, __VA_ARGS__); break;                        \
+    default: lp_launch(KERNEL<8>, MMA_GRID, __VA_ARGS__); break;                       \
   }
 
 extern "C" {
@@ -373,7 +380,7 @@ int lpb_mma_prepare(long long n, int m, double* x, const double* xmin, const dou
 int lpb_mma_sub_init(long long n, const double* alfa, const double* beta, double* xs, double* xsi, double* eta,
                      void* stream) {
   if (n < 1 || !alfa || !beta || !xs || !xsi || !eta) return LP_ERR_ARG;
-  k_mma_sub_init<<<MMA_GRID>>>(n, alfa, beta, xs, xsi, eta);
+  lp_launch(k_mma_sub_init, MMA_GRID, n, alfa, beta, xs, xsi, eta);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -440,7 +447,7 @@ int lpb_mma_trial(long long n, int m, const double* low, const double* upp, cons
 int lpb_mma_finish(long long n, const double* xs, const double* x, const double* alfa, const double* beta,
                    double* xnew, void* stream) {
   if (n < 1 || !xs || !x || !alfa || !beta || !xnew) return LP_ERR_ARG;
-  k_mma_finish<<<MMA_GRID>>>(n, xs, x, alfa, beta, xnew);
+  lp_launch(k_mma_finish, MMA_GRID, n, xs, x, alfa, beta, xnew);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }

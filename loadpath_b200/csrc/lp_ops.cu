@@ -49,6 +49,7 @@ __device__ __forceinline__ void gather24(const T* __restrict__ u, const uint8_t*
 template <typename T, int KIND>
 __global__ void k_apply_level(T* __restrict__ out, const T* __restrict__ u, const uint8_t* __restrict__ mask,
                               LpGrid g, LevelArgs<T> a, int mask_in, int finish) {
+  lp_after_launch();
   extern __shared__ unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
   // stage the level's fixed matrices in shared memory
@@ -149,7 +150,7 @@ int launch_apply(T* out, const T* u, const uint8_t* mask, LpGrid g, LevelArgs<T>
   int threads = 256;
   int blocks = lp_blocks(total, threads);
   if (blocks > 148 * 64) blocks = 148 * 64;
-  k_apply_level<T, KIND><<<blocks, threads, smem, st>>>(out, u, mask, g, a, mask_in, finish);
+  lp_launch(k_apply_level<T, KIND>, blocks, threads, smem, st, out, u, mask, g, a, mask_in, finish);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -157,6 +158,7 @@ int launch_apply(T* out, const T* u, const uint8_t* mask, LpGrid g, LevelArgs<T>
 // diagonal of the unmasked K, float64 (3, nodes)
 template <typename T, int KIND>
 __global__ void k_diag_level(double* __restrict__ d, LpGrid g, LevelArgs<T> a) {
+  lp_after_launch();
   const long long total = g.nodes_padded();
   const long long cs = g.comp_stride();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
@@ -193,7 +195,7 @@ template <typename T, int KIND>
 int launch_diag(double* d, LpGrid g, LevelArgs<T> a, cudaStream_t st) {
   if (!lp_grid_ok(g) || !d) return LP_ERR_ARG;
   long long total = g.nodes_padded();
-  k_diag_level<T, KIND><<<lp_blocks(total, 256), 256, 0, st>>>(d, g, a);
+  lp_launch(k_diag_level<T, KIND>, lp_blocks(total, 256), 256, 0, st, d, g, a);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -208,6 +210,7 @@ __global__ void k_masks(uint8_t* __restrict__ mask, double* __restrict__ dinv64,
                         const double* __restrict__ d, const uint8_t* __restrict__ held_bits,
                         const float* __restrict__ kept, LpGrid g, double alive_thr, double live_thr,
                         const double* __restrict__ thr_scale) {
+  lp_after_launch();
   if (thr_scale) {
     const double sc = fmax(*thr_scale, 1e-300);
     alive_thr *= sc;
@@ -242,6 +245,7 @@ __global__ void k_masks(uint8_t* __restrict__ mask, double* __restrict__ dinv64,
 // of the caller, which reads back one value per block)
 __global__ void k_max_abs_diff_partial(const double* __restrict__ a, const double* __restrict__ b, long long n,
                                        double* __restrict__ part) {
+  lp_after_launch();
   __shared__ double sh[32];
   double m = 0.0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -257,6 +261,7 @@ __global__ void k_max_abs_diff_partial(const double* __restrict__ a, const doubl
 }
 
 __global__ void k_max_partial(const double* __restrict__ a, long long n, double* __restrict__ part) {
+  lp_after_launch();
   __shared__ double sh[32];
   double m = -1e308;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -272,6 +277,7 @@ __global__ void k_max_partial(const double* __restrict__ a, long long n, double*
 }
 
 __global__ void k_max_final(const double* __restrict__ part, int n, double* __restrict__ out) {
+  lp_after_launch();
   __shared__ double sh[32];
   double m = -1e308;
   for (int i = threadIdx.x; i < n; i += blockDim.x) m = fmax(m, part[i]);
@@ -299,6 +305,7 @@ __device__ __forceinline__ void lp_count_store(double c, double* part) {
 
 // cells with modulus > 0 (all padded cells; the padding holds zeros)
 __global__ void k_count_pos(const double* __restrict__ e, long long n, double* __restrict__ part) {
+  lp_after_launch();
   double c = 0.0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     c += e[i] > 0.0 ? 1.0 : 0.0;
@@ -309,6 +316,7 @@ __global__ void k_count_pos(const double* __restrict__ e, long long n, double* _
 template <typename T>
 __global__ void k_count_weights(const T* __restrict__ w, const int* __restrict__ patch_id, LpGrid g,
                                 double* __restrict__ part) {
+  lp_after_launch();
   const long long ncp = g.cells_padded();
   double c = 0.0;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < ncp;
@@ -326,6 +334,7 @@ __global__ void k_count_weights(const T* __restrict__ w, const int* __restrict__
 // explicit-level cells whose 24 x 24 matrix has a non-zero entry; one warp per cell
 template <typename T>
 __global__ void k_count_explicit(const T* __restrict__ k, LpGrid g, double* __restrict__ part) {
+  lp_after_launch();
   const long long total = g.cells_padded();
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
@@ -344,6 +353,7 @@ __global__ void k_count_explicit(const T* __restrict__ k, LpGrid g, double* __re
 // positions where two byte arrays differ
 __global__ void k_count_ne_u8(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b, long long n,
                               double* __restrict__ part) {
+  lp_after_launch();
   double c = 0.0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     c += a[i] != b[i] ? 1.0 : 0.0;
@@ -351,6 +361,7 @@ __global__ void k_count_ne_u8(const uint8_t* __restrict__ a, const uint8_t* __re
 }
 
 __global__ void k_count_final(const double* __restrict__ part, int n, double* __restrict__ out) {
+  lp_after_launch();
   __shared__ double sh[32];
   double s = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += part[i];
@@ -456,7 +467,7 @@ int lpb_masks(uint8_t* mask, double* dinv64, float* dinv32, const double* d, con
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !mask || !d) return LP_ERR_ARG;
   long long total = g.nodes_padded();
-  k_masks<<<lp_blocks(total, 256), 256, 0, (cudaStream_t)stream>>>(mask, dinv64, dinv32, d, held_bits, kept, g,
+  lp_launch(k_masks, lp_blocks(total, 256), 256, 0, (cudaStream_t)stream, mask, dinv64, dinv32, d, held_bits, kept, g,
                                                                    alive_thr, live_thr, thr_scale);
   LP_LAUNCH_CHECK();
   return LP_OK;
@@ -467,8 +478,8 @@ int lpb_max_f64(const double* a, long long n, double* part, double* out, void* s
   if (!a || !part || !out || n < 0) return LP_ERR_ARG;
   int blocks = lp_blocks(n, 256);
   if (blocks > 1024) blocks = 1024;
-  k_max_partial<<<blocks, 256, 0, (cudaStream_t)stream>>>(a, n, part);
-  k_max_final<<<1, 1024, 0, (cudaStream_t)stream>>>(part, blocks, out);
+  lp_launch(k_max_partial, blocks, 256, 0, (cudaStream_t)stream, a, n, part);
+  lp_launch(k_max_final, 1, 1024, 0, (cudaStream_t)stream, part, blocks, out);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -478,8 +489,8 @@ int lpb_max_abs_diff_f64(const double* a, const double* b, long long n, double* 
   if (!a || !b || !part || !out || n < 0) return LP_ERR_ARG;
   int blocks = lp_blocks(n, 256);
   if (blocks > 1024) blocks = 1024;
-  k_max_abs_diff_partial<<<blocks, 256, 0, (cudaStream_t)stream>>>(a, b, n, part);
-  k_max_final<<<1, 1024, 0, (cudaStream_t)stream>>>(part, blocks, out);
+  lp_launch(k_max_abs_diff_partial, blocks, 256, 0, (cudaStream_t)stream, a, b, n, part);
+  lp_launch(k_max_final, 1, 1024, 0, (cudaStream_t)stream, part, blocks, out);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -487,8 +498,8 @@ int lpb_max_abs_diff_f64(const double* a, const double* b, long long n, double* 
 // ---- counts into a device scalar; part: scratch of at least 592 doubles ----------------
 int lpb_count_positive_f64(const double* e, long long n, double* part, double* out, void* stream) {
   if (!e || !part || !out || n < 0) return LP_ERR_ARG;
-  k_count_pos<<<LP_COUNT_BLOCKS, 256, 0, (cudaStream_t)stream>>>(e, n, part);
-  k_count_final<<<1, 1024, 0, (cudaStream_t)stream>>>(part, LP_COUNT_BLOCKS, out);
+  lp_launch(k_count_pos, LP_COUNT_BLOCKS, 256, 0, (cudaStream_t)stream, e, n, part);
+  lp_launch(k_count_final, 1, 1024, 0, (cudaStream_t)stream, part, LP_COUNT_BLOCKS, out);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -497,8 +508,8 @@ int lpb_count_active_weights_f32(const float* w, const int* patch_id, LP_GRID_AR
                                  void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !w || !part || !out) return LP_ERR_ARG;
-  k_count_weights<float><<<LP_COUNT_BLOCKS, 256, 0, (cudaStream_t)stream>>>(w, patch_id, g, part);
-  k_count_final<<<1, 1024, 0, (cudaStream_t)stream>>>(part, LP_COUNT_BLOCKS, out);
+  lp_launch(k_count_weights<float>, LP_COUNT_BLOCKS, 256, 0, (cudaStream_t)stream, w, patch_id, g, part);
+  lp_launch(k_count_final, 1, 1024, 0, (cudaStream_t)stream, part, LP_COUNT_BLOCKS, out);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -507,8 +518,8 @@ int lpb_count_active_weights_f64(const double* w, const int* patch_id, LP_GRID_A
                                  void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !w || !part || !out) return LP_ERR_ARG;
-  k_count_weights<double><<<LP_COUNT_BLOCKS, 256, 0, (cudaStream_t)stream>>>(w, patch_id, g, part);
-  k_count_final<<<1, 1024, 0, (cudaStream_t)stream>>>(part, LP_COUNT_BLOCKS, out);
+  lp_launch(k_count_weights<double>, LP_COUNT_BLOCKS, 256, 0, (cudaStream_t)stream, w, patch_id, g, part);
+  lp_launch(k_count_final, 1, 1024, 0, (cudaStream_t)stream, part, LP_COUNT_BLOCKS, out);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -516,8 +527,8 @@ int lpb_count_active_weights_f64(const double* w, const int* patch_id, LP_GRID_A
 int lpb_count_active_explicit_f32(const float* k, LP_GRID_ARGS, double* part, double* out, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !k || !part || !out) return LP_ERR_ARG;
-  k_count_explicit<float><<<LP_COUNT_BLOCKS, 256, 0, (cudaStream_t)stream>>>(k, g, part);
-  k_count_final<<<1, 1024, 0, (cudaStream_t)stream>>>(part, LP_COUNT_BLOCKS, out);
+  lp_launch(k_count_explicit<float>, LP_COUNT_BLOCKS, 256, 0, (cudaStream_t)stream, k, g, part);
+  lp_launch(k_count_final, 1, 1024, 0, (cudaStream_t)stream, part, LP_COUNT_BLOCKS, out);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -525,16 +536,16 @@ int lpb_count_active_explicit_f32(const float* k, LP_GRID_ARGS, double* part, do
 int lpb_count_active_explicit_f64(const double* k, LP_GRID_ARGS, double* part, double* out, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !k || !part || !out) return LP_ERR_ARG;
-  k_count_explicit<double><<<LP_COUNT_BLOCKS, 256, 0, (cudaStream_t)stream>>>(k, g, part);
-  k_count_final<<<1, 1024, 0, (cudaStream_t)stream>>>(part, LP_COUNT_BLOCKS, out);
+  lp_launch(k_count_explicit<double>, LP_COUNT_BLOCKS, 256, 0, (cudaStream_t)stream, k, g, part);
+  lp_launch(k_count_final, 1, 1024, 0, (cudaStream_t)stream, part, LP_COUNT_BLOCKS, out);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_count_ne_u8(const uint8_t* a, const uint8_t* b, long long n, double* part, double* out, void* stream) {
   if (!a || !b || !part || !out || n < 0) return LP_ERR_ARG;
-  k_count_ne_u8<<<LP_COUNT_BLOCKS, 256, 0, (cudaStream_t)stream>>>(a, b, n, part);
-  k_count_final<<<1, 1024, 0, (cudaStream_t)stream>>>(part, LP_COUNT_BLOCKS, out);
+  lp_launch(k_count_ne_u8, LP_COUNT_BLOCKS, 256, 0, (cudaStream_t)stream, a, b, n, part);
+  lp_launch(k_count_final, 1, 1024, 0, (cudaStream_t)stream, part, LP_COUNT_BLOCKS, out);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }

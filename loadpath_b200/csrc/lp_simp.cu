@@ -13,6 +13,7 @@ namespace {
 
 // e = emin + x^p (1 - emin) on the grid's cells (padding untouched)
 __global__ void k_simp_law(double* __restrict__ e, const double* __restrict__ x, double penal, double emin, LpGrid g) {
+  lp_after_launch();
   const long long total = g.cells_padded();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int x_, y_, z;
@@ -31,6 +32,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) k_element_energy(double* __restrict__ ce, const T* __restrict__ u,
                                                         const T* __restrict__ v, const double* __restrict__ ke,
                                                         LpGrid g) {
+  lp_after_launch();
   __shared__ double kh[576];
   __shared__ double wmax[4];
   constexpr int rows[LP_MODAL_NNZ] = LP_MODAL_ROWS;
@@ -103,6 +105,7 @@ __global__ void __launch_bounds__(128) k_element_energy(double* __restrict__ ce,
 __global__ void k_sensitivity(double* __restrict__ dc, const double* __restrict__ xphys, const double* __restrict__ ce,
                               const double* __restrict__ e, double penal, double emin, double scale, int accumulate,
                               LpGrid g, double* __restrict__ part) {
+  lp_after_launch();
   __shared__ double sh[32];
   const long long total = g.cells_padded();
   double acc = 0.0;
@@ -144,6 +147,7 @@ __global__ void __launch_bounds__(256, 2) k_oc_volumes(const double* __restrict_
                                                        const double* __restrict__ dv, const double* __restrict__ gv,
                                                        const double* __restrict__ lam, double move, LpGrid g,
                                                        double* __restrict__ part) {
+  lp_after_launch();
   __shared__ double s_isl[NL];
   __shared__ double sacc[NL][8];
   if (threadIdx.x < NL) s_isl[threadIdx.x] = 1.0 / sqrt(lam[threadIdx.x]);
@@ -194,6 +198,7 @@ __global__ void __launch_bounds__(256, 2) k_oc_volumes(const double* __restrict_
 // the nl volumes from the blocks' partial sums: one warp per multiplier, its lanes striding over
 // the blocks, then a shuffle tree (a fixed order, so the sums are the same every run)
 __global__ void k_oc_final(const double* __restrict__ part, int nblocks, int nl, double* __restrict__ out) {
+  lp_after_launch();
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   for (int j = threadIdx.x >> 5; j < nl; j += nw) {
     double s = 0.0;
@@ -215,6 +220,7 @@ __global__ void k_oc_final(const double* __restrict__ part, int nblocks, int nl,
 __global__ void k_oc_walk(cudaGraphConditionalHandle handle, int use_handle, double* __restrict__ state,
                           const double* __restrict__ vols, double* __restrict__ cands, double target, double tol,
                           int absorb) {
+  lp_after_launch();
   double l1 = state[0], l2 = state[1], below = state[2], above = state[3], lmid = state[4], passes = state[5];
   if (absorb) {
     for (int j = 0; j < 31; ++j) {
@@ -268,6 +274,7 @@ __global__ void k_oc_walk(cudaGraphConditionalHandle handle, int use_handle, dou
 }
 
 __global__ void k_oc_walk_init(double* __restrict__ state, double l2) {
+  lp_after_launch();
   state[0] = 0.0;
   state[1] = l2;
   state[2] = __longlong_as_double(0x7ff0000000000000LL);    // +inf
@@ -282,6 +289,7 @@ __global__ void k_oc_walk_init(double* __restrict__ state, double l2) {
 __global__ void k_oc_apply(double* __restrict__ xnew, const double* __restrict__ x, const double* __restrict__ dc,
                            const double* __restrict__ dv, double lam_h, const double* __restrict__ lam_dev,
                            double move, LpGrid g, double* __restrict__ part) {
+  lp_after_launch();
   __shared__ double sh[32];
   const double lam = lam_dev ? *lam_dev : lam_h;
   const long long total = g.cells_padded();
@@ -307,6 +315,7 @@ __global__ void k_oc_apply(double* __restrict__ xnew, const double* __restrict__
 }
 
 __global__ void k_max_final2(const double* __restrict__ part, int n, double* __restrict__ out) {
+  lp_after_launch();
   double m = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) m = fmax(m, part[i]);
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
@@ -321,6 +330,7 @@ __global__ void k_max_final2(const double* __restrict__ part, int n, double* __r
 }
 
 __global__ void k_sum_final_s(const double* __restrict__ part, int n, double* __restrict__ out) {
+  lp_after_launch();
   __shared__ double sh[32];
   double s = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += part[i];
@@ -339,6 +349,7 @@ __global__ void k_sum_final_s(const double* __restrict__ part, int n, double* __
 __global__ void k_project(double* __restrict__ xp, double* __restrict__ dxp, const double* __restrict__ xt,
                           double beta, double eta, double tbe, double den, const uint8_t* __restrict__ flags,
                           const double* __restrict__ w, LpGrid g, double* __restrict__ part) {
+  lp_after_launch();
   __shared__ double sh[32];
   const long long total = g.cells_padded();
   double acc = 0.0;
@@ -370,6 +381,7 @@ __global__ void k_project(double* __restrict__ xp, double* __restrict__ dxp, con
 __global__ void k_oc_stepped(double* __restrict__ xn, const double* __restrict__ x, const double* __restrict__ dc,
                              const double* __restrict__ dv, double lm, double move, const uint8_t* __restrict__ flags,
                              LpGrid g) {
+  lp_after_launch();
   const double sl = sqrt(lm);
   const long long total = g.cells_padded();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -387,6 +399,7 @@ __global__ void k_oc_stepped(double* __restrict__ xn, const double* __restrict__
 // out = a * b (zero where the flags hold a cell); with clip0, out = min(out, 0)
 __global__ void k_cell_product(double* __restrict__ out, const double* __restrict__ a, const double* __restrict__ b,
                                const uint8_t* __restrict__ flags, int clip0, LpGrid g) {
+  lp_after_launch();
   const long long total = g.cells_padded();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int x_, y_, z;
@@ -404,6 +417,7 @@ __global__ void k_cell_product(double* __restrict__ out, const double* __restric
 // has a mirror): one thread per pair, the cell below the mid-plane; the middle cell of an odd
 // extent is its own image and keeps its value.
 __global__ void k_mirror_average(double* __restrict__ v, int axis, LpGrid g) {
+  lp_after_launch();
   const long long total = g.cells_padded();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int x, y, z;
@@ -426,6 +440,7 @@ __global__ void k_mirror_average(double* __restrict__ v, int axis, LpGrid g) {
 // caller has checked every index against the vectors' length.
 __global__ void k_energy_edof(double* __restrict__ ce, const double* __restrict__ u, const double* __restrict__ v,
                               const long long* __restrict__ edof, const double* __restrict__ ke, long long ne) {
+  lp_after_launch();
   __shared__ double sk[576];
   for (int i = threadIdx.x; i < 576; i += blockDim.x) sk[i] = ke[i];
   __syncthreads();
@@ -463,7 +478,7 @@ int lpb_simp_law(double* e, const double* x, double penal, double emin, LP_GRID_
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !e || !x) return LP_ERR_ARG;
   long long total = g.cells_padded();
-  k_simp_law<<<lp_blocks(total, 256), 256, 0, LP_ST>>>(e, x, penal, emin, g);
+  lp_launch(k_simp_law, lp_blocks(total, 256), 256, 0, LP_ST, e, x, penal, emin, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -472,7 +487,7 @@ int lpb_element_energy_edof(double* ce, const double* u, const double* v, const 
                             long long ne, void* stream) {
   if (!ce || !u || !edof || !ke || ne < 0) return LP_ERR_ARG;
   if (ne == 0) return LP_OK;
-  k_energy_edof<<<lp_blocks(ne, 128), 128, 0, LP_ST>>>(ce, u, v, edof, ke, ne);
+  lp_launch(k_energy_edof, lp_blocks(ne, 128), 128, 0, LP_ST, ce, u, v, edof, ke, ne);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -482,7 +497,7 @@ int lpb_element_energy_f64(double* ce, const double* u, const double* v, const d
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !ce || !u || !ke) return LP_ERR_ARG;
   long long total = g.cells_padded();
-  k_element_energy<double><<<(int)std::min<long long>(lp_blocks(total, 128), LP_ENERGY_BLOCKS), 128, 0, LP_ST>>>(
+  lp_launch(k_element_energy<double>, (int)std::min<long long>(lp_blocks(total, 128), LP_ENERGY_BLOCKS), 128, 0, LP_ST, 
       ce, u, v, ke, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
@@ -492,7 +507,7 @@ int lpb_element_energy_f32(double* ce, const float* u, const float* v, const dou
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !ce || !u || !ke) return LP_ERR_ARG;
   long long total = g.cells_padded();
-  k_element_energy<float><<<(int)std::min<long long>(lp_blocks(total, 128), LP_ENERGY_BLOCKS), 128, 0, LP_ST>>>(
+  lp_launch(k_element_energy<float>, (int)std::min<long long>(lp_blocks(total, 128), LP_ENERGY_BLOCKS), 128, 0, LP_ST, 
       ce, u, v, ke, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
@@ -503,8 +518,8 @@ int lpb_sensitivity(double* dc, const double* xphys, const double* ce, const dou
                     double scale, int accumulate, double* part, double* comp, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !dc || !xphys || !ce || !part) return LP_ERR_ARG;
-  k_sensitivity<<<LP_SIMP_BLOCKS, 256, 0, LP_ST>>>(dc, xphys, ce, e, penal, emin, scale, accumulate, g, part);
-  if (comp) k_sum_final_s<<<1, 1024, 0, LP_ST>>>(part, LP_SIMP_BLOCKS, comp);
+  lp_launch(k_sensitivity, LP_SIMP_BLOCKS, 256, 0, LP_ST, dc, xphys, ce, e, penal, emin, scale, accumulate, g, part);
+  if (comp) lp_launch(k_sum_final_s, 1, 1024, 0, LP_ST, part, LP_SIMP_BLOCKS, comp);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -513,8 +528,8 @@ int lpb_sensitivity(double* dc, const double* xphys, const double* ce, const dou
 // cands) and one step after a volumes pass; handle: the conditional of a graph WHILE node or 0
 int lpb_oc_walk_init(double* state, double* cands, double l2, double target, double tol, void* stream) {
   if (!state || !cands || !(l2 > 0.0)) return LP_ERR_ARG;
-  k_oc_walk_init<<<1, 1, 0, LP_ST>>>(state, l2);
-  k_oc_walk<<<1, 1, 0, LP_ST>>>(cudaGraphConditionalHandle{}, 0, state, nullptr, cands, target, tol, 0);
+  lp_launch(k_oc_walk_init, 1, 1, 0, LP_ST, state, l2);
+  lp_launch(k_oc_walk, 1, 1, 0, LP_ST, cudaGraphConditionalHandle{}, 0, state, nullptr, cands, target, tol, 0);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -522,7 +537,7 @@ int lpb_oc_walk_init(double* state, double* cands, double l2, double target, dou
 int lpb_oc_walk(long long handle, double* state, const double* vols, double* cands, double target, double tol,
                 void* stream) {
   if (!state || !vols || !cands) return LP_ERR_ARG;
-  k_oc_walk<<<1, 1, 0, LP_ST>>>((cudaGraphConditionalHandle)handle, handle != 0, state, vols, cands, target, tol, 1);
+  lp_launch(k_oc_walk, 1, 1, 0, LP_ST, (cudaGraphConditionalHandle)handle, handle != 0, state, vols, cands, target, tol, 1);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -534,8 +549,8 @@ int lpb_oc_volumes(double* volumes, const double* x, const double* dc, const dou
   if (!lp_grid_ok(g) || nl < 1 || nl > LP_MAX_LAMBDA || !volumes || !x || !dc || !dv || !gv || !lam || !part)
     return LP_ERR_ARG;
   if (nl != 31) return LP_ERR_ARG;
-  k_oc_volumes<31><<<LP_SIMP_BLOCKS, 256, 0, LP_ST>>>(x, dc, dv, gv, lam, move, g, part);
-  k_oc_final<<<1, 1024, 0, LP_ST>>>(part, LP_SIMP_BLOCKS, nl, volumes);
+  lp_launch(k_oc_volumes<31>, LP_SIMP_BLOCKS, 256, 0, LP_ST, x, dc, dv, gv, lam, move, g, part);
+  lp_launch(k_oc_final, 1, 1024, 0, LP_ST, part, LP_SIMP_BLOCKS, nl, volumes);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -544,8 +559,8 @@ int lpb_oc_apply(double* xnew, const double* x, const double* dc, const double* 
                  double* part, double* change, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !xnew || !x || !dc || !dv || !part || !change) return LP_ERR_ARG;
-  k_oc_apply<<<LP_SIMP_BLOCKS, 256, 0, LP_ST>>>(xnew, x, dc, dv, lam, nullptr, move, g, part);
-  k_max_final2<<<1, 1024, 0, LP_ST>>>(part, LP_SIMP_BLOCKS, change);
+  lp_launch(k_oc_apply, LP_SIMP_BLOCKS, 256, 0, LP_ST, xnew, x, dc, dv, lam, nullptr, move, g, part);
+  lp_launch(k_max_final2, 1, 1024, 0, LP_ST, part, LP_SIMP_BLOCKS, change);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -555,8 +570,8 @@ int lpb_oc_apply_at(double* xnew, const double* x, const double* dc, const doubl
                     double move, double* part, double* change, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !xnew || !x || !dc || !dv || !lam || !part || !change) return LP_ERR_ARG;
-  k_oc_apply<<<LP_SIMP_BLOCKS, 256, 0, LP_ST>>>(xnew, x, dc, dv, 0.0, lam, move, g, part);
-  k_max_final2<<<1, 1024, 0, LP_ST>>>(part, LP_SIMP_BLOCKS, change);
+  lp_launch(k_oc_apply, LP_SIMP_BLOCKS, 256, 0, LP_ST, xnew, x, dc, dv, 0.0, lam, move, g, part);
+  lp_launch(k_max_final2, 1, 1024, 0, LP_ST, part, LP_SIMP_BLOCKS, change);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -568,8 +583,8 @@ int lpb_project(double* xp, double* dxp, const double* xt, double beta, double e
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !xt || (w && (!part || !vol))) return LP_ERR_ARG;
   const double tbe = tanh(beta * eta), den = tbe + tanh(beta * (1.0 - eta));
-  k_project<<<LP_SIMP_BLOCKS, 256, 0, LP_ST>>>(xp, dxp, xt, beta, eta, tbe, den, flags, w, g, w ? part : nullptr);
-  if (w) k_sum_final_s<<<1, 1024, 0, LP_ST>>>(part, LP_SIMP_BLOCKS, vol);
+  lp_launch(k_project, LP_SIMP_BLOCKS, 256, 0, LP_ST, xp, dxp, xt, beta, eta, tbe, den, flags, w, g, w ? part : nullptr);
+  if (w) lp_launch(k_sum_final_s, 1, 1024, 0, LP_ST, part, LP_SIMP_BLOCKS, vol);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -578,7 +593,7 @@ int lpb_oc_stepped(double* xn, const double* x, const double* dc, const double* 
                    const uint8_t* flags, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !xn || !x || !dc || !dv || !(lm > 0.0)) return LP_ERR_ARG;
-  k_oc_stepped<<<lp_blocks(g.cells_padded(), 256), 256, 0, LP_ST>>>(xn, x, dc, dv, lm, move, flags, g);
+  lp_launch(k_oc_stepped, lp_blocks(g.cells_padded(), 256), 256, 0, LP_ST, xn, x, dc, dv, lm, move, flags, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -587,7 +602,7 @@ int lpb_oc_stepped(double* xn, const double* x, const double* dc, const double* 
 int lpb_mirror_average(double* v, int axis, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !v || axis < 0 || axis > 2) return LP_ERR_ARG;
-  k_mirror_average<<<lp_blocks(g.cells_padded(), 256), 256, 0, LP_ST>>>(v, axis, g);
+  lp_launch(k_mirror_average, lp_blocks(g.cells_padded(), 256), 256, 0, LP_ST, v, axis, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -597,7 +612,7 @@ int lpb_cell_product(double* out, const double* a, const double* b, const uint8_
                      void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !out || !a || clip0 < 0 || clip0 > 2) return LP_ERR_ARG;
-  k_cell_product<<<lp_blocks(g.cells_padded(), 256), 256, 0, LP_ST>>>(out, a, b, flags, clip0, g);
+  lp_launch(k_cell_product, lp_blocks(g.cells_padded(), 256), 256, 0, LP_ST, out, a, b, flags, clip0, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }

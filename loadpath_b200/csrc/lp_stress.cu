@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(ST_THREADS) k_stress_pass(const double* __rest
                                                             double pm, double kappa, double nc, LpGrid g,
                                                             double* __restrict__ part, double* __restrict__ gxe,
                                                             double* __restrict__ fe) {
+  lp_after_launch();
   __shared__ double cb[8 * 6 * 24];
   __shared__ double sh[32];
   __shared__ double sfv[MODE == 2 ? ST_THREADS * 25 : 1];
@@ -135,6 +136,7 @@ __global__ void __launch_bounds__(ST_THREADS) k_stress_pass(const double* __rest
 
 // the max (mode 0) or the sum (mode 1) of the block partials
 __global__ void k_stress_final(int mode, const double* __restrict__ part, int n, double* __restrict__ out) {
+  lp_after_launch();
   __shared__ double sh[32];
   double a = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) a = mode == 0 ? fmax(a, part[i]) : a + part[i];
@@ -156,6 +158,7 @@ __global__ void k_stress_final(int mode, const double* __restrict__ part, int n,
 // out (node field, all three components) = each node's share of its cells' 24-vectors fe
 // (cells_padded x 24, dof 3 q + component at corner q = (q & 1, q >> 1 & 1, q >> 2 & 1))
 __global__ void k_cell_vectors_to_nodes(double* __restrict__ out, const double* __restrict__ fe, LpGrid g) {
+  lp_after_launch();
   const long long total = g.nodes_padded();
   const long long cs = g.comp_stride();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -198,12 +201,12 @@ int lpb_stress_pass(int mode, const double* u, const double* xe, const uint8_t* 
   if (mode == 1 && !(sc > 0.0)) return LP_ERR_ARG;
   if (mode == 2 && (!gxe || !fe || !(nc > 0.0))) return LP_ERR_ARG;
   if (mode == 0)
-    k_stress_pass<0><<<ST_BLOCKS, ST_THREADS, 0, LP_ST>>>(u, xe, counted, cb, lim, sc, pm, kappa, nc, g, part, gxe, fe);
+    lp_launch(k_stress_pass<0>, ST_BLOCKS, ST_THREADS, 0, LP_ST, u, xe, counted, cb, lim, sc, pm, kappa, nc, g, part, gxe, fe);
   else if (mode == 1)
-    k_stress_pass<1><<<ST_BLOCKS, ST_THREADS, 0, LP_ST>>>(u, xe, counted, cb, lim, sc, pm, kappa, nc, g, part, gxe, fe);
+    lp_launch(k_stress_pass<1>, ST_BLOCKS, ST_THREADS, 0, LP_ST, u, xe, counted, cb, lim, sc, pm, kappa, nc, g, part, gxe, fe);
   else
-    k_stress_pass<2><<<ST_BLOCKS, ST_THREADS, 0, LP_ST>>>(u, xe, counted, cb, lim, sc, pm, kappa, nc, g, part, gxe, fe);
-  if (mode < 2) k_stress_final<<<1, 1024, 0, LP_ST>>>(mode, part, ST_BLOCKS, out);
+    lp_launch(k_stress_pass<2>, ST_BLOCKS, ST_THREADS, 0, LP_ST, u, xe, counted, cb, lim, sc, pm, kappa, nc, g, part, gxe, fe);
+  if (mode < 2) lp_launch(k_stress_final, 1, 1024, 0, LP_ST, mode, part, ST_BLOCKS, out);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -212,7 +215,7 @@ int lpb_stress_pass(int mode, const double* u, const double* xe, const uint8_t* 
 int lpb_cell_vectors_to_nodes(double* out, const double* fe, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !out || !fe) return LP_ERR_ARG;
-  k_cell_vectors_to_nodes<<<lp_blocks(g.nodes_padded(), 256), 256, 0, LP_ST>>>(out, fe, g);
+  lp_launch(k_cell_vectors_to_nodes, lp_blocks(g.nodes_padded(), 256), 256, 0, LP_ST, out, fe, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }

@@ -43,6 +43,7 @@ struct V4ld<double> {
 template <typename Ta, typename Tb>
 __global__ void k_dot_partial(const Ta* __restrict__ a, const Tb* __restrict__ b, long long n,
                               double* __restrict__ part) {
+  lp_after_launch();
   __shared__ double sh[32];
   double s = 0.0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -53,6 +54,7 @@ __global__ void k_dot_partial(const Ta* __restrict__ a, const Tb* __restrict__ b
 
 // out[0] = sum(part); optional: out_sqrt = sqrt(sum)
 __global__ void k_sum_final(const double* __restrict__ part, int n, double* __restrict__ out) {
+  lp_after_launch();
   __shared__ double sh[32];
   double s = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += part[i];
@@ -64,6 +66,7 @@ __global__ void k_sum_final(const double* __restrict__ part, int n, double* __re
 __global__ void k_cg_step(double* __restrict__ x, double* __restrict__ r, const double* __restrict__ p,
                           const double* __restrict__ ap, float* __restrict__ r32, long long n,
                           const double* __restrict__ num, const double* __restrict__ den, double* __restrict__ part) {
+  lp_after_launch();
   __shared__ double sh[32];
   const double alpha = (*num) / (*den);
   double s = 0.0;
@@ -82,6 +85,7 @@ __global__ void k_cg_step(double* __restrict__ x, double* __restrict__ r, const 
 template <typename Tz>
 __global__ void k_xpby(double* __restrict__ p, const Tz* __restrict__ z, long long n, const double* __restrict__ num,
                        const double* __restrict__ den) {
+  lp_after_launch();
   const double beta = (*num) / (*den);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     p[i] = (double)z[i] + beta * p[i];
@@ -89,6 +93,7 @@ __global__ void k_xpby(double* __restrict__ p, const Tz* __restrict__ z, long lo
 
 template <typename Ta, typename Tb>
 __global__ void k_cast(Tb* __restrict__ out, const Ta* __restrict__ a, long long n) {
+  lp_after_launch();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     out[i] = (Tb)a[i];
 }
@@ -96,6 +101,7 @@ __global__ void k_cast(Tb* __restrict__ out, const Ta* __restrict__ a, long long
 // out = a x + b y
 template <typename T>
 __global__ void k_axpby(T* __restrict__ out, T a, const T* __restrict__ x, T b, const T* __restrict__ y, long long n) {
+  lp_after_launch();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     out[i] = a * x[i] + (y ? b * y[i] : T(0));
 }
@@ -108,6 +114,7 @@ __global__ void k_axpby(T* __restrict__ out, T a, const T* __restrict__ x, T b, 
 template <typename T>
 __global__ void k_cheb_start(const T* __restrict__ b, const T* __restrict__ dinv, const double* __restrict__ coef,
                              T* __restrict__ x, T* __restrict__ r, T* __restrict__ d, long long n) {
+  lp_after_launch();
   const T s = (T)coef[1];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     T bi = b[i];
@@ -121,6 +128,7 @@ __global__ void k_cheb_start(const T* __restrict__ b, const T* __restrict__ dinv
 template <typename T>
 __global__ void k_residual_scaled(const T* __restrict__ b, const T* __restrict__ ax, const T* __restrict__ dinv,
                                   const double* __restrict__ coef, T* __restrict__ r, T* __restrict__ d, long long n) {
+  lp_after_launch();
   const T s = (T)coef[1];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     T ri, di;
@@ -134,6 +142,7 @@ __global__ void k_residual_scaled(const T* __restrict__ b, const T* __restrict__
 template <typename T>
 __global__ void k_cheb(T* __restrict__ x, T* __restrict__ d, T* __restrict__ r, const T* __restrict__ ad,
                        const T* __restrict__ dinv, const double* __restrict__ coef, int step, int last, long long n) {
+  lp_after_launch();
   const T c1 = (T)coef[2 + 2 * step], c2 = (T)coef[3 + 2 * step];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     T di = d[i];
@@ -151,6 +160,7 @@ __global__ void k_cheb(T* __restrict__ x, T* __restrict__ d, T* __restrict__ r, 
 // the interval is [lmax / 30, lmax]. One thread, float64 throughout.
 __global__ void k_cheb_coef(double* __restrict__ coef, const double* __restrict__ vv, const double* __restrict__ vav,
                             int its, int degree, double safety) {
+  lp_after_launch();
   bool zero = false;
   for (int k = 0; k < its; ++k) zero = zero || vv[k] == 0.0;
   const double lam = vav[its - 1];
@@ -177,6 +187,7 @@ __global__ void k_cheb_coef(double* __restrict__ coef, const double* __restrict_
 template <typename T>
 __global__ void k_cheb_d_start(const T* __restrict__ b, const T* __restrict__ dinv, const double* __restrict__ coef,
                                T* __restrict__ d, long long n) {
+  lp_after_launch();
   const T s = (T)coef[1];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     d[i] = (dinv[i] * b[i]) * s;
@@ -187,6 +198,7 @@ template <typename T>
 __global__ void k_cheb2_zero(T* __restrict__ x, const T* __restrict__ b, const T* __restrict__ ad,
                              const T* __restrict__ d, const T* __restrict__ dinv, const double* __restrict__ coef,
                              long long n) {
+  lp_after_launch();
   const T c1 = (T)coef[2], c2 = (T)coef[3];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     x[i] = lp_cheb2_zero_v(d[i], b[i], ad[i], dinv[i], c1, c2);
@@ -197,6 +209,7 @@ __global__ void k_cheb2_zero(T* __restrict__ x, const T* __restrict__ b, const T
 template <typename T>
 __global__ void k_cheb2(T* __restrict__ x, const T* __restrict__ d, const T* __restrict__ r, const T* __restrict__ ad,
                         const T* __restrict__ dinv, const double* __restrict__ coef, long long n) {
+  lp_after_launch();
   const T c1 = (T)coef[2], c2 = (T)coef[3];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     x[i] = lp_cheb2_v(x[i], d[i], r[i], ad[i], dinv[i], c1, c2);
@@ -206,6 +219,7 @@ __global__ void k_cheb2(T* __restrict__ x, const T* __restrict__ d, const T* __r
 template <typename T>
 __global__ void k_jacobi(T* __restrict__ x, const T* __restrict__ b, const T* __restrict__ ax,
                          const T* __restrict__ dinv, T omega, int from_zero, long long n) {
+  lp_after_launch();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     if (from_zero)
       x[i] = omega * dinv[i] * b[i];
@@ -229,6 +243,7 @@ constexpr int R4_COLS = 15;   // coarse columns per warp
 template <typename T>
 __global__ void k_restrict4(T* __restrict__ rc, const T* __restrict__ b, const T* __restrict__ ax,
                             const uint8_t* __restrict__ m, const uint8_t* __restrict__ cm, LpGrid gf, LpGrid gc) {
+  lp_after_launch();
   const int CX = gc.NX(), CY = gc.NY(), CZ4 = gc.pz / 4;
   const int FX = gf.NX(), FY = gf.NY();
   const int ngx = (CX + R4_COLS - 1) / R4_COLS;
@@ -326,6 +341,7 @@ __global__ void k_restrict4(T* __restrict__ rc, const T* __restrict__ b, const T
 template <typename T>
 __global__ void k_prolong4(T* __restrict__ xf, const T* __restrict__ xc, const uint8_t* __restrict__ cm,
                            const uint8_t* __restrict__ m, LpGrid gf, LpGrid gc) {
+  lp_after_launch();
   const long long total = gf.nodes_padded() / 4;
   const long long fcs = gf.comp_stride(), ccs = gc.comp_stride();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -388,6 +404,7 @@ __global__ void k_prolong4(T* __restrict__ xf, const T* __restrict__ xc, const u
 template <typename T>
 __global__ void k_mask_field(T* __restrict__ out, const T* __restrict__ u, const uint8_t* __restrict__ m, LpGrid g,
                              int bitshift) {
+  lp_after_launch();
   const long long nq = g.nodes_padded() >> 2;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < 3 * nq; i += (long long)gridDim.x * blockDim.x) {
     const int c = i >= nq ? (i >= 2 * nq ? 2 : 1) : 0;
@@ -406,6 +423,7 @@ __global__ void k_mask_field(T* __restrict__ out, const T* __restrict__ u, const
 // v *= 1 / sqrt(*nrm2) (power iteration normalisation); leaves v alone when the norm is 0
 template <typename T>
 __global__ void k_scale_rsqrt(T* __restrict__ v, long long n, const double* __restrict__ nrm2) {
+  lp_after_launch();
   double s = *nrm2;
   if (s <= 0.0) return;
   T f = (T)(1.0 / sqrt(s));
@@ -417,6 +435,7 @@ __global__ void k_scale_rsqrt(T* __restrict__ v, long long n, const double* __re
 // av = dinv * av * mask, four nodes per step as k_mask_field
 template <typename T>
 __global__ void k_dinv_mask(T* __restrict__ av, const T* __restrict__ dinv, const uint8_t* __restrict__ m, LpGrid g) {
+  lp_after_launch();
   const long long nq = g.nodes_padded() >> 2;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < 3 * nq; i += (long long)gridDim.x * blockDim.x) {
     const int c = i >= nq ? (i >= 2 * nq ? 2 : 1) : 0;
@@ -440,6 +459,7 @@ __device__ __forceinline__ double lp_warm_scale(const double* sc) { return sc[5]
 
 __global__ void k_warm_residual(double* __restrict__ rs, const double* __restrict__ b, const double* __restrict__ ax,
                                 const double* __restrict__ sc, long long n) {
+  lp_after_launch();
   const double s = lp_warm_scale(sc);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     rs[i] = b[i] - s * ax[i];
@@ -448,6 +468,7 @@ __global__ void k_warm_residual(double* __restrict__ rs, const double* __restric
 // keep the scaled warm start when s > 0 and |rs| < |b| (x = s x, r = rs), else x = 0, r = b
 __global__ void k_warm_select(double* __restrict__ x, double* __restrict__ r, const double* __restrict__ b,
                               const double* __restrict__ rs, const double* __restrict__ sc, long long n) {
+  lp_after_launch();
   const double s = lp_warm_scale(sc);
   const bool keep = s > 0.0 && sqrt(sc[7]) < sqrt(sc[0]);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -462,6 +483,7 @@ __global__ void k_warm_select(double* __restrict__ x, double* __restrict__ r, co
 __global__ void k_cg_step_r(double* __restrict__ r, const double* __restrict__ ap, float* __restrict__ r32,
                             long long n, const double* __restrict__ num, const double* __restrict__ den,
                             double* __restrict__ part) {
+  lp_after_launch();
   __shared__ double sh[32];
   const double alpha = (*num) / (*den);
   double s = 0.0;
@@ -480,6 +502,7 @@ template <typename Tz>
 __global__ void k_xpby_x(double* __restrict__ p, double* __restrict__ x, const Tz* __restrict__ z, long long n,
                          const double* __restrict__ rz, const double* __restrict__ pap,
                          const double* __restrict__ rz_new) {
+  lp_after_launch();
   const double alpha = (*rz) / (*pap), beta = (*rz_new) / (*rz);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const double pi = p[i];
@@ -513,24 +536,24 @@ int lpb_event_record(void* event, void* stream) {
 
 int lpb_dot_f64(const double* a, const double* b, long long n, double* part, double* out, void* stream) {
   if (!a || !b || !part || !out || n < 0) return LP_ERR_ARG;
-  k_dot_partial<double, double><<<LP_RED_BLOCKS, LP_RED_THREADS, 0, LP_ST>>>(a, b, n, part);
-  k_sum_final<<<1, 1024, 0, LP_ST>>>(part, LP_RED_BLOCKS, out);
+  lp_launch(k_dot_partial<double, double>, LP_RED_BLOCKS, LP_RED_THREADS, 0, LP_ST, a, b, n, part);
+  lp_launch(k_sum_final, 1, 1024, 0, LP_ST, part, LP_RED_BLOCKS, out);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_dot_f32(const float* a, const float* b, long long n, double* part, double* out, void* stream) {
   if (!a || !b || !part || !out || n < 0) return LP_ERR_ARG;
-  k_dot_partial<float, float><<<LP_RED_BLOCKS, LP_RED_THREADS, 0, LP_ST>>>(a, b, n, part);
-  k_sum_final<<<1, 1024, 0, LP_ST>>>(part, LP_RED_BLOCKS, out);
+  lp_launch(k_dot_partial<float, float>, LP_RED_BLOCKS, LP_RED_THREADS, 0, LP_ST, a, b, n, part);
+  lp_launch(k_sum_final, 1, 1024, 0, LP_ST, part, LP_RED_BLOCKS, out);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_dot_f64_f32(const double* a, const float* b, long long n, double* part, double* out, void* stream) {
   if (!a || !b || !part || !out || n < 0) return LP_ERR_ARG;
-  k_dot_partial<double, float><<<LP_RED_BLOCKS, LP_RED_THREADS, 0, LP_ST>>>(a, b, n, part);
-  k_sum_final<<<1, 1024, 0, LP_ST>>>(part, LP_RED_BLOCKS, out);
+  lp_launch(k_dot_partial<double, float>, LP_RED_BLOCKS, LP_RED_THREADS, 0, LP_ST, a, b, n, part);
+  lp_launch(k_sum_final, 1, 1024, 0, LP_ST, part, LP_RED_BLOCKS, out);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -538,50 +561,50 @@ int lpb_dot_f64_f32(const double* a, const float* b, long long n, double* part, 
 int lpb_cg_step(double* x, double* r, const double* p, const double* ap, float* r32, long long n, const double* num,
                 const double* den, double* part, double* rr, void* stream) {
   if (!x || !r || !p || !ap || !num || !den || !part || !rr) return LP_ERR_ARG;
-  k_cg_step<<<LP_RED_BLOCKS, LP_RED_THREADS, 0, LP_ST>>>(x, r, p, ap, r32, n, num, den, part);
-  k_sum_final<<<1, 1024, 0, LP_ST>>>(part, LP_RED_BLOCKS, rr);
+  lp_launch(k_cg_step, LP_RED_BLOCKS, LP_RED_THREADS, 0, LP_ST, x, r, p, ap, r32, n, num, den, part);
+  lp_launch(k_sum_final, 1, 1024, 0, LP_ST, part, LP_RED_BLOCKS, rr);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_xpby_f32(double* p, const float* z, long long n, const double* num, const double* den, void* stream) {
   if (!p || !z || !num || !den) return LP_ERR_ARG;
-  k_xpby<float><<<LP_VEC_GRID(n)>>>(p, z, n, num, den);
+  lp_launch(k_xpby<float>, LP_VEC_GRID(n), p, z, n, num, den);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_xpby_f64(double* p, const double* z, long long n, const double* num, const double* den, void* stream) {
   if (!p || !z || !num || !den) return LP_ERR_ARG;
-  k_xpby<double><<<LP_VEC_GRID(n)>>>(p, z, n, num, den);
+  lp_launch(k_xpby<double>, LP_VEC_GRID(n), p, z, n, num, den);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_axpby_f64(double* out, double a, const double* x, double b, const double* y, long long n, void* stream) {
   if (!out || !x) return LP_ERR_ARG;
-  k_axpby<double><<<LP_VEC_GRID(n)>>>(out, a, x, b, y, n);
+  lp_launch(k_axpby<double>, LP_VEC_GRID(n), out, a, x, b, y, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_axpby_f32(float* out, float a, const float* x, float b, const float* y, long long n, void* stream) {
   if (!out || !x) return LP_ERR_ARG;
-  k_axpby<float><<<LP_VEC_GRID(n)>>>(out, a, x, b, y, n);
+  lp_launch(k_axpby<float>, LP_VEC_GRID(n), out, a, x, b, y, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_cast_f64_f32(float* out, const double* a, long long n, void* stream) {
   if (!out || !a) return LP_ERR_ARG;
-  k_cast<double, float><<<LP_VEC_GRID(n)>>>(out, a, n);
+  lp_launch(k_cast<double, float>, LP_VEC_GRID(n), out, a, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_cast_f32_f64(double* out, const float* a, long long n, void* stream) {
   if (!out || !a) return LP_ERR_ARG;
-  k_cast<float, double><<<LP_VEC_GRID(n)>>>(out, a, n);
+  lp_launch(k_cast<float, double>, LP_VEC_GRID(n), out, a, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -589,7 +612,7 @@ int lpb_cast_f32_f64(double* out, const float* a, long long n, void* stream) {
 int lpb_cheb_coef(double* coef, const double* vv, const double* vav, int its, int degree, double safety,
                   void* stream) {
   if (!coef || !vv || !vav || its < 1 || degree < 1 || degree > LP_CHEB_MAX_DEGREE) return LP_ERR_ARG;
-  k_cheb_coef<<<1, 1, 0, LP_ST>>>(coef, vv, vav, its, degree, safety);
+  lp_launch(k_cheb_coef, 1, 1, 0, LP_ST, coef, vv, vav, its, degree, safety);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -597,7 +620,7 @@ int lpb_cheb_coef(double* coef, const double* vv, const double* vav, int its, in
 int lpb_cheb_start_f32(const float* b, const float* dinv, const double* coef, float* x, float* r, float* d,
                        long long n, void* stream) {
   if (!b || !dinv || !coef || !x || !r || !d) return LP_ERR_ARG;
-  k_cheb_start<float><<<LP_VEC_GRID(n)>>>(b, dinv, coef, x, r, d, n);
+  lp_launch(k_cheb_start<float>, LP_VEC_GRID(n), b, dinv, coef, x, r, d, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -605,7 +628,7 @@ int lpb_cheb_start_f32(const float* b, const float* dinv, const double* coef, fl
 int lpb_cheb_start_f64(const double* b, const double* dinv, const double* coef, double* x, double* r, double* d,
                        long long n, void* stream) {
   if (!b || !dinv || !coef || !x || !r || !d) return LP_ERR_ARG;
-  k_cheb_start<double><<<LP_VEC_GRID(n)>>>(b, dinv, coef, x, r, d, n);
+  lp_launch(k_cheb_start<double>, LP_VEC_GRID(n), b, dinv, coef, x, r, d, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -613,7 +636,7 @@ int lpb_cheb_start_f64(const double* b, const double* dinv, const double* coef, 
 int lpb_residual_scaled_f32(const float* b, const float* ax, const float* dinv, const double* coef, float* r,
                             float* d, long long n, void* stream) {
   if (!b || !ax || !dinv || !coef || !r || !d) return LP_ERR_ARG;
-  k_residual_scaled<float><<<LP_VEC_GRID(n)>>>(b, ax, dinv, coef, r, d, n);
+  lp_launch(k_residual_scaled<float>, LP_VEC_GRID(n), b, ax, dinv, coef, r, d, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -621,7 +644,7 @@ int lpb_residual_scaled_f32(const float* b, const float* ax, const float* dinv, 
 int lpb_residual_scaled_f64(const double* b, const double* ax, const double* dinv, const double* coef, double* r,
                             double* d, long long n, void* stream) {
   if (!b || !ax || !dinv || !coef || !r || !d) return LP_ERR_ARG;
-  k_residual_scaled<double><<<LP_VEC_GRID(n)>>>(b, ax, dinv, coef, r, d, n);
+  lp_launch(k_residual_scaled<double>, LP_VEC_GRID(n), b, ax, dinv, coef, r, d, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -629,7 +652,7 @@ int lpb_residual_scaled_f64(const double* b, const double* ax, const double* din
 int lpb_cheb_f32(float* x, float* d, float* r, const float* ad, const float* dinv, const double* coef, int step,
                  int last, long long n, void* stream) {
   if (!x || !d || !r || !ad || !dinv || !coef || step < 0 || step >= LP_CHEB_MAX_DEGREE) return LP_ERR_ARG;
-  k_cheb<float><<<LP_VEC_GRID(n)>>>(x, d, r, ad, dinv, coef, step, last, n);
+  lp_launch(k_cheb<float>, LP_VEC_GRID(n), x, d, r, ad, dinv, coef, step, last, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -637,7 +660,7 @@ int lpb_cheb_f32(float* x, float* d, float* r, const float* ad, const float* din
 int lpb_cheb_f64(double* x, double* d, double* r, const double* ad, const double* dinv, const double* coef, int step,
                  int last, long long n, void* stream) {
   if (!x || !d || !r || !ad || !dinv || !coef || step < 0 || step >= LP_CHEB_MAX_DEGREE) return LP_ERR_ARG;
-  k_cheb<double><<<LP_VEC_GRID(n)>>>(x, d, r, ad, dinv, coef, step, last, n);
+  lp_launch(k_cheb<double>, LP_VEC_GRID(n), x, d, r, ad, dinv, coef, step, last, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -645,21 +668,21 @@ int lpb_cheb_f64(double* x, double* d, double* r, const double* ad, const double
 #define LP_CHEB2_ENTRIES(T, SFX)                                                                            \
   int lpb_cheb_d_start_##SFX(const T* b, const T* dinv, const double* coef, T* d, long long n, void* stream) { \
     if (!b || !dinv || !coef || !d) return LP_ERR_ARG;                                                   \
-    k_cheb_d_start<T><<<LP_VEC_GRID(n)>>>(b, dinv, coef, d, n);                                          \
+    lp_launch(k_cheb_d_start<T>, LP_VEC_GRID(n), b, dinv, coef, d, n);                                          \
     LP_LAUNCH_CHECK();                                                                                    \
     return LP_OK;                                                                                         \
   }                                                                                                       \
   int lpb_cheb2_zero_##SFX(T* x, const T* b, const T* ad, const T* d, const T* dinv, const double* coef,  \
                            long long n, void* stream) {                                                  \
     if (!x || !b || !ad || !d || !dinv || !coef) return LP_ERR_ARG;                                     \
-    k_cheb2_zero<T><<<LP_VEC_GRID(n)>>>(x, b, ad, d, dinv, coef, n);                                     \
+    lp_launch(k_cheb2_zero<T>, LP_VEC_GRID(n), x, b, ad, d, dinv, coef, n);                                     \
     LP_LAUNCH_CHECK();                                                                                    \
     return LP_OK;                                                                                         \
   }                                                                                                       \
   int lpb_cheb2_##SFX(T* x, const T* d, const T* r, const T* ad, const T* dinv, const double* coef,       \
                       long long n, void* stream) {                                                       \
     if (!x || !d || !r || !ad || !dinv || !coef) return LP_ERR_ARG;                                     \
-    k_cheb2<T><<<LP_VEC_GRID(n)>>>(x, d, r, ad, dinv, coef, n);                                          \
+    lp_launch(k_cheb2<T>, LP_VEC_GRID(n), x, d, r, ad, dinv, coef, n);                                          \
     LP_LAUNCH_CHECK();                                                                                    \
     return LP_OK;                                                                                         \
   }
@@ -669,8 +692,8 @@ LP_CHEB2_ENTRIES(double, f64)
 int lpb_cg_step_r(double* r, const double* ap, float* r32, long long n, const double* num, const double* den,
                   double* part, double* rr, void* stream) {
   if (!r || !ap || !num || !den || !part || !rr) return LP_ERR_ARG;
-  k_cg_step_r<<<LP_RED_BLOCKS, LP_RED_THREADS, 0, LP_ST>>>(r, ap, r32, n, num, den, part);
-  k_sum_final<<<1, 1024, 0, LP_ST>>>(part, LP_RED_BLOCKS, rr);
+  lp_launch(k_cg_step_r, LP_RED_BLOCKS, LP_RED_THREADS, 0, LP_ST, r, ap, r32, n, num, den, part);
+  lp_launch(k_sum_final, 1, 1024, 0, LP_ST, part, LP_RED_BLOCKS, rr);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -678,7 +701,7 @@ int lpb_cg_step_r(double* r, const double* ap, float* r32, long long n, const do
 int lpb_xpby_x_f32(double* p, double* x, const float* z, long long n, const double* rz, const double* pap,
                    const double* rz_new, void* stream) {
   if (!p || !x || !z || !rz || !pap || !rz_new) return LP_ERR_ARG;
-  k_xpby_x<float><<<LP_VEC_GRID(n)>>>(p, x, z, n, rz, pap, rz_new);
+  lp_launch(k_xpby_x<float>, LP_VEC_GRID(n), p, x, z, n, rz, pap, rz_new);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -686,21 +709,21 @@ int lpb_xpby_x_f32(double* p, double* x, const float* z, long long n, const doub
 int lpb_xpby_x_f64(double* p, double* x, const double* z, long long n, const double* rz, const double* pap,
                    const double* rz_new, void* stream) {
   if (!p || !x || !z || !rz || !pap || !rz_new) return LP_ERR_ARG;
-  k_xpby_x<double><<<LP_VEC_GRID(n)>>>(p, x, z, n, rz, pap, rz_new);
+  lp_launch(k_xpby_x<double>, LP_VEC_GRID(n), p, x, z, n, rz, pap, rz_new);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_jacobi_f32(float* x, const float* b, const float* ax, const float* dinv, float omega, int from_zero,
                    long long n, void* stream) {
-  k_jacobi<float><<<LP_VEC_GRID(n)>>>(x, b, ax, dinv, omega, from_zero, n);
+  lp_launch(k_jacobi<float>, LP_VEC_GRID(n), x, b, ax, dinv, omega, from_zero, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_jacobi_f64(double* x, const double* b, const double* ax, const double* dinv, double omega, int from_zero,
                    long long n, void* stream) {
-  k_jacobi<double><<<LP_VEC_GRID(n)>>>(x, b, ax, dinv, omega, from_zero, n);
+  lp_launch(k_jacobi<double>, LP_VEC_GRID(n), x, b, ax, dinv, omega, from_zero, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -724,7 +747,7 @@ int lpb_restrict_residual_f32(float* rc, const float* b, const float* ax, const 
   if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || !rc || !b || !ax || !m || !cm) return LP_ERR_ARG;
   if (!lp_pair_ok(gf, gc)) return LP_ERR_ARG;
   const long long nw = (long long)((gc.NX() + R4_COLS - 1) / R4_COLS) * gc.NY() * (gc.pz / 4);
-  k_restrict4<float><<<lp_blocks(32 * nw, 128), 128, 0, LP_ST>>>(rc, b, ax, m, cm, gf, gc);
+  lp_launch(k_restrict4<float>, lp_blocks(32 * nw, 128), 128, 0, LP_ST, rc, b, ax, m, cm, gf, gc);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -735,7 +758,7 @@ int lpb_restrict_residual_f64(double* rc, const double* b, const double* ax, con
   if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || !rc || !b || !ax || !m || !cm) return LP_ERR_ARG;
   if (!lp_pair_ok(gf, gc)) return LP_ERR_ARG;
   const long long nw = (long long)((gc.NX() + R4_COLS - 1) / R4_COLS) * gc.NY() * (gc.pz / 4);
-  k_restrict4<double><<<lp_blocks(32 * nw, 128), 128, 0, LP_ST>>>(rc, b, ax, m, cm, gf, gc);
+  lp_launch(k_restrict4<double>, lp_blocks(32 * nw, 128), 128, 0, LP_ST, rc, b, ax, m, cm, gf, gc);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -745,7 +768,7 @@ int lpb_prolong_add_f32(float* x, const float* xc, const uint8_t* cm, const uint
   if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || !x || !xc || !m || !cm) return LP_ERR_ARG;
   if (!lp_pair_ok(gf, gc)) return LP_ERR_ARG;
   const long long t4 = gf.nodes_padded() / 4;
-  k_prolong4<float><<<lp_blocks(t4, 128), 128, 0, LP_ST>>>(x, xc, cm, m, gf, gc);
+  lp_launch(k_prolong4<float>, lp_blocks(t4, 128), 128, 0, LP_ST, x, xc, cm, m, gf, gc);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -755,7 +778,7 @@ int lpb_prolong_add_f64(double* x, const double* xc, const uint8_t* cm, const ui
   if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || !x || !xc || !m || !cm) return LP_ERR_ARG;
   if (!lp_pair_ok(gf, gc)) return LP_ERR_ARG;
   const long long t4 = gf.nodes_padded() / 4;
-  k_prolong4<double><<<lp_blocks(t4, 128), 128, 0, LP_ST>>>(x, xc, cm, m, gf, gc);
+  lp_launch(k_prolong4<double>, lp_blocks(t4, 128), 128, 0, LP_ST, x, xc, cm, m, gf, gc);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -763,7 +786,7 @@ int lpb_prolong_add_f64(double* x, const double* xc, const uint8_t* cm, const ui
 int lpb_mask_field_f32(float* out, const float* u, const uint8_t* m, LP_GRID_ARGS, int bitshift, void* stream) {
   LpGrid g = LP_GRID;
   long long n = 3 * g.nodes_padded();
-  k_mask_field<float><<<LP_VEC_GRID(n / 4)>>>(out, u, m, g, bitshift);
+  lp_launch(k_mask_field<float>, LP_VEC_GRID(n / 4), out, u, m, g, bitshift);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -771,19 +794,19 @@ int lpb_mask_field_f32(float* out, const float* u, const uint8_t* m, LP_GRID_ARG
 int lpb_mask_field_f64(double* out, const double* u, const uint8_t* m, LP_GRID_ARGS, int bitshift, void* stream) {
   LpGrid g = LP_GRID;
   long long n = 3 * g.nodes_padded();
-  k_mask_field<double><<<LP_VEC_GRID(n / 4)>>>(out, u, m, g, bitshift);
+  lp_launch(k_mask_field<double>, LP_VEC_GRID(n / 4), out, u, m, g, bitshift);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_scale_rsqrt_f32(float* v, long long n, const double* nrm2, void* stream) {
-  k_scale_rsqrt<float><<<LP_VEC_GRID(n)>>>(v, n, nrm2);
+  lp_launch(k_scale_rsqrt<float>, LP_VEC_GRID(n), v, n, nrm2);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_scale_rsqrt_f64(double* v, long long n, const double* nrm2, void* stream) {
-  k_scale_rsqrt<double><<<LP_VEC_GRID(n)>>>(v, n, nrm2);
+  lp_launch(k_scale_rsqrt<double>, LP_VEC_GRID(n), v, n, nrm2);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -791,7 +814,7 @@ int lpb_scale_rsqrt_f64(double* v, long long n, const double* nrm2, void* stream
 int lpb_dinv_mask_f32(float* av, const float* dinv, const uint8_t* m, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   long long n = 3 * g.nodes_padded();
-  k_dinv_mask<float><<<LP_VEC_GRID(n / 4)>>>(av, dinv, m, g);
+  lp_launch(k_dinv_mask<float>, LP_VEC_GRID(n / 4), av, dinv, m, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -799,14 +822,14 @@ int lpb_dinv_mask_f32(float* av, const float* dinv, const uint8_t* m, LP_GRID_AR
 int lpb_dinv_mask_f64(double* av, const double* dinv, const uint8_t* m, LP_GRID_ARGS, void* stream) {
   LpGrid g = LP_GRID;
   long long n = 3 * g.nodes_padded();
-  k_dinv_mask<double><<<LP_VEC_GRID(n / 4)>>>(av, dinv, m, g);
+  lp_launch(k_dinv_mask<double>, LP_VEC_GRID(n / 4), av, dinv, m, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
 
 int lpb_warm_residual(double* rs, const double* b, const double* ax, const double* sc, long long n, void* stream) {
   if (!rs || !b || !ax || !sc || n < 0) return LP_ERR_ARG;
-  k_warm_residual<<<LP_VEC_GRID(n)>>>(rs, b, ax, sc, n);
+  lp_launch(k_warm_residual, LP_VEC_GRID(n), rs, b, ax, sc, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -814,7 +837,7 @@ int lpb_warm_residual(double* rs, const double* b, const double* ax, const doubl
 int lpb_warm_select(double* x, double* r, const double* b, const double* rs, const double* sc, long long n,
                     void* stream) {
   if (!x || !r || !b || !rs || !sc || n < 0) return LP_ERR_ARG;
-  k_warm_select<<<LP_VEC_GRID(n)>>>(x, r, b, rs, sc, n);
+  lp_launch(k_warm_select, LP_VEC_GRID(n), x, r, b, rs, sc, n);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
