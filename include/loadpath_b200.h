@@ -50,11 +50,16 @@ int lpb_apply_fine_f32(float* out, const float* u, const float* e, const uint8_t
  * apply it, same bits): mode 1 (u = d) x = d + (c1 d + c2 dinv (b - A d)); mode 2 (u = x)
  * r = b - A x, d = s dinv r; mode 3 (u = d) x = (x + d) + (c1 d + c2 dinv (r - A d)). */
 int lpb_apply_fine_cheb_f32(int mode, float* x, float* r, float* d, const float* u, const float* b, const float* dinv, const double* coef, const float* e, const uint8_t* mask, const double* kmodal, int* err, int nx, int ny, int nz, int pz, int cpz, void* stream);
+/* the same (mode 0: out = m K u) for cols columns, each field's columns one after the other */
+int lpb_apply_fine_cols_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b, const float* dinv, const double* coef, const float* e, const uint8_t* mask, const double* kmodal, int* err, int nx, int ny, int nz, int pz, int cpz, int cols, void* stream);
 int lpb_apply_fine_f64(double* out, const double* u, const double* e, const uint8_t* mask, const double* kmodal, int* err, int nx, int ny, int nz, int pz, int cpz, void* stream);
 /* the float64 fine apply that also forms u . out over the level's nodes into *dot (device),
  * for the PCG's p . A p: per-block partials in part (part_len doubles, -3 when short), summed in
  * a fixed order */
 int lpb_apply_fine_dot_f64(double* out, const double* u, const double* e, const uint8_t* mask, const double* kmodal, int* err, double* part, long long part_len, double* dot, int nx, int ny, int nz, int pz, int cpz, void* stream);
+/* the same for cols columns (each field's columns one after the other) with the block partials left in
+ * part for the next pass, *nparts (host) of them per column */
+int lpb_apply_fine_dot_part_f64(double* out, const double* u, const double* e, const uint8_t* mask, const double* kmodal, int* err, double* part, long long part_len, int* nparts, int nx, int ny, int nz, int pz, int cpz, int cols, void* stream);
 /* the element matrix (24 x 24, float64, host pointer) in the corner-parity basis that
  * lpb_apply_fine_* reads (45 coefficients, host pointer out); returns the count or < 0 */
 int lpb_modal_ke(const double* ke, double* kmodal_out);
@@ -89,6 +94,9 @@ int lpb_patch_modal_f32(float* pm, const float* pk, long long npatch, void* stre
 int lpb_patch_modal_f64(double* pm, const double* pk, long long npatch, void* stream);
 int lpb_apply_level1_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b, const float* dinv, const double* coef, const float* wc, const int* patch_id, const float* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, void* stream);
 int lpb_apply_level1_f64(int mode, double* out, double* x, double* r, double* d, const double* u, const double* b, const double* dinv, const double* coef, const double* wc, const int* patch_id, const double* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, void* stream);
+/* the same for cols columns */
+int lpb_apply_level1_cols_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b, const float* dinv, const double* coef, const float* wc, const int* patch_id, const float* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, int cols, void* stream);
+int lpb_apply_level1_cols_f64(int mode, double* out, double* x, double* r, double* d, const double* u, const double* b, const double* dinv, const double* coef, const double* wc, const int* patch_id, const double* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, int cols, void* stream);
 /* explicit levels in the cell's corner-parity basis: K^ = T K T^T / 64 has the level-1 pattern
  * (150 upper entries) at every level of the plain hierarchy; lpb_pack_modal_f32 stores them
  * (km: (150, cells)) and lists the cells with off-pattern weight (children with masked patch
@@ -103,6 +111,8 @@ int lpb_apply_explicit_modal_f32(float* out, const float* u, const float* km, co
  * mode 1 (u = d) x = d + (c1 d + c2 dinv (b - A d)); mode 2 (u = x) r = b - A x, d = s dinv r;
  * mode 3 (u = d) x = (x + d) + (c1 d + c2 dinv (r - A d)); coef: the level's coefficients. */
 int lpb_apply_explicit_modal_cheb_f32(int mode, float* x, float* r, float* d, const float* u, const float* b, const float* dinv, const double* coef, const float* km, const float* kpc, const int* glist, const int* gcount, float* ft, const uint8_t* mask, int nx, int ny, int nz, int pz, int cpz, void* stream);
+/* both (mode 0: out = m K u) for cols columns; ft: 24 * cells scratch per column */
+int lpb_apply_explicit_modal_cols_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b, const float* dinv, const double* coef, const float* km, const float* kpc, const int* glist, const int* gcount, float* ft, const uint8_t* mask, int nx, int ny, int nz, int pz, int cpz, int cols, void* stream);
 int lpb_apply_explicit_sym_f32(float* out, const float* u, const float* kp, float* ft, const uint8_t* mask, int nx, int ny, int nz, int pz, int cpz, void* stream);
 int lpb_apply_explicit_sym_f64(double* out, const double* u, const double* kp, double* ft, const uint8_t* mask, int nx, int ny, int nz, int pz, int cpz, void* stream);
 /* lpb_apply_explicit_sym_f32 for callers that cannot allocate device memory (a host that owns
@@ -242,6 +252,12 @@ int lpb_restrict_residual_f32(float* rc, const float* b, const float* ax, const 
 int lpb_restrict_residual_f64(double* rc, const double* b, const double* ax, const uint8_t* m, const uint8_t* cm, int fnx, int fny, int fnz, int fpz, int fcpz, int cnx, int cny, int cnz, int cpz_, int ccpz, void* stream);
 int lpb_prolong_add_f32(float* x, const float* xc, const uint8_t* cm, const uint8_t* m, int fnx, int fny, int fnz, int fpz, int fcpz, int cnx, int cny, int cnz, int cpz_, int ccpz, void* stream);
 int lpb_prolong_add_f64(double* x, const double* xc, const uint8_t* cm, const uint8_t* m, int fnx, int fny, int fnz, int fpz, int fcpz, int cnx, int cny, int cnz, int cpz_, int ccpz, void* stream);
+/* the same for cols columns (each field's columns one after the other); lpb_restrict_start also
+ * forms the smoother's first direction on the coarse level, d = (dinv rc) coef[1] (d may be NULL) */
+int lpb_restrict_start_f32(float* rc, float* d, const float* dinv, const double* coef, const float* b, const float* ax, const uint8_t* m, const uint8_t* cm, int fnx, int fny, int fnz, int fpz, int fcpz, int cnx, int cny, int cnz, int cpz_, int ccpz, int cols, void* stream);
+int lpb_restrict_start_f64(double* rc, double* d, const double* dinv, const double* coef, const double* b, const double* ax, const uint8_t* m, const uint8_t* cm, int fnx, int fny, int fnz, int fpz, int fcpz, int cnx, int cny, int cnz, int cpz_, int ccpz, int cols, void* stream);
+int lpb_prolong_add_cols_f32(float* x, const float* xc, const uint8_t* cm, const uint8_t* m, int fnx, int fny, int fnz, int fpz, int fcpz, int cnx, int cny, int cnz, int cpz_, int ccpz, int cols, void* stream);
+int lpb_prolong_add_cols_f64(double* x, const double* xc, const uint8_t* cm, const uint8_t* m, int fnx, int fny, int fnz, int fpz, int fcpz, int cnx, int cny, int cnz, int cpz_, int ccpz, int cols, void* stream);
 
 /* ---- PCG and power-iteration vector passes (loadpath/mgops.py:346-360, :557-585; mg.py:771-794,
  * :872-926). Reductions are deterministic: part needs lpb_reduce_blocks() doubles; results land
@@ -263,6 +279,31 @@ int lpb_xpby_f64(double* p, const double* z, long long n, const double* num, con
 int lpb_cg_step_r(double* r, const double* ap, float* r32, long long n, const double* num, const double* den, double* part, double* rr, void* stream);
 int lpb_xpby_x_f32(double* p, double* x, const float* z, long long n, const double* rz, const double* pap, const double* rz_new, void* stream);
 int lpb_xpby_x_f64(double* p, double* x, const double* z, long long n, const double* rz, const double* pap, const double* rz_new, void* stream);
+/* the PCG's passes with the reductions left as partials for the next pass, cols columns at a time
+ * (column j's fields n values after column j - 1's, sc 8 scalars a column: [0] b.b, [1] r.z the step
+ * sizes use, [2] r.z newest, [3] p.Ap, [4] |r|^2; n a multiple of 4, fields on 16 bytes).
+ * lpb_cg_parts: partials a pass leaves per column. lpb_cg_r: alpha = sc[2] / p.Ap from npap
+ * partials, r -= alpha ap, its float32 copy r32 (may be NULL), d = (dinv r) coef[1] (d may be NULL),
+ * partials of |r|^2; lpb_cg_rr: sc[4] from them; lpb_cg_test: the same and the device loop's stopping
+ * test, state (cols + 1, 2) as lpb_cg_continue_cols; lpb_cg_rz: partials of r.z; lpb_cg_p:
+ * x += (sc[1] / sc[3]) p, p = z + (r.z / sc[1]) p, sc[2] = r.z. */
+int lpb_cg_parts(long long n);
+int lpb_cg_r_f32(double* r, const double* ap, float* r32, float* d, const float* dinv, const double* coef, long long n, double* sc, const double* pap_part, int npap, double* part, int cols, void* stream);
+int lpb_cg_r_f64(double* r, const double* ap, float* r32, double* d, const double* dinv, const double* coef, long long n, double* sc, const double* pap_part, int npap, double* part, int cols, void* stream);
+int lpb_cg_rr(double* sc, const double* part, long long n, int cols, void* stream);
+int lpb_cg_test(long long handle, double* sc, const double* part, long long n, long long* state, int cols, double rtol, long long maxiter, void* stream);
+int lpb_cg_rz_f32(const double* r, const float* z, long long n, double* part, int cols, void* stream);
+int lpb_cg_rz_f64(const double* r, const double* z, long long n, double* part, int cols, void* stream);
+int lpb_cg_p_f32(double* p, double* x, const float* z, long long n, double* sc, const double* part, int cols, void* stream);
+int lpb_cg_p_f64(double* p, double* x, const double* z, long long n, double* sc, const double* part, int cols, void* stream);
+/* power iteration on D^-1 A: start v = m v0; after av = A v, step k: av = m dinv av / |v|,
+ * vv[k] = |v|^2, and the fields trade places; coef: the Chebyshev coefficients after its steps.
+ * part: 4 * lpb_cg_parts(n) doubles. */
+int lpb_pw_start_f32(float* v, const float* v0, const uint8_t* m, int nx, int ny, int nz, int pz, int cpz, double* part, void* stream);
+int lpb_pw_start_f64(double* v, const double* v0, const uint8_t* m, int nx, int ny, int nz, int pz, int cpz, double* part, void* stream);
+int lpb_pw_step_f32(float* av, const float* v, const float* dinv, const uint8_t* m, int nx, int ny, int nz, int pz, int cpz, int step, double* part, double* vv, void* stream);
+int lpb_pw_step_f64(double* av, const double* v, const double* dinv, const uint8_t* m, int nx, int ny, int nz, int pz, int cpz, int step, double* part, double* vv, void* stream);
+int lpb_pw_coef(double* coef, const double* vv, const double* part, long long n, int its, int degree, double safety, void* stream);
 /* warm start of the PCG on the device (loadpath/mg.py:878-895); sc holds [0] b.b, [5] x.Ax,
  * [6] b.x, [7] |rs|^2 and s = b.x / x.Ax (0 unless x.Ax > 0). lpb_warm_residual: rs = b - s Ax;
  * lpb_warm_select: x = s x, r = rs when s > 0 and |rs| < |b|, else x = 0, r = b. */
@@ -364,6 +405,7 @@ int lpb_cg_continue(long long handle, const double* sc, long long* state, double
  * lpb_snapshot_converged writes m x of column col into out in the iteration it converges. */
 int lpb_cg_continue_cols(long long handle, const double* sc, long long* state, int k, double rtol, long long maxiter, void* stream);
 int lpb_snapshot_converged(double* out, const double* x, const uint8_t* mask, const long long* state, int col, int k, int nx, int ny, int nz, int pz, int cpz, void* stream);
+int lpb_snapshot_converged_cols(double* out, const double* x, const uint8_t* mask, const long long* state, int k, int nx, int ny, int nz, int pz, int cpz, void* stream);
 int lpb_memcpy_async(void* dst, const void* src, long long bytes, void* stream);
 int lpb_memset_async(void* dst, int value, long long bytes, void* stream);
 

@@ -236,9 +236,9 @@ struct FineCheb {
 __device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 
 template <int MODE>
-__device__ __forceinline__ void cheb_store(const FineCheb& ch, long long i, const float4 ad4, float s, float c1,
+__device__ __forceinline__ void cheb_store(const FineCheb& ch, long long n, long long i, const float4 ad4, float s, float c1,
                                            float c2) {
-  const float4 dv4 = ldg4(ch.dinv + i);
+  const float4 dv4 = ldg4(ch.dinv + n);
   const float* ad = &ad4.x;
   const float* dv = &dv4.x;
   if constexpr (MODE == 1) {
@@ -304,6 +304,8 @@ k_apply_fine(const __grid_constant__ FineMaps maps, T* __restrict__ out, const u
   const long long units = (long long)gx * gy * nchunks;
   const long long u0 = units * blockIdx.x / gridDim.x, u1 = units * (blockIdx.x + 1) / gridDim.x;
   const long long cs = g.comp_stride(), zcs = g.node_zc_stride();
+  const long long co = 3 * cs * blockIdx.y;   // the column's fields (a launch of several right-hand sides)
+  if (dotp) dotp += (long long)gridDim.x * blockIdx.y;
   constexpr uint32_t UBYTES = 3 * BOX * BOX * 4 * sizeof(T);
   constexpr uint32_t EBYTES = TXC * TYC * 4 * sizeof(T);
   if (u0 >= u1) {
@@ -367,7 +369,7 @@ k_apply_fine(const __grid_constant__ FineMaps maps, T* __restrict__ out, const u
     pst = pst + 1 == NST ? 0 : pst + 1;
     const int x0 = (ps.tile % gx) * (TXC - 1), y0 = (ps.tile / gx) * (TYC - 1);
     lp_mbar_expect_tx(&sm.full[s], UBYTES + EBYTES);
-    lp_tma_load_4d(sm.u[s].v, &maps.u, 4 * (x0 - 1), y0 - 1, ps.cstart + pk, 0, &sm.full[s]);
+    lp_tma_load_4d(sm.u[s].v, &maps.u, 4 * (x0 - 1), y0 - 1, ps.cstart + pk, 3 * (int)blockIdx.y, &sm.full[s]);
     lp_tma_load_3d(sm.e[s].v, &maps.e, 4 * (x0 - 1), y0 - 1, ps.cstart + pk, &sm.full[s]);
     ++pk;
     ++issued;
@@ -488,7 +490,7 @@ k_apply_fine(const __grid_constant__ FineMaps maps, T* __restrict__ out, const u
             if (!((mb4 >> (8 * t + cc)) & 1u)) o[t] = T(0);
           const long long idx = cc * cs + obase + c * zcs;
           if constexpr (MODE == 0) {
-            store4(out + idx, o);
+            store4(out + co + idx, o);
             if constexpr (sizeof(T) == 8) {
               if (dotp) {
 #pragma unroll
@@ -496,7 +498,7 @@ k_apply_fine(const __grid_constant__ FineMaps maps, T* __restrict__ out, const u
               }
             }
           } else if constexpr (sizeof(T) == 4) {
-            cheb_store<MODE>(ch, idx, make_float4(o[0], o[1], o[2], o[3]), cs_s, cs_c1, cs_c2);
+            cheb_store<MODE>(ch, idx, co + idx, make_float4(o[0], o[1], o[2], o[3]), cs_s, cs_c1, cs_c2);
           }
         }
       }
@@ -613,7 +615,9 @@ static bool modal_sym_classes(const double* km, double out[7]) {
 template <typename T>
 static int launch_fine(T* out, const T* u, const T* e, const uint8_t* mask, const double* kmodal_host, int* err,
                        LpGrid g, cudaStream_t st, double* part = nullptr, long long part_len = 0,
-                       double* dot_out = nullptr, int mode = 0, const FineCheb* ch = nullptr) {
+                       double* dot_out = nullptr, int mode = 0, const FineCheb* ch = nullptr,
+                       int* nparts = nullptr, int cols = 1) {
+  if (cols < 1 || cols > 65535) return LP_ERR_ARG;
   if (!fine_args_ok(g) || !out || !u || !e || !mask || !kmodal_host || !err || out == u) return LP_ERR_ARG;
   if (mode != 0 && (sizeof(T) != 4 || !ch || mode < 0 || mode > 3)) return LP_ERR_ARG;
   double cls[7];
@@ -622,7 +626,7 @@ static int launch_fine(T* out, const T* u, const T* e, const uint8_t* mask, cons
   for (int n = 0; n < 7; ++n) ks.c[n] = (T)cls[n];
   const uint32_t zc = 4;
   FineMaps maps;
-  const uint64_t nd[4] = {zc * (uint64_t)g.NX(), (uint64_t)g.NY(), (uint64_t)g.pz / zc, 3};
+  const uint64_t nd[4] = {zc * (uint64_t)g.NX(), (uint64_t)g.NY(), (uint64_t)g.pz / zc, 3 * (uint64_t)cols};
   const uint64_t cd[3] = {zc * (uint64_t)g.nx, (uint64_t)g.ny, (uint64_t)g.cpz / zc};
   const uint32_t bin[4] = {zc * BOX, BOX, 1, 3};
   const uint32_t be[3] = {zc * TXC, TYC, 1};
@@ -658,10 +662,10 @@ static int launch_fine(T* out, const T* u, const T* e, const uint8_t* mask, cons
   const FineCheb& c = ch ? *ch : none;
   double* dp = nullptr;
   if (part) {
-    if (nb > part_len) return LP_ERR_SIZE;
+    if (nb * cols > part_len) return LP_ERR_SIZE;
     dp = part;
   }
-  const dim3 grid((unsigned)nb);
+  const dim3 grid((unsigned)nb, cols);
   if constexpr (sizeof(T) == 4) {
     if (mode == 1)
       lp_launch(k_apply_fine<float, 1>, grid, TXC * TYC, smem, st, maps, out, mask, ks, g, nchunks, err, c, nullptr);
@@ -674,7 +678,8 @@ static int launch_fine(T* out, const T* u, const T* e, const uint8_t* mask, cons
   } else {
     lp_launch(k_apply_fine<double, 0>, grid, TXC * TYC, smem, st, maps, out, mask, ks, g, nchunks, err, c, dp);
   }
-  if (dp) lp_launch(k_fine_dot_final, 1, 1024, 0, st, dp, nb, dot_out);
+  if (nparts) *nparts = (int)nb;
+  else if (dp) lp_launch(k_fine_dot_final, 1, 1024, 0, st, dp, nb, dot_out);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -724,18 +729,33 @@ int lpb_apply_fine_f64(double* out, const double* u, const double* e, const uint
 // x = d + (c1 d + c2 dinv (b - A d)); mode 2 (u = x) r = b - A x, d = s dinv r; mode 3 (u = d)
 // x = (x + d) + (c1 d + c2 dinv (r - A d)); coef: the level's Chebyshev coefficients (device);
 // the fields a mode does not name may be NULL
-int lpb_apply_fine_cheb_f32(int mode, float* x, float* r, float* d, const float* u, const float* b, const float* dinv,
-                            const double* coef, const float* e, const uint8_t* mask, const double* kmodal, int* err,
-                            int nx, int ny, int nz, int pz, int cpz, void* stream) {
-  if (!u || !dinv || !coef) return LP_ERR_ARG;
-  float* out = nullptr;
+static int fine_cheb(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b,
+                     const float* dinv, const double* coef, const float* e, const uint8_t* mask, const double* kmodal,
+                     int* err, LpGrid g, int cols, cudaStream_t st) {
+  if (!u || (mode && (!dinv || !coef))) return LP_ERR_ARG;
+  if (mode) out = nullptr;
   if (mode == 1 && x && d && b && u == d && x != d) out = x;
   if (mode == 2 && r && d && b && u == x && r != u && d != u && r != d) out = r;
   if (mode == 3 && x && d && r && u == d && x != d && r != d && r != x) out = x;
   if (!out) return LP_ERR_ARG;
   const FineCheb ch{x, r, d, b, dinv, coef};
-  return launch_fine<float>(out, u, e, mask, kmodal, err, lp_grid(nx, ny, nz, pz, cpz), (cudaStream_t)stream, nullptr,
-                            0, nullptr, mode, &ch);
+  return launch_fine<float>(out, u, e, mask, kmodal, err, g, st, nullptr, 0, nullptr, mode, &ch, nullptr, cols);
+}
+int lpb_apply_fine_cheb_f32(int mode, float* x, float* r, float* d, const float* u, const float* b, const float* dinv,
+                            const double* coef, const float* e, const uint8_t* mask, const double* kmodal, int* err,
+                            int nx, int ny, int nz, int pz, int cpz, void* stream) {
+  if (mode < 1) return LP_ERR_ARG;
+  return fine_cheb(mode, nullptr, x, r, d, u, b, dinv, coef, e, mask, kmodal, err, lp_grid(nx, ny, nz, pz, cpz), 1,
+                   (cudaStream_t)stream);
+}
+
+// the same (mode 0: out = m K u) for cols columns, each field's columns one after the other
+int lpb_apply_fine_cols_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b,
+                            const float* dinv, const double* coef, const float* e, const uint8_t* mask,
+                            const double* kmodal, int* err, int nx, int ny, int nz, int pz, int cpz, int cols,
+                            void* stream) {
+  return fine_cheb(mode, out, x, r, d, u, b, dinv, coef, e, mask, kmodal, err, lp_grid(nx, ny, nz, pz, cpz), cols,
+                   (cudaStream_t)stream);
 }
 
 // lpb_apply_fine_f64 that also forms u . out over the level's nodes into *dot (float64, device):
@@ -747,6 +767,16 @@ int lpb_apply_fine_dot_f64(double* out, const double* u, const double* e, const 
   if (!part || !dot || part_len <= 0) return LP_ERR_ARG;
   return launch_fine<double>(out, u, e, mask, kmodal, err, lp_grid(nx, ny, nz, pz, cpz), (cudaStream_t)stream, part,
                              part_len, dot);
+}
+
+// the same for cols columns (each field's columns one after the other) with the partials left for the
+// pass that uses the dot: *nparts (host) of them per column
+int lpb_apply_fine_dot_part_f64(double* out, const double* u, const double* e, const uint8_t* mask,
+                                const double* kmodal, int* err, double* part, long long part_len, int* nparts, int nx,
+                                int ny, int nz, int pz, int cpz, int cols, void* stream) {
+  if (!part || !nparts || part_len <= 0) return LP_ERR_ARG;
+  return launch_fine<double>(out, u, e, mask, kmodal, err, lp_grid(nx, ny, nz, pz, cpz), (cudaStream_t)stream, part,
+                             part_len, nullptr, 0, nullptr, nparts, cols);
 }
 
 }  // extern "C"

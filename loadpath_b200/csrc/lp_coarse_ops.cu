@@ -678,7 +678,7 @@ k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split sp
     const int s = issued % LST;
     const int x0 = (ps.tile % gx) * (LX - 1), y0 = (ps.tile / gx) * (LY - 1);
     lp_mbar_expect_tx(&sm.full[s], UBYTES + WBYTES);
-    lp_tma_load_4d(sm.u[s].v, &maps.u, 4 * (x0 - 1), y0 - 1, ps.cstart + pk, 0, &sm.full[s]);
+    lp_tma_load_4d(sm.u[s].v, &maps.u, 4 * (x0 - 1), y0 - 1, ps.cstart + pk, 3 * (int)blockIdx.y, &sm.full[s]);
     if constexpr (staged_w) lp_tma_load_4d(sm.w[s], &maps.w, 0, x0 - 1, y0 - 1, ps.cstart + pk, &sm.full[s]);
     ++pk;
     ++issued;
@@ -686,6 +686,7 @@ k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split sp
   if (tid == 0)
     while (issued < LST && issued < total) issue_next();
   const long long wstride = 32LL * g.nx * g.ny, cs = g.comp_stride(), zcs = g.node_zc_stride();
+  const long long co = 3 * cs * blockIdx.y;   // the column's fields (a launch of several right-hand sides)
   bool ok = true, failed = false;
   int n = 0, it = 0;   // the load in hand, chunks processed
   for (long long u = u0; u < u1 && !failed;) {
@@ -835,12 +836,12 @@ k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split sp
           const T val = sm.own[it & 1][cc][t][tid] + sm.red[it & 1][cc][t][tid - LX];
           o[t] = ((mb >> (8 * t + cc)) & 1u) ? val : T(0);
         }
-        const long long idx = cc * cs + obase + c * zcs;
+        const long long at = cc * cs + obase + c * zcs, idx = co + at;
         if constexpr (MODE == 0) {
           lp_st4(out + idx, o);
         } else {
           T dv[4], d[4];
-          lp_ld4(ch.dinv + idx, dv);
+          lp_ld4(ch.dinv + at, dv);
           if constexpr (MODE == 1) {
             T b[4], x[4];
             lp_ld4(ch.d + idx, d);
@@ -1241,6 +1242,8 @@ __global__ void __launch_bounds__(128, 4) k_explicit_modal_cells(float* __restri
                                                                 const int* __restrict__ gcount, LpGrid g,
                                                                 int modal_blocks) {
   lp_after_launch();
+  ft += 24 * g.cells_padded() * blockIdx.y;   // the column
+  u += 3 * g.comp_stride() * blockIdx.y;
   __shared__ float sk[4][300];
   __shared__ float su[4][24];
   if ((int)blockIdx.x < modal_blocks) {
@@ -1256,6 +1259,8 @@ __global__ void k_explicit_gather(T* __restrict__ out, const T* __restrict__ ft,
   lp_after_launch();
   const long long total = g.nodes_padded();
   const long long ncp = g.cells_padded(), cs = g.comp_stride();
+  ft += 24 * ncp * blockIdx.y;   // the column
+  out += 3 * cs * blockIdx.y;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int x, y, z;
     if (!g.node_at(t, x, y, z)) continue;
@@ -1293,7 +1298,8 @@ __global__ void k_explicit_gather_cheb(const T* __restrict__ ft, const uint8_t* 
                                        ChebArgs<T> a) {
   lp_after_launch();
   const long long total = g.nodes_padded();
-  const long long ncp = g.cells_padded(), cs = g.comp_stride();
+  const long long ncp = g.cells_padded(), cs = g.comp_stride(), co = 3 * cs * blockIdx.y;
+  ft += 24 * ncp * blockIdx.y;   // the column
   const T s = (T)a.coef[1], c1 = (T)a.coef[2], c2 = (T)a.coef[3];
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int x, y, z;
@@ -1311,17 +1317,17 @@ __global__ void k_explicit_gather_cheb(const T* __restrict__ ft, const uint8_t* 
     const uint8_t mb = mask[n];
 #pragma unroll
     for (int cc = 0; cc < 3; ++cc) {
-      const long long i = cc * cs + n;
+      const long long i = co + cc * cs + n;
       const T adi = ((mb >> cc) & 1) ? acc[cc] : T(0);
       if (MODE == 1) {
-        a.x[i] = lp_cheb2_zero_v(a.d[i], a.b[i], adi, a.dinv[i], c1, c2);
+        a.x[i] = lp_cheb2_zero_v(a.d[i], a.b[i], adi, a.dinv[i - co], c1, c2);
       } else if (MODE == 2) {
         T ri, di;
-        lp_residual_scaled_v(a.b[i], adi, a.dinv[i], s, ri, di);
+        lp_residual_scaled_v(a.b[i], adi, a.dinv[i - co], s, ri, di);
         a.r[i] = ri;
         a.d[i] = di;
       } else {
-        a.x[i] = lp_cheb2_v(a.x[i], a.d[i], a.r[i], adi, a.dinv[i], c1, c2);
+        a.x[i] = lp_cheb2_v(a.x[i], a.d[i], a.r[i], adi, a.dinv[i - co], c1, c2);
       }
     }
   }
@@ -1365,13 +1371,14 @@ static const int G1_COLS[279] = {3, 7, 14, 10, 17, 9, 20, 23, 15, 19, 22, 21, 4,
 template <typename T, int MODE>
 static int launch_level1(T* out, const T* u, const T* wc, const int* pid, const T* pm, const uint8_t* mask,
                          const double* g1_host, const int* pbox, int* err, LpGrid g, cudaStream_t st,
-                         const L1Cheb<T>& ch) {
+                         const L1Cheb<T>& ch, int cols = 1) {
+  if (cols < 1 || cols > 65535) return LP_ERR_ARG;
   if (!lp_grid_ok(g) || g.pz % 4 || g.cpz != g.pz || !out || !u || !wc || !mask || !g1_host || !err)
     return LP_ERR_ARG;
   G1<T> gc;
   for (int i = 0; i < 279; ++i) gc.c[i] = (T)g1_host[i];
   L1Maps maps;
-  const uint64_t nd[4] = {4 * (uint64_t)g.NX(), (uint64_t)g.NY(), (uint64_t)g.pz / 4, 3};
+  const uint64_t nd[4] = {4 * (uint64_t)g.NX(), (uint64_t)g.NY(), (uint64_t)g.pz / 4, 3 * (uint64_t)cols};
   const uint32_t bin[4] = {4 * LBX, LBY, 1, 3};
   if (!lp_make_map(&maps.u, u, 4, nd, bin, sizeof(T))) return LP_ERR_ARG;
   memset(&maps.w, 0, sizeof(maps.w));
@@ -1424,7 +1431,7 @@ static int launch_level1(T* out, const T* u, const T* wc, const int* pid, const 
     done += (long long)w * nchunks;
   }
   for (; b <= nb; ++b) split.u0[b] = (int)units;
-  lp_launch(k_level1<T, MODE>, (unsigned)nb, LCOL, smem, st, maps, split, out, wc, patches ? pid : nullptr, pm, mask, gc, g,
+  lp_launch(k_level1<T, MODE>, dim3((unsigned)nb, cols), LCOL, smem, st, maps, split, out, wc, patches ? pid : nullptr, pm, mask, gc, g,
                                                       nchunks, err, ch, box);
   LP_LAUNCH_CHECK();
   return LP_OK;
@@ -1449,17 +1456,17 @@ static int apply_weights_tma(T* out, const T* u, const T* wc, const int* pid, co
 template <typename T>
 static int apply_level1(int mode, T* out, T* x, T* r, T* d, const T* u, const T* b, const T* dinv, const double* coef,
                         const T* wc, const int* pid, const T* pm, const uint8_t* mask, const double* g1, const int* pbox,
-                        int* err, LpGrid g, cudaStream_t st) {
+                        int* err, LpGrid g, int cols, cudaStream_t st) {
   if (!u || mode < 0 || mode > 3 || (mode && (!dinv || !coef))) return LP_ERR_ARG;
   const L1Cheb<T> ch{x, r, d, b, dinv, coef};
   if (mode == 0 && out && out != u)
-    return launch_level1<T, 0>(out, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch);
+    return launch_level1<T, 0>(out, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch, cols);
   if (mode == 1 && x && d && b && u == d && x != d)
-    return launch_level1<T, 1>(x, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch);
+    return launch_level1<T, 1>(x, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch, cols);
   if (mode == 2 && r && d && b && u == x && r != u && d != u && r != d)
-    return launch_level1<T, 2>(r, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch);
+    return launch_level1<T, 2>(r, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch, cols);
   if (mode == 3 && x && d && r && u == d && x != d && r != d && r != x)
-    return launch_level1<T, 3>(x, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch);
+    return launch_level1<T, 3>(x, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch, cols);
   return LP_ERR_ARG;
 }
 
@@ -1471,6 +1478,31 @@ static int launch_explicit(T* out, const T* u, const T* kp, T* ft, const uint8_t
     return LP_ERR_LAUNCH;
   lp_launch(k_explicit_cells<T>, lp_blocks(g.cells_padded(), 32), 32 * EX_WARPS, smem, st, ft, u, kp, g);
   lp_launch(k_explicit_gather<T>, lp_blocks(g.nodes_padded(), 256), 256, 0, st, out, ft, mask, g);
+  LP_LAUNCH_CHECK();
+  return LP_OK;
+}
+
+static int launch_explicit_modal(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b,
+                                 const float* dinv, const double* coef, const float* km, const float* kpc,
+                                 const int* glist, const int* gcount, float* ft, const uint8_t* mask, LpGrid g, int cols,
+                                 cudaStream_t st) {
+  if (!lp_grid_ok(g) || !u || !km || !kpc || !glist || !gcount || !ft || !mask) return LP_ERR_ARG;
+  if (cols < 1 || cols > 65535) return LP_ERR_ARG;
+  if (mode == 0 && (!out || out == u)) return LP_ERR_ARG;
+  if (mode != 0 && (!dinv || !coef)) return LP_ERR_ARG;
+  if (mode == 1 && (!x || !d || !b || u != d || x == d)) return LP_ERR_ARG;
+  if (mode == 2 && (!r || !d || !b || u == r || u == d || r == d)) return LP_ERR_ARG;
+  if (mode == 3 && (!x || !d || !r || u != d || x == d)) return LP_ERR_ARG;
+  if (mode < 0 || mode > 3) return LP_ERR_ARG;
+  const int modal_blocks = lp_blocks(g.cells_padded(), 128);
+  lp_launch(k_explicit_modal_cells, dim3(modal_blocks + 148, cols), 128, 0, st, ft, u, km, kpc, glist, gcount, g,
+            modal_blocks);
+  const ChebArgs<float> a{x, r, d, b, dinv, coef};
+  const dim3 nb(lp_blocks(g.nodes_padded(), 256), cols);
+  if (mode == 0) lp_launch(k_explicit_gather<float>, nb, 256, 0, st, out, ft, mask, g);
+  else if (mode == 1) lp_launch(k_explicit_gather_cheb<float, 1>, nb, 256, 0, st, ft, mask, g, a);
+  else if (mode == 2) lp_launch(k_explicit_gather_cheb<float, 2>, nb, 256, 0, st, ft, mask, g, a);
+  else lp_launch(k_explicit_gather_cheb<float, 3>, nb, 256, 0, st, ft, mask, g, a);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -1616,7 +1648,16 @@ int lpb_apply_level1_f32(int mode, float* out, float* x, float* r, float* d, con
                          const float* dinv, const double* coef, const float* wc, const int* patch_id,
                          const float* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err,
                          LP_GRID_ARGS, void* stream) {
-  return apply_level1<float>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, mask, g1, pbox, err, LP_GRID,
+  return apply_level1<float>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, mask, g1, pbox, err, LP_GRID, 1,
+                             LP_ST);
+}
+
+// the same for cols columns (each field's columns one after the other)
+int lpb_apply_level1_cols_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b,
+                         const float* dinv, const double* coef, const float* wc, const int* patch_id,
+                         const float* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err,
+                         LP_GRID_ARGS, int cols, void* stream) {
+  return apply_level1<float>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, mask, g1, pbox, err, LP_GRID, cols,
                              LP_ST);
 }
 
@@ -1624,7 +1665,16 @@ int lpb_apply_level1_f64(int mode, double* out, double* x, double* r, double* d,
                          const double* dinv, const double* coef, const double* wc, const int* patch_id,
                          const double* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err,
                          LP_GRID_ARGS, void* stream) {
-  return apply_level1<double>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, mask, g1, pbox, err, LP_GRID,
+  return apply_level1<double>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, mask, g1, pbox, err, LP_GRID, 1,
+                              LP_ST);
+}
+
+// the same for cols columns (each field's columns one after the other)
+int lpb_apply_level1_cols_f64(int mode, double* out, double* x, double* r, double* d, const double* u, const double* b,
+                         const double* dinv, const double* coef, const double* wc, const int* patch_id,
+                         const double* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err,
+                         LP_GRID_ARGS, int cols, void* stream) {
+  return apply_level1<double>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, mask, g1, pbox, err, LP_GRID, cols,
                               LP_ST);
 }
 
@@ -1673,13 +1723,8 @@ int lpb_pack_modal_f32(float* km, int* glist, int* gcount, float* kpc, const flo
 // node-basis entries kpc (both from lpb_pack_modal_f32); ft: 24 * cells scratch
 int lpb_apply_explicit_modal_f32(float* out, const float* u, const float* km, const float* kpc, const int* glist,
                                  const int* gcount, float* ft, const uint8_t* mask, LP_GRID_ARGS, void* stream) {
-  LpGrid g = LP_GRID;
-  if (!lp_grid_ok(g) || !out || !u || !km || !kpc || !glist || !gcount || !ft || !mask || out == u) return LP_ERR_ARG;
-  const int modal_blocks = lp_blocks(g.cells_padded(), 128);
-  lp_launch(k_explicit_modal_cells, modal_blocks + 148, 128, 0, LP_ST, ft, u, km, kpc, glist, gcount, g, modal_blocks);
-  lp_launch(k_explicit_gather<float>, lp_blocks(g.nodes_padded(), 256), 256, 0, LP_ST, out, ft, mask, g);
-  LP_LAUNCH_CHECK();
-  return LP_OK;
+  return launch_explicit_modal(0, out, nullptr, nullptr, nullptr, u, nullptr, nullptr, nullptr, km, kpc, glist, gcount, ft,
+                               mask, LP_GRID, 1, LP_ST);
 }
 
 // the explicit level's A u (modal form, as lpb_apply_explicit_modal_f32) with a degree-2 Chebyshev
@@ -1690,21 +1735,19 @@ int lpb_apply_explicit_modal_cheb_f32(int mode, float* x, float* r, float* d, co
                                       const float* dinv, const double* coef, const float* km, const float* kpc,
                                       const int* glist, const int* gcount, float* ft, const uint8_t* mask,
                                       LP_GRID_ARGS, void* stream) {
-  LpGrid g = LP_GRID;
-  if (!lp_grid_ok(g) || !u || !km || !kpc || !glist || !gcount || !ft || !mask || !dinv || !coef) return LP_ERR_ARG;
-  if (mode == 1 && (!x || !d || !b || u != d || x == d)) return LP_ERR_ARG;
-  if (mode == 2 && (!r || !d || !b || u == r || u == d || r == d)) return LP_ERR_ARG;
-  if (mode == 3 && (!x || !d || !r || u != d || x == d)) return LP_ERR_ARG;
-  if (mode < 1 || mode > 3) return LP_ERR_ARG;
-  const int modal_blocks = lp_blocks(g.cells_padded(), 128);
-  lp_launch(k_explicit_modal_cells, modal_blocks + 148, 128, 0, LP_ST, ft, u, km, kpc, glist, gcount, g, modal_blocks);
-  const ChebArgs<float> a{x, r, d, b, dinv, coef};
-  const int nb = lp_blocks(g.nodes_padded(), 256);
-  if (mode == 1) lp_launch(k_explicit_gather_cheb<float, 1>, nb, 256, 0, LP_ST, ft, mask, g, a);
-  else if (mode == 2) lp_launch(k_explicit_gather_cheb<float, 2>, nb, 256, 0, LP_ST, ft, mask, g, a);
-  else lp_launch(k_explicit_gather_cheb<float, 3>, nb, 256, 0, LP_ST, ft, mask, g, a);
-  LP_LAUNCH_CHECK();
-  return LP_OK;
+  if (mode < 1) return LP_ERR_ARG;
+  return launch_explicit_modal(mode, nullptr, x, r, d, u, b, dinv, coef, km, kpc, glist, gcount, ft, mask, LP_GRID, 1,
+                               LP_ST);
+}
+
+// both (mode 0: out = m K u) for cols columns, each field's columns one after the other; ft: 24 * cells
+// scratch per column
+int lpb_apply_explicit_modal_cols_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b,
+                                      const float* dinv, const double* coef, const float* km, const float* kpc,
+                                      const int* glist, const int* gcount, float* ft, const uint8_t* mask,
+                                      LP_GRID_ARGS, int cols, void* stream) {
+  return launch_explicit_modal(mode, out, x, r, d, u, b, dinv, coef, km, kpc, glist, gcount, ft, mask, LP_GRID, cols,
+                               LP_ST);
 }
 
 int lpb_pack_sym_f32(float* kp, const float* k, long long ncells, void* stream) {

@@ -96,6 +96,27 @@ __device__ __forceinline__ void lp_residual_scaled_v(T bi, T axi, T dinvi, T s, 
   d = s * dinvi * ri;
 }
 
+#define LP_CHEB_MAX_DEGREE 7   // coefficient block of 16 doubles per level
+
+// a level's block of Chebyshev coefficients from the power iteration's Rayleigh value lam: the interval
+// [lmax / 30, lmax] with lmax = safety * max(lam, 1e-12), or 2 when an iterate vanished
+// (loadpath/mg.py:771-794, :796-821)
+__device__ __forceinline__ void lp_cheb_coef(double* coef, double lam, bool zero, int degree, double safety) {
+  const double hi = zero ? 2.0 : safety * (lam > 1e-12 ? lam : 1e-12);
+  const double lo = hi / 30.0;
+  const double theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo);
+  const double sigma = theta / delta;
+  double rho = 1.0 / sigma;
+  coef[0] = hi;
+  coef[1] = 1.0 / theta;
+  for (int k = 0; k < degree; ++k) {
+    const double rho_new = 1.0 / (2.0 * sigma - rho);
+    coef[2 + 2 * k] = rho_new * rho;
+    coef[3 + 2 * k] = 2.0 * rho_new / delta;
+    rho = rho_new;
+  }
+}
+
 static inline int lp_blocks(long long n, int threads) {
   long long b = (n + threads - 1) / threads;
   if (b < 1) b = 1;

@@ -55,13 +55,17 @@ __global__ void k_cg_continue_cols(cudaGraphConditionalHandle handle, const doub
   cudaGraphSetConditional(handle, (running && it < maxiter) ? 1u : 0u);
 }
 
-// out = m x (the solved bits) when column col converged at this iteration (state as above)
+// out = m x (the solved bits) of column col + blockIdx.y (the columns' fields one after the other) when it
+// converged at this iteration (state as above)
 __global__ void k_snapshot_converged(double* __restrict__ out, const double* __restrict__ x,
                                      const uint8_t* __restrict__ m, const long long* __restrict__ state, int col,
                                      int k, LpGrid g) {
   lp_after_launch();
+  col += blockIdx.y;
   if (state[2 * col + 1] != 1 || state[2 * col] != state[2 * k]) return;
   const long long nn = g.nodes_padded();
+  out += 3 * nn * blockIdx.y;
+  x += 3 * nn * blockIdx.y;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < 3 * nn; t += (long long)gridDim.x * blockDim.x) {
     const int c = t >= nn ? (t >= 2 * nn ? 2 : 1) : 0;
     out[t] = ((m[t - c * nn] >> c) & 1) ? x[t] : 0.0;
@@ -225,6 +229,16 @@ int lpb_snapshot_converged(double* out, const double* x, const uint8_t* mask, co
   LpGrid g = LP_GRID;
   if (!lp_grid_ok(g) || !out || !x || !mask || !state || col < 0 || col >= k || out == x) return LP_ERR_ARG;
   lp_launch(k_snapshot_converged, lp_blocks(3 * g.nodes_padded(), 256), 256, 0, LP_ST, out, x, mask, state, col, k, g);
+  LP_LAUNCH_CHECK();
+  return LP_OK;
+}
+
+// the same for every column of a k-column block solve: out, x (k, field)
+int lpb_snapshot_converged_cols(double* out, const double* x, const uint8_t* mask, const long long* state, int k,
+                                LP_GRID_ARGS, void* stream) {
+  LpGrid g = LP_GRID;
+  if (!lp_grid_ok(g) || !out || !x || !mask || !state || k < 1 || k > 65535) return LP_ERR_ARG;
+  lp_launch(k_snapshot_converged, dim3(lp_blocks(3 * g.nodes_padded(), 256), k), 256, 0, LP_ST, out, x, mask, state, 0, k, g);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }

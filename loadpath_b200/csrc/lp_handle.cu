@@ -307,7 +307,7 @@ struct Mg {
   void* mcat_d = nullptr;
   void* nkq_d = nullptr;
   int* err = nullptr;
-  double* part = nullptr;
+  double *part = nullptr, *part_cg = nullptr;
   long long part_len = 0;
   double *scal = nullptr, *chk = nullptr, *pw = nullptr, *coef = nullptr;
   double* host = nullptr;   // pinned: the CG scalars the host tests
@@ -361,11 +361,6 @@ struct Mg {
 };
 
 // dispatch helpers over the V-cycle precision
-int dot_v(bool f32, const void* a, const void* b, long long n, double* part, double* out, cudaStream_t st) {
-  return f32 ? lpb_dot_f32((const float*)a, (const float*)b, n, part, out, st)
-             : lpb_dot_f64((const double*)a, (const double*)b, n, part, out, st);
-}
-
 // the weights level's march (mode 0 out = m K u, 1..3 a Chebyshev update; lpb_apply_level1_*)
 void level1(Mg& m, Level& lv, int mode, void* out, const void* u, void* x = nullptr, void* r = nullptr,
             void* d = nullptr, const void* b = nullptr) {
@@ -613,22 +608,18 @@ void estimate_lmax(Mg& m, int i, int its = 12) {
   void *v, *av, *keep;
   lmax_vectors(m, i, v, av, keep);
   const bool f = lv.f32;
-  m.ok(f ? lpb_mask_field_f32((float*)v, (const float*)keep, lv.mask, HG(g), 0, m.st)
-         : lpb_mask_field_f64((double*)v, (const double*)keep, lv.mask, HG(g), 0, m.st));
   const long long n = g.nnode();
   double* pw = m.pw + 32 * i;
+  m.ok(f ? lpb_pw_start_f32((float*)v, (const float*)keep, lv.mask, HG(g), m.part, m.st)
+         : lpb_pw_start_f64((double*)v, (const double*)keep, lv.mask, HG(g), m.part, m.st));
   for (int it = 0; it < its; ++it) {
-    m.ok(dot_v(f, v, v, n, m.part, pw + it, m.st));
-    m.ok(f ? lpb_scale_rsqrt_f32((float*)v, n, pw + it, m.st) : lpb_scale_rsqrt_f64((double*)v, n, pw + it, m.st));
     apply(m, lv, av, v);
-    m.ok(f ? lpb_dinv_mask_f32((float*)av, (const float*)lv.dinv, lv.mask, HG(g), m.st)
-           : lpb_dinv_mask_f64((double*)av, (const double*)lv.dinv, lv.mask, HG(g), m.st));
-    m.ok(dot_v(f, v, av, n, m.part, pw + 16 + it, m.st));
+    m.ok(f ? lpb_pw_step_f32((float*)av, (const float*)v, (const float*)lv.dinv, lv.mask, HG(g), it, m.part, pw, m.st)
+           : lpb_pw_step_f64((double*)av, (const double*)v, (const double*)lv.dinv, lv.mask, HG(g), it, m.part, pw, m.st));
     std::swap(v, av);
   }
-  m.ok(f ? lpb_mask_field_f32((float*)keep, (const float*)v, lv.mask, HG(g), 0, m.st)
-         : lpb_mask_field_f64((double*)keep, (const double*)v, lv.mask, HG(g), 0, m.st));
-  m.ok(lpb_cheb_coef(m.coef + 16 * i, pw, pw + 16, its, std::max(m.degree, 1), LMAX_SAFETY, m.st));
+  cudaMemcpyAsync(keep, v, (f ? 4 : 8) * (size_t)n, cudaMemcpyDeviceToDevice, m.st);
+  m.ok(lpb_pw_coef(m.coef + 16 * i, pw, m.part, n, its, std::max(m.degree, 1), LMAX_SAFETY, m.st));
 }
 
 // one hierarchy build (loadpath/mg.py:515-591); false when the coarsest factor is singular
@@ -728,8 +719,9 @@ void set_moduli(Mg& m) {
   }
 }
 
-// Chebyshev smoothing of level i (degree 2; the fused forms of the Python class)
-void smooth(Mg& m, int i, const void* b, void* x, bool from_zero) {
+// Chebyshev smoothing of level i (degree 2; the fused forms of the Python class); started: from zero, and
+// the pass that formed b left the first direction in the level's d
+void smooth(Mg& m, int i, const void* b, void* x, bool from_zero, bool started = false) {
   Level& lv = m.op(i);
   const HGrid& g = lv.g;
   const bool f = lv.f32;
@@ -739,6 +731,9 @@ void smooth(Mg& m, int i, const void* b, void* x, bool from_zero) {
   void* t = m.field("t" + s, g, f);
   const long long n = g.nnode();
   const double* coef = lv.coef;
+  if (from_zero && !started)
+    m.ok(f ? lpb_cheb_d_start_f32((const float*)b, (const float*)lv.dinv, coef, (float*)d, n, m.st)
+           : lpb_cheb_d_start_f64((const double*)b, (const double*)lv.dinv, coef, (double*)d, n, m.st));
   if (lv.kind == K_SCALED && f) {
     auto fused = [&](int mode, const void* u) {
       m.ok(lpb_apply_fine_cheb_f32(mode, (float*)x, (float*)r, (float*)d, (const float*)u, (const float*)b,
@@ -746,7 +741,6 @@ void smooth(Mg& m, int i, const void* b, void* x, bool from_zero) {
                                    m.st));
     };
     if (from_zero) {
-      m.ok(lpb_cheb_d_start_f32((const float*)b, (const float*)lv.dinv, coef, (float*)d, n, m.st));
       fused(1, d);
     } else {
       fused(2, x);
@@ -756,8 +750,6 @@ void smooth(Mg& m, int i, const void* b, void* x, bool from_zero) {
   }
   if (lv.kind == K_WEIGHTS) {
     if (from_zero) {
-      m.ok(f ? lpb_cheb_d_start_f32((const float*)b, (const float*)lv.dinv, coef, (float*)d, n, m.st)
-             : lpb_cheb_d_start_f64((const double*)b, (const double*)lv.dinv, coef, (double*)d, n, m.st));
       level1(m, lv, 1, nullptr, d, x, nullptr, d, b);
     } else {
       level1(m, lv, 2, nullptr, x, x, r, d, b);
@@ -772,7 +764,6 @@ void smooth(Mg& m, int i, const void* b, void* x, bool from_zero) {
                                              lv.glist, lv.gcount, (float*)lv.ft, lv.mask, HG(g), m.st));
     };
     if (from_zero) {
-      m.ok(lpb_cheb_d_start_f32((const float*)b, (const float*)lv.dinv, coef, (float*)d, n, m.st));
       fused(1, d);
     } else {
       fused(2, x);
@@ -781,8 +772,6 @@ void smooth(Mg& m, int i, const void* b, void* x, bool from_zero) {
     return;
   }
   if (from_zero) {
-    m.ok(f ? lpb_cheb_d_start_f32((const float*)b, (const float*)lv.dinv, coef, (float*)d, n, m.st)
-           : lpb_cheb_d_start_f64((const double*)b, (const double*)lv.dinv, coef, (double*)d, n, m.st));
     apply(m, lv, t, d);
     m.ok(f ? lpb_cheb2_zero_f32((float*)x, (const float*)b, (const float*)t, (const float*)d, (const float*)lv.dinv, coef,
                                 n, m.st)
@@ -802,8 +791,11 @@ void smooth(Mg& m, int i, const void* b, void* x, bool from_zero) {
   }
 }
 
-// x = V(b) on level i (loadpath/mg.py:837-860); with r64 also *dot = r64 . x
-void* vcycle(Mg& m, int i, const void* b, const double* r64 = nullptr, double* dot = nullptr) {
+// whether level i's smoothing from zero can be handed its first direction
+bool starts(const Mg& m, int i) { return i + 1 < (int)m.levels.size() || !m.has_coarse; }
+
+// x = V(b) on level i (loadpath/mg.py:837-860); started: see smooth
+void* vcycle(Mg& m, int i, const void* b, bool started = false) {
   Level& lv = m.op(i);
   const HGrid& g = lv.g;
   const bool f = lv.f32;
@@ -818,26 +810,27 @@ void* vcycle(Mg& m, int i, const void* b, const double* r64 = nullptr, double* d
         m.ok(f ? lpb_band_solve_f32((float*)x, (const float*)b, m.ainv, m.cv, HG(g), m.st)
                : lpb_band_solve_f64((double*)x, (const double*)b, m.ainv, m.cv, HG(g), m.st));
     } else {
-      smooth(m, i, b, x, true);
+      smooth(m, i, b, x, true, started);
       smooth(m, i, b, x, false);
     }
-    if (r64) m.ok(lpb_dot_f64_f32(r64, (const float*)x, g.nnode(), m.part, dot, m.st));
     return x;
   }
-  smooth(m, i, b, x, true);
+  smooth(m, i, b, x, true, started);
   void* t = m.field("t" + s, g, f);
   apply(m, lv, t, x);
   Level& nxt = m.op(i + 1);
   const HGrid& gc = nxt.g;
   void* bc = m.field("b" + std::to_string(i + 1), gc, f);
-  m.ok(f ? lpb_restrict_residual_f32((float*)bc, (const float*)b, (const float*)t, lv.mask, nxt.mask, HG(g), HG(gc), m.st)
-         : lpb_restrict_residual_f64((double*)bc, (const double*)b, (const double*)t, lv.mask, nxt.mask, HG(g), HG(gc),
-                                     m.st));
-  void* xc = vcycle(m, i + 1, bc);
+  const bool go = starts(m, i + 1);
+  void* dc = go ? m.field("d" + std::to_string(i + 1), gc, f) : nullptr;
+  m.ok(f ? lpb_restrict_start_f32((float*)bc, (float*)dc, (const float*)nxt.dinv, nxt.coef, (const float*)b,
+                                  (const float*)t, lv.mask, nxt.mask, HG(g), HG(gc), 1, m.st)
+         : lpb_restrict_start_f64((double*)bc, (double*)dc, (const double*)nxt.dinv, nxt.coef, (const double*)b,
+                                  (const double*)t, lv.mask, nxt.mask, HG(g), HG(gc), 1, m.st));
+  void* xc = vcycle(m, i + 1, bc, go);
   m.ok(f ? lpb_prolong_add_f32((float*)x, (const float*)xc, nxt.mask, lv.mask, HG(g), HG(gc), m.st)
          : lpb_prolong_add_f64((double*)x, (const double*)xc, nxt.mask, lv.mask, HG(g), HG(gc), m.st));
   smooth(m, i, b, x, false);
-  if (r64) m.ok(lpb_dot_f64_f32(r64, (const float*)x, g.nnode(), m.part, dot, m.st));
   return x;
 }
 
@@ -874,6 +867,9 @@ double* pcg(Mg& m, const double* x0, int& iters, bool& ok) {
   double* rs = (double*)m.field("cg_rs", g, false);
   float* r32 = m.f32 ? (float*)m.field("cg_r32", g, true) : nullptr;
   double* src = (double*)m.field("cg_b", g, false);
+  Level& lv0 = m.op(0);
+  const bool go = starts(m, 0);
+  void* d0 = go ? m.field("d0", g, m.f32) : nullptr;
   if (x0) cudaMemcpyAsync(x, x0, nb, cudaMemcpyDeviceToDevice, m.st);
   // set-up: the warm start chosen on the device (loadpath/mg.py:880-896)
   m.ok(lpb_dot_f64(src, src, n, m.part, sc + 0, m.st));
@@ -890,29 +886,31 @@ double* pcg(Mg& m, const double* x0, int& iters, bool& ok) {
   }
   precondition(m, r, z);
   cudaMemcpyAsync(p, z, nb, cudaMemcpyDeviceToDevice, m.st);
-  m.ok(lpb_dot_f64(r, z, n, m.part, sc + 1, m.st));
+  m.ok(lpb_dot_f64(r, z, n, m.part, sc + 2, m.st));
   double tol = -1.0;
   cudaEvent_t ev;
   cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
   ok = false;
   iters = m.maxiter;
   for (int it = 1; it <= m.maxiter && m.status == LP_OK; ++it) {
-    // head: ap = A p with p . A p, r -= alpha ap (and its float32 copy), |r|^2
-    m.ok(lpb_apply_fine_dot_f64(ap, p, m.e0, a.mask, m.kmodal, m.err, m.part, m.part_len, sc + 3, HG(g), m.st));
-    m.ok(lpb_cg_step_r(r, ap, r32, n, sc + 1, sc + 3, m.part, sc + 4, m.st));
+    // head: ap = A p with p . A p, r -= alpha ap (and its float32 copy, and the V-cycle's first
+    // direction), |r|^2; dots are left as partials for the pass that uses them
+    int npap = 0;
+    m.ok(lpb_apply_fine_dot_part_f64(ap, p, m.e0, a.mask, m.kmodal, m.err, m.part, m.part_len, &npap, HG(g), 1, m.st));
+    m.ok(m.f32 ? lpb_cg_r_f32(r, ap, r32, (float*)d0, (const float*)lv0.dinv, lv0.coef, n, sc, m.part, npap, m.part_cg, 1,
+                              m.st)
+               : lpb_cg_r_f64(r, ap, nullptr, (double*)d0, (const double*)lv0.dinv, lv0.coef, n, sc, m.part, npap,
+                              m.part_cg, 1, m.st));
+    m.ok(lpb_cg_rr(sc, m.part_cg, n, 1, m.st));
     cudaMemcpyAsync(m.host, sc + 3, 16, cudaMemcpyDeviceToHost, m.st);
     cudaMemcpyAsync(m.host + 2, sc, 8, cudaMemcpyDeviceToHost, m.st);
     cudaEventRecord(ev, m.st);
     // tail, queued before the test: z = V(r), x += alpha p, p = z + beta p
-    if (r32) {
-      float* xv = (float*)vcycle(m, 0, r32, r, sc + 2);
-      m.ok(lpb_xpby_x_f32(p, x, xv, n, sc + 1, sc + 3, sc + 2, m.st));
-    } else {
-      precondition(m, r, z);
-      m.ok(lpb_dot_f64(r, z, n, m.part, sc + 2, m.st));
-      m.ok(lpb_xpby_x_f64(p, x, z, n, sc + 1, sc + 3, sc + 2, m.st));
-    }
-    cudaMemcpyAsync(sc + 1, sc + 2, 8, cudaMemcpyDeviceToDevice, m.st);
+    void* zv = vcycle(m, 0, r32 ? (const void*)r32 : (const void*)r, go);
+    m.ok(r32 ? lpb_cg_rz_f32(r, (const float*)zv, n, m.part_cg, 1, m.st)
+             : lpb_cg_rz_f64(r, (const double*)zv, n, m.part_cg, 1, m.st));
+    m.ok(r32 ? lpb_cg_p_f32(p, x, (const float*)zv, n, sc, m.part_cg, 1, m.st)
+             : lpb_cg_p_f64(p, x, (const double*)zv, n, sc, m.part_cg, 1, m.st));
     cudaEventSynchronize(ev);
     if (tol < 0.0) {
       const double bb = m.host[2];
@@ -1075,8 +1073,9 @@ void* lpb_mg_create(int nx, int ny, int nz, const uint8_t* fixed, const double* 
   }
   m->err = (int*)m->buf("err", 4);
   const long long fine_blocks = ((g.NX() + 14) / 15) * (long long)((g.NY() + 14) / 15) * (g.pz / 4);
-  m->part_len = std::max(std::max(2LL * lpb_reduce_blocks(), 2048LL), fine_blocks);
+  m->part_len = std::max(std::max(4LL * lpb_reduce_blocks(), 2048LL), fine_blocks);
   m->part = (double*)m->buf("part", 8 * (size_t)m->part_len);
+  m->part_cg = (double*)m->buf("part_cg", 8 * (size_t)lpb_reduce_blocks());
   m->scal = (double*)m->buf("scal", 8 * 64);
   m->chk = (double*)m->buf("chk", 8 * 64);
   m->pw = (double*)m->buf("pw", 8 * 32 * 32);

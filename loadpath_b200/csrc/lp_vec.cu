@@ -11,7 +11,6 @@
 
 #define LP_RED_BLOCKS 592   // 4 per SM on 148 SMs
 #define LP_RED_THREADS 512
-#define LP_CHEB_MAX_DEGREE 7   // coefficient block of 16 doubles per level
 
 namespace {
 
@@ -163,20 +162,7 @@ __global__ void k_cheb_coef(double* __restrict__ coef, const double* __restrict_
   lp_after_launch();
   bool zero = false;
   for (int k = 0; k < its; ++k) zero = zero || vv[k] == 0.0;
-  const double lam = vav[its - 1];
-  const double hi = zero ? 2.0 : safety * (lam > 1e-12 ? lam : 1e-12);
-  const double lo = hi / 30.0;
-  const double theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo);
-  const double sigma = theta / delta;
-  double rho = 1.0 / sigma;
-  coef[0] = hi;
-  coef[1] = 1.0 / theta;
-  for (int k = 0; k < degree; ++k) {
-    const double rho_new = 1.0 / (2.0 * sigma - rho);
-    coef[2 + 2 * k] = rho_new * rho;
-    coef[3 + 2 * k] = 2.0 * rho_new / delta;
-    rho = rho_new;
-  }
+  lp_cheb_coef(coef, vav[its - 1], zero, degree, safety);
 }
 
 // Degree-2 Chebyshev in two passes per smoothing (the reference's default degree). With
@@ -237,13 +223,21 @@ __global__ void k_jacobi(T* __restrict__ x, const T* __restrict__ b, const T* __
 // coarse columns X0..X0+14 of one coarse row Y and chunk C (coarse planes 4C..4C+3): lane l
 // reads fine column x = 2 X0 - 1 + l (rows 2Y - 1 .. 2Y + 1, fine planes 8C - 1 .. 8C + 7), so a
 // warp's loads are 32 consecutive 16-byte chunk rows; the lane restricts z and y in registers,
-// and the odd lanes (x = 2X) finish x with their two neighbours' sums by shuffles and store.
+// and the odd lanes (x = 2X) finish x with their two neighbours' sums by shuffles and store, with d
+// also the first direction d = (dinv rc) s of the smoothing that starts from rc (k_cheb_d_start's
+// values: a pass over the coarse field less, 3 us on the coarse levels). blockIdx.y: the column.
 constexpr int R4_COLS = 15;   // coarse columns per warp
 
 template <typename T>
-__global__ void k_restrict4(T* __restrict__ rc, const T* __restrict__ b, const T* __restrict__ ax,
+__global__ void k_restrict4(T* __restrict__ rc, T* __restrict__ d, const T* __restrict__ dinv,
+                            const double* __restrict__ coef, const T* __restrict__ b, const T* __restrict__ ax,
                             const uint8_t* __restrict__ m, const uint8_t* __restrict__ cm, LpGrid gf, LpGrid gc) {
   lp_after_launch();
+  rc += 3 * gc.comp_stride() * blockIdx.y;
+  d += d ? 3 * gc.comp_stride() * blockIdx.y : 0;
+  b += 3 * gf.comp_stride() * blockIdx.y;
+  ax += 3 * gf.comp_stride() * blockIdx.y;
+  const T sd = d ? (T)coef[1] : T(0);
   const int CX = gc.NX(), CY = gc.NY(), CZ4 = gc.pz / 4;
   const int FX = gf.NX(), FY = gf.NY();
   const int ngx = (CX + R4_COLS - 1) / R4_COLS;
@@ -331,17 +325,27 @@ __global__ void k_restrict4(T* __restrict__ rc, const T* __restrict__ b, const T
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) ov[kk] = ((cms[kk] >> i) & 1) ? o[i][kk] : T(0);
         V4ld<T>::st(rc + i * ccs + cn, ov);
+        if (d) {
+          T dv[4];
+          V4ld<T>::ld(dinv + i * ccs + cn, dv);
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) dv[kk] = (dv[kk] * ov[kk]) * sd;
+          V4ld<T>::st(d + i * ccs + cn, dv);
+        }
       }
     }
   }
 }
 
 // x += prolong(xc * cm) * m for fine nodes (x, y, 4c..4c+3): coarse planes 2c, 2c + 1, 2c + 2 of
-// the one, two or four coarse columns around (x / 2, y / 2)   (loadpath/mgops.py:714-750)
+// the one, two or four coarse columns around (x / 2, y / 2)   (loadpath/mgops.py:714-750); blockIdx.y:
+// the column
 template <typename T>
 __global__ void k_prolong4(T* __restrict__ xf, const T* __restrict__ xc, const uint8_t* __restrict__ cm,
                            const uint8_t* __restrict__ m, LpGrid gf, LpGrid gc) {
   lp_after_launch();
+  xf += 3 * gf.comp_stride() * blockIdx.y;
+  xc += 3 * gc.comp_stride() * blockIdx.y;
   const long long total = gf.nodes_padded() / 4;
   const long long fcs = gf.comp_stride(), ccs = gc.comp_stride();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -517,6 +521,40 @@ __global__ void k_xpby_x(double* __restrict__ p, double* __restrict__ x, const T
 #define LP_GRID lp_grid(nx, ny, nz, pz, cpz)
 #define LP_ST ((cudaStream_t)stream)
 #define LP_VEC_GRID(n) lp_blocks((n), 256) > 148 * 32 ? 148 * 32 : lp_blocks((n), 256), 256, 0, LP_ST
+
+namespace {
+// a fine level and the level below it: on each axis the coarse cells are ceil(fine cells / 2),
+// or one more when the coarse count is padded to even (loadpath/mg.py:607); the prolongation
+// reads coarse nodes up to ceil(fine / 2), the restriction checks its fine reads against the fine
+// grid
+bool lp_axis_ok(int f, int c) { return c >= (f + 1) / 2 && c <= (f + 1) / 2 + 1; }
+bool lp_pair_ok(const LpGrid& gf, const LpGrid& gc) {
+  return lp_axis_ok(gf.nx, gc.nx) && lp_axis_ok(gf.ny, gc.ny) && lp_axis_ok(gf.nz, gc.nz);
+}
+
+template <typename T>
+int launch_restrict(T* rc, T* d, const T* dinv, const double* coef, const T* b, const T* ax, const uint8_t* m,
+                    const uint8_t* cm, const LpGrid& gf, const LpGrid& gc, int cols, cudaStream_t st) {
+  if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || !rc || !b || !ax || !m || !cm || cols < 1 || cols > 65535) return LP_ERR_ARG;
+  if (d && (!dinv || !coef)) return LP_ERR_ARG;
+  if (!lp_pair_ok(gf, gc)) return LP_ERR_ARG;
+  const long long nw = (long long)((gc.NX() + R4_COLS - 1) / R4_COLS) * gc.NY() * (gc.pz / 4);
+  lp_launch(k_restrict4<T>, dim3(lp_blocks(32 * nw, 128), cols), 128, 0, st, rc, d, dinv, coef, b, ax, m, cm, gf, gc);
+  LP_LAUNCH_CHECK();
+  return LP_OK;
+}
+
+template <typename T>
+int launch_prolong(T* x, const T* xc, const uint8_t* cm, const uint8_t* m, const LpGrid& gf, const LpGrid& gc, int cols,
+                   cudaStream_t st) {
+  if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || !x || !xc || !m || !cm || cols < 1 || cols > 65535) return LP_ERR_ARG;
+  if (!lp_pair_ok(gf, gc)) return LP_ERR_ARG;
+  const long long t4 = gf.nodes_padded() / 4;
+  lp_launch(k_prolong4<T>, dim3(lp_blocks(t4, 128), cols), 128, 0, st, x, xc, cm, m, gf, gc);
+  LP_LAUNCH_CHECK();
+  return LP_OK;
+}
+}  // namespace
 
 extern "C" {
 
@@ -732,55 +770,48 @@ int lpb_jacobi_f64(double* x, const double* b, const double* ax, const double* d
 #define LP_GF lp_grid(fnx, fny, fnz, fpz, fcpz)
 #define LP_GC lp_grid(cnx, cny, cnz, cpz_, ccpz)
 
-// a fine level and the level below it: on each axis the coarse cells are ceil(fine cells / 2),
-// or one more when the coarse count is padded to even (loadpath/mg.py:607); the prolongation
-// reads coarse nodes up to ceil(fine / 2), the restriction checks its fine reads against the fine
-// grid
-static bool lp_axis_ok(int f, int c) { return c >= (f + 1) / 2 && c <= (f + 1) / 2 + 1; }
-static bool lp_pair_ok(const LpGrid& gf, const LpGrid& gc) {
-  return lp_axis_ok(gf.nx, gc.nx) && lp_axis_ok(gf.ny, gc.ny) && lp_axis_ok(gf.nz, gc.nz);
-}
-
 int lpb_restrict_residual_f32(float* rc, const float* b, const float* ax, const uint8_t* m, const uint8_t* cm,
                               LP_FC_ARGS, void* stream) {
-  LpGrid gf = LP_GF, gc = LP_GC;
-  if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || !rc || !b || !ax || !m || !cm) return LP_ERR_ARG;
-  if (!lp_pair_ok(gf, gc)) return LP_ERR_ARG;
-  const long long nw = (long long)((gc.NX() + R4_COLS - 1) / R4_COLS) * gc.NY() * (gc.pz / 4);
-  lp_launch(k_restrict4<float>, lp_blocks(32 * nw, 128), 128, 0, LP_ST, rc, b, ax, m, cm, gf, gc);
-  LP_LAUNCH_CHECK();
-  return LP_OK;
+  return launch_restrict<float>(rc, nullptr, nullptr, nullptr, b, ax, m, cm, LP_GF, LP_GC, 1, LP_ST);
+}
+
+// the same for cols columns (each field's columns one after the other), with the smoother's first
+// direction on the coarse level, d = (dinv rc) coef[1] (d NULL: none)
+int lpb_restrict_start_f32(float* rc, float* d, const float* dinv, const double* coef, const float* b, const float* ax,
+                           const uint8_t* m, const uint8_t* cm, LP_FC_ARGS, int cols, void* stream) {
+  return launch_restrict<float>(rc, d, dinv, coef, b, ax, m, cm, LP_GF, LP_GC, cols, LP_ST);
 }
 
 int lpb_restrict_residual_f64(double* rc, const double* b, const double* ax, const uint8_t* m, const uint8_t* cm,
                               LP_FC_ARGS, void* stream) {
-  LpGrid gf = LP_GF, gc = LP_GC;
-  if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || !rc || !b || !ax || !m || !cm) return LP_ERR_ARG;
-  if (!lp_pair_ok(gf, gc)) return LP_ERR_ARG;
-  const long long nw = (long long)((gc.NX() + R4_COLS - 1) / R4_COLS) * gc.NY() * (gc.pz / 4);
-  lp_launch(k_restrict4<double>, lp_blocks(32 * nw, 128), 128, 0, LP_ST, rc, b, ax, m, cm, gf, gc);
-  LP_LAUNCH_CHECK();
-  return LP_OK;
+  return launch_restrict<double>(rc, nullptr, nullptr, nullptr, b, ax, m, cm, LP_GF, LP_GC, 1, LP_ST);
+}
+
+// the same for cols columns (each field's columns one after the other), with the smoother's first
+// direction on the coarse level, d = (dinv rc) coef[1] (d NULL: none)
+int lpb_restrict_start_f64(double* rc, double* d, const double* dinv, const double* coef, const double* b, const double* ax,
+                           const uint8_t* m, const uint8_t* cm, LP_FC_ARGS, int cols, void* stream) {
+  return launch_restrict<double>(rc, d, dinv, coef, b, ax, m, cm, LP_GF, LP_GC, cols, LP_ST);
 }
 
 int lpb_prolong_add_f32(float* x, const float* xc, const uint8_t* cm, const uint8_t* m, LP_FC_ARGS, void* stream) {
-  LpGrid gf = LP_GF, gc = LP_GC;
-  if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || !x || !xc || !m || !cm) return LP_ERR_ARG;
-  if (!lp_pair_ok(gf, gc)) return LP_ERR_ARG;
-  const long long t4 = gf.nodes_padded() / 4;
-  lp_launch(k_prolong4<float>, lp_blocks(t4, 128), 128, 0, LP_ST, x, xc, cm, m, gf, gc);
-  LP_LAUNCH_CHECK();
-  return LP_OK;
+  return launch_prolong<float>(x, xc, cm, m, LP_GF, LP_GC, 1, LP_ST);
+}
+
+// the same for cols columns
+int lpb_prolong_add_cols_f32(float* x, const float* xc, const uint8_t* cm, const uint8_t* m, LP_FC_ARGS, int cols,
+                             void* stream) {
+  return launch_prolong<float>(x, xc, cm, m, LP_GF, LP_GC, cols, LP_ST);
 }
 
 int lpb_prolong_add_f64(double* x, const double* xc, const uint8_t* cm, const uint8_t* m, LP_FC_ARGS, void* stream) {
-  LpGrid gf = LP_GF, gc = LP_GC;
-  if (!lp_grid_ok(gf) || !lp_grid_ok(gc) || !x || !xc || !m || !cm) return LP_ERR_ARG;
-  if (!lp_pair_ok(gf, gc)) return LP_ERR_ARG;
-  const long long t4 = gf.nodes_padded() / 4;
-  lp_launch(k_prolong4<double>, lp_blocks(t4, 128), 128, 0, LP_ST, x, xc, cm, m, gf, gc);
-  LP_LAUNCH_CHECK();
-  return LP_OK;
+  return launch_prolong<double>(x, xc, cm, m, LP_GF, LP_GC, 1, LP_ST);
+}
+
+// the same for cols columns
+int lpb_prolong_add_cols_f64(double* x, const double* xc, const uint8_t* cm, const uint8_t* m, LP_FC_ARGS, int cols,
+                             void* stream) {
+  return launch_prolong<double>(x, xc, cm, m, LP_GF, LP_GC, cols, LP_ST);
 }
 
 int lpb_mask_field_f32(float* out, const float* u, const uint8_t* m, LP_GRID_ARGS, int bitshift, void* stream) {

@@ -233,9 +233,10 @@ class DevLevel:
                                                   self.mask.data_ptr(), self.g1.ctypes.data, self.pbox.ctypes.data,
                                                   self.err.data_ptr(), *self.grid.args, stream_handle())
 
-    def apply_dot(self, out, u, part, dot):
+    def apply_dot(self, out, u, part, dot=None, cols=1):
         """out = m K u on the float64 fine level (u zero on masked dofs) and *dot = u . out, in one
-        pass (the PCG's A p and p . A p)."""
+        pass (the PCG's A p and p . A p). dot None: the dots of cols columns are left as partials in
+        part, their count per column returned."""
         L = lib()
         g = self.grid
         st = stream_handle()
@@ -243,16 +244,22 @@ class DevLevel:
         if probe is not None:
             a, b = probe.take()
             L.lpb_event_record(a.cuda_event, st)
-        L.lpb_apply_fine_dot_f64(out.data_ptr(), u.data_ptr(), self.e.data_ptr(), self.mask.data_ptr(),
-                                 self.kmodal.ctypes.data, self.err.data_ptr(), part.data_ptr(), part.numel(),
-                                 dot.data_ptr(), *g.args, st)
+        count = ctypes.c_int(0)
+        if dot is None:
+            L.lpb_apply_fine_dot_part_f64(out.data_ptr(), u.data_ptr(), self.e.data_ptr(), self.mask.data_ptr(),
+                                          self.kmodal.ctypes.data, self.err.data_ptr(), part.data_ptr(),
+                                          part.numel(), ctypes.addressof(count), *g.args, cols, st)
+        else:
+            L.lpb_apply_fine_dot_f64(out.data_ptr(), u.data_ptr(), self.e.data_ptr(), self.mask.data_ptr(),
+                                     self.kmodal.ctypes.data, self.err.data_ptr(), part.data_ptr(), part.numel(),
+                                     dot.data_ptr(), *g.args, st)
         if probe is not None:
             L.lpb_event_record(b.cuda_event, st)
             if probe.capture is not None:
                 probe.capture.append((self.dtype, a, b))
             else:
                 probe.pending.append((self.dtype, a, b))
-        return out
+        return out if dot is not None else count.value
 
     def diagonal(self, d):
         L = lib()
@@ -378,12 +385,13 @@ class GridElasticity:
         # apply with p . A p (15 x 15 node columns by z segments of at least two chunks)
         g0 = self.g0
         fine_blocks = ((g0.NX + 14) // 15) * ((g0.NY + 14) // 15) * (g0.pz // 4)
-        self._part = torch.zeros(max(lib().lpb_reduce_blocks() * 2, 2048, fine_blocks), dtype=torch.float64,
+        self._part = torch.zeros(max(lib().lpb_reduce_blocks() * 4, 2048, fine_blocks), dtype=torch.float64,
                                  device=self.device)
+        self._part_cg = torch.zeros(lib().lpb_reduce_blocks(), dtype=torch.float64, device=self.device)
         self._host = torch.zeros(8, dtype=torch.float64, pin_memory=True)
         # the device-side CG loop: its stopping test's state (iterations, status) and its copy
-        self._loop_state = torch.zeros(2, dtype=torch.int64, device=self.device)
-        self._loop_out = torch.zeros(2, dtype=torch.int64, pin_memory=True)
+        self._loop_state = torch.zeros((2, 2), dtype=torch.int64, device=self.device)
+        self._loop_out = torch.zeros((2, 2), dtype=torch.int64, pin_memory=True)
         self.device_loop = True  # graphed solves test convergence on the device (no host read per iteration)
         self._work = {}
         self._e_dev = None
@@ -398,14 +406,14 @@ class GridElasticity:
         self._pw_stream = torch.cuda.Stream(device=self.device)             # coarse power iterations
         self._ev_pw_fork = torch.cuda.Event()
         self._ev_pw_join = torch.cuda.Event()
-        self._part_pw = torch.zeros(lib().lpb_reduce_blocks() * 2, dtype=torch.float64, device=self.device)
+        self._part_pw = torch.zeros(lib().lpb_reduce_blocks() * 4, dtype=torch.float64, device=self.device)
         # the fine two levels' power iterations: on the working stream, or (a planned rebuild) on a
         # stream of their own as soon as level 1 is built, beside the coarser levels' Galerkin
         # products; their own reduction scratch either way
         self._pw01_stream = torch.cuda.Stream(device=self.device)
         self._ev_pw01_fork = torch.cuda.Event()
         self._ev_pw01_join = torch.cuda.Event()
-        self._part_pw01 = torch.zeros(lib().lpb_reduce_blocks() * 2, dtype=torch.float64, device=self.device)
+        self._part_pw01 = torch.zeros(lib().lpb_reduce_blocks() * 4, dtype=torch.float64, device=self.device)
         self._pw01_early = False
         self._joined = True
 
@@ -848,28 +856,24 @@ class GridElasticity:
         buffers come from _lmax_vectors), so a level's iterations can be one graph."""
         L = lib()
         st = stream_handle()
-        part = self._part if part is None else part
+        part = self._part if part is None else part   # (4 * lpb_reduce_blocks() doubles)
         lv = self._op(i)
         g = lv.grid
         dt = lv.dtype
         sfx = "f32" if dt == torch.float32 else "f64"
         v, av, keep = self._lmax_vectors(i)
-        getattr(L, f"lpb_mask_field_{sfx}")(v.data_ptr(), keep.data_ptr(), lv.mask.data_ptr(), *g.args, 0, st)
         n = g.n_node_field
         pw = self._pw[32 * i:32 * (i + 1)]
+        getattr(L, f"lpb_pw_start_{sfx}")(v.data_ptr(), keep.data_ptr(), lv.mask.data_ptr(), *g.args, part.data_ptr(), st)
         for it in range(its):
-            getattr(L, f"lpb_dot_{sfx}")(v.data_ptr(), v.data_ptr(), n, part.data_ptr(),
-                                         pw[it:].data_ptr(), st)
-            getattr(L, f"lpb_scale_rsqrt_{sfx}")(v.data_ptr(), n, pw[it:].data_ptr(), st)
             lv.apply(av, v)
-            getattr(L, f"lpb_dinv_mask_{sfx}")(av.data_ptr(), lv.dinv.data_ptr(), lv.mask.data_ptr(), *g.args, st)
-            getattr(L, f"lpb_dot_{sfx}")(v.data_ptr(), av.data_ptr(), n, part.data_ptr(),
-                                         pw[16 + it:].data_ptr(), st)
+            getattr(L, f"lpb_pw_step_{sfx}")(av.data_ptr(), v.data_ptr(), lv.dinv.data_ptr(), lv.mask.data_ptr(),
+                                             *g.args, it, part.data_ptr(), pw.data_ptr(), st)
             v, av = av, v
         # the final vector is kept for the next hierarchy (already masked)
-        getattr(L, f"lpb_mask_field_{sfx}")(keep.data_ptr(), v.data_ptr(), lv.mask.data_ptr(), *g.args, 0, st)
-        L.lpb_cheb_coef(self._coef[16 * i:].data_ptr(), pw.data_ptr(), pw[16:].data_ptr(), its,
-                        max(self.degree, 1), LMAX_SAFETY, st)
+        L.lpb_memcpy_async(keep.data_ptr(), v.data_ptr(), v.numel() * v.element_size(), st)
+        L.lpb_pw_coef(self._coef[16 * i:].data_ptr(), pw.data_ptr(), part.data_ptr(), n, its, max(self.degree, 1),
+                      LMAX_SAFETY, st)
 
     def _run_lmax(self, i, nl, part):
         if self.use_graphs:
@@ -920,8 +924,13 @@ class GridElasticity:
             torch.cuda.current_stream().wait_event(self._ev_pw_join)
 
     # --- V-cycle (loadpath/mg.py:796-864) -----------------------------------------------
-    def _smooth(self, i, b, x, from_zero):
-        """Chebyshev (or damped Jacobi) smoothing of level i."""
+    def _starts(self, i):
+        """Whether level i's smoothing from zero can be handed its first direction."""
+        return self.smoother != "jacobi" and self.degree == 2 and (i + 1 < len(self.levels) or self._coarse is None)
+
+    def _smooth(self, i, b, x, from_zero, started=False):
+        """Chebyshev (or damped Jacobi) smoothing of level i. started: from zero, and the pass that
+        formed b left the first direction in the level's d (see _starts)."""
         L = lib()
         st = stream_handle()
         lv = self._op(i)
@@ -944,6 +953,8 @@ class GridElasticity:
                                                     0, n, st)
             return x
         coef = lv.coef.data_ptr()
+        if self.degree == 2 and from_zero and not started:
+            getattr(L, f"lpb_cheb_d_start_{sfx}")(b.data_ptr(), lv.dinv.data_ptr(), coef, d.data_ptr(), n, st)
         if self.degree == 2 and lv.kind == "scaled" and dt == torch.float32:
             # the fine float32 level forms each update where its tiled apply stores A u
             def fused(mode, u):
@@ -958,7 +969,6 @@ class GridElasticity:
                     L.lpb_event_record(eb.cuda_event, st)
                     (probe.capture if probe.capture is not None else probe.pending).append((f"f32c{mode}", ea, eb))
             if from_zero:
-                getattr(L, f"lpb_cheb_d_start_{sfx}")(b.data_ptr(), lv.dinv.data_ptr(), coef, d.data_ptr(), n, st)
                 fused(1, d)
             else:
                 fused(2, x)
@@ -972,7 +982,6 @@ class GridElasticity:
                                                     lv.kpc.data_ptr(), lv.glist.data_ptr(), lv.gcount.data_ptr(),
                                                     lv.ft.data_ptr(), lv.mask.data_ptr(), *g.args, st)
             if from_zero:
-                getattr(L, f"lpb_cheb_d_start_{sfx}")(b.data_ptr(), lv.dinv.data_ptr(), coef, d.data_ptr(), n, st)
                 fused(1, d)
             else:
                 fused(2, x)
@@ -981,7 +990,6 @@ class GridElasticity:
         if self.degree == 2 and lv.kind == "weights":
             # the first coarse level too, where its march stores A u
             if from_zero:
-                getattr(L, f"lpb_cheb_d_start_{sfx}")(b.data_ptr(), lv.dinv.data_ptr(), coef, d.data_ptr(), n, st)
                 lv.level1(1, None, d, x=x, d=d, b=b, coef=coef)
             else:
                 lv.level1(2, None, x, x=x, r=r, d=d, b=b, coef=coef)
@@ -990,7 +998,6 @@ class GridElasticity:
         if self.degree == 2:
             # the two Chebyshev steps in two passes (same bits as the step-by-step form)
             if from_zero:
-                getattr(L, f"lpb_cheb_d_start_{sfx}")(b.data_ptr(), lv.dinv.data_ptr(), coef, d.data_ptr(), n, st)
                 lv.apply(t, d)
                 getattr(L, f"lpb_cheb2_zero_{sfx}")(x.data_ptr(), b.data_ptr(), t.data_ptr(), d.data_ptr(),
                                                     lv.dinv.data_ptr(), coef, n, st)
@@ -1017,9 +1024,8 @@ class GridElasticity:
                                           lv.dinv.data_ptr(), coef, it, int(last), n, st)
         return x
 
-    def _vcycle(self, i, b, dot=None):
-        """x = V(b) on level i; b and the result live in level-i buffers. dot = (r64, out): also
-        out = r64 . x (the PCG's r . z)."""
+    def _vcycle(self, i, b, started=False):
+        """x = V(b) on level i; b and the result live in level-i buffers. started: see _smooth."""
         L = lib()
         st = stream_handle()
         lv = self._op(i)
@@ -1036,28 +1042,24 @@ class GridElasticity:
                     getattr(L, f"lpb_band_solve_{sfx}")(x.data_ptr(), b.data_ptr(), c["ainv"].data_ptr(),
                                                         c["v"].data_ptr(), *g.args, st)
             else:
-                self._smooth(i, b, x, True)
+                self._smooth(i, b, x, True, started)
                 self._smooth(i, b, x, False)
-            if dot is not None:
-                L.lpb_dot_f64_f32(dot[0].data_ptr(), x.data_ptr(), x.numel(), self._part.data_ptr(),
-                                  dot[1].data_ptr(), st)
             return x
-        self._smooth(i, b, x, True)
+        self._smooth(i, b, x, True, started)
         t = self._buf(f"t{i}", g, dt)
         lv.apply(t, x)
         nxt = self._op(i + 1)
         gc = nxt.grid
         bc = self._buf(f"b{i + 1}", gc, dt)
-        getattr(L, f"lpb_restrict_residual_{sfx}")(bc.data_ptr(), b.data_ptr(), t.data_ptr(), lv.mask.data_ptr(),
-                                                   nxt.mask.data_ptr(), *g.args, *gc.args, st)
-        xc = self._vcycle(i + 1, bc)
+        starts = self._starts(i + 1)
+        getattr(L, f"lpb_restrict_start_{sfx}")(bc.data_ptr(), ptr(self._buf(f"d{i + 1}", gc, dt)) if starts else None,
+                                                nxt.dinv.data_ptr() if starts else None,
+                                                nxt.coef.data_ptr() if starts else None, b.data_ptr(), t.data_ptr(),
+                                                lv.mask.data_ptr(), nxt.mask.data_ptr(), *g.args, *gc.args, 1, st)
+        xc = self._vcycle(i + 1, bc, starts)
         getattr(L, f"lpb_prolong_add_{sfx}")(x.data_ptr(), xc.data_ptr(), nxt.mask.data_ptr(), lv.mask.data_ptr(),
                                              *g.args, *gc.args, st)
         self._smooth(i, b, x, False)
-        if dot is not None:
-            # its own pass: folded into the last smoothing pass it evicts that pass's inputs from
-            # L2 (the float64 r is 103 MB at 256 x 128 x 128) and runs slower than the two
-            L.lpb_dot_f64_f32(dot[0].data_ptr(), x.data_ptr(), x.numel(), self._part.data_ptr(), dot[1].data_ptr(), st)
         return x
 
     def precondition_device(self, r64, z_out):
@@ -1177,6 +1179,9 @@ class GridElasticity:
         r32 = self._buf("cg_r32", g, torch.float32) if self.tdtype == torch.float32 else None
         host = self._host
         nb = 8 * n
+        part = self._part_cg
+        sfx = "f64" if r32 is None else "f32"
+        starts = self._starts(0)
         src = self._buf("cg_b", g, torch.float64)
         if b.data_ptr() != src.data_ptr():
             L.lpb_memcpy_async(src.data_ptr(), b.data_ptr(), nb, stream_handle())
@@ -1198,32 +1203,34 @@ class GridElasticity:
                 L.lpb_memcpy_async(r.data_ptr(), src.data_ptr(), nb, st)
             self.precondition_device(r, z)
             L.lpb_memcpy_async(p.data_ptr(), z.data_ptr(), nb, st)
-            self._dot64(r, z, 1)
+            self._dot64(r, z, 2)
+
+        def step():
+            # ap = A p and p.Ap in one pass; r -= alpha ap (and its float32 copy, and the V-cycle's
+            # first direction); |r|^2. Dots are left as partials for the pass that uses them.
+            # x += alpha p waits for the tail's pass over p.
+            npap = a.apply_dot(ap, p, self._part)
+            lv0 = self._op(0)
+            d0 = self._buf("d0", g, self.tdtype) if starts else None
+            getattr(L, f"lpb_cg_r_{sfx}")(r.data_ptr(), ap.data_ptr(), ptr(r32), ptr(d0), ptr(lv0.dinv) if starts else None,
+                                          ptr(lv0.coef) if starts else None, n, sc.data_ptr(), self._part.data_ptr(), npap,
+                                          part.data_ptr(), 1, stream_handle())
 
         def head():
-            # ap = A p and pap in one pass; r -= alpha ap (and its float32 copy); |r|^2; scalars
-            # out. x += alpha p waits for the tail's pass over p.
+            # the step, |r|^2 and the scalars out
             st = stream_handle()
-            a.apply_dot(ap, p, self._part, sc[3])
-            L.lpb_cg_step_r(r.data_ptr(), ap.data_ptr(), ptr(r32), n, sc[1].data_ptr(), sc[3].data_ptr(),
-                            self._part.data_ptr(), sc[4].data_ptr(), st)
+            step()
+            L.lpb_cg_rr(sc.data_ptr(), part.data_ptr(), n, 1, st)
             L.lpb_memcpy_async(host.data_ptr(), sc[3:5].data_ptr(), 16, st)
             L.lpb_memcpy_async(host[2:].data_ptr(), sc[0:1].data_ptr(), 8, st)
 
         def tail():
-            # z = V(r) and rz_new (formed by the V-cycle's last pass); x += alpha p;
-            # p = z + (rz_new / rz) p; rz = rz_new
+            # z = V(r); r.z; x += alpha p; p = z + (rz_new / rz) p
             st = stream_handle()
-            if r32 is not None:
-                xv = self._vcycle(0, r32, dot=(r, sc[2]))
-                L.lpb_xpby_x_f32(p.data_ptr(), x.data_ptr(), xv.data_ptr(), n, sc[1].data_ptr(), sc[3].data_ptr(),
-                                 sc[2].data_ptr(), st)
-            else:
-                self.precondition_device(r, z)
-                self._dot64(r, z, 2)
-                L.lpb_xpby_x_f64(p.data_ptr(), x.data_ptr(), z.data_ptr(), n, sc[1].data_ptr(), sc[3].data_ptr(),
-                                 sc[2].data_ptr(), st)
-            L.lpb_memcpy_async(sc[1:2].data_ptr(), sc[2:3].data_ptr(), 8, st)
+            z = self._vcycle(0, r if r32 is None else r32, starts)
+            getattr(L, f"lpb_cg_rz_{sfx}")(r.data_ptr(), z.data_ptr(), n, part.data_ptr(), 1, st)
+            getattr(L, f"lpb_cg_p_{sfx}")(p.data_ptr(), x.data_ptr(), z.data_ptr(), n, sc.data_ptr(), part.data_ptr(), 1,
+                                          st)
 
         warm = x0 is not None
         probe = _PROBE[0]
@@ -1237,21 +1244,19 @@ class GridElasticity:
             rtol, maxiter = float(self.rtol), int(self.maxiter)
 
             def body(handle):
-                stb = stream_handle()
-                a.apply_dot(ap, p, self._part, sc[3])
-                L.lpb_cg_step_r(r.data_ptr(), ap.data_ptr(), ptr(r32), n, sc[1].data_ptr(), sc[3].data_ptr(),
-                                self._part.data_ptr(), sc[4].data_ptr(), stb)
-                L.lpb_cg_continue(handle, sc.data_ptr(), state.data_ptr(), rtol, maxiter, stb)
+                step()
+                L.lpb_cg_test(handle, sc.data_ptr(), part.data_ptr(), n, state.data_ptr(), 1, rtol, maxiter,
+                              stream_handle())
                 tail()
 
             g_pre = self._graph(("pre", warm), lambda: pre(warm))
             g_loop = self._graph(("loop", rtol, maxiter), body, loop=True)
-            L.lpb_memset_async(state.data_ptr(), 0, 16, st)
+            L.lpb_memset_async(state.data_ptr(), 0, 32, st)
             self._replay(g_pre)
             self._replay(g_loop)
-            L.lpb_memcpy_async(self._loop_out.data_ptr(), state.data_ptr(), 16, st)
+            L.lpb_memcpy_async(self._loop_out.data_ptr(), state.data_ptr(), 32, st)
             torch.cuda.current_stream().synchronize()
-            it, status = int(self._loop_out[0]), int(self._loop_out[1])
+            it, status = int(self._loop_out[1, 0]), int(self._loop_out[0, 1])
             add_launches(g_loop[2] * (it - 1))          # the body ran `it` times
             if status == 2:
                 L.lpb_memset_async(x.data_ptr(), 0, nb, st)
@@ -1392,6 +1397,17 @@ class GridElasticity:
             self._work[key] = t
         return t
 
+    def _batched(self, i, k):
+        """Whether level i's smoothing of k columns runs with the columns in one launch (float32,
+        degree 2): a small grid's launches are a few us whatever they hold, so k columns cost
+        little more than one (a step with 8 loads on 96 x 48 x 48 cells: 39.2 ms with the columns
+        launched one after the other, 17.2 ms so). Where the columns' r, d and t would take over 1 GiB, one column fills the GPU by
+        itself, and the columns take turns in one set of them."""
+        lv = self._op(i)
+        return (self.smoother != "jacobi" and self.degree == 2 and lv.dtype == torch.float32
+                and lv.kind in ("scaled", "weights", "explicit") and (lv.kind != "explicit" or lv.km is not None)
+                and i + 1 < len(self.levels) and 12 * k * lv.grid.n_node_field <= 1 << 30)
+
     def _block_buffers(self, k):
         g = self.g0
         bufs = {key: self._blk(f"bcg_{key}", k, g, torch.float64) for key in ("x", "r", "p", "ap", "rs", "b", "snap")}
@@ -1400,18 +1416,49 @@ class GridElasticity:
             self._blk(f"bx{i}", k, lv.grid, self.tdtype)
             self._blk(f"bb{i}", k, lv.grid, self.tdtype)
             for key in ("r", "d", "t"):
-                self._buf(f"{key}{i}", lv.grid, self.tdtype)
+                if self._batched(i, k):
+                    self._blk(f"b{key}{i}", k, lv.grid, lv.dtype)
+                else:
+                    self._buf(f"{key}{i}", lv.grid, self.tdtype)
+            if self._batched(i, k) and lv.kind == "explicit":
+                self._flat_buf(f"bft{i}", k * lv.ft.numel(), lv.dtype)
         if self._coarse is not None and self._coarse["chain"] is None:
             self._flat_buf("band_vcols", k * self._coarse["v"].numel(), torch.float64)
         bufs["sc"] = self._tbuf("bcg_sc", (k, 8), torch.float64)
+        self._flat_buf("bcg_pap", k * self._part.numel(), torch.float64)
+        self._flat_buf("bcg_part", k * lib().lpb_reduce_blocks(), torch.float64)
         if getattr(self, "_bhost", None) is None or self._bhost.shape[0] != k:
             self._bhost = torch.zeros((k, 8), dtype=torch.float64, pin_memory=True)
             self._gen += 1               # graphs that copy into the old one are not replayed again
         return bufs
 
-    def _vcycle_cols(self, i, bb, dots=None):
+    def _apply_cols(self, i, mode, out, u, x=None, r=None, d=None, b=None):
+        """Level i's A u (mode 0) or a Chebyshev update formed where it is stored (modes 1..3, as in
+        _smooth) for every column of the blocks."""
+        L = lib()
+        st = stream_handle()
+        lv = self._op(i)
+        g = lv.grid
+        k = u.shape[0]
+        fields = (ptr(out), ptr(x), ptr(r), ptr(d), u.data_ptr(), ptr(b))
+        smooth = (lv.dinv.data_ptr(), lv.coef.data_ptr()) if mode else (None, None)
+        if lv.kind == "scaled":
+            L.lpb_apply_fine_cols_f32(mode, *fields, *smooth, lv.e.data_ptr(), lv.mask.data_ptr(), lv.kmodal.ctypes.data,
+                                      lv.err.data_ptr(), *g.args, k, st)
+        elif lv.kind == "weights":
+            L.lpb_apply_level1_cols_f32(mode, *fields, *smooth, lv.wc.data_ptr(), ptr(lv.patch_id) if lv.npatch else None,
+                                        ptr(lv.patch_m), lv.mask.data_ptr(), lv.g1.ctypes.data, lv.pbox.ctypes.data,
+                                        lv.err.data_ptr(), *g.args, k, st)
+        else:
+            L.lpb_apply_explicit_modal_cols_f32(mode, *fields, *smooth, lv.km.data_ptr(), lv.kpc.data_ptr(),
+                                                lv.glist.data_ptr(), lv.gcount.data_ptr(),
+                                                self._flat_buf(f"bft{i}", k * lv.ft.numel(), lv.dtype).data_ptr(),
+                                                lv.mask.data_ptr(), *g.args, k, st)
+
+    def _vcycle_cols(self, i, bb, started=False):
         """The V-cycle of level i for every column of bb (a (k, field) level-i block); returns
-        the level's x block. dots: [(r64, out)] per column, out = r64 . x."""
+        the level's x block. started: the level is batched and its first directions are in its d
+        block (see _smooth)."""
         L = lib()
         st = stream_handle()
         lv = self._op(i)
@@ -1434,26 +1481,43 @@ class GridElasticity:
                 for j in range(k):
                     self._smooth(i, bb[j], xb[j], True)
                     self._smooth(i, bb[j], xb[j], False)
+            return xb
+        nxt = self._op(i + 1)
+        gc = nxt.grid
+        bc = self._blk(f"bb{i + 1}", k, gc, dt)
+        starts = self._batched(i + 1, k)
+        dc = self._blk(f"bd{i + 1}", k, gc, dt) if starts else None
+
+        def restrict(bcs, dcs, bs, ts, cols):
+            getattr(L, f"lpb_restrict_start_{sfx}")(bcs.data_ptr(), ptr(dcs), nxt.dinv.data_ptr() if starts else None,
+                                                    nxt.coef.data_ptr() if starts else None, bs.data_ptr(), ts.data_ptr(),
+                                                    lv.mask.data_ptr(), nxt.mask.data_ptr(), *g.args, *gc.args, cols, st)
+
+        batched = self._batched(i, k)
+        if batched:
+            r, d, t = (self._blk(f"b{key}{i}", k, g, dt) for key in ("r", "d", "t"))
+            if not started:
+                for j in range(k):
+                    getattr(L, f"lpb_cheb_d_start_{sfx}")(bb[j].data_ptr(), lv.dinv.data_ptr(), lv.coef.data_ptr(),
+                                                          d[j].data_ptr(), g.n_node_field, st)
+            self._apply_cols(i, 1, None, d, x=xb, d=d, b=bb)
+            self._apply_cols(i, 0, t, xb)
+            restrict(bc, dc, bb, t, k)
         else:
             t = self._buf(f"t{i}", g, dt)
-            nxt = self._op(i + 1)
-            gc = nxt.grid
-            bc = self._blk(f"bb{i + 1}", k, gc, dt)
             for j in range(k):
                 self._smooth(i, bb[j], xb[j], True)
                 lv.apply(t, xb[j])
-                getattr(L, f"lpb_restrict_residual_{sfx}")(bc[j].data_ptr(), bb[j].data_ptr(), t.data_ptr(),
-                                                           lv.mask.data_ptr(), nxt.mask.data_ptr(), *g.args,
-                                                           *gc.args, st)
-            xc = self._vcycle_cols(i + 1, bc)
+                restrict(bc[j], None if dc is None else dc[j], bb[j], t, 1)
+        xc = self._vcycle_cols(i + 1, bc, starts)
+        getattr(L, f"lpb_prolong_add_cols_{sfx}")(xb.data_ptr(), xc.data_ptr(), nxt.mask.data_ptr(), lv.mask.data_ptr(),
+                                                  *g.args, *gc.args, k, st)
+        if batched:
+            self._apply_cols(i, 2, None, xb, x=xb, r=r, d=d, b=bb)
+            self._apply_cols(i, 3, None, d, x=xb, r=r, d=d)
+        else:
             for j in range(k):
-                getattr(L, f"lpb_prolong_add_{sfx}")(xb[j].data_ptr(), xc[j].data_ptr(), nxt.mask.data_ptr(),
-                                                     lv.mask.data_ptr(), *g.args, *gc.args, st)
                 self._smooth(i, bb[j], xb[j], False)
-        if dots is not None:
-            dot = L.lpb_dot_f64_f32 if dt == torch.float32 else L.lpb_dot_f64
-            for j, (r64, out) in enumerate(dots):
-                dot(r64.data_ptr(), xb[j].data_ptr(), xb[j].numel(), self._part.data_ptr(), out.data_ptr(), st)
         return xb
 
     def _pcg_block(self, bs, x0s, outs):
@@ -1473,7 +1537,11 @@ class GridElasticity:
             host = self._bhost
             nb = 8 * n
             f32 = self.tdtype == torch.float32
+            sfx = "f32" if f32 else "f64"
             bb0 = self._blk("bb0", k, g, self.tdtype)
+            starts = self._batched(0, k)
+            part = self._flat_buf("bcg_part", k * L.lpb_reduce_blocks(), torch.float64)
+            pap = self._flat_buf("bcg_pap", k * self._part.numel(), torch.float64)
             for j in range(k):
                 L.lpb_memcpy_async(src[j].data_ptr(), bs[j].data_ptr(), nb, stream_handle())
                 if x0s[j] is not None:
@@ -1486,11 +1554,10 @@ class GridElasticity:
             def precondition_all():
                 # z = V(r) for every column, z left in the level-0 x block
                 st = stream_handle()
-                for j in range(k):
-                    if f32:
-                        L.lpb_cast_f64_f32(bb0[j].data_ptr(), r[j].data_ptr(), n, st)
-                    else:
-                        L.lpb_memcpy_async(bb0[j].data_ptr(), r[j].data_ptr(), nb, st)
+                if f32:
+                    L.lpb_cast_f64_f32(bb0.data_ptr(), r.data_ptr(), k * n, st)
+                else:
+                    L.lpb_memcpy_async(bb0.data_ptr(), r.data_ptr(), k * nb, st)
                 return self._vcycle_cols(0, bb0)
 
             def pre():
@@ -1516,33 +1583,29 @@ class GridElasticity:
                         L.lpb_cast_f32_f64(p[j].data_ptr(), z[j].data_ptr(), n, st)
                     else:
                         L.lpb_memcpy_async(p[j].data_ptr(), z[j].data_ptr(), nb, st)
-                    dot(r[j], p[j], sc[j][1])
+                    dot(r[j], p[j], sc[j][2])
 
-            def head(to_host=True):
+            def step():
+                # _pcg_device's step, every column in each launch
+                npap = a.apply_dot(ap, p, pap, cols=k)
+                lv0 = self._op(0)
+                d0 = self._blk("bd0", k, g, self.tdtype) if starts else None
+                getattr(L, f"lpb_cg_r_{sfx}")(r.data_ptr(), ap.data_ptr(), bb0.data_ptr() if f32 else None, ptr(d0),
+                                              ptr(lv0.dinv) if starts else None, ptr(lv0.coef) if starts else None, n,
+                                              sc.data_ptr(), pap.data_ptr(), npap, part.data_ptr(), k, stream_handle())
+
+            def head():
                 st = stream_handle()
-                for j in range(k):
-                    s = sc[j]
-                    a.apply_dot(ap[j], p[j], self._part, s[3])
-                    L.lpb_cg_step_r(r[j].data_ptr(), ap[j].data_ptr(), bb0[j].data_ptr() if f32 else None, n,
-                                    s[1].data_ptr(), s[3].data_ptr(), self._part.data_ptr(), s[4].data_ptr(), st)
-                if to_host:
-                    L.lpb_memcpy_async(host.data_ptr(), sc.data_ptr(), 8 * 8 * k, st)
+                step()
+                L.lpb_cg_rr(sc.data_ptr(), part.data_ptr(), n, k, st)
+                L.lpb_memcpy_async(host.data_ptr(), sc.data_ptr(), 8 * 8 * k, st)
 
             def tail():
                 st = stream_handle()
-                if f32:
-                    # cg_step_r left each column's float32 residual in the level-0 b block
-                    z = self._vcycle_cols(0, bb0, dots=[(r[j], sc[j][2]) for j in range(k)])
-                else:
-                    z = precondition_all()
-                    for j in range(k):
-                        dot(r[j], z[j], sc[j][2])
-                for j in range(k):
-                    s = sc[j]
-                    getattr(L, "lpb_xpby_x_f32" if f32 else "lpb_xpby_x_f64")(
-                        p[j].data_ptr(), x[j].data_ptr(), z[j].data_ptr(), n, s[1].data_ptr(), s[3].data_ptr(),
-                        s[2].data_ptr(), st)
-                    L.lpb_memcpy_async(s[1].data_ptr(), s[2].data_ptr(), 8, st)
+                z = self._vcycle_cols(0, bb0 if f32 else r, starts)
+                getattr(L, f"lpb_cg_rz_{sfx}")(r.data_ptr(), z.data_ptr(), n, part.data_ptr(), k, st)
+                getattr(L, f"lpb_cg_p_{sfx}")(p.data_ptr(), x.data_ptr(), z.data_ptr(), n, sc.data_ptr(), part.data_ptr(),
+                                              k, st)
 
             graphed = self.use_graphs and self.maxiter > 1
             if graphed and self.device_loop:
@@ -1558,12 +1621,10 @@ class GridElasticity:
 
                 def body(handle):
                     stb = stream_handle()
-                    head(to_host=False)
-                    L.lpb_cg_continue_cols(handle, sc.data_ptr(), state.data_ptr(), k, rtol, maxiter, stb)
+                    step()
+                    L.lpb_cg_test(handle, sc.data_ptr(), part.data_ptr(), n, state.data_ptr(), k, rtol, maxiter, stb)
                     tail()
-                    for j in range(k):
-                        L.lpb_snapshot_converged(snap[j].data_ptr(), x[j].data_ptr(), mk, state.data_ptr(), j, k,
-                                                 *g.args, stb)
+                    L.lpb_snapshot_converged_cols(snap.data_ptr(), x.data_ptr(), mk, state.data_ptr(), k, *g.args, stb)
 
                 g_pre = self._graph(("bpre", k, warm), pre)
                 g_loop = self._graph(("bloop", k, rtol, maxiter), body, loop=True)
