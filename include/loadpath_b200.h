@@ -458,6 +458,14 @@ int lpb_mma_newton_b(long long n, int m, const double* low, const double* upp, c
  * out = [sum of squares, largest magnitude of the residual's n-sized rows, gvec (M)] */
 int lpb_mma_trial(long long n, int m, const double* low, const double* upp, const double* alfa, const double* beta, const double* p0, const double* q0, const double* P, const double* Q, const double* xs0, const double* xsi0, const double* eta0, const double* dx, const double* dxsi, const double* deta, double steg, const double* lam, double epsi, double* xs, double* xsi, double* eta, double* part, double* out, void* stream);
 /* xnew = clip(finite(xs) ? xs : x, alfa, beta)   (loadpath/mma.py:104-108) */
+/* the subproblem's loops on the device: lpb_mma_loop_begin writes the starting state (b = bsum - f; a, c,
+ * d, f HOST pointers to m doubles), lpb_mma_loop_body records one body (four launches) between
+ * lpb_while_begin and lpb_while_end, the sets (x0, xsi0, eta0) from lpb_mma_sub_init and (x1, ...) scratch.
+ * state: lpb_mma_state_len() doubles, after the loop [0, m) lam, [8] status (1 done, 2 singular Newton
+ * system), [9] the set that holds the result, [10] bodies run. */
+int lpb_mma_state_len(void);
+int lpb_mma_loop_begin(int m, double* state, const double* bsum, const double* a, const double* c, const double* d, const double* f, double a0, double epsimin, void* stream);
+int lpb_mma_loop_body(long long handle, long long n, int m, const double* low, const double* upp, const double* alfa, const double* beta, const double* p0, const double* q0, const double* P, const double* Q, double* x0, double* xsi0, double* eta0, double* x1, double* xsi1, double* eta1, double* state, double* part, void* stream);
 int lpb_mma_finish(long long n, const double* xs, const double* x, const double* alfa, const double* beta, double* xnew, void* stream);
 
 

@@ -12,7 +12,10 @@
 //   lpb_mma_trial     x, xsi, eta = old + steg * d and the residual's n-sized parts at the new
 //                     point (sum of squares, largest magnitude, gvec)
 //   lpb_mma_finish    non-finite results back to the old design, clip to [alfa, beta]
-// The host runs the loops, the m-sized parts of the residual and the (m + 1) x (m + 1) solve.
+//   lpb_mma_loop_*    the whole subproblem on the device: the loops as a graph's while node, the m-sized
+//                     variables and the (m + 1) system in a state block (below)
+// With newton_a, newton_b and trial the host runs the loops, the m-sized parts of the residual and the
+// (m + 1) x (m + 1) solve.
 // Reductions go through fixed per-block partials summed in order (the same bits every run).
 #include <math.h>
 
@@ -294,6 +297,419 @@ __global__ void __launch_bounds__(LP_MMA_THREADS) k_mma_trial(long long n, int m
   block_reduce<K>(acc, is_max, part);
 }
 
+// ---- the subproblem's loops on the device ------------------------------------------------------
+// A Newton step is two passes over the variables: k_mma_maxima forms the directions and their step-length
+// maxima, k_mma_move forms them again, moves the point by steg and leaves at the new point the residual's
+// sums and the sums of the next Newton system. Nothing n-sized is stored between them: the directions are
+// recomputed from the point and dlam, so a step reads 11 arrays and then reads 11 and writes 3, where
+// newton_a, newton_b and trial move 44. Between the passes one block each (k_mma_steg, k_mma_test) does
+// what the host did: step length, line search, epsi's descent, the (m + 1) system. The passes are bound by
+// memory (14 MB an array at 192 x 96 x 96 variables); quotients that share a divisor share its
+// reciprocal, since with each division of its own the float64 units took as long as the memory. An update
+// there takes 2.73 ms, with the host between the passes it took 9.98 ms (half of it waiting for results).
+constexpr int MMA_LOOP_BLOCKS = 296;   // two per SM
+
+struct MmaState {
+  double lam[LP_MMA_MAXM];
+  double status, which, passes;        // status: 0 running, 1 done, 2 singular system
+  double y[LP_MMA_MAXM], mu[LP_MMA_MAXM], s[LP_MMA_MAXM], z, zet;
+  double ty[LP_MMA_MAXM], tlam[LP_MMA_MAXM], tmu[LP_MMA_MAXM], ts[LP_MMA_MAXM], tz, tzet;   // the trial point's
+  double dy[LP_MMA_MAXM], dlam[LP_MMA_MAXM], dmu[LP_MMA_MAXM], ds[LP_MMA_MAXM], dz, dzet;
+  double a[LP_MMA_MAXM], b[LP_MMA_MAXM], c[LP_MMA_MAXM], d[LP_MMA_MAXM], a0;
+  double epsi, epsimin, norm, steg;
+  int it, halvings, fresh, move;       // fresh: a new direction (its maxima are wanted); move: a trial step
+};
+
+struct MmaInit {
+  double a[LP_MMA_MAXM], c[LP_MMA_MAXM], d[LP_MMA_MAXM], f[LP_MMA_MAXM], a0, epsimin;
+};
+
+struct MmaSets {
+  double* v[2][3];   // x, xsi, eta of the two points
+};
+
+__global__ void k_mma_begin(MmaState* __restrict__ st, const double* __restrict__ bsum, MmaInit in, int m) {
+  lp_after_launch();
+  const int i = threadIdx.x;
+  if (i < LP_MMA_MAXM) {
+    const bool on = i < m;
+    st->y[i] = st->lam[i] = st->s[i] = on ? 1.0 : 0.0;
+    st->mu[i] = on ? (0.5 * in.c[i] > 1.0 || isnan(in.c[i]) ? 0.5 * in.c[i] : 1.0) : 0.0;
+    st->a[i] = in.a[i];
+    st->c[i] = in.c[i];
+    st->d[i] = in.d[i];
+    st->b[i] = on ? bsum[i] - in.f[i] : 0.0;
+  }
+  if (i == 0) {
+    st->z = st->zet = 1.0;
+    st->a0 = in.a0;
+    st->epsi = 1.0;
+    st->epsimin = in.epsimin;
+    st->status = st->which = st->passes = 0.0;
+    st->it = st->halvings = st->fresh = st->move = 0;
+  }
+}
+
+// One variable: its constants, point and the reciprocals of its distances
+struct MmaVar {
+  double x, s, e, up, lo, al, be;
+  double iux, ixl, ixa, ibx;
+  __device__ __forceinline__ void reciprocals() {
+    iux = 1.0 / (up - x);
+    ixl = 1.0 / (x - lo);
+    ixa = 1.0 / (x - al);
+    ibx = 1.0 / (be - x);
+  }
+  // delx and diagx at p.lam, q.lam
+  __device__ __forceinline__ void newton(double plam, double qlam, double epsi, double& delx, double& diagx) const {
+    const double pu = plam * (iux * iux), ql = qlam * (ixl * ixl);
+    delx = pu - ql - epsi * ixa + epsi * ibx;
+    diagx = 2.0 * (pu * iux + ql * ixl) + s * ixa + e * ibx;
+  }
+};
+
+// the direction of variable j: (dx, dxsi, deta) from dlam
+__device__ __forceinline__ void mma_direction(const MmaVar& v, double plam, double qlam, double gp, double gq, double epsi,
+                                              double& dx, double& ds, double& de) {
+  double delx, diagx;
+  v.newton(plam, qlam, epsi, delx, diagx);
+  const double gtl = gp * (v.iux * v.iux) - gq * (v.ixl * v.ixl);   // (GG^T dlam)_j
+  dx = -(delx + gtl) / diagx;
+  ds = -v.s + epsi * v.ixa - v.s * dx * v.ixa;
+  de = -v.e + epsi * v.ibx + v.e * dx * v.ibx;
+}
+
+__device__ __forceinline__ MmaVar mma_var(const MmaArrays& A, const MmaSets& sets, int which, long long j) {
+  MmaVar v;
+  v.x = (which ? sets.v[1][0] : sets.v[0][0])[j];
+  v.s = (which ? sets.v[1][1] : sets.v[0][1])[j];
+  v.e = (which ? sets.v[1][2] : sets.v[0][2])[j];
+  v.up = A.upp[j];
+  v.lo = A.low[j];
+  v.al = A.alfa[j];
+  v.be = A.beta[j];
+  return v;
+}
+
+// maxima of -1.01 dxsi / xsi, -1.01 deta / eta, -1.01 dx / (x - alfa), 1.01 dx / (beta - x)
+template <int M>
+__global__ void __launch_bounds__(LP_MMA_THREADS, M > 2 ? 1 : 2) k_mma_maxima(long long n, int m, MmaArrays A, MmaSets sets,
+                                                                  const MmaState* __restrict__ st,
+                                                                  double* __restrict__ part) {
+  lp_after_launch();
+  if (!st->fresh) return;
+  __shared__ double lam[M], dlam[M];
+  if (threadIdx.x < M) {
+    lam[threadIdx.x] = st->lam[threadIdx.x];
+    dlam[threadIdx.x] = st->dlam[threadIdx.x];
+  }
+  __syncthreads();
+  const double epsi = st->epsi;
+  const int which = (int)st->which;
+  double acc[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  const bool is_max[4] = {true, true, true, true};
+  for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x) {
+    MmaVar v = mma_var(A, sets, which, j);
+    double plam = A.p0[j], qlam = A.q0[j], gp = 0.0, gq = 0.0;
+#pragma unroll
+    for (int i = 0; i < M; ++i)
+      if (i < m) {
+        const double P = A.P[(long long)i * n + j], Q = A.Q[(long long)i * n + j];
+        plam += P * lam[i];
+        qlam += Q * lam[i];
+        gp += P * dlam[i];
+        gq += Q * dlam[i];
+      }
+    v.reciprocals();
+    double dx, ds, de;
+    mma_direction(v, plam, qlam, gp, gq, epsi, dx, ds, de);
+    acc[0] = fmax(acc[0], -1.01 * ds / v.s);
+    acc[1] = fmax(acc[1], -1.01 * de / v.e);
+    acc[2] = fmax(acc[2], -1.01 * dx * v.ixa);
+    acc[3] = fmax(acc[3], 1.01 * dx * v.ibx);
+  }
+  block_reduce<4>(acc, is_max, part);
+}
+
+// warp sum or maximum of a value's partials (every lane gets it)
+__device__ __forceinline__ double mma_part(const double* __restrict__ part, int k, bool mx) {
+  double x = mx ? -INFINITY : 0.0;
+  for (int b = threadIdx.x & 31; b < MMA_LOOP_BLOCKS; b += 32) {
+    const double y = part[k * MMA_LOOP_BLOCKS + b];
+    x = mx ? fmax(x, y) : x + y;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double y = __shfl_xor_sync(0xffffffffu, x, o);
+    x = mx ? fmax(x, y) : x + y;
+  }
+  return x;
+}
+
+// the step length of a fresh direction (the largest keeping the variables positive and inside their
+// limits, at most 1), and the trial point's m-sized variables
+__global__ void __launch_bounds__(128) k_mma_steg(MmaState* __restrict__ st, const double* __restrict__ part, int m) {
+  lp_after_launch();
+  if (!st->move) return;
+  __shared__ double mx[4];
+  const int w = threadIdx.x >> 5;
+  if (st->fresh) {
+    const double v = mma_part(part, w, true);
+    if ((threadIdx.x & 31) == 0) mx[w] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x) return;
+  if (st->fresh) {
+    // (comparisons in this order: a NaN among the m-sized ratios never shortens the step)
+    double t = -INFINITY;
+    bool nan = false;
+    auto ratio = [&](double d, double v) {
+      const double r = -1.01 * d / v;
+      nan = nan || isnan(r);
+      if (r > t) t = r;
+    };
+    for (int i = 0; i < m; ++i) {
+      ratio(st->dy[i], st->y[i]);
+      ratio(st->dlam[i], st->lam[i]);
+      ratio(st->dmu[i], st->mu[i]);
+      ratio(st->ds[i], st->s[i]);
+    }
+    ratio(st->dz, st->z);
+    ratio(st->dzet, st->zet);
+    double top = mx[2];
+    if (mx[3] > top) top = mx[3];
+    if (!nan) {
+      if (mx[0] > t) t = mx[0];
+      if (mx[1] > t) t = mx[1];
+      if (t > top) top = t;
+    }
+    if (1.0 > top) top = 1.0;
+    st->steg = 1.0 / top;
+  }
+  const double g = st->steg;
+  for (int i = 0; i < m; ++i) {
+    st->ty[i] = st->y[i] + g * st->dy[i];
+    st->tlam[i] = st->lam[i] + g * st->dlam[i];
+    st->tmu[i] = st->mu[i] + g * st->dmu[i];
+    st->ts[i] = st->s[i] + g * st->ds[i];
+  }
+  st->tz = st->z + g * st->dz;
+  st->tzet = st->zet + g * st->dzet;
+}
+
+// the point moved by steg along its direction (move) into the other set, or as it is; sums there: the residual's
+// squares, its largest magnitude, gvec (M), GG (delx / diagx) (M), (GG / diagx) GG^T (upper triangle)
+template <int M>
+__global__ void __launch_bounds__(LP_MMA_THREADS, M > 2 ? 1 : 2) k_mma_move(long long n, int m, MmaArrays A, MmaSets sets,
+                                                                const MmaState* __restrict__ st,
+                                                                double* __restrict__ part) {
+  lp_after_launch();
+  constexpr int K = 2 + 2 * M + M * (M + 1) / 2;
+  const bool move = st->move;
+  __shared__ double lam[M], dlam[M], tlam[M];
+  if (threadIdx.x < M) {
+    lam[threadIdx.x] = st->lam[threadIdx.x];
+    dlam[threadIdx.x] = st->dlam[threadIdx.x];
+    tlam[threadIdx.x] = move ? st->tlam[threadIdx.x] : st->lam[threadIdx.x];
+  }
+  __syncthreads();
+  const double epsi = st->epsi, steg = st->steg;
+  const int which = (int)st->which;
+  double acc[K];
+  bool is_max[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    acc[k] = 0.0;
+    is_max[k] = k == 1;
+  }
+  for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x) {
+    MmaVar v = mma_var(A, sets, which, j);
+    const double p0 = A.p0[j], q0 = A.q0[j];
+    double plam = p0, qlam = q0, gp = 0.0, gq = 0.0, pnew = p0, qnew = q0, P[M], Q[M];
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      P[i] = Q[i] = 0.0;
+      if (i < m) {
+        P[i] = A.P[(long long)i * n + j];
+        Q[i] = A.Q[(long long)i * n + j];
+        plam += P[i] * lam[i];
+        qlam += Q[i] * lam[i];
+        gp += P[i] * dlam[i];
+        gq += Q[i] * dlam[i];
+        pnew += P[i] * tlam[i];
+        qnew += Q[i] * tlam[i];
+      }
+    }
+    if (move) {
+      v.reciprocals();
+      double dx, ds, de;
+      mma_direction(v, plam, qlam, gp, gq, epsi, dx, ds, de);
+      v.x += steg * dx;
+      v.s += steg * ds;
+      v.e += steg * de;
+      (which ? sets.v[0][0] : sets.v[1][0])[j] = v.x;
+      (which ? sets.v[0][1] : sets.v[1][1])[j] = v.s;
+      (which ? sets.v[0][2] : sets.v[1][2])[j] = v.e;
+    }
+    v.reciprocals();
+    const double iux2 = v.iux * v.iux, ixl2 = v.ixl * v.ixl;
+    const double r1 = pnew * iux2 - qnew * ixl2 - v.s + v.e;
+    const double r5 = v.s * (v.x - v.al) - epsi, r6 = v.e * (v.be - v.x) - epsi;
+    acc[0] += r1 * r1 + r5 * r5 + r6 * r6;
+    acc[1] = fmax(acc[1], fmax(fabs(r1), fmax(fabs(r5), fabs(r6))));
+    double delx, diagx;
+    v.newton(pnew, qnew, epsi, delx, diagx);
+    const double idg = 1.0 / diagx, t = delx * idg;
+    int k = 2 + 2 * M;
+    double gg[M];
+#pragma unroll
+    for (int i = 0; i < M; ++i) gg[i] = P[i] * iux2 - Q[i] * ixl2;
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      acc[2 + i] += P[i] * v.iux + Q[i] * v.ixl;
+      acc[2 + M + i] += gg[i] * t;
+      const double h = gg[i] * idg;
+#pragma unroll
+      for (int i2 = i; i2 < M; ++i2) acc[k++] += h * gg[i2];
+    }
+  }
+  block_reduce<K>(acc, is_max, part);
+}
+
+// (m + 1) x (m + 1) system by elimination with partial pivoting; false when a pivot is exactly zero
+__device__ bool mma_solve(double (*a)[LP_MMA_MAXM + 2], int n) {
+  for (int k = 0; k < n; ++k) {
+    int p = k;
+    for (int r = k + 1; r < n; ++r)
+      if (fabs(a[r][k]) > fabs(a[p][k])) p = r;
+    if (a[p][k] == 0.0) return false;
+    if (p != k)
+      for (int c = k; c <= n; ++c) {
+        const double t = a[k][c];
+        a[k][c] = a[p][c];
+        a[p][c] = t;
+      }
+    for (int r = k + 1; r < n; ++r) {
+      const double f = a[r][k] / a[k][k];
+      for (int c = k + 1; c <= n; ++c) a[r][c] -= f * a[k][c];
+    }
+  }
+  for (int k = n - 1; k >= 0; --k) {
+    double t = a[k][n];
+    for (int c = k + 1; c < n; ++c) t -= a[k][c] * a[c][n];
+    a[k][n] = t / a[k][k];
+  }
+  return true;
+}
+
+// After k_mma_move: accept the trial point or halve its step; then the next Newton system, or the next epsi
+// (loadpath/mma.py:126-214, the loops flattened: one pass of them per body of the while node)
+__global__ void __launch_bounds__(256) k_mma_test(cudaGraphConditionalHandle handle, MmaState* __restrict__ st,
+                                                  const double* __restrict__ part, int m, int M) {
+  lp_after_launch();
+  __shared__ double o[2 + 2 * LP_MMA_MAXM + LP_MMA_MAXM * (LP_MMA_MAXM + 1) / 2];
+  __shared__ double sys[LP_MMA_MAXM + 1][LP_MMA_MAXM + 2];
+  const int K = 2 + 2 * M + M * (M + 1) / 2;
+  for (int k = threadIdx.x >> 5; k < K; k += 8) {
+    const double v = mma_part(part, k, k == 1);
+    if ((threadIdx.x & 31) == 0) o[k] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x) return;
+  const bool move = st->move;
+  const double *y = move ? st->ty : st->y, *lam = move ? st->tlam : st->lam, *mu = move ? st->tmu : st->mu;
+  const double *s = move ? st->ts : st->s, z = move ? st->tz : st->z, zet = move ? st->tzet : st->zet;
+  const double epsi = st->epsi, *gvec = o + 2, *bl = o + 2 + M;
+  st->passes += 1.0;
+  // norm and largest magnitude of the residual
+  double ss = 0.0, top = 0.0, al = 0.0;
+  bool nan = false;
+  auto part_of = [&](double r) {
+    ss += r * r;
+    nan = nan || isnan(r);
+    if (fabs(r) > top) top = fabs(r);
+  };
+  for (int i = 0; i < m; ++i) {
+    part_of(st->c[i] + st->d[i] * y[i] - mu[i] - lam[i]);
+    al += st->a[i] * lam[i];
+    part_of(gvec[i] - st->a[i] * z - y[i] + s[i] - st->b[i]);
+    part_of(mu[i] * y[i] - epsi);
+    part_of(lam[i] * s[i] - epsi);
+  }
+  part_of(st->a0 - zet - al);
+  part_of(zet * z - epsi);
+  const double norm = sqrt(o[0] + ss), rmax = !nan && top > o[1] ? top : o[1];
+  bool go = true;
+  if (move) {
+    if (!(norm < 2.0 * st->norm) && ++st->halvings < 50) {
+      st->steg *= 0.5;
+      st->fresh = 0;
+      cudaGraphSetConditional(handle, 1u);
+      return;
+    }
+    for (int i = 0; i < m; ++i) {
+      st->y[i] = y[i];
+      st->lam[i] = lam[i];
+      st->mu[i] = mu[i];
+      st->s[i] = s[i];
+    }
+    st->z = z;
+    st->zet = zet;
+    st->which = 1.0 - st->which;
+  } else {
+    st->it = 0;
+  }
+  st->norm = norm;
+  y = st->y;
+  lam = st->lam;
+  mu = st->mu;
+  s = st->s;
+  if (rmax > 0.9 * epsi && st->it < 200) {
+    st->it += 1;
+    const int n = m + 1;
+    int k = 2 + 2 * M;
+    for (int i = 0; i < M; ++i)
+      for (int j = i; j < M; ++j, ++k)
+        if (j < m) sys[i][j] = sys[j][i] = o[k];
+    for (int i = 0; i < m; ++i) {
+      const double dely = st->c[i] + st->d[i] * y[i] - lam[i] - epsi / y[i], diagy = st->d[i] + mu[i] / y[i];
+      const double dellam = gvec[i] - st->a[i] * z - y[i] - st->b[i] + epsi / lam[i];
+      sys[i][i] += s[i] / lam[i] + 1.0 / diagy;
+      sys[i][n] = dellam + dely / diagy - bl[i];
+      sys[i][m] = sys[m][i] = st->a[i];
+    }
+    sys[m][m] = -zet / z;
+    sys[m][n] = st->a0 - al - epsi / z;
+    if (mma_solve(sys, n)) {
+      const double dz = sys[m][n];
+      for (int i = 0; i < m; ++i) {
+        const double dl = sys[i][n];
+        const double dely = st->c[i] + st->d[i] * y[i] - lam[i] - epsi / y[i], diagy = st->d[i] + mu[i] / y[i];
+        const double dy = -dely / diagy + dl / diagy;
+        st->dlam[i] = dl;
+        st->dy[i] = dy;
+        st->dmu[i] = -mu[i] + epsi / y[i] - mu[i] * dy / y[i];
+        st->ds[i] = -s[i] + epsi / lam[i] - s[i] * dl / lam[i];
+      }
+      st->dz = dz;
+      st->dzet = -zet + epsi / z - zet * dz / z;
+      st->fresh = st->move = 1;
+      st->halvings = 0;
+    } else {
+      st->status = 2.0;
+      go = false;
+    }
+  } else {
+    st->epsi = epsi * 0.1;
+    st->fresh = st->move = 0;
+    if (!(st->epsi > st->epsimin)) {
+      st->status = 1.0;
+      go = false;
+    }
+  }
+  cudaGraphSetConditional(handle, go ? 1u : 0u);
+}
+
 __global__ void k_mma_finish(long long n, const double* __restrict__ xs, const double* __restrict__ x,
                              const double* __restrict__ alfa, const double* __restrict__ beta,
                              double* __restrict__ xnew) {
@@ -440,6 +856,57 @@ int lpb_mma_trial(long long n, int m, const double* low, const double* upp, cons
   const MVec lv = mvec(lam, m);
   MMA_DISPATCH(k_mma_trial, n, m, A, xs0, xsi0, eta0, dx, dxsi, deta, steg, lv, epsi, xs, xsi, eta, part)
   final_reduce(part, 2 + mma_m_template(m), mask, out, LP_ST);
+  LP_LAUNCH_CHECK();
+  return LP_OK;
+}
+
+// ---- the subproblem as a device-side loop ----
+// doubles of the state block: [0, m) lam, [8] status (1 done, 2 singular Newton system), [9] the set that
+// holds the result, [10] bodies run
+int lpb_mma_state_len(void) { return (int)((sizeof(MmaState) + 7) / 8); }
+
+// the starting state: b = bsum - f, y = lam = s = z = zet = 1, mu = max(1, c / 2); a, c, d, f: HOST pointers to m
+int lpb_mma_loop_begin(int m, double* state, const double* bsum, const double* a, const double* c, const double* d,
+                       const double* f, double a0, double epsimin, void* stream) {
+  if (m < 1 || m > LP_MMA_MAXM || !state || !bsum || !a || !c || !d || !f) return LP_ERR_ARG;
+  MmaInit in{};
+  for (int i = 0; i < m; ++i) {
+    in.a[i] = a[i];
+    in.c[i] = c[i];
+    in.d[i] = d[i];
+    in.f[i] = f[i];
+  }
+  in.a0 = a0;
+  in.epsimin = epsimin;
+  lp_launch(k_mma_begin, 1, 32, 0, LP_ST, reinterpret_cast<MmaState*>(state), bsum, in, m);
+  LP_LAUNCH_CHECK();
+  return LP_OK;
+}
+
+// one body of the loop (four launches), recorded between lpb_while_begin, which gave handle, and
+// lpb_while_end; the first set holds the starting point, part: lpb_mma_part_len(m) doubles
+int lpb_mma_loop_body(long long handle, long long n, int m, const double* low, const double* upp, const double* alfa,
+                      const double* beta, const double* p0, const double* q0, const double* P, const double* Q,
+                      double* x0, double* xsi0, double* eta0, double* x1, double* xsi1, double* eta1, double* state,
+                      double* part, void* stream) {
+  if (n < 1 || m < 1 || m > LP_MMA_MAXM || !low || !upp || !alfa || !beta || !p0 || !q0 || !P || !Q || !x0 || !xsi0 ||
+      !eta0 || !x1 || !xsi1 || !eta1 || !state || !part)
+    return LP_ERR_ARG;
+  const MmaArrays A = {low, upp, alfa, beta, p0, q0, P, Q};
+  const MmaSets sets = {{{x0, xsi0, eta0}, {x1, xsi1, eta1}}};
+  MmaState* st = reinterpret_cast<MmaState*>(state);
+  const int M = mma_m_template(m);
+#define MMA_LOOP(KERNEL)                                                                                       \
+  switch (M) {                                                                                                 \
+    case 1: lp_launch(KERNEL<1>, MMA_LOOP_BLOCKS, LP_MMA_THREADS, 0, LP_ST, n, m, A, sets, st, part); break;   \
+    case 2: lp_launch(KERNEL<2>, MMA_LOOP_BLOCKS, LP_MMA_THREADS, 0, LP_ST, n, m, A, sets, st, part); break;   \
+    case 4: lp_launch(KERNEL<4>, MMA_LOOP_BLOCKS, LP_MMA_THREADS, 0, LP_ST, n, m, A, sets, st, part); break;   \
+    default: lp_launch(KERNEL<8>, MMA_LOOP_BLOCKS, LP_MMA_THREADS, 0, LP_ST, n, m, A, sets, st, part); break;  \
+  }
+  MMA_LOOP(k_mma_maxima)
+  lp_launch(k_mma_steg, 1, 128, 0, LP_ST, st, part, m);
+  MMA_LOOP(k_mma_move)
+  lp_launch(k_mma_test, 1, 256, 0, LP_ST, (cudaGraphConditionalHandle)handle, st, part, m, M);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }

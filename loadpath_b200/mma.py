@@ -8,21 +8,23 @@
 
 with a0 = 1, a_i = 0, d_i = 1, solved each iteration by Svanberg's primal-dual interior-point
 method on the convex separable approximation built from moving asymptotes. The design, the
-asymptotes, the approximation's terms and the subsolver's n-sized variables (x, xsi, eta and their
-Newton directions) live on the device; each pass over them is one of lp_mma.cu's kernels with its
-reductions. The host keeps the m-sized variables (y, z, lam, mu, zet, s), runs the loops (epsi from
-1 down to 1e-7, Newton steps, the line search of up to 50 halvings) and solves the (m + 1) x (m + 1)
-Newton system, exactly as the reference orders them. m <= 8.
+asymptotes, the approximation's terms and the subsolver's variables live on the device, and so do its
+loops (epsi from 1 down to 1e-7, Newton steps, the line search of up to 50 halvings), in the
+reference's order: a graph's while node whose body is two passes over the n-sized variables
+(lp_mma.cu), each followed by one block that does the m-sized part and the (m + 1) x (m + 1) Newton
+system. The host launches it and reads the outcome once. m <= 8.
 
 x, df0 and df may be numpy arrays (copied to the device; the result comes back as numpy) or
 float64 CUDA tensors (the result is a CUDA tensor).
 """
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import torch
 
-from ._lib import lib
+from ._lib import add_launches, launches, lib
 from .grid import stream_handle
 
 __all__ = ["MMA"]
@@ -63,9 +65,10 @@ class MMA:
         self._P, self._Q, self._df = z(m, n), z(m, n), z(m, n)
         self._df0, self._xnew = z(), z()
         self._sets = [(z(), z(), z()), (z(), z(), z())]   # (x, xsi, eta) of the subsolver, two sets
-        self._dx, self._dxsi, self._deta, self._delx, self._diagx = z(), z(), z(), z(), z()
         self._part = torch.zeros(int(lib().lpb_mma_part_len(m)), **dev)
         self._out = torch.zeros(64, **dev)
+        self._state = torch.zeros(int(lib().lpb_mma_state_len()), **dev)
+        self._exec = None
         self._have_asy = False
         self._have_old = False
 
@@ -95,8 +98,7 @@ class MMA:
                           self._beta.data_ptr(), self._p0.data_ptr(), self._q0.data_ptr(), self._P.data_ptr(),
                           self._Q.data_ptr(), self._part.data_ptr(), self._out.data_ptr(), st)
         self._have_asy = True
-        b = self._out[:m].cpu().numpy() - f
-        xs = self._subsolv(b)
+        xs = self._subsolv(f)
         L.lpb_mma_finish(n, xs.data_ptr(), self._x.data_ptr(), self._alfa.data_ptr(), self._beta.data_ptr(),
                          self._xnew.data_ptr(), st)
         self._xold2.copy_(self._xold1 if self._have_old else self._x)
@@ -105,106 +107,51 @@ class MMA:
         return self._xnew.cpu().numpy() if host else self._xnew.clone()
 
     # -- the subproblem (loadpath/mma.py:114-214) ---------------------------------------------
-    def _arrays(self):
-        return (self.low.data_ptr(), self.upp.data_ptr(), self._alfa.data_ptr(), self._beta.data_ptr())
+    def _loop(self):
+        """The interior-point loops as a graph with one while node (every buffer it names lives as
+        long as this object), captured at the first update."""
+        if self._exec is None:
+            L = lib()
+            c0 = launches()
+            with torch.cuda.device(self.device), torch.cuda.stream(torch.cuda.Stream(self.device)):
+                st = stream_handle()
+                handle, outer, exec_ = ctypes.c_longlong(), ctypes.c_void_p(), ctypes.c_void_p()
+                L.lpb_while_begin(st, ctypes.byref(handle), ctypes.byref(outer))
+                try:
+                    L.lpb_mma_loop_body(handle.value, self.n, self.m, self.low.data_ptr(), self.upp.data_ptr(),
+                                        self._alfa.data_ptr(), self._beta.data_ptr(), self._p0.data_ptr(),
+                                        self._q0.data_ptr(), self._P.data_ptr(), self._Q.data_ptr(),
+                                        *(t.data_ptr() for s in self._sets for t in s), self._state.data_ptr(),
+                                        self._part.data_ptr(), st)
+                finally:
+                    L.lpb_while_end(st, outer, ctypes.byref(exec_))
+            self._body = launches() - c0
+            add_launches(-self._body)      # recorded, not run
+            self._exec = exec_
+        return self._exec
 
-    def _residual(self, cur, nxt, d, steg, lam, y, z, mu, zet, s, epsi, b):
-        """Norm and largest magnitude of the KKT residual; with d given, the point cur + steg d
-        is written to nxt first (the device part), the m-sized part from the host values."""
-        L = lib()
-        m = self.m
-        dx = d[0].data_ptr() if d is not None else None
-        dxsi = d[1].data_ptr() if d is not None else None
-        deta = d[2].data_ptr() if d is not None else None
-        L.lpb_mma_trial(self.n, m, *self._arrays(), self._p0.data_ptr(), self._q0.data_ptr(), self._P.data_ptr(),
-                        self._Q.data_ptr(), cur[0].data_ptr(), cur[1].data_ptr(), cur[2].data_ptr(), dx, dxsi, deta,
-                        float(steg), np.ascontiguousarray(lam, float).ctypes.data, float(epsi),
-                        nxt[0].data_ptr(), nxt[1].data_ptr(), nxt[2].data_ptr(), self._part.data_ptr(),
-                        self._out.data_ptr(), stream_handle())
-        o = self._out[:2 + self.M].cpu().numpy()
-        gvec = o[2:2 + m]
-        small = np.concatenate([self.c + self.d * y - mu - lam, [self.a0 - zet - self.a @ lam],
-                                gvec - self.a * z - y + s - b, mu * y - epsi, [zet * z - epsi], lam * s - epsi])
-        norm = np.sqrt(o[0] + small @ small)
-        rmax = max(o[1], np.abs(small).max())
-        return norm, rmax
-
-    def _subsolv(self, b, epsimin=1e-7):
+    def _subsolv(self, f, epsimin=1e-7):
+        """The subproblem of b = out - f; returns the solution's x."""
         L = lib()
         st = stream_handle()
-        n, m, M = self.n, self.m, self.M
-        a0, a, c, d = self.a0, self.a, self.c, self.d
-        cur, nxt = self._sets
-        L.lpb_mma_sub_init(n, self._alfa.data_ptr(), self._beta.data_ptr(), cur[0].data_ptr(), cur[1].data_ptr(),
-                           cur[2].data_ptr(), st)
-        y = np.ones(m)
-        z = 1.0
-        lam = np.ones(m)
-        mu = np.maximum(1.0, 0.5 * c)
-        zet = 1.0
-        s = np.ones(m)
-        epsi = 1.0
-        dvec = (self._dx, self._dxsi, self._deta)
-        ntri = M * (M + 1) // 2
-        iu = np.triu_indices(M)
-        while epsi > epsimin:
-            norm, rmax = self._residual(cur, cur, None, 0.0, lam, y, z, mu, zet, s, epsi, b)
-            it = 0
-            while rmax > 0.9 * epsi and it < 200:
-                it += 1
-                L.lpb_mma_newton_a(n, m, *self._arrays(), self._p0.data_ptr(), self._q0.data_ptr(),
-                                   self._P.data_ptr(), self._Q.data_ptr(), cur[0].data_ptr(), cur[1].data_ptr(),
-                                   cur[2].data_ptr(), np.ascontiguousarray(lam, float).ctypes.data, float(epsi),
-                                   self._delx.data_ptr(), self._diagx.data_ptr(), self._part.data_ptr(),
-                                   self._out.data_ptr(), st)
-                o = self._out[:2 * M + ntri].cpu().numpy()
-                gvec, bl = o[:m], o[M:M + m]
-                tri = np.zeros((M, M))
-                tri[iu] = o[2 * M:2 * M + ntri]
-                gg = (tri + np.triu(tri, 1).T)[:m, :m]
-                dely = c + d * y - lam - epsi / y
-                delz = a0 - a @ lam - epsi / z
-                dellam = gvec - a * z - y - b + epsi / lam
-                diagy = d + mu / y
-                diaglamyi = s / lam + 1.0 / diagy
-                blam = dellam + dely / diagy - bl
-                alam = np.diag(diaglamyi) + gg
-                aa = np.zeros((m + 1, m + 1))
-                aa[:m, :m] = alam
-                aa[:m, m] = a
-                aa[m, :m] = a
-                aa[m, m] = -zet / z
-                sol = np.linalg.solve(aa, np.concatenate([blam, [delz]]))
-                dlam, dz = sol[:m], sol[m]
-                L.lpb_mma_newton_b(n, m, *self._arrays(), self._P.data_ptr(), self._Q.data_ptr(), cur[0].data_ptr(),
-                                   cur[1].data_ptr(), cur[2].data_ptr(), self._delx.data_ptr(), self._diagx.data_ptr(),
-                                   np.ascontiguousarray(dlam, float).ctypes.data, float(epsi), self._dx.data_ptr(),
-                                   self._dxsi.data_ptr(), self._deta.data_ptr(), self._part.data_ptr(),
-                                   self._out.data_ptr(), st)
-                mx = self._out[:4].cpu().numpy()
-                dy = -dely / diagy + dlam / diagy
-                dmu = -mu + epsi / y - mu * dy / y
-                dzet = -zet + epsi / z - zet * dz / z
-                ds = -s + epsi / lam - s * dlam / lam
-                xx = np.concatenate([y, [z], lam, mu, [zet], s])
-                dxx = np.concatenate([dy, [dz], dlam, dmu, [dzet], ds])
-                stmxx = max(np.max(-1.01 * dxx / xx), mx[0], mx[1])
-                steg = 1.0 / max(mx[2], mx[3], stmxx, 1.0)
-                old = (y, z, lam, mu, zet, s)
-                for _ in range(50):
-                    y = old[0] + steg * dy
-                    z = old[1] + steg * dz
-                    lam = old[2] + steg * dlam
-                    mu = old[3] + steg * dmu
-                    zet = old[4] + steg * dzet
-                    s = old[5] + steg * ds
-                    newnorm, newmax = self._residual(cur, nxt, dvec, steg, lam, y, z, mu, zet, s, epsi, b)
-                    if newnorm < 2.0 * norm:
-                        break
-                    steg /= 2.0
-                cur, nxt = nxt, cur
-                norm, rmax = newnorm, newmax
-            epsi *= 0.1
-        self._sets = [cur, nxt]
-        self.lam = lam
-        return cur[0]
+        x0, xsi0, eta0 = self._sets[0]
+        host = [np.ascontiguousarray(v, float) for v in (self.a, self.c, self.d, f)]
+        L.lpb_mma_sub_init(self.n, self._alfa.data_ptr(), self._beta.data_ptr(), x0.data_ptr(), xsi0.data_ptr(),
+                           eta0.data_ptr(), st)
+        L.lpb_mma_loop_begin(self.m, self._state.data_ptr(), self._out.data_ptr(), *(v.ctypes.data for v in host),
+                             float(self.a0), float(epsimin), st)
+        L.lpb_graph_launch(self._loop(), st)
+        o = self._state[:16].cpu().numpy()
+        add_launches(self._body * int(o[10]))
+        if o[8] == 2:
+            raise np.linalg.LinAlgError("Singular matrix")
+        self.lam = o[:self.m].copy()
+        return self._sets[int(o[9])][0]
+
+    def __del__(self):
+        if getattr(self, "_exec", None) is not None:
+            try:
+                torch.cuda.synchronize(self.device)
+                lib().lpb_graph_free(self._exec)
+            except Exception:
+                pass
