@@ -115,7 +115,8 @@ def test_power_passes(dims, dtype, zero):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
-@pytest.mark.parametrize("dims,cdims", [((14, 6, 6), (7, 3, 3)), ((62, 9, 17), (31, 5, 9))])
+@pytest.mark.parametrize("dims,cdims", [((14, 6, 6), (7, 3, 3)), ((62, 9, 17), (31, 5, 9)),
+                                        ((62, 40, 60), (31, 20, 30))])   # (the last: one column and three fall on either side of a rule)
 def test_transfers_with_columns(dtype, dims, cdims):
     """Three columns at once and the first direction, to the bit as one column's passes."""
     from loadpath_b200._lib import lib
