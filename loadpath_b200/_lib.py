@@ -36,7 +36,8 @@ _KERNELS = {"lpb_modal_ke": 0, "lpb_modal_g1": 0, "lpb_reduce_blocks": 0, "lpb_c
             "lpb_mma_part_len": 0, "lpb_mma_state_len": 0, "lpb_mma_loop_body": 4, "lpb_mma_prepare": 2, "lpb_mma_newton_a": 2, "lpb_mma_newton_b": 2,
             "lpb_mma_trial": 2, "lpb_project": 2, "lpb_oc_trial": 2, "lpb_live_seed": 2, "lpb_live_outside": 2,
             "lpb_dead_loads": 2, "lpb_apply_rf_f32": 2, "lpb_apply_explicit_modal_f32": 2,
-            "lpb_apply_explicit_modal_cheb_f32": 2, "lpb_apply_explicit_modal_cols_f32": 2, "lpb_modal_sym": 0, "lpb_hex8_ke": 0,
+            "lpb_apply_explicit_modal_cheb_f32": 2, "lpb_apply_explicit_modal_cols_f32": 2, "lpb_pack_modal_f32": 2, "lpb_pack_sym_f32": 2, "lpb_pack_sym_f64": 2,
+            "lpb_apply_explicit_sym_f32": 2, "lpb_apply_explicit_sym_f64": 2, "lpb_apply_explicit_sym_cheb_f64": 2, "lpb_modal_sym": 0, "lpb_hex8_ke": 0,
             "lpb_level1_products": 0, "lpb_uniform_numpy": 0, "lpb_layout_dims": 0, "lpb_layout_nodes_f64": 0,
             "lpb_unlayout_nodes_f64": 0, "lpb_layout_cells_f64": 0, "lpb_mg_levels": 0, "lpb_mg_strict": 0,
             "lpb_mg_destroy": 0,

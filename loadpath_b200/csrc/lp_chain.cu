@@ -662,7 +662,6 @@ __global__ void __launch_bounds__(256) k_chain_y(double* __restrict__ ws, const 
 // x_s = S^-1 g
 template <typename T, int NC>
 __global__ void __launch_bounds__(256) k_chain_s(double* __restrict__ ws, T* __restrict__ f, long long cstride, Chain c) {
-  lp_after_launch();
   extern __shared__ __align__(16) unsigned char sv_raw[];
   double* v = reinterpret_cast<double*>(sv_raw);   // [NC][MS]
   const int* idx = reinterpret_cast<const int*>(ws + c.idx);
@@ -670,7 +669,9 @@ __global__ void __launch_bounds__(256) k_chain_s(double* __restrict__ ws, T* __r
   const int r = SOLVE_ROWS * blockIdx.x + w, n = (c.nS + 1) & ~1;
   const double* a = ws + c.s + (long long)min(r, c.nS - 1) * c.MS;
   RowAhead h;
-  h.load(a, 0, n);
+  h.load(a, 0, n);   // (the matrix was complete before the launch ahead, k_chain_y)
+  lp_wait_prior();
+  lp_release_next();
 #pragma unroll
   for (int q = 0; q < NC; ++q)
     for (int i = threadIdx.x; i < c.MS; i += 256) v[q * c.MS + i] = i < c.nS ? ws[c.g + q * (long long)c.MS + i] : 0.0;
@@ -690,7 +691,6 @@ __global__ void __launch_bounds__(256) k_chain_s(double* __restrict__ ws, T* __r
 // x_I = y - W x_s
 template <typename T, int NC>
 __global__ void __launch_bounds__(256) k_chain_x(double* __restrict__ ws, T* __restrict__ f, long long cstride, Chain c) {
-  lp_after_launch();
   extern __shared__ __align__(16) unsigned char sv_raw[];
   double* v = reinterpret_cast<double*>(sv_raw);   // [NC][2b]: the segment's left and right separator
   const int* idx = reinterpret_cast<const int*>(ws + c.idx);
@@ -706,6 +706,8 @@ __global__ void __launch_bounds__(256) k_chain_x(double* __restrict__ ws, T* __r
   const double* a = ws + c.w + ((long long)j * c.M + min(r, m - 1)) * n;
   RowAhead h;
   h.load(a, 0, n);
+  lp_wait_prior();
+  lp_release_next();
 #pragma unroll
   for (int q = 0; q < NC; ++q)
     for (int k = threadIdx.x; k < n; k += 256)

@@ -958,7 +958,8 @@ __host__ __device__ __forceinline__ int sym_index(int i, int j) {  // i <= j
 
 // A block takes 32 consecutive cells, a lane per cell, and its eight warps share the 300 entries of their
 // matrices (entry p of consecutive cells coalesced): each warp loads its 37 or 38 entries before the
-// corner values are staged, forms its part of the 24 corner forces, and the parts are added in order.
+// corner values are staged, forms its part of the 24 corner forces, and the parts are added in order. The
+// matrices are older than the launch ahead (lpb_pack_sym_* see to it), so they are loaded while it runs.
 // What bounds it is how many of those loads are in flight: with one thread per cell (a few
 // thousand cells on a coarse level) the apply of 32 x 16 x 16 cells took 25.7 us in float64, shared by
 // eight warps 11.7 us, of 64 x 32 x 32 cells 69 and 50 us (157 MB of entries from DRAM: 22 us).
@@ -989,11 +990,16 @@ __device__ __forceinline__ void sym_forces(const T (&k)[38], const T (&u)[24][32
     }
 }
 template <int W, typename T>
-__device__ __forceinline__ void sym_warp(ExCells<T>& sm, const T* __restrict__ kc, long long ncp) {
+__device__ __forceinline__ void sym_warp(ExCells<T>& sm, const T* __restrict__ kc, long long ncp,
+                                         const T* __restrict__ u, long long cs, bool in) {
   const int lane = threadIdx.x & 31;
   T k[38], f[24];
   sym_part<W, T>(kc, ncp, k);
-  __syncthreads();   // the corner values are staged
+  lp_wait_prior();
+  lp_release_next();
+#pragma unroll
+  for (int cc = 0; cc < 3; ++cc) sm.u[3 * W + cc][lane] = in ? u[cc * cs] : T(0);   // corner W
+  __syncthreads();
 #pragma unroll
   for (int r = 0; r < 24; ++r) f[r] = T(0);
   sym_forces<W, T>(k, sm.u, f);
@@ -1006,7 +1012,6 @@ __global__ void __launch_bounds__(32 * EX_WARPS)
 k_explicit_cells(T* __restrict__ ft, const T* __restrict__ u, const T* __restrict__ kp, LpGrid g) {
   extern __shared__ __align__(16) unsigned char ex_raw[];
   ExCells<T>& sm = *reinterpret_cast<ExCells<T>*>(ex_raw);
-  lp_after_launch();
   const long long ncp = g.cells_padded(), cs = g.comp_stride();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long c = blockIdx.x * 32LL + lane;
@@ -1016,18 +1021,16 @@ k_explicit_cells(T* __restrict__ ft, const T* __restrict__ u, const T* __restric
   const long long n0 = in ? g.node(x, y, z) : 0;
   const long long oy = 4LL * g.NX(), oz = (z & 3) == 3 ? g.node_zc_stride() - 3 : 1;
   const long long n = n0 + (w & 1 ? 4 : 0) + (w & 2 ? oy : 0) + (w & 4 ? oz : 0);
-#pragma unroll
-  for (int cc = 0; cc < 3; ++cc) sm.u[3 * w + cc][lane] = in ? u[cc * cs + n] : T(0);
   const T* kc = kp + (in ? c : 0);
   switch (w) {
-    case 0: sym_warp<0, T>(sm, kc, ncp); break;
-    case 1: sym_warp<1, T>(sm, kc, ncp); break;
-    case 2: sym_warp<2, T>(sm, kc, ncp); break;
-    case 3: sym_warp<3, T>(sm, kc, ncp); break;
-    case 4: sym_warp<4, T>(sm, kc, ncp); break;
-    case 5: sym_warp<5, T>(sm, kc, ncp); break;
-    case 6: sym_warp<6, T>(sm, kc, ncp); break;
-    default: sym_warp<7, T>(sm, kc, ncp); break;
+    case 0: sym_warp<0, T>(sm, kc, ncp, u + n, cs, in); break;
+    case 1: sym_warp<1, T>(sm, kc, ncp, u + n, cs, in); break;
+    case 2: sym_warp<2, T>(sm, kc, ncp, u + n, cs, in); break;
+    case 3: sym_warp<3, T>(sm, kc, ncp, u + n, cs, in); break;
+    case 4: sym_warp<4, T>(sm, kc, ncp, u + n, cs, in); break;
+    case 5: sym_warp<5, T>(sm, kc, ncp, u + n, cs, in); break;
+    case 6: sym_warp<6, T>(sm, kc, ncp, u + n, cs, in); break;
+    default: sym_warp<7, T>(sm, kc, ncp, u + n, cs, in); break;
   }
   __syncthreads();
   if (!in) return;
@@ -1156,19 +1159,28 @@ __device__ __forceinline__ void walsh8(float (&a)[8]) {
       }
 }
 
-// ft (24, cells) = T^T (K^ (T u_c)) for every cell (listed cells are rewritten afterwards)
+// ft (24, cells) = T^T (K^ (T u_c)) for every cell (listed cells are rewritten afterwards). The matrices
+// are older than the launch ahead (lpb_pack_modal_f32 sees to it), so a cell's first MODAL_AHEAD entries
+// are loaded while that launch still runs; u is read after it.
+constexpr int MODAL_AHEAD = 64;
 __device__ __forceinline__ void modal_cell(float* __restrict__ ft, const float* __restrict__ u,
                                            const float* __restrict__ km, const LpGrid& g, long long t) {
   const long long ncp = g.cells_padded();
   const long long cs = g.comp_stride();
-  if (t >= ncp) return;
   int x, y, z;
-  if (!g.cell_at(t, x, y, z)) return;
-  if (isnan(__ldg(km + t))) return;                // a listed cell (its entry 0 holds the marker)
-  const long long n0 = g.node(x, y, z);
-  const long long oy = 4LL * g.NX(), oz = (z & 3) == 3 ? g.node_zc_stride() - 3 : 1;
+  const bool on = t < ncp && g.cell_at(t, x, y, z);
   constexpr int MUP_R[MODAL_UP] = MUP_ROWS;
   constexpr int MUP_C[MODAL_UP] = MUP_COLS;
+  const float* kc = km + t;
+  float ahead[MODAL_AHEAD];
+  if (on)
+#pragma unroll
+    for (int p = 0; p < MODAL_AHEAD; ++p) ahead[p] = __ldg(kc + (long long)p * ncp);
+  lp_wait_prior();
+  lp_release_next();
+  if (!on || isnan(ahead[0])) return;              // a listed cell's entry 0 holds the marker
+  const long long n0 = g.node(x, y, z);
+  const long long oy = 4LL * g.NX(), oz = (z & 3) == 3 ? g.node_zc_stride() - 3 : 1;
   float uh[24], fh[24];
 #pragma unroll
   for (int cc = 0; cc < 3; ++cc) {
@@ -1182,10 +1194,9 @@ __device__ __forceinline__ void modal_cell(float* __restrict__ ft, const float* 
   }
 #pragma unroll
   for (int r = 0; r < 24; ++r) fh[r] = 0.0f;
-  const float* kc = km + t;
 #pragma unroll
   for (int p = 0; p < MODAL_UP; ++p) {
-    const float v = __ldg(kc + (long long)p * ncp);
+    const float v = p < MODAL_AHEAD ? ahead[p < MODAL_AHEAD ? p : 0] : __ldg(kc + (long long)p * ncp);
     fh[MUP_R[p]] += v * uh[MUP_C[p]];
     if (MUP_R[p] != MUP_C[p]) fh[MUP_C[p]] += v * uh[MUP_R[p]];
   }
@@ -1241,7 +1252,6 @@ __global__ void __launch_bounds__(128, 4) k_explicit_modal_cells(float* __restri
                                                                 const int* __restrict__ glist,
                                                                 const int* __restrict__ gcount, LpGrid g,
                                                                 int modal_blocks) {
-  lp_after_launch();
   ft += 24 * g.cells_padded() * blockIdx.y;   // the column
   u += 3 * g.comp_stride() * blockIdx.y;
   __shared__ float sk[4][300];
@@ -1249,9 +1259,14 @@ __global__ void __launch_bounds__(128, 4) k_explicit_modal_cells(float* __restri
   if ((int)blockIdx.x < modal_blocks) {
     modal_cell(ft, u, km, g, blockIdx.x * (long long)blockDim.x + threadIdx.x);
   } else {
+    lp_after_launch();
     listed_cells(ft, u, kpc, glist, gcount, g, blockIdx.x - modal_blocks, gridDim.x - modal_blocks, sk, su);
   }
 }
+
+// nothing: a launch of its own behind lpb_pack_modal_f32's and lpb_pack_sym_*'s, after which that one is complete for whatever is
+// launched next, started early or not
+__global__ void k_settled() { lp_after_launch(); }
 
 template <typename T>
 __global__ void k_explicit_gather(T* __restrict__ out, const T* __restrict__ ft, const uint8_t* __restrict__ mask,
@@ -1294,41 +1309,53 @@ struct ChebArgs {
 };
 
 template <typename T, int MODE>
-__global__ void k_explicit_gather_cheb(const T* __restrict__ ft, const uint8_t* __restrict__ mask, LpGrid g,
-                                       ChebArgs<T> a) {
-  lp_after_launch();
-  const long long total = g.nodes_padded();
+__global__ void __launch_bounds__(128)
+k_explicit_gather_cheb(const T* __restrict__ ft, const uint8_t* __restrict__ mask, LpGrid g, ChebArgs<T> a) {
   const long long ncp = g.cells_padded(), cs = g.comp_stride(), co = 3 * cs * blockIdx.y;
   ft += 24 * ncp * blockIdx.y;   // the column
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  int x, y, z;
+  const bool on = t < g.nodes_padded() && g.node_at(t, x, y, z);
   const T s = (T)a.coef[1], c1 = (T)a.coef[2], c2 = (T)a.coef[3];
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    int x, y, z;
-    if (!g.node_at(t, x, y, z)) continue;
-    T acc[3] = {T(0), T(0), T(0)};
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int cx = x - cx_(k), cy = y - cy_(k), cz = z - cz_(k);
-      if (cx < 0 || cy < 0 || cz < 0 || cx >= g.nx || cy >= g.ny || cz >= g.nz) continue;
-      const long long c = g.cell(cx, cy, cz);
-#pragma unroll
-      for (int cc = 0; cc < 3; ++cc) acc[cc] += ft[(long long)(3 * k + cc) * ncp + c];
-    }
-    const long long n = g.node(x, y, z);
-    const uint8_t mb = mask[n];
+  // all but the cells' forces was complete before the launch ahead (the cells')
+  uint8_t mb = 0;
+  T dv[3], v0[3], v1[3], v2[3];   // mode 1: d, b; mode 2: b; mode 3: x, d, r
+  if (on) {
+    mb = mask[t];
 #pragma unroll
     for (int cc = 0; cc < 3; ++cc) {
-      const long long i = co + cc * cs + n;
-      const T adi = ((mb >> cc) & 1) ? acc[cc] : T(0);
-      if (MODE == 1) {
-        a.x[i] = lp_cheb2_zero_v(a.d[i], a.b[i], adi, a.dinv[i - co], c1, c2);
-      } else if (MODE == 2) {
-        T ri, di;
-        lp_residual_scaled_v(a.b[i], adi, a.dinv[i - co], s, ri, di);
-        a.r[i] = ri;
-        a.d[i] = di;
-      } else {
-        a.x[i] = lp_cheb2_v(a.x[i], a.d[i], a.r[i], adi, a.dinv[i - co], c1, c2);
-      }
+      const long long i = co + cc * cs + t;
+      dv[cc] = a.dinv[i - co];
+      v0[cc] = MODE == 1 ? a.d[i] : MODE == 2 ? a.b[i] : a.x[i];
+      if (MODE != 2) v1[cc] = MODE == 1 ? a.b[i] : a.d[i];
+      if (MODE == 3) v2[cc] = a.r[i];
+    }
+  }
+  lp_wait_prior();
+  lp_release_next();
+  if (!on) return;
+  T acc[3] = {T(0), T(0), T(0)};
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int cx = x - cx_(k), cy = y - cy_(k), cz = z - cz_(k);
+    if (cx < 0 || cy < 0 || cz < 0 || cx >= g.nx || cy >= g.ny || cz >= g.nz) continue;
+    const long long c = g.cell(cx, cy, cz);
+#pragma unroll
+    for (int cc = 0; cc < 3; ++cc) acc[cc] += ft[(long long)(3 * k + cc) * ncp + c];
+  }
+#pragma unroll
+  for (int cc = 0; cc < 3; ++cc) {
+    const long long i = co + cc * cs + t;
+    const T adi = ((mb >> cc) & 1) ? acc[cc] : T(0);
+    if (MODE == 1) {
+      a.x[i] = lp_cheb2_zero_v(v0[cc], v1[cc], adi, dv[cc], c1, c2);
+    } else if (MODE == 2) {
+      T ri, di;
+      lp_residual_scaled_v(v0[cc], adi, dv[cc], s, ri, di);
+      a.r[i] = ri;
+      a.d[i] = di;
+    } else {
+      a.x[i] = lp_cheb2_v(v0[cc], v1[cc], v2[cc], adi, dv[cc], c1, c2);
     }
   }
 }
@@ -1471,15 +1498,33 @@ static int apply_level1(int mode, T* out, T* x, T* r, T* d, const T* u, const T*
 }
 
 template <typename T>
-static int launch_explicit(T* out, const T* u, const T* kp, T* ft, const uint8_t* mask, LpGrid g, cudaStream_t st) {
-  if (!lp_grid_ok(g) || !out || !u || !kp || !ft || !mask || out == u) return LP_ERR_ARG;
+static int launch_explicit(T* out, const T* u, const T* kp, T* ft, const uint8_t* mask, LpGrid g, cudaStream_t st,
+                           int mode = 0, const ChebArgs<T>* ch = nullptr) {
+  if (!lp_grid_ok(g) || !u || !kp || !ft || !mask) return LP_ERR_ARG;
+  if (mode == 0 && (!out || out == u)) return LP_ERR_ARG;
   constexpr int smem = (int)sizeof(ExCells<T>);   // above the 48 KB default in float64
   if (cudaFuncSetAttribute(k_explicit_cells<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return LP_ERR_LAUNCH;
   lp_launch(k_explicit_cells<T>, lp_blocks(g.cells_padded(), 32), 32 * EX_WARPS, smem, st, ft, u, kp, g);
-  lp_launch(k_explicit_gather<T>, lp_blocks(g.nodes_padded(), 256), 256, 0, st, out, ft, mask, g);
+  if (mode == 0) {
+    lp_launch(k_explicit_gather<T>, lp_blocks(g.nodes_padded(), 256), 256, 0, st, out, ft, mask, g);
+  } else {
+    const ChebArgs<T> a = *ch;
+    const int nb = lp_blocks(g.nodes_padded(), 128);
+    if (mode == 1) lp_launch(k_explicit_gather_cheb<T, 1>, nb, 128, 0, st, ft, mask, g, a);
+    else if (mode == 2) lp_launch(k_explicit_gather_cheb<T, 2>, nb, 128, 0, st, ft, mask, g, a);
+    else lp_launch(k_explicit_gather_cheb<T, 3>, nb, 128, 0, st, ft, mask, g, a);
+  }
   LP_LAUNCH_CHECK();
   return LP_OK;
+}
+
+template <typename T>
+static bool explicit_cheb_ok(int mode, const ChebArgs<T>& a, const T* u) {
+  if (mode < 1 || mode > 3 || !a.dinv || !a.coef) return false;
+  if (mode == 1) return a.x && a.d && a.b && u == a.d && a.x != a.d;
+  if (mode == 2) return a.r && a.d && a.b && u != a.r && u != a.d && a.r != a.d;
+  return a.x && a.d && a.r && u == a.d && a.x != a.d;
 }
 
 static int launch_explicit_modal(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b,
@@ -1489,20 +1534,16 @@ static int launch_explicit_modal(int mode, float* out, float* x, float* r, float
   if (!lp_grid_ok(g) || !u || !km || !kpc || !glist || !gcount || !ft || !mask) return LP_ERR_ARG;
   if (cols < 1 || cols > 65535) return LP_ERR_ARG;
   if (mode == 0 && (!out || out == u)) return LP_ERR_ARG;
-  if (mode != 0 && (!dinv || !coef)) return LP_ERR_ARG;
-  if (mode == 1 && (!x || !d || !b || u != d || x == d)) return LP_ERR_ARG;
-  if (mode == 2 && (!r || !d || !b || u == r || u == d || r == d)) return LP_ERR_ARG;
-  if (mode == 3 && (!x || !d || !r || u != d || x == d)) return LP_ERR_ARG;
-  if (mode < 0 || mode > 3) return LP_ERR_ARG;
+  const ChebArgs<float> a{x, r, d, b, dinv, coef};
+  if (mode != 0 && !explicit_cheb_ok(mode, a, u)) return LP_ERR_ARG;
   const int modal_blocks = lp_blocks(g.cells_padded(), 128);
   lp_launch(k_explicit_modal_cells, dim3(modal_blocks + 148, cols), 128, 0, st, ft, u, km, kpc, glist, gcount, g,
             modal_blocks);
-  const ChebArgs<float> a{x, r, d, b, dinv, coef};
-  const dim3 nb(lp_blocks(g.nodes_padded(), 256), cols);
+  const dim3 nb(lp_blocks(g.nodes_padded(), 256), cols), nbc(lp_blocks(g.nodes_padded(), 128), cols);
   if (mode == 0) lp_launch(k_explicit_gather<float>, nb, 256, 0, st, out, ft, mask, g);
-  else if (mode == 1) lp_launch(k_explicit_gather_cheb<float, 1>, nb, 256, 0, st, ft, mask, g, a);
-  else if (mode == 2) lp_launch(k_explicit_gather_cheb<float, 2>, nb, 256, 0, st, ft, mask, g, a);
-  else lp_launch(k_explicit_gather_cheb<float, 3>, nb, 256, 0, st, ft, mask, g, a);
+  else if (mode == 1) lp_launch(k_explicit_gather_cheb<float, 1>, nbc, 128, 0, st, ft, mask, g, a);
+  else if (mode == 2) lp_launch(k_explicit_gather_cheb<float, 2>, nbc, 128, 0, st, ft, mask, g, a);
+  else lp_launch(k_explicit_gather_cheb<float, 3>, nbc, 128, 0, st, ft, mask, g, a);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -1688,6 +1729,16 @@ int lpb_apply_explicit_sym_f64(double* out, const double* u, const double* kp, d
   return launch_explicit<double>(out, u, kp, ft, mask, LP_GRID, LP_ST);
 }
 
+// lpb_apply_explicit_sym_f64 with a degree-2 Chebyshev update in its gather (modes 1..3, as
+// lpb_apply_explicit_modal_cheb_f32)
+int lpb_apply_explicit_sym_cheb_f64(int mode, double* x, double* r, double* d, const double* u, const double* b,
+                                    const double* dinv, const double* coef, const double* kp, double* ft,
+                                    const uint8_t* mask, LP_GRID_ARGS, void* stream) {
+  const ChebArgs<double> a{x, r, d, b, dinv, coef};
+  if (!explicit_cheb_ok(mode, a, u)) return LP_ERR_ARG;
+  return launch_explicit<double>(nullptr, u, kp, ft, mask, LP_GRID, LP_ST, mode, &a);
+}
+
 // lpb_apply_explicit_sym_f32 with its (24, cells) scratch in the library's static array: no
 // allocation by the caller or the library. Grids with more than LP_NOALLOC_MAX_CELLS padded
 // cells return LP_ERR_SIZE. The first call on a device looks the array's address up (it should
@@ -1715,6 +1766,7 @@ int lpb_pack_modal_f32(float* km, int* glist, int* gcount, float* kpc, const flo
   const long long blocks = (ncells + 3) / 4;
   lp_launch(k_pack_modal<float>, (unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 128, 0, LP_ST, km, glist, gcount, kpc,
                                                                                           k, ncells, tol);
+  lp_launch(k_settled, 1, 32, 0, LP_ST);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -1753,6 +1805,7 @@ int lpb_apply_explicit_modal_cols_f32(int mode, float* out, float* x, float* r, 
 int lpb_pack_sym_f32(float* kp, const float* k, long long ncells, void* stream) {
   if (!kp || !k || ncells < 0) return LP_ERR_ARG;
   lp_launch(k_pack_sym<float, float>, lp_blocks(300 * ncells, 256), 256, 0, LP_ST, kp, k, ncells);
+  lp_launch(k_settled, 1, 32, 0, LP_ST);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -1760,6 +1813,7 @@ int lpb_pack_sym_f32(float* kp, const float* k, long long ncells, void* stream) 
 int lpb_pack_sym_f64(double* kp, const double* k, long long ncells, void* stream) {
   if (!kp || !k || ncells < 0) return LP_ERR_ARG;
   lp_launch(k_pack_sym<double, double>, lp_blocks(300 * ncells, 256), 256, 0, LP_ST, kp, k, ncells);
+  lp_launch(k_settled, 1, 32, 0, LP_ST);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }

@@ -206,6 +206,10 @@ __device__ __forceinline__ void lp_after_launch() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// The two halves, for a kernel whose launch ahead is always one of the library's own that begins with
+// lp_after_launch: what was complete when that one began may be read before lp_wait_prior.
+__device__ __forceinline__ void lp_release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void lp_wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... P, typename... A>
 static inline void lp_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchAttribute attr[1];

@@ -757,8 +757,14 @@ void smooth(Mg& m, int i, const void* b, void* x, bool from_zero, bool started =
     }
     return;
   }
-  if (lv.kind == K_EXPLICIT && lv.km) {
+  if (lv.kind == K_EXPLICIT && (lv.km || !f)) {
     auto fused = [&](int mode, const void* u) {
+      if (!lv.km) {
+        m.ok(lpb_apply_explicit_sym_cheb_f64(mode, (double*)x, (double*)r, (double*)d, (const double*)u, (const double*)b,
+                                             (const double*)lv.dinv, coef, (const double*)lv.kp, (double*)lv.ft, lv.mask,
+                                             HG(g), m.st));
+        return;
+      }
       m.ok(lpb_apply_explicit_modal_cheb_f32(mode, (float*)x, (float*)r, (float*)d, (const float*)u, (const float*)b,
                                              (const float*)lv.dinv, coef, (const float*)lv.km, (const float*)lv.kpc,
                                              lv.glist, lv.gcount, (float*)lv.ft, lv.mask, HG(g), m.st));

@@ -65,11 +65,19 @@ class DevGrid:
     def node_field(self, dtype) -> torch.Tensor:
         return torch.zeros((3, self.pz // 4, self.NY, self.NX, 4), dtype=dtype, device=self.device)
 
+    def node_empty(self, dtype) -> torch.Tensor:
+        """A node field for a pass that writes all of it, the padding included."""
+        return torch.empty((3, self.pz // 4, self.NY, self.NX, 4), dtype=dtype, device=self.device)
+
     def cell_field(self, dtype) -> torch.Tensor:
         return torch.zeros((self.cpz // 4, self.ny, self.nx, 4), dtype=dtype, device=self.device)
 
+    @property
+    def mask_shape(self):
+        return (self.pz // 4, self.NY, self.NX, 4)
+
     def mask_field(self) -> torch.Tensor:
-        return torch.zeros((self.pz // 4, self.NY, self.NX, 4), dtype=torch.uint8, device=self.device)
+        return torch.zeros(self.mask_shape, dtype=torch.uint8, device=self.device)
 
     # layout <-> grid order (torch, on either side) ---------------------------------------
     def node_grid(self, t: torch.Tensor) -> torch.Tensor:

@@ -513,7 +513,7 @@ class GridElasticity:
         l0.err = self._err
         d0 = self._buf("diag0", g0, torch.float64)
         L.lpb_diag_scaled_f64(d0.data_ptr(), e_dev.data_ptr(), self.ke64.data_ptr(), *g0.args, st)
-        l0.mask = self._tbuf("mask0", g0.mask_field().shape, torch.uint8)
+        l0.mask = self._tbuf("mask0", g0.mask_shape, torch.uint8)
         l0.dinv = self._buf("dinv0_64", g0, torch.float64)
         dinv32 = self._buf("dinv0_32", g0, torch.float32) if dt == torch.float32 else None
         L.lpb_masks(l0.mask.data_ptr(), l0.dinv.data_ptr(), ptr(dinv32), d0.data_ptr(), self.fixed_bits.data_ptr(),
@@ -556,12 +556,12 @@ class GridElasticity:
             L.lpb_max_f64(d.data_ptr(), d.numel(), part.data_ptr(), chk[40 + depth:].data_ptr(), st)
             held_c = kept = None
             if self.strict:
-                held_c = self._tbuf(f"held{depth}", gc.mask_field().shape, torch.uint8)
+                held_c = self._tbuf(f"held{depth}", gc.mask_shape, torch.uint8)
                 kept = self._buf(f"kept{depth}", gc, torch.float32)
                 L.lpb_strict_held_kept(held_c.data_ptr(), kept.data_ptr(), held.data_ptr(), fine.mask.data_ptr(),
                                        *fine.grid.args, *gc.args, st)
                 held = held_c
-            coarse.mask = self._tbuf(f"mask{depth}", gc.mask_field().shape, torch.uint8)
+            coarse.mask = self._tbuf(f"mask{depth}", gc.mask_shape, torch.uint8)
             coarse.dinv = self._buf(f"dinv{depth}", gc, dt)
             d64 = coarse.dinv if dt == torch.float64 else None
             d32 = coarse.dinv if dt == torch.float32 else None
@@ -974,9 +974,14 @@ class GridElasticity:
                 fused(2, x)
                 fused(3, d)
             return x
-        if self.degree == 2 and lv.kind == "explicit" and lv.km is not None:
+        if self.degree == 2 and lv.kind == "explicit" and (lv.km is not None or (lv.kp is not None and sfx == "f64")):
             # the explicit levels form each update in the gather of A u (the same expressions)
             def fused(mode, u):
+                if lv.km is None:
+                    L.lpb_apply_explicit_sym_cheb_f64(mode, x.data_ptr(), r.data_ptr(), d.data_ptr(), u.data_ptr(),
+                                                      b.data_ptr(), lv.dinv.data_ptr(), coef, lv.kp.data_ptr(),
+                                                      lv.ft.data_ptr(), lv.mask.data_ptr(), *g.args, st)
+                    return
                 L.lpb_apply_explicit_modal_cheb_f32(mode, x.data_ptr(), r.data_ptr(), d.data_ptr(), u.data_ptr(),
                                                     b.data_ptr(), lv.dinv.data_ptr(), coef, lv.km.data_ptr(),
                                                     lv.kpc.data_ptr(), lv.glist.data_ptr(), lv.gcount.data_ptr(),
@@ -1357,7 +1362,7 @@ class GridElasticity:
         if not ok:
             raise RuntimeError(f"linear solve did not converge ({it} iterations); "
                                "the structure may be a mechanism (check supports)")
-        out = g.node_field(torch.float64)
+        out = g.node_empty(torch.float64)
         L.lpb_mask_field_f64(out.data_ptr(), x.data_ptr(), m.data_ptr(), *g.args, 0, st)
         return out
 
@@ -1401,8 +1406,8 @@ class GridElasticity:
         """Whether level i's smoothing of k columns runs with the columns in one launch (float32,
         degree 2): a small grid's launches are a few us whatever they hold, so k columns cost
         little more than one (a step with 8 loads on 96 x 48 x 48 cells: 39.2 ms with the columns
-        launched one after the other, 17.2 ms so). Where the columns' r, d and t would take over 1 GiB, one column fills the GPU by
-        itself, and the columns take turns in one set of them."""
+        launched one after the other, 17.2 ms so). Where the columns' r, d and t would take over
+        1 GiB, one column fills the GPU by itself, and the columns take turns in one set of them."""
         lv = self._op(i)
         return (self.smoother != "jacobi" and self.degree == 2 and lv.dtype == torch.float32
                 and lv.kind in ("scaled", "weights", "explicit") and (lv.kind != "explicit" or lv.km is not None)
@@ -1715,11 +1720,11 @@ class GridElasticity:
         x0s = list(x0s) if x0s is not None else [None] * k
         bm, x0m, outs = [], [], []
         for j in range(k):
-            b = g.node_field(torch.float64)
+            b = g.node_empty(torch.float64)
             L.lpb_mask_field_f64(b.data_ptr(), bs[j].data_ptr(), m.data_ptr(), *g.args, 0, st)
             bm.append(b)
             if x0s[j] is not None:
-                x0 = g.node_field(torch.float64)
+                x0 = g.node_empty(torch.float64)
                 L.lpb_mask_field_f64(x0.data_ptr(), x0s[j].data_ptr(), m.data_ptr(), *g.args, 0, st)
                 x0m.append(x0)
             else:

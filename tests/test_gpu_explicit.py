@@ -89,3 +89,54 @@ def test_explicit_apply(dims, dtype):
     want = _assembled(kk, u, dims)
     err = np.abs(g.nodes_to_host(out) - want).max()
     assert err <= 1.3e-3 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (11, 3, 4), (8, 4, 12)])
+def test_float64_updates_match_two_launches(dims):
+    """The Chebyshev updates in the float64 gather, to the bit as the apply and the vector kernel."""
+    from loadpath_b200._lib import lib
+    from loadpath_b200.grid import DevGrid
+
+    L, st = lib(), torch.cuda.current_stream().cuda_stream
+    rng = np.random.default_rng(sum(dims))
+    g = DevGrid(dims)
+    k = rng.standard_normal(dims + (24, 24))
+    kd = _cells_dev(g, k + np.swapaxes(k, -1, -2), torch.float64)
+    ncp = kd.shape[0]
+    kp = torch.empty(300, ncp, device="cuda", dtype=torch.float64)
+    ft = torch.empty(24, ncp, device="cuda", dtype=torch.float64)
+    L.lpb_pack_sym_f64(kp.data_ptr(), kd.data_ptr(), ncp, st)
+    b, d0, x0, r0, dinv = (g.nodes_to_dev(rng.standard_normal(g.node_shape), torch.float64) for _ in range(5))
+    mask = torch.randint(0, 8, b.shape[1:], device="cuda", dtype=torch.uint8)
+    coef = torch.rand(16, device="cuda", dtype=torch.float64)
+    n = b.numel()
+
+    def fused(mode, x, r, d, u):
+        assert L.lpb_apply_explicit_sym_cheb_f64(mode, x.data_ptr(), r.data_ptr(), d.data_ptr(), u.data_ptr(),
+                                                 b.data_ptr(), dinv.data_ptr(), coef.data_ptr(), kp.data_ptr(),
+                                                 ft.data_ptr(), mask.data_ptr(), *g.args, st) == 0
+
+    def apply(u):
+        t = torch.zeros_like(u)
+        L.lpb_apply_explicit_sym_f64(t.data_ptr(), u.data_ptr(), kp.data_ptr(), ft.data_ptr(), mask.data_ptr(), *g.args, st)
+        return t
+
+    def same(a, w):   # (the padding aside: the fused form leaves it)
+        assert np.array_equal(g.nodes_to_host(a), g.nodes_to_host(w))
+
+    xa, xb = x0.clone(), x0.clone()
+    fused(1, xa, r0.clone(), d0, d0)
+    L.lpb_cheb2_zero_f64(xb.data_ptr(), b.data_ptr(), apply(d0).data_ptr(), d0.data_ptr(), dinv.data_ptr(),
+                         coef.data_ptr(), n, st)
+    same(xa, xb)
+    ra, da, rb, db = r0.clone(), d0.clone(), r0.clone(), d0.clone()
+    fused(2, x0, ra, da, x0)
+    L.lpb_residual_scaled_f64(b.data_ptr(), apply(x0).data_ptr(), dinv.data_ptr(), coef.data_ptr(), rb.data_ptr(),
+                              db.data_ptr(), n, st)
+    same(ra, rb)
+    same(da, db)
+    xa, xb = x0.clone(), x0.clone()
+    fused(3, xa, r0, d0, d0)
+    L.lpb_cheb2_f64(xb.data_ptr(), d0.data_ptr(), r0.data_ptr(), apply(d0).data_ptr(), dinv.data_ptr(),
+                    coef.data_ptr(), n, st)
+    same(xa, xb)
