@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(TXC * TYC, (sizeof(T) == 4 ? 2 : 1))
 k_apply_fine(const __grid_constant__ FineMaps maps, T* __restrict__ out, const uint8_t* __restrict__ mask,
              const KSym<T> ks, LpGrid g, int nchunks, int* __restrict__ err, const FineCheb ch,
              double* __restrict__ dotp) {
-  lp_after_launch();
+  // nothing global is touched before lp_after_launch: the set-up overlaps the launch ahead
   typedef PairOps<T> O;
   typedef Pair<T> P;
   extern __shared__ unsigned char smem_raw[];
@@ -309,6 +309,7 @@ k_apply_fine(const __grid_constant__ FineMaps maps, T* __restrict__ out, const u
   constexpr uint32_t UBYTES = 3 * BOX * BOX * 4 * sizeof(T);
   constexpr uint32_t EBYTES = TXC * TYC * 4 * sizeof(T);
   if (u0 >= u1) {
+    lp_after_launch();
     if (dotp && tid == 0) dotp[blockIdx.x] = 0.0;
     return;
   }
@@ -335,14 +336,9 @@ k_apply_fine(const __grid_constant__ FineMaps maps, T* __restrict__ out, const u
   }
   __syncthreads();
   if (bad) {
+    lp_after_launch();
     if (dotp && tid == 0) dotp[blockIdx.x] = 0.0;
     return;
-  }
-  float cs_s = 0.0f, cs_c1 = 0.0f, cs_c2 = 0.0f;
-  if constexpr (MODE != 0) {
-    cs_s = (float)ch.coef[1];
-    cs_c1 = (float)ch.coef[2];
-    cs_c2 = (float)ch.coef[3];
   }
   // the producer (thread 0) walks the block's loads: its segment, the loads issued in it and in all
   int total = 0;
@@ -359,6 +355,13 @@ k_apply_fine(const __grid_constant__ FineMaps maps, T* __restrict__ out, const u
     lp_fence_barrier_init();
   }
   __syncthreads();
+  lp_after_launch();
+  float cs_s = 0.0f, cs_c1 = 0.0f, cs_c2 = 0.0f;
+  if constexpr (MODE != 0) {
+    cs_s = (float)ch.coef[1];
+    cs_c1 = (float)ch.coef[2];
+    cs_c2 = (float)ch.coef[3];
+  }
   auto issue_next = [&]() {
     if (pk == ps.nload) {
       pu += ps.ce - ps.cb;

@@ -545,12 +545,14 @@ __global__ void __launch_bounds__(256) k_chain_schur(double* __restrict__ ws, co
 constexpr int ROW_AHEAD = 8;
 struct RowAhead {
   double2 x[ROW_AHEAD];
+  template <bool EARLY = false>   // EARLY: before lp_wait_prior
   __device__ __forceinline__ void load(const double* __restrict__ a, int k0, int n) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int u = 0; u < ROW_AHEAD; ++u) {
       const int k = k0 + 64 * u + 2 * lane;
-      x[u] = k < n ? __ldg(reinterpret_cast<const double2*>(a + k)) : make_double2(0.0, 0.0);
+      const double2* p = reinterpret_cast<const double2*>(a + k);
+      x[u] = k < n ? (EARLY ? __ldcg(p) : __ldg(p)) : make_double2(0.0, 0.0);
     }
   }
   // s[c] += row . v_c over the loaded entries (v_c: NC shared vectors at stride vs); n even
@@ -592,10 +594,13 @@ constexpr int SOLVE_ROWS = 8;   // rows per block, one per warp
 constexpr int SEG_ROWS = 16;    // rows of a segment's inverse per block, two per warp: half as many blocks stage b
 
 // rows of y = A_I^-1 b_I (blocks of each segment in turn), then of g = b_s - W^T b_I
+// nothing: behind the factor's launches, so that they are complete for whatever is launched next, started
+// early or not
+__global__ void k_chain_settled() { lp_after_launch(); }
+
 template <typename T, int NC>
 __global__ void __launch_bounds__(256) k_chain_y(double* __restrict__ ws, const T* __restrict__ f, long long cstride,
                                                  Chain c) {
-  lp_after_launch();
   extern __shared__ __align__(16) unsigned char sv_raw[];
   double* v = reinterpret_cast<double*>(sv_raw);   // [2][NC][M]
   const int* idx = reinterpret_cast<const int*>(ws + c.idx);
@@ -619,8 +624,9 @@ __global__ void __launch_bounds__(256) k_chain_y(double* __restrict__ ws, const 
     const double* a0 = ws + c.ai + ((long long)j * c.M + min(r, m - 1)) * c.M;
     const double* a1 = ws + c.ai + ((long long)j * c.M + min(r + 1, m - 1)) * c.M;
     RowAhead h0, h1;
-    h0.load(a0, 0, n);
-    h1.load(a1, 0, n);
+    h0.load<true>(a0, 0, n);
+    h1.load<true>(a1, 0, n);   // (the matrices are older than the launch ahead: lpb_chain_factor sees to it)
+    lp_after_launch();
     stage(v, j);
     __syncthreads();
     if (r >= m) return;
@@ -644,8 +650,9 @@ __global__ void __launch_bounds__(256) k_chain_y(double* __restrict__ ws, const 
   const double* wr = ws + c.wt + (2LL * (k + 1) * c.b + rr) * c.M;       // segment k + 1, its left separator
   const int nl = (c.size(k) + 1) & ~1, nr = (c.size(k + 1) + 1) & ~1;
   RowAhead hl, hr;
-  hl.load(wl, 0, nl);
-  hr.load(wr, 0, nr);
+  hl.load<true>(wl, 0, nl);
+  hr.load<true>(wr, 0, nr);
+  lp_after_launch();
   stage(v, k);
   stage(v + NC * c.M, k + 1);
   __syncthreads();
@@ -669,7 +676,7 @@ __global__ void __launch_bounds__(256) k_chain_s(double* __restrict__ ws, T* __r
   const int r = SOLVE_ROWS * blockIdx.x + w, n = (c.nS + 1) & ~1;
   const double* a = ws + c.s + (long long)min(r, c.nS - 1) * c.MS;
   RowAhead h;
-  h.load(a, 0, n);   // (the matrix was complete before the launch ahead, k_chain_y)
+  h.load<true>(a, 0, n);   // (the matrix was complete before the launch ahead, k_chain_y)
   lp_wait_prior();
   lp_release_next();
 #pragma unroll
@@ -705,7 +712,7 @@ __global__ void __launch_bounds__(256) k_chain_x(double* __restrict__ ws, T* __r
   const int r = SOLVE_ROWS * blk + w, n = 2 * c.b;
   const double* a = ws + c.w + ((long long)j * c.M + min(r, m - 1)) * n;
   RowAhead h;
-  h.load(a, 0, n);
+  h.load<true>(a, 0, n);
   lp_wait_prior();
   lp_release_next();
 #pragma unroll
@@ -805,7 +812,7 @@ long long lpb_chain_dims(int nx, int ny, int nz, long long* out) {
     out[1] = c.b;
     out[2] = c.M;
     out[3] = c.nS;
-    out[4] = 7 + (c.size(0) + 31) / 32 + (c.nS + 31) / 32;
+    out[4] = 8 + (c.size(0) + 31) / 32 + (c.nS + 31) / 32;
   }
   return c.total;
 }
@@ -841,7 +848,11 @@ int lpb_chain_factor(double* ws, const double* t, int* info, LP_GRID_ARGS, void*
   job.n = 1;
   job.diag = ws + c.diag + (long long)c.P * c.M;
   job.steps[0] = (short)((c.nS + 31) / 32);
-  return sweep_all(job, LP_ST);
+  rc = sweep_all(job, LP_ST);
+  if (rc != LP_OK) return rc;
+  lp_launch(k_chain_settled, 1, 32, 0, LP_ST);
+  LP_LAUNCH_CHECK();
+  return LP_OK;
 }
 
 // f_out = A^-1 f_in on the coarsest level from lpb_chain_factor's ws (whose solve scratch it uses: solves

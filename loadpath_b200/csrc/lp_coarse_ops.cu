@@ -614,7 +614,7 @@ k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split sp
          const T* __restrict__ wc, const int* __restrict__ pid, const T* __restrict__ pm,
          const uint8_t* __restrict__ mask, const __grid_constant__ G1<T> gc, LpGrid g, int nchunks, int* __restrict__ err,
          const L1Cheb<T> ch, const L1Box pbox) {
-  lp_after_launch();
+  // nothing global is touched before lp_after_launch: the set-up overlaps the launch ahead
   extern __shared__ unsigned char wsm_raw[];
   const uint32_t raw_off = lp_smem_addr(wsm_raw);
   L1Smem<T>& sm = *reinterpret_cast<L1Smem<T>*>(wsm_raw + ((1024u - (raw_off & 1023u)) & 1023u));
@@ -625,7 +625,10 @@ k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split sp
   const long long u0 = split.u0[blockIdx.x], u1 = split.u0[blockIdx.x + 1];
   constexpr uint32_t UBYTES = 3 * LBX * LBY * 4 * sizeof(T);
   constexpr uint32_t WBYTES = staged_w ? 32 * LCOL * sizeof(T) : 0;
-  if (u0 >= u1) return;
+  if (u0 >= u1) {
+    lp_after_launch();
+    return;
+  }
   __shared__ int bad;
   if (tid == 0) {
     int code = 0;
@@ -648,12 +651,9 @@ k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split sp
     if (code) atomicExch(err, code);
   }
   __syncthreads();
-  if (bad) return;
-  T cs_s = T(0), cs_c1 = T(0), cs_c2 = T(0);
-  if constexpr (MODE != 0) {
-    cs_s = (T)ch.coef[1];
-    cs_c1 = (T)ch.coef[2];
-    cs_c2 = (T)ch.coef[3];
+  if (bad) {
+    lp_after_launch();
+    return;
   }
   // thread 0 issues the block's loads in order: its segment, the loads issued in it and in all
   int total = 0, issued = 0, pk = 0;
@@ -669,6 +669,13 @@ k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split sp
     lp_fence_barrier_init();
   }
   __syncthreads();
+  lp_after_launch();
+  T cs_s = T(0), cs_c1 = T(0), cs_c2 = T(0);
+  if constexpr (MODE != 0) {
+    cs_s = (T)ch.coef[1];
+    cs_c1 = (T)ch.coef[2];
+    cs_c2 = (T)ch.coef[3];
+  }
   auto issue_next = [&]() {
     if (pk == ps.nload) {
       pu += ps.ce - ps.cb;
@@ -973,7 +980,7 @@ template <int W, typename T>
 __device__ __forceinline__ void sym_part(const T* __restrict__ kc, long long ncp, T (&k)[38]) {
   constexpr int LO = 300 * W / EX_WARPS, HI = 300 * (W + 1) / EX_WARPS;
 #pragma unroll
-  for (int p = LO; p < HI; ++p) k[p - LO] = __ldg(kc + (long long)p * ncp);
+  for (int p = LO; p < HI; ++p) k[p - LO] = __ldcg(kc + (long long)p * ncp);
 }
 template <int W, typename T>
 __device__ __forceinline__ void sym_forces(const T (&k)[38], const T (&u)[24][32], T (&f)[24]) {
@@ -1175,7 +1182,7 @@ __device__ __forceinline__ void modal_cell(float* __restrict__ ft, const float* 
   float ahead[MODAL_AHEAD];
   if (on)
 #pragma unroll
-    for (int p = 0; p < MODAL_AHEAD; ++p) ahead[p] = __ldg(kc + (long long)p * ncp);
+    for (int p = 0; p < MODAL_AHEAD; ++p) ahead[p] = __ldcg(kc + (long long)p * ncp);
   lp_wait_prior();
   lp_release_next();
   if (!on || isnan(ahead[0])) return;              // a listed cell's entry 0 holds the marker
@@ -1316,19 +1323,19 @@ k_explicit_gather_cheb(const T* __restrict__ ft, const uint8_t* __restrict__ mas
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   int x, y, z;
   const bool on = t < g.nodes_padded() && g.node_at(t, x, y, z);
-  const T s = (T)a.coef[1], c1 = (T)a.coef[2], c2 = (T)a.coef[3];
+  const T s = (T)__ldcg(a.coef + 1), c1 = (T)__ldcg(a.coef + 2), c2 = (T)__ldcg(a.coef + 3);
   // all but the cells' forces was complete before the launch ahead (the cells')
   uint8_t mb = 0;
   T dv[3], v0[3], v1[3], v2[3];   // mode 1: d, b; mode 2: b; mode 3: x, d, r
   if (on) {
-    mb = mask[t];
+    mb = __ldcg(mask + t);
 #pragma unroll
     for (int cc = 0; cc < 3; ++cc) {
       const long long i = co + cc * cs + t;
-      dv[cc] = a.dinv[i - co];
-      v0[cc] = MODE == 1 ? a.d[i] : MODE == 2 ? a.b[i] : a.x[i];
-      if (MODE != 2) v1[cc] = MODE == 1 ? a.b[i] : a.d[i];
-      if (MODE == 3) v2[cc] = a.r[i];
+      dv[cc] = __ldcg(a.dinv + i - co);
+      v0[cc] = __ldcg((MODE == 1 ? a.d : MODE == 2 ? a.b : a.x) + i);
+      if (MODE != 2) v1[cc] = __ldcg((MODE == 1 ? a.b : a.d) + i);
+      if (MODE == 3) v2[cc] = __ldcg(a.r + i);
     }
   }
   lp_wait_prior();

@@ -207,7 +207,8 @@ __device__ __forceinline__ void lp_after_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 // The two halves, for a kernel whose launch ahead is always one of the library's own that begins with
-// lp_after_launch: what was complete when that one began may be read before lp_wait_prior.
+// lp_after_launch: what was complete when that one began may be read before lp_wait_prior, by loads that
+// pass the L1 by (__ldcg): only the wait makes sure that no line there is older.
 __device__ __forceinline__ void lp_release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void lp_wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... P, typename... A>
