@@ -86,17 +86,18 @@ int lpb_walsh_chunks_f32(float* wc, const float* w, int nx, int ny, int nz, int 
 int lpb_walsh_chunks_f64(double* wc, const double* w, int nx, int ny, int nz, int pz, int cpz, void* stream);
 int lpb_apply_weights_tma_f32(float* out, const float* u, const float* wc, const int* patch_id, const float* patch_k, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, void* stream);
 int lpb_apply_weights_tma_f64(double* out, const double* u, const double* wc, const int* patch_id, const double* patch_k, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, void* stream);
-/* The level-1 apply with its patch cells in the same launch (patch_m: lpb_patch_modal_* of patch_k, the
- * (npatch, 24, 24) matrices in the corner-parity basis): mode 0 out = m K u; modes 1..3
- * the Chebyshev updates of lpb_apply_fine_cheb_f32 formed where K u is stored (out not used; the
- * fields a mode does not name may be NULL). */
+/* The level-1 apply with its patch cells (patch_k, and patch_m: lpb_patch_modal_* of it, the (npatch, 24, 24)
+ * matrices in the corner-parity basis): mode 0 out = m K u; modes 1..3 the Chebyshev updates of
+ * lpb_apply_fine_cheb_f32 formed where K u is stored (the fields a mode does not name may be NULL).
+ * Small grids take the patch cells in a launch of their own behind the march; modes 1..3 do so only
+ * with out given, a field of scratch of its own (any content). */
 int lpb_patch_modal_f32(float* pm, const float* pk, long long npatch, void* stream);
 int lpb_patch_modal_f64(double* pm, const double* pk, long long npatch, void* stream);
-int lpb_apply_level1_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b, const float* dinv, const double* coef, const float* wc, const int* patch_id, const float* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, void* stream);
-int lpb_apply_level1_f64(int mode, double* out, double* x, double* r, double* d, const double* u, const double* b, const double* dinv, const double* coef, const double* wc, const int* patch_id, const double* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, void* stream);
+int lpb_apply_level1_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b, const float* dinv, const double* coef, const float* wc, const int* patch_id, const float* patch_m, const float* patch_k, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, void* stream);
+int lpb_apply_level1_f64(int mode, double* out, double* x, double* r, double* d, const double* u, const double* b, const double* dinv, const double* coef, const double* wc, const int* patch_id, const double* patch_m, const double* patch_k, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, void* stream);
 /* the same for cols columns */
-int lpb_apply_level1_cols_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b, const float* dinv, const double* coef, const float* wc, const int* patch_id, const float* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, int cols, void* stream);
-int lpb_apply_level1_cols_f64(int mode, double* out, double* x, double* r, double* d, const double* u, const double* b, const double* dinv, const double* coef, const double* wc, const int* patch_id, const double* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, int cols, void* stream);
+int lpb_apply_level1_cols_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b, const float* dinv, const double* coef, const float* wc, const int* patch_id, const float* patch_m, const float* patch_k, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, int cols, void* stream);
+int lpb_apply_level1_cols_f64(int mode, double* out, double* x, double* r, double* d, const double* u, const double* b, const double* dinv, const double* coef, const double* wc, const int* patch_id, const double* patch_m, const double* patch_k, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, int cols, void* stream);
 /* explicit levels in the cell's corner-parity basis: K^ = T K T^T / 64 has the level-1 pattern
  * (150 upper entries) at every level of the plain hierarchy; lpb_pack_modal_f32 stores them
  * (km: (150, cells)) and lists the cells with off-pattern weight (children with masked patch

@@ -477,6 +477,11 @@ struct L1Box {
   int x, hx, y, hy;
 };
 
+// nodes of columns [x, hx) x [y, hy) and chunks [c, hc) whose patch cells' part comes from k_patch_nodes
+struct L1Nodes {
+  int x, hx, y, hy, c, hc;
+};
+
 template <typename T>
 struct L1Cheb {
   T* x;
@@ -613,7 +618,7 @@ __global__ void __launch_bounds__(LCOL, 2)
 k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split split, T* __restrict__ out,
          const T* __restrict__ wc, const int* __restrict__ pid, const T* __restrict__ pm,
          const uint8_t* __restrict__ mask, const __grid_constant__ G1<T> gc, LpGrid g, int nchunks, int* __restrict__ err,
-         const L1Cheb<T> ch, const L1Box pbox) {
+         const L1Cheb<T> ch, const L1Box pbox, const L1Nodes apart) {
   // nothing global is touched before lp_after_launch: the set-up overlaps the launch ahead
   extern __shared__ unsigned char wsm_raw[];
   const uint32_t raw_off = lp_smem_addr(wsm_raw);
@@ -640,7 +645,7 @@ k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split sp
     if ((so & 127) || (staged_w && (sw & 1023))) code = 20;
     else if (staged_w && (reinterpret_cast<uintptr_t>(&maps.w) & 63)) code = 26;
     else if (reinterpret_cast<uintptr_t>(&maps.u) & 63) code = 21;
-    else if (MODE == 0 && (reinterpret_cast<uintptr_t>(out) & 15)) code = 22;
+    else if ((MODE == 0 || apart.hx > apart.x) && (reinterpret_cast<uintptr_t>(out) & 15)) code = 22;
     else if (MODE != 0 && ((reinterpret_cast<uintptr_t>(ch.x) | reinterpret_cast<uintptr_t>(ch.r) |
                             reinterpret_cast<uintptr_t>(ch.d) | reinterpret_cast<uintptr_t>(ch.b) |
                             reinterpret_cast<uintptr_t>(ch.dinv)) & 15)) code = 27;
@@ -706,6 +711,7 @@ k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split sp
     // the tile's cells reach into the box of the patch cells
     const bool tile_patches = pid && x0 - 1 < pbox.hx && x0 - 1 + LX > pbox.x && y0 - 1 < pbox.hy && y0 - 1 + LY > pbox.y;
     const bool writer = i >= 1 && j >= 1 && cx < g.NX() && cy < g.NY();   // owns the node column (cx, cy)
+    const bool raw_col = MODE != 0 && cx >= apart.x && cx < apart.hx && cy >= apart.y && cy < apart.hy;
     const long long obase = writer ? g.node(cx, cy, 0) : 0;               // chunk c at obase + c * zcs
     const long long pstride = g.cell_zc_stride();
     const int* pcol = pid + (cell_ok ? g.cell(cx, cy, 0) : 0);
@@ -835,6 +841,7 @@ k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split sp
       if (tid == 0 && issued < total && issued < n + 1 + LST) issue_next();
       if (halo) continue;   // uniform across the block
       if (!writer) continue;
+      const bool raw = raw_col && c >= apart.c && c < apart.hc;
 #pragma unroll
       for (int cc = 0; cc < 3; ++cc) {
         T o[4];
@@ -844,7 +851,7 @@ k_level1(const __grid_constant__ L1Maps maps, const __grid_constant__ L1Split sp
           o[t] = ((mb >> (8 * t + cc)) & 1u) ? val : T(0);
         }
         const long long at = cc * cs + obase + c * zcs, idx = co + at;
-        if constexpr (MODE == 0) {
+        if (MODE == 0 || raw) {
           lp_st4(out + idx, o);
         } else {
           T dv[4], d[4];
@@ -909,52 +916,85 @@ __global__ void __launch_bounds__(192) k_patch_modal(T* __restrict__ pm, const T
   }
 }
 
-// patch cells (weights zero, an explicit masked matrix): out += m * sum of their rows times
-// u, node by node over the box of nodes they touch (one warp per node: the lanes split the
-// 8 cells x 24 columns); runs after k_weights_tma
-template <typename T>
-__global__ void k_patch_add(T* __restrict__ out, const T* __restrict__ u, const int* __restrict__ pid,
-                            const T* __restrict__ pk, const uint8_t* __restrict__ mask, LpGrid g, int bx0, int by0,
-                            int bz0, int bnx, int bny, int bnz) {
-  lp_after_launch();
+// Patch cells (weights zero, an explicit masked matrix) after a march without them, node by node over the
+// nodes they touch (one warp per node: the lanes split the 8 cells x 24 columns): MODE 0 out += m * sum of
+// their rows times u; modes 1..3 the Chebyshev update from out, which the march left there, and that
+// sum (the vector kernels' expressions). All it reads but out is older than the march, the launch ahead,
+// so the products are formed while that one runs. bz0 and bnz are whole chunks in modes 1..3.
+template <typename T, int MODE>
+__global__ void __launch_bounds__(256)
+k_patch_nodes(T* __restrict__ out, const T* __restrict__ u, const int* __restrict__ pid, const T* __restrict__ pk,
+              const uint8_t* __restrict__ mask, LpGrid g, int bx0, int by0, int bz0, int bnx, int bny, int bnz,
+              L1Cheb<T> ch) {
   const long long total = (long long)bnx * bny * bnz;
-  const long long cs = g.comp_stride();
+  const long long cs = g.comp_stride(), co = 3 * cs * blockIdx.y;   // (the column)
   const int lane = threadIdx.x & 31;
   const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  if (warp >= total) return;
+  if (warp >= total) {
+    lp_after_launch();
+    return;
+  }
   const int z = bz0 + (int)(warp % bnz);
   const long long q = warp / bnz;
   const int y = by0 + (int)(q % bny), x = bx0 + (int)(q / bny);
+  const long long n = g.node(x, y, z);
+  const uint8_t mb = __ldcg(mask + n);
   // a node with no solved component keeps its output (the held nodes of a support face are
   // half of a patch box): the whole warp leaves
-  const uint8_t mb0 = mask[g.node(x, y, z)];
-  if (!(mb0 & 7)) return;
+  if (MODE == 0 && !(mb & 7)) {
+    lp_after_launch();
+    return;
+  }
   // lane -> (cell corner kk = lane / 4, column block of 6 = lane % 4)
   const int kk = lane >> 2, cb = lane & 3;
   T a[3] = {T(0), T(0), T(0)};
   const int cx = x - cx_(kk), cy = y - cy_(kk), cz = z - cz_(kk);
   int p = -1;
-  if (cx >= 0 && cy >= 0 && cz >= 0 && cx < g.nx && cy < g.ny && cz < g.nz) p = pid[g.cell(cx, cy, cz)];
+  if (cx >= 0 && cy >= 0 && cz >= 0 && cx < g.nx && cy < g.ny && cz < g.nz) p = __ldcg(pid + g.cell(cx, cy, cz));
   if (p >= 0) {
     const T* kp = pk + (long long)p * 576;
 #pragma unroll
     for (int c6 = 0; c6 < 6; ++c6) {
       const int col = 6 * cb + c6, q2 = col / 3, c2 = col % 3;
-      const T uv = u[c2 * cs + g.node(cx + cx_(q2), cy + cy_(q2), cz + cz_(q2))];
+      const T uv = __ldcg(u + co + c2 * cs + g.node(cx + cx_(q2), cy + cy_(q2), cz + cz_(q2)));
 #pragma unroll
-      for (int cc = 0; cc < 3; ++cc) a[cc] += kp[(3 * kk + cc) * 24 + col] * uv;
+      for (int cc = 0; cc < 3; ++cc) a[cc] += __ldcg(kp + (3 * kk + cc) * 24 + col) * uv;
     }
   }
-  const unsigned any = __ballot_sync(0xffffffffu, p >= 0);
-  if (!any) return;
+  const bool any = __any_sync(0xffffffffu, p >= 0);
 #pragma unroll
   for (int cc = 0; cc < 3; ++cc)
-    for (int o = 16; o > 0; o >>= 1) a[cc] += __shfl_down_sync(0xffffffffu, a[cc], o);
-  if (lane == 0) {
-    const long long n = g.node(x, y, z);
-#pragma unroll
-    for (int cc = 0; cc < 3; ++cc)
-      if ((mb0 >> cc) & 1) out[cc * cs + n] += a[cc];
+    for (int o = 16; o > 0; o >>= 1) a[cc] += __shfl_xor_sync(0xffffffffu, a[cc], o);
+  const T av = lane == 0 ? a[0] : lane == 1 ? a[1] : a[2];   // lane cc < 3 finishes component cc
+  const long long at = (lane < 3 ? lane : 0) * cs + n, i = co + at;
+  T dv = T(0), v0 = T(0), v1 = T(0), v2 = T(0), s = T(0), c1 = T(0), c2 = T(0);
+  if constexpr (MODE != 0) {
+    s = (T)__ldcg(ch.coef + 1);
+    c1 = (T)__ldcg(ch.coef + 2);
+    c2 = (T)__ldcg(ch.coef + 3);
+    dv = __ldcg(ch.dinv + at);
+    v0 = __ldcg((MODE == 1 ? ch.d : MODE == 2 ? ch.b : ch.x) + i);
+    if (MODE != 2) v1 = __ldcg((MODE == 1 ? ch.b : ch.d) + i);
+    if (MODE == 3) v2 = __ldcg(ch.r + i);
+  }
+  lp_wait_prior();
+  lp_release_next();
+  if (lane >= 3) return;
+  const bool on = (mb >> lane) & 1;
+  if constexpr (MODE == 0) {
+    if (any && on) out[i] += av;
+  } else {
+    const T raw = out[i], ad = any && on ? raw + av : raw;
+    if constexpr (MODE == 1) {
+      ch.x[i] = lp_cheb2_zero_v(v0, v1, ad, dv, c1, c2);
+    } else if constexpr (MODE == 2) {
+      T ri, di;
+      lp_residual_scaled_v(v0, ad, dv, s, ri, di);
+      ch.r[i] = ri;
+      ch.d[i] = di;
+    } else {
+      ch.x[i] = lp_cheb2_v(v0, v1, v2, ad, dv, c1, c2);
+    }
   }
 }
 
@@ -1403,11 +1443,11 @@ static const int G1_COLS[279] = {3, 7, 14, 10, 17, 9, 20, 23, 15, 19, 22, 21, 4,
 
 // pbox: the node box of the patch cells (host, 6 ints), which the split weighs
 template <typename T, int MODE>
-static int launch_level1(T* out, const T* u, const T* wc, const int* pid, const T* pm, const uint8_t* mask,
+static int launch_level1(T* out, const T* u, const T* wc, const int* pid, const T* pm, const T* pk, const uint8_t* mask,
                          const double* g1_host, const int* pbox, int* err, LpGrid g, cudaStream_t st,
                          const L1Cheb<T>& ch, int cols = 1) {
   if (cols < 1 || cols > 65535) return LP_ERR_ARG;
-  if (!lp_grid_ok(g) || g.pz % 4 || g.cpz != g.pz || !out || !u || !wc || !mask || !g1_host || !err)
+  if (!lp_grid_ok(g) || g.pz % 4 || g.cpz != g.pz || (MODE == 0 && !out) || !u || !wc || !mask || !g1_host || !err)
     return LP_ERR_ARG;
   G1<T> gc;
   for (int i = 0; i < 279; ++i) gc.c[i] = (T)g1_host[i];
@@ -1440,11 +1480,17 @@ static int launch_level1(T* out, const T* u, const T* wc, const int* pid, const 
   if (tuned >= 1 && (long long)tuned * nsm < nb) nb = (long long)tuned * nsm;
   const long long units = (long long)gx * gy * nchunks;
   if (units > 2147483647LL) return LP_ERR_SIZE;
+  // The patch cells' products are a chunk's latency over again, which a march of a few units a block does not
+  // hide: their own launch, overlapping the march, is then the faster form (applies in us, in the march and
+  // apart: 64 x 32 x 32 cells 13.8 and 9.7 in float32, 27.2 and 17.0 in float64; 96 x 48 x 48, 2.2
+  // units a block, 21.0 and 19.7, 41.7 and 34.4; 128 x 64 x 64, 5.2 units, 32.7 and 35.8, 69.7 and 71.4)
+  const bool have_patches = pid && pm && pbox && pbox[3] > 0 && pbox[4] > 0 && pbox[5] > 0;
+  const bool apart = have_patches && pk && out && out != u && units <= 3 * nb;
   if (nb > units) nb = units;
   // block b starts where b / nb of the total weight is reached: a chunk weighs 4, 8 in a tile that holds
   // patch cells (measured: with equal weights the support face's blocks ran 1.8x as long as the mean,
   // 47 us against 36 at 128 x 64 x 64)
-  const bool patches = pid && pm && pbox && pbox[3] > 0 && pbox[4] > 0 && pbox[5] > 0;
+  const bool patches = have_patches && !apart;
   const L1Box box = patches ? L1Box{pbox[0], pbox[0] + pbox[3] - 1, pbox[1], pbox[1] + pbox[4] - 1} : L1Box{};
   auto weight = [&](int tile) {
     const int x0 = (tile % gx) * (LX - 1) - 1, y0 = (tile / gx) * (LY - 1) - 1;
@@ -1465,8 +1511,18 @@ static int launch_level1(T* out, const T* u, const T* wc, const int* pid, const 
     done += (long long)w * nchunks;
   }
   for (; b <= nb; ++b) split.u0[b] = (int)units;
-  lp_launch(k_level1<T, MODE>, dim3((unsigned)nb, cols), LCOL, smem, st, maps, split, out, wc, patches ? pid : nullptr, pm, mask, gc, g,
-                                                      nchunks, err, ch, box);
+  L1Nodes nodes{};
+  int z0 = 0, nz = 0;
+  if (apart) {
+    z0 = MODE ? pbox[2] & ~3 : pbox[2];
+    nz = (MODE ? (pbox[2] + pbox[5] + 3) & ~3 : pbox[2] + pbox[5]) - z0;
+    if (MODE) nodes = L1Nodes{pbox[0], pbox[0] + pbox[3], pbox[1], pbox[1] + pbox[4], z0 >> 2, (z0 + nz) >> 2};
+  }
+  lp_launch(k_level1<T, MODE>, dim3((unsigned)nb, cols), LCOL, smem, st, maps, split, out, wc, patches ? pid : nullptr, pm, mask,
+            gc, g, nchunks, err, ch, box, nodes);
+  if (apart)
+    lp_launch(k_patch_nodes<T, MODE>, dim3(lp_blocks((long long)pbox[3] * pbox[4] * nz * 32, 256), cols), 256, 0, st, out, u,
+              pid, pk, mask, g, pbox[0], pbox[1], z0, pbox[3], pbox[4], nz, ch);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -1476,12 +1532,12 @@ template <typename T>
 static int apply_weights_tma(T* out, const T* u, const T* wc, const int* pid, const T* pk, const uint8_t* mask,
                              const double* g1, const int* pbox, int* err, LpGrid g, cudaStream_t st) {
   if (out == u) return LP_ERR_ARG;
-  const int rc = launch_level1<T, 0>(out, u, wc, nullptr, nullptr, mask, g1, nullptr, err, g, st, L1Cheb<T>{});
+  const int rc = launch_level1<T, 0>(out, u, wc, nullptr, nullptr, nullptr, mask, g1, nullptr, err, g, st, L1Cheb<T>{});
   if (rc != LP_OK) return rc;
   if (pid && pk && pbox && pbox[3] > 0 && pbox[4] > 0 && pbox[5] > 0) {
     const long long nb = (long long)pbox[3] * pbox[4] * pbox[5];
-    lp_launch(k_patch_add<T>, lp_blocks(nb * 32, 256), 256, 0, st, out, u, pid, pk, mask, g, pbox[0], pbox[1], pbox[2],
-                                                            pbox[3], pbox[4], pbox[5]);
+    lp_launch(k_patch_nodes<T, 0>, lp_blocks(nb * 32, 256), 256, 0, st, out, u, pid, pk, mask, g, pbox[0], pbox[1], pbox[2],
+              pbox[3], pbox[4], pbox[5], L1Cheb<T>{});
     LP_LAUNCH_CHECK();
   }
   return LP_OK;
@@ -1489,18 +1545,18 @@ static int apply_weights_tma(T* out, const T* u, const T* wc, const int* pid, co
 
 template <typename T>
 static int apply_level1(int mode, T* out, T* x, T* r, T* d, const T* u, const T* b, const T* dinv, const double* coef,
-                        const T* wc, const int* pid, const T* pm, const uint8_t* mask, const double* g1, const int* pbox,
-                        int* err, LpGrid g, int cols, cudaStream_t st) {
+                        const T* wc, const int* pid, const T* pm, const T* pk, const uint8_t* mask, const double* g1,
+                        const int* pbox, int* err, LpGrid g, int cols, cudaStream_t st) {
   if (!u || mode < 0 || mode > 3 || (mode && (!dinv || !coef))) return LP_ERR_ARG;
   const L1Cheb<T> ch{x, r, d, b, dinv, coef};
   if (mode == 0 && out && out != u)
-    return launch_level1<T, 0>(out, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch, cols);
+    return launch_level1<T, 0>(out, u, wc, pid, pm, pk, mask, g1, pbox, err, g, st, ch, cols);
   if (mode == 1 && x && d && b && u == d && x != d)
-    return launch_level1<T, 1>(x, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch, cols);
+    return launch_level1<T, 1>(out, u, wc, pid, pm, pk, mask, g1, pbox, err, g, st, ch, cols);
   if (mode == 2 && r && d && b && u == x && r != u && d != u && r != d)
-    return launch_level1<T, 2>(r, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch, cols);
+    return launch_level1<T, 2>(out, u, wc, pid, pm, pk, mask, g1, pbox, err, g, st, ch, cols);
   if (mode == 3 && x && d && r && u == d && x != d && r != d && r != x)
-    return launch_level1<T, 3>(x, u, wc, pid, pm, mask, g1, pbox, err, g, st, ch, cols);
+    return launch_level1<T, 3>(out, u, wc, pid, pm, pk, mask, g1, pbox, err, g, st, ch, cols);
   return LP_ERR_ARG;
 }
 
@@ -1694,35 +1750,35 @@ int lpb_patch_modal_f64(double* pm, const double* pk, long long npatch, void* st
 // not name may be NULL)
 int lpb_apply_level1_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b,
                          const float* dinv, const double* coef, const float* wc, const int* patch_id,
-                         const float* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err,
+                         const float* patch_m, const float* patch_k, const uint8_t* mask, const double* g1, const int* pbox, int* err,
                          LP_GRID_ARGS, void* stream) {
-  return apply_level1<float>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, mask, g1, pbox, err, LP_GRID, 1,
+  return apply_level1<float>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, patch_k, mask, g1, pbox, err, LP_GRID, 1,
                              LP_ST);
 }
 
 // the same for cols columns (each field's columns one after the other)
 int lpb_apply_level1_cols_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b,
                          const float* dinv, const double* coef, const float* wc, const int* patch_id,
-                         const float* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err,
+                         const float* patch_m, const float* patch_k, const uint8_t* mask, const double* g1, const int* pbox, int* err,
                          LP_GRID_ARGS, int cols, void* stream) {
-  return apply_level1<float>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, mask, g1, pbox, err, LP_GRID, cols,
+  return apply_level1<float>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, patch_k, mask, g1, pbox, err, LP_GRID, cols,
                              LP_ST);
 }
 
 int lpb_apply_level1_f64(int mode, double* out, double* x, double* r, double* d, const double* u, const double* b,
                          const double* dinv, const double* coef, const double* wc, const int* patch_id,
-                         const double* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err,
+                         const double* patch_m, const double* patch_k, const uint8_t* mask, const double* g1, const int* pbox, int* err,
                          LP_GRID_ARGS, void* stream) {
-  return apply_level1<double>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, mask, g1, pbox, err, LP_GRID, 1,
+  return apply_level1<double>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, patch_k, mask, g1, pbox, err, LP_GRID, 1,
                               LP_ST);
 }
 
 // the same for cols columns (each field's columns one after the other)
 int lpb_apply_level1_cols_f64(int mode, double* out, double* x, double* r, double* d, const double* u, const double* b,
                          const double* dinv, const double* coef, const double* wc, const int* patch_id,
-                         const double* patch_m, const uint8_t* mask, const double* g1, const int* pbox, int* err,
+                         const double* patch_m, const double* patch_k, const uint8_t* mask, const double* g1, const int* pbox, int* err,
                          LP_GRID_ARGS, int cols, void* stream) {
-  return apply_level1<double>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, mask, g1, pbox, err, LP_GRID, cols,
+  return apply_level1<double>(mode, out, x, r, d, u, b, dinv, coef, wc, patch_id, patch_m, patch_k, mask, g1, pbox, err, LP_GRID, cols,
                               LP_ST);
 }
 

@@ -370,11 +370,11 @@ void level1(Mg& m, Level& lv, int mode, void* out, const void* u, void* x = null
   const double* coef = mode ? lv.coef : nullptr;
   const void* dinv = mode ? lv.dinv : nullptr;
   m.ok(lv.f32 ? lpb_apply_level1_f32(mode, (float*)out, (float*)x, (float*)r, (float*)d, (const float*)u, (const float*)b,
-                                     (const float*)dinv, coef, (const float*)lv.wc, pid, (const float*)pm, lv.mask, m.g1,
+                                     (const float*)dinv, coef, (const float*)lv.wc, pid, (const float*)pm, (const float*)lv.patch_k, lv.mask, m.g1,
                                      lv.pbox, m.err, HG(g), m.st)
               : lpb_apply_level1_f64(mode, (double*)out, (double*)x, (double*)r, (double*)d, (const double*)u,
                                      (const double*)b, (const double*)dinv, coef, (const double*)lv.wc, pid,
-                                     (const double*)pm, lv.mask, m.g1, lv.pbox, m.err, HG(g), m.st));
+                                     (const double*)pm, (const double*)lv.patch_k, lv.mask, m.g1, lv.pbox, m.err, HG(g), m.st));
 }
 
 void apply(Mg& m, Level& lv, void* out, const void* u) {
@@ -750,10 +750,10 @@ void smooth(Mg& m, int i, const void* b, void* x, bool from_zero, bool started =
   }
   if (lv.kind == K_WEIGHTS) {
     if (from_zero) {
-      level1(m, lv, 1, nullptr, d, x, nullptr, d, b);
+      level1(m, lv, 1, t, d, x, nullptr, d, b);
     } else {
-      level1(m, lv, 2, nullptr, x, x, r, d, b);
-      level1(m, lv, 3, nullptr, d, x, r, d);
+      level1(m, lv, 2, t, x, x, r, d, b);
+      level1(m, lv, 3, t, d, x, r, d);
     }
     return;
   }

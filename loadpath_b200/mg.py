@@ -155,6 +155,7 @@ class DevLevel:
         self.wc = None           # weights: Walsh coefficients (cpz/4, ny, nx, 4, 8)
         self.pbox = None         # weights: node box of the patch cells (host, 6 ints)
         self.patch_m = None      # weights: the patch cells' matrices in the corner-parity basis
+        self.scratch = None      # weights: level1's
         self.mask = None
         self.dinv = None
         self.coef = None         # device: lmax and the Chebyshev coefficients (lpb_cheb_coef)
@@ -204,7 +205,12 @@ class DevLevel:
                                                        int(mask_in), 1, st)
         elif self.kind == "weights":
             if fine_kernel and not mask_in:
-                self.level1(0, out, u)
+                fn = L.lpb_apply_level1_f32 if sfx == "f32" else L.lpb_apply_level1_f64
+                n = self.npatch
+                fn(0, out.data_ptr(), None, None, None, u.data_ptr(), None, None, None, self.wc.data_ptr(),
+                   self.patch_id.data_ptr() if n else None, self.patch_m.data_ptr() if n else None,
+                   self.patch_k.data_ptr() if n else None, self.mask.data_ptr(), self.g1.ctypes.data,
+                   self.pbox.ctypes.data, self.err.data_ptr(), *g.args, st)
             else:
                 getattr(L, f"lpb_apply_weights_{sfx}")(out.data_ptr(), u.data_ptr(), self.w.data_ptr(),
                                                         self.mcat.data_ptr(), ptr(self.patch_id),
@@ -225,12 +231,16 @@ class DevLevel:
 
     def level1(self, mode, out, u, x=None, r=None, d=None, b=None, coef=None):
         """The weights level's march: mode 0 out = m K u (u zero on masked dofs), modes 1..3 a Chebyshev
-        update formed where K u is stored (lpb_apply_level1_*)."""
+        update formed where K u is stored (lpb_apply_level1_*; out: scratch, the level's own when not given)."""
         sfx = self._sfx()
+        if out is None:
+            if self.scratch is None:
+                self.scratch = self.grid.node_field(self.dtype)
+            out = self.scratch
         getattr(lib(), f"lpb_apply_level1_{sfx}")(mode, ptr(out), ptr(x), ptr(r), ptr(d), u.data_ptr(), ptr(b),
                                                   self.dinv.data_ptr() if mode else None, coef, self.wc.data_ptr(),
                                                   ptr(self.patch_id) if self.npatch else None, ptr(self.patch_m),
-                                                  self.mask.data_ptr(), self.g1.ctypes.data, self.pbox.ctypes.data,
+                                                  ptr(self.patch_k), self.mask.data_ptr(), self.g1.ctypes.data, self.pbox.ctypes.data,
                                                   self.err.data_ptr(), *self.grid.args, stream_handle())
 
     def apply_dot(self, out, u, part, dot=None, cols=1):
@@ -995,10 +1005,10 @@ class GridElasticity:
         if self.degree == 2 and lv.kind == "weights":
             # the first coarse level too, where its march stores A u
             if from_zero:
-                lv.level1(1, None, d, x=x, d=d, b=b, coef=coef)
+                lv.level1(1, t, d, x=x, d=d, b=b, coef=coef)
             else:
-                lv.level1(2, None, x, x=x, r=r, d=d, b=b, coef=coef)
-                lv.level1(3, None, d, x=x, r=r, d=d, coef=coef)
+                lv.level1(2, t, x, x=x, r=r, d=d, b=b, coef=coef)
+                lv.level1(3, t, d, x=x, r=r, d=d, coef=coef)
             return x
         if self.degree == 2:
             # the two Chebyshev steps in two passes (same bits as the step-by-step form)
@@ -1439,7 +1449,7 @@ class GridElasticity:
 
     def _apply_cols(self, i, mode, out, u, x=None, r=None, d=None, b=None):
         """Level i's A u (mode 0) or a Chebyshev update formed where it is stored (modes 1..3, as in
-        _smooth) for every column of the blocks."""
+        _smooth, out scratch) for every column of the blocks."""
         L = lib()
         st = stream_handle()
         lv = self._op(i)
@@ -1452,7 +1462,7 @@ class GridElasticity:
                                       lv.err.data_ptr(), *g.args, k, st)
         elif lv.kind == "weights":
             L.lpb_apply_level1_cols_f32(mode, *fields, *smooth, lv.wc.data_ptr(), ptr(lv.patch_id) if lv.npatch else None,
-                                        ptr(lv.patch_m), lv.mask.data_ptr(), lv.g1.ctypes.data, lv.pbox.ctypes.data,
+                                        ptr(lv.patch_m), ptr(lv.patch_k), lv.mask.data_ptr(), lv.g1.ctypes.data, lv.pbox.ctypes.data,
                                         lv.err.data_ptr(), *g.args, k, st)
         else:
             L.lpb_apply_explicit_modal_cols_f32(mode, *fields, *smooth, lv.km.data_ptr(), lv.kpc.data_ptr(),
@@ -1505,7 +1515,7 @@ class GridElasticity:
                 for j in range(k):
                     getattr(L, f"lpb_cheb_d_start_{sfx}")(bb[j].data_ptr(), lv.dinv.data_ptr(), lv.coef.data_ptr(),
                                                           d[j].data_ptr(), g.n_node_field, st)
-            self._apply_cols(i, 1, None, d, x=xb, d=d, b=bb)
+            self._apply_cols(i, 1, t, d, x=xb, d=d, b=bb)
             self._apply_cols(i, 0, t, xb)
             restrict(bc, dc, bb, t, k)
         else:
@@ -1518,8 +1528,8 @@ class GridElasticity:
         getattr(L, f"lpb_prolong_add_cols_{sfx}")(xb.data_ptr(), xc.data_ptr(), nxt.mask.data_ptr(), lv.mask.data_ptr(),
                                                   *g.args, *gc.args, k, st)
         if batched:
-            self._apply_cols(i, 2, None, xb, x=xb, r=r, d=d, b=bb)
-            self._apply_cols(i, 3, None, d, x=xb, r=r, d=d)
+            self._apply_cols(i, 2, t, xb, x=xb, r=r, d=d, b=bb)
+            self._apply_cols(i, 3, t, d, x=xb, r=r, d=d)
         else:
             for j in range(k):
                 self._smooth(i, bb[j], xb[j], False)
