@@ -394,9 +394,8 @@ int lpb_graph_free(void* exec);
  * lpb_cg_continue (sc: the PCG scalars, [0] |b|^2, [3] p.Ap, [4] |r|^2; state: iterations,
  * status) ends the loop once |r| <= rtol |b|, p.Ap <= 0, b = 0 or maxiter iterations ran. */
 /* Launch-geometry tuning (no reference counterpart), per grid of nx x ny x nz cells: the
- * persistent blocks per SM of the fine float32 (knob 1) and float64 (2) apply, and the z-segment
- * length, in chunks of four planes, of the level-1 float32 (3) and float64 (4) apply; 0 clears it
- * (the launcher decides). Set by loadpath_b200.tune from timed candidates; results are the same
+ * persistent blocks per SM of the fine float32 (knob 1) and float64 (2) apply and of the level-1
+ * float32 (3) and float64 (4) apply; 0 clears it (the launcher decides). Set by loadpath_b200.tune from timed candidates; results are the same
  * operator, the last bit of a float32 sum can differ at segment boundaries. */
 int lpb_tune_set(int knob, int nx, int ny, int nz, int value);
 int lpb_tune_get(int knob, int nx, int ny, int nz);

@@ -1009,7 +1009,8 @@ __host__ __device__ __forceinline__ int sym_index(int i, int j) {  // i <= j
 // matrices are older than the launch ahead (lpb_pack_sym_* see to it), so they are loaded while it runs.
 // What bounds it is how many of those loads are in flight: with one thread per cell (a few
 // thousand cells on a coarse level) the apply of 32 x 16 x 16 cells took 25.7 us in float64, shared by
-// eight warps 11.7 us, of 64 x 32 x 32 cells 69 and 50 us (157 MB of entries from DRAM: 22 us).
+// eight warps 11.7 us, of 64 x 32 x 32 cells 69 and 50 us (157 MB of entries from DRAM: 22 us); with the
+// loads ahead 9.3 us.
 constexpr int EX_WARPS = 8;
 template <typename T>
 struct ExCells {

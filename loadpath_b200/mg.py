@@ -1396,9 +1396,9 @@ class GridElasticity:
     # columns advance together: one traversal of the hierarchy per PCG iteration runs every
     # column's smoothing, transfers and operator applies level by level (so a level's
     # coefficients - moduli, level-1 weights, explicit matrices - are read from L2 by the
-    # columns after the first), one kernel solves the coarsest level for all columns (its
-    # dense inverse read once per eight), and the host reads every column's scalars with one
-    # copy per iteration. Each column keeps its own scalars and stopping test and runs the
+    # columns after the first; float32 levels take all columns in one launch, see _batched), and
+    # the coarsest level is solved for four columns per pass over its stored blocks. Each
+    # column keeps its own scalars and stopping test and runs the
     # same kernels on the same data as a lone solve, so a column's answer has the same bits.
     def _blk(self, key, k, grid: DevGrid, dtype):
         """k node fields of a level as one (k, field) tensor; [j] is column j's field."""
