@@ -604,7 +604,7 @@ __device__ __noinline__ void patch_alone(const T* __restrict__ pm, int patch, co
 // warps per scheduler issue them; what can be cut is the waiting and the rest: two blocks of four
 // warps per SM, whose barriers do not meet, instead of one of eight; one barrier per chunk; masks and
 // patch indices loaded a chunk ahead of their use; the patch cells (dense products) shared by a
-// warp's lanes in the same launch; units split evenly over the SMs instead of whole z segments. Sharing a
+// block's threads in the same launch, or in one behind it on small grids; units split evenly over the SMs instead of whole z segments. Sharing a
 // cell's rows between two warps (half the registers, twice the warps) ran 1.2x slower: the modes and
 // indices formed twice cost more issue slots than the extra warps filled.
 //
@@ -1209,7 +1209,9 @@ __device__ __forceinline__ void walsh8(float (&a)[8]) {
 
 // ft (24, cells) = T^T (K^ (T u_c)) for every cell (listed cells are rewritten afterwards). The matrices
 // are older than the launch ahead (lpb_pack_modal_f32 sees to it), so a cell's first MODAL_AHEAD entries
-// are loaded while that launch still runs; u is read after it.
+// are loaded while that launch still runs; u is read after it (an update of 32 x 16 x 16 cells 7.3 -> 6.6 us,
+// and 8.2 -> 7.3 by the gather's loads ahead; a cell's entries shared by four warps
+// won 0.4 us there and lost 2.0 us at 64 x 32 x 32).
 constexpr int MODAL_AHEAD = 64;
 __device__ __forceinline__ void modal_cell(float* __restrict__ ft, const float* __restrict__ u,
                                            const float* __restrict__ km, const LpGrid& g, long long t) {
