@@ -163,13 +163,16 @@ __global__ void k_chain_gather(double* __restrict__ ws, const double* __restrict
   }
 }
 
-// 1 / d from the hardware's approximation x (23 bits) by one step of the cubic form of Newton's iteration,
-// x <- x + x (e + e^2), e = 1 - d x (a pivot waits for it; a division takes twice as long)
-__device__ __forceinline__ double cubic_inverse(double d) {
+// 1 / d by the Newton-Raphson iteration for a reciprocal, x <- x + x (1 - d x), which squares the relative
+// error: two steps from the hardware's approximation (20 bits) pass a double's 53. A pivot waits for it;
+// d is a tested pivot, so the special cases that a division looks after do not arise (a zero, an infinity
+// or a NaN gives a NaN that the caller's test reports).
+__device__ __forceinline__ double pivot_inverse(double d) {
   double x;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
-  const double e = fma(-d, x, 1.0);
-  return fma(x, fma(e, e, e), x);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) x = fma(x, fma(-d, x, 1.0), x);
+  return x;
 }
 
 // The 32 x 32 matrix in s (row stride CLD) to its inverse in p (32 x 32), by warp 0: lane r holds row r
@@ -197,7 +200,7 @@ __device__ __forceinline__ void invert32(double (&s)[32][CLD], PivotCols& col, d
     c0[(lane - k) & 31] = x[0];
     c1[(lane - k) & 31] = x[1];
     __syncwarp();
-    const double det = fma(d0, d1, -e * e), inv = cubic_inverse(det);
+    const double det = fma(d0, d1, -e * e), inv = pivot_inverse(det);
     // the pivots are d0 and det / d0 (a NaN fails either test)
     if (lane == k && !(d0 > keep && d0 < 1e300)) bad = row0 + k + 1;
     if (lane == k + 1 && !(det > keep * d0 && det < 1e300)) bad = row0 + k + 2;
@@ -593,11 +596,11 @@ __device__ __forceinline__ void lane_sums(double (&s)[NC]) {
 constexpr int SOLVE_ROWS = 8;   // rows per block, one per warp
 constexpr int SEG_ROWS = 16;    // rows of a segment's inverse per block, two per warp: half as many blocks stage b
 
-// rows of y = A_I^-1 b_I (blocks of each segment in turn), then of g = b_s - W^T b_I
 // nothing: behind the factor's launches, so that they are complete for whatever is launched next, started
 // early or not
 __global__ void k_chain_settled() { lp_after_launch(); }
 
+// rows of y = A_I^-1 b_I (blocks of each segment in turn), then of g = b_s - W^T b_I
 template <typename T, int NC>
 __global__ void __launch_bounds__(256) k_chain_y(double* __restrict__ ws, const T* __restrict__ f, long long cstride,
                                                  Chain c) {
