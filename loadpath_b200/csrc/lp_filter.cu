@@ -44,6 +44,8 @@ constexpr int FT_THREADS = 32 * FT_Y;
 constexpr int FT_XH = 40;        // staged columns per row, from 4 below the tile
 constexpr int FT_BLOCKS = 296;   // two resident blocks on each of 148 SMs (one at reach 3)
 
+constexpr double TRIAL_EXP_BETA = 0.5;   // smallest slope of the projection that a volume trial takes by exp
+
 // The operation on a cell before the taps are applied.
 struct FilterIn {
   const double* v;
@@ -53,7 +55,8 @@ struct FilterIn {
 // WRITE: the accepted design, with the expressions of k_oc_stepped and k_project (lp_simp.cu). A trial
 // that only measures the volume forms the step and the projection from products with the inverses
 // and 1 - 2 / (exp(2 t) + 1) for tanh t, each within a rounding or two of those (the divisions and
-// tanh took half of its time).
+// tanh took half of its time). 1 - 2 / (exp(2 t) + 1) is off by a rounding of 1, which the division by
+// den, about beta on a slope below 1, would make large: there tanh stays.
 template <bool WRITE>
 struct TrialIn {
   const double* ts;      // x sqrt(-dc / dv)
@@ -159,6 +162,7 @@ __device__ __forceinline__ void finish(const TrialOut<WRITE>& o, const TrialIn<W
   for (int q = 0; q < 4; ++q) {
     xt[q] = r[q] / h[q];
     if constexpr (WRITE) xp[q] = (o.tbe + tanh(o.beta * (xt[q] - o.eta))) / o.den;
+    else if (o.beta < TRIAL_EXP_BETA) xp[q] = (o.tbe + tanh(o.beta * (xt[q] - o.eta))) * o.iden;
     else xp[q] = (o.tbe + (1.0 - 2.0 / (exp(2.0 * o.beta * (xt[q] - o.eta)) + 1.0))) * o.iden;
     if (q < n) {
       if (o.flags) {

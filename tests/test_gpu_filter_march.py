@@ -88,3 +88,31 @@ def test_fused_trial_equals_separate_passes(dims, radius):
         assert abs(out.item() - vol) <= w.size * EPS * vol
     for got, want in ((xn, pd.xn), (xt, pd.xt), (xp, pd.xp)):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("beta", [1e-7, 0.499, 0.5, 64.0])
+def test_trial_volume_at_any_slope(beta):
+    """A volume trial alone, at slopes on both sides of where it leaves tanh, against the projection in
+    extended precision: a cell's share is within 16 roundings (the filter's sum and division, the
+    argument's, tanh's two, den's) of its own size or, on a steep slope, beta / 2 roundings of xt."""
+    from loadpath_b200._lib import lib
+    from loadpath_b200.grid import DevGrid, stream_handle
+    from loadpath_b200.simp import DeviceFilter, ProjectedDesign
+
+    dims, eta = (33, 17, 5), 0.5
+    rng = np.random.default_rng(6)
+    g = DevGrid(dims)
+    w = rng.random(dims)
+    pd = ProjectedDesign(DeviceFilter(g, 2.0, pad=True), w=g.cells_to_dev(w, torch.float64))
+    x, ts = rng.random(dims), 0.5 * rng.random(dims)
+    xd, td = (g.cells_to_dev(a, torch.float64) for a in (x, ts))
+    out = torch.zeros(1, dtype=torch.float64, device="cuda")
+    lib().lpb_oc_trial(None, None, None, td.data_ptr(), xd.data_ptr(), 1.0, 0.2, None, pd.flt.toff.data_ptr(),
+                       pd.flt.tw.data_ptr(), pd.flt.ntaps, pd.flt.reach, pd.flt.hs.data_ptr(), beta, eta,
+                       pd.w.data_ptr(), pd._part.data_ptr(), out.data_ptr(), *g.args, stream_handle())
+    xn = g.set_cells(g.cell_field(torch.float64), torch.from_numpy(np.clip(ts, np.maximum(0, x - 0.2), np.minimum(1, x + 0.2))))
+    xt = g.cells_to_host(pd.flt.apply(g.cell_field(torch.float64), xn, hs_out=pd.flt.hs)).astype(np.longdouble)
+    b, e = np.longdouble(beta), np.longdouble(eta)
+    xp = (np.tanh(b * e) + np.tanh(b * (xt - e))) / (np.tanh(b * e) + np.tanh(b * (1 - e)))
+    want = (xp * w).sum()
+    assert abs(out.item() - want) <= (16 + beta / 2) * EPS * w.sum()
