@@ -112,9 +112,13 @@ int lpb_apply_explicit_modal_f32(float* out, const float* u, const float* km, co
  * mode 1 (u = d) x = d + (c1 d + c2 dinv (b - A d)); mode 2 (u = x) r = b - A x, d = s dinv r;
  * mode 3 (u = d) x = (x + d) + (c1 d + c2 dinv (r - A d)); coef: the level's coefficients. */
 int lpb_apply_explicit_modal_cheb_f32(int mode, float* x, float* r, float* d, const float* u, const float* b, const float* dinv, const double* coef, const float* km, const float* kpc, const int* glist, const int* gcount, float* ft, const uint8_t* mask, int nx, int ny, int nz, int pz, int cpz, void* stream);
-/* both (mode 0: out = m K u) for cols columns; ft: 24 * cells scratch per column */
+/* both (mode 0: out = m K u) for cols columns; ft: 24 * cells scratch per column. Loads km, kpc, glist and
+ * gcount beside the launch ahead: they are to be lpb_pack_modal_f32's, or complete before the last launch on
+ * the stream was made (the single-column entries above, and lpb_apply_explicit_sym_*, take matrices that the
+ * last launch wrote) */
 int lpb_apply_explicit_modal_cols_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b, const float* dinv, const double* coef, const float* km, const float* kpc, const int* glist, const int* gcount, float* ft, const uint8_t* mask, int nx, int ny, int nz, int pz, int cpz, int cols, void* stream);
-/* lpb_apply_explicit_sym_f64 with the update in its gather, modes 1..3 */
+/* lpb_apply_explicit_sym_f64 with the update in its gather, modes 1..3; kp, like the matrices of
+ * lpb_apply_explicit_modal_cols_f32, lpb_pack_sym_f64's, or complete before the last launch */
 int lpb_apply_explicit_sym_cheb_f64(int mode, double* x, double* r, double* d, const double* u, const double* b, const double* dinv, const double* coef, const double* kp, double* ft, const uint8_t* mask, int nx, int ny, int nz, int pz, int cpz, void* stream);
 int lpb_apply_explicit_sym_f32(float* out, const float* u, const float* kp, float* ft, const uint8_t* mask, int nx, int ny, int nz, int pz, int cpz, void* stream);
 int lpb_apply_explicit_sym_f64(double* out, const double* u, const double* kp, double* ft, const uint8_t* mask, int nx, int ny, int nz, int pz, int cpz, void* stream);

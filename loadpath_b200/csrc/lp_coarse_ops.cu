@@ -1005,8 +1005,9 @@ __host__ __device__ __forceinline__ int sym_index(int i, int j) {  // i <= j
 
 // A block takes 32 consecutive cells, a lane per cell, and its eight warps share the 300 entries of their
 // matrices (entry p of consecutive cells coalesced): each warp loads its 37 or 38 entries before the
-// corner values are staged, forms its part of the 24 corner forces, and the parts are added in order. The
-// matrices are older than the launch ahead (lpb_pack_sym_* see to it), so they are loaded while it runs.
+// corner values are staged, forms its part of the 24 corner forces, and the parts are added in order. Where the
+// matrices are older than the launch ahead (lpb_pack_sym_* see to it) they are loaded while it runs; where the
+// caller may have written them by the launch ahead, the launch is in stream order.
 // What bounds it is how many of those loads are in flight: with one thread per cell (a few
 // thousand cells on a coarse level) the apply of 32 x 16 x 16 cells took 25.7 us in float64, shared by
 // eight warps 11.7 us, of 64 x 32 x 32 cells 69 and 50 us (157 MB of entries from DRAM: 22 us); with the
@@ -1207,9 +1208,9 @@ __device__ __forceinline__ void walsh8(float (&a)[8]) {
       }
 }
 
-// ft (24, cells) = T^T (K^ (T u_c)) for every cell (listed cells are rewritten afterwards). The matrices
-// are older than the launch ahead (lpb_pack_modal_f32 sees to it), so a cell's first MODAL_AHEAD entries
-// are loaded while that launch still runs; u is read after it (an update of 32 x 16 x 16 cells 7.3 -> 6.6 us,
+// ft (24, cells) = T^T (K^ (T u_c)) for every cell (listed cells are rewritten afterwards). Where the matrices
+// are older than the launch ahead (lpb_pack_modal_f32 sees to it) a cell's first MODAL_AHEAD entries
+// are loaded while that launch still runs (elsewhere the launch is in stream order); u is read after it (an update of 32 x 16 x 16 cells 7.3 -> 6.6 us,
 // and 8.2 -> 7.3 by the gather's loads ahead; a cell's entries shared by four warps
 // won 0.4 us there and lost 2.0 us at 64 x 32 x 32).
 constexpr int MODAL_AHEAD = 64;
@@ -1563,15 +1564,16 @@ static int apply_level1(int mode, T* out, T* x, T* r, T* d, const T* u, const T*
   return LP_ERR_ARG;
 }
 
+// settled: kp was complete before the launch ahead began, so the cells may load it beside that launch
 template <typename T>
-static int launch_explicit(T* out, const T* u, const T* kp, T* ft, const uint8_t* mask, LpGrid g, cudaStream_t st,
-                           int mode = 0, const ChebArgs<T>* ch = nullptr) {
+static int launch_explicit(bool settled, T* out, const T* u, const T* kp, T* ft, const uint8_t* mask, LpGrid g,
+                           cudaStream_t st, int mode = 0, const ChebArgs<T>* ch = nullptr) {
   if (!lp_grid_ok(g) || !u || !kp || !ft || !mask) return LP_ERR_ARG;
   if (mode == 0 && (!out || out == u)) return LP_ERR_ARG;
   constexpr int smem = (int)sizeof(ExCells<T>);   // above the 48 KB default in float64
   if (cudaFuncSetAttribute(k_explicit_cells<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return LP_ERR_LAUNCH;
-  lp_launch(k_explicit_cells<T>, lp_blocks(g.cells_padded(), 32), 32 * EX_WARPS, smem, st, ft, u, kp, g);
+  lp_launch_as(settled, k_explicit_cells<T>, lp_blocks(g.cells_padded(), 32), 32 * EX_WARPS, smem, st, ft, u, kp, g);
   if (mode == 0) {
     lp_launch(k_explicit_gather<T>, lp_blocks(g.nodes_padded(), 256), 256, 0, st, out, ft, mask, g);
   } else {
@@ -1593,7 +1595,8 @@ static bool explicit_cheb_ok(int mode, const ChebArgs<T>& a, const T* u) {
   return a.x && a.d && a.r && u == a.d && a.x != a.d;
 }
 
-static int launch_explicit_modal(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b,
+// settled: as launch_explicit's, of km, kpc, glist and gcount
+static int launch_explicit_modal(bool settled, int mode, float* out, float* x, float* r, float* d, const float* u, const float* b,
                                  const float* dinv, const double* coef, const float* km, const float* kpc,
                                  const int* glist, const int* gcount, float* ft, const uint8_t* mask, LpGrid g, int cols,
                                  cudaStream_t st) {
@@ -1603,8 +1606,8 @@ static int launch_explicit_modal(int mode, float* out, float* x, float* r, float
   const ChebArgs<float> a{x, r, d, b, dinv, coef};
   if (mode != 0 && !explicit_cheb_ok(mode, a, u)) return LP_ERR_ARG;
   const int modal_blocks = lp_blocks(g.cells_padded(), 128);
-  lp_launch(k_explicit_modal_cells, dim3(modal_blocks + 148, cols), 128, 0, st, ft, u, km, kpc, glist, gcount, g,
-            modal_blocks);
+  lp_launch_as(settled, k_explicit_modal_cells, dim3(modal_blocks + 148, cols), 128, 0, st, ft, u, km, kpc, glist, gcount,
+               g, modal_blocks);
   const dim3 nb(lp_blocks(g.nodes_padded(), 256), cols), nbc(lp_blocks(g.nodes_padded(), 128), cols);
   if (mode == 0) lp_launch(k_explicit_gather<float>, nb, 256, 0, st, out, ft, mask, g);
   else if (mode == 1) lp_launch(k_explicit_gather_cheb<float, 1>, nbc, 128, 0, st, ft, mask, g, a);
@@ -1787,22 +1790,23 @@ int lpb_apply_level1_cols_f64(int mode, double* out, double* x, double* r, doubl
 
 int lpb_apply_explicit_sym_f32(float* out, const float* u, const float* kp, float* ft, const uint8_t* mask,
                                LP_GRID_ARGS, void* stream) {
-  return launch_explicit<float>(out, u, kp, ft, mask, LP_GRID, LP_ST);
+  return launch_explicit<float>(false, out, u, kp, ft, mask, LP_GRID, LP_ST);
 }
 
 int lpb_apply_explicit_sym_f64(double* out, const double* u, const double* kp, double* ft, const uint8_t* mask,
                                LP_GRID_ARGS, void* stream) {
-  return launch_explicit<double>(out, u, kp, ft, mask, LP_GRID, LP_ST);
+  return launch_explicit<double>(false, out, u, kp, ft, mask, LP_GRID, LP_ST);
 }
 
 // lpb_apply_explicit_sym_f64 with a degree-2 Chebyshev update in its gather (modes 1..3, as
-// lpb_apply_explicit_modal_cheb_f32)
+// lpb_apply_explicit_modal_cheb_f32), kp loaded before the launch ahead has ended: it must have been complete
+// when that one began (lpb_pack_sym_f64 ends with a launch that sees to it)
 int lpb_apply_explicit_sym_cheb_f64(int mode, double* x, double* r, double* d, const double* u, const double* b,
                                     const double* dinv, const double* coef, const double* kp, double* ft,
                                     const uint8_t* mask, LP_GRID_ARGS, void* stream) {
   const ChebArgs<double> a{x, r, d, b, dinv, coef};
   if (!explicit_cheb_ok(mode, a, u)) return LP_ERR_ARG;
-  return launch_explicit<double>(nullptr, u, kp, ft, mask, LP_GRID, LP_ST, mode, &a);
+  return launch_explicit<double>(true, nullptr, u, kp, ft, mask, LP_GRID, LP_ST, mode, &a);
 }
 
 // lpb_apply_explicit_sym_f32 with its (24, cells) scratch in the library's static array: no
@@ -1818,7 +1822,7 @@ int lpb_apply_explicit_sym_noalloc_f32(float* out, const float* u, const float* 
   if (g.cells_padded() > LP_NOALLOC_MAX_CELLS) return LP_ERR_SIZE;
   float* ft = explicit_scratch_address();
   if (!ft) return LP_ERR_LAUNCH;
-  return launch_explicit<float>(out, u, kp, ft, mask, g, LP_ST);
+  return launch_explicit<float>(false, out, u, kp, ft, mask, g, LP_ST);
 }
 
 // km (150, ncells) = the pattern entries of each cell's K^ = T K T^T / 64 (symmetric part); cells
@@ -1841,7 +1845,7 @@ int lpb_pack_modal_f32(float* km, int* glist, int* gcount, float* kpc, const flo
 // node-basis entries kpc (both from lpb_pack_modal_f32); ft: 24 * cells scratch
 int lpb_apply_explicit_modal_f32(float* out, const float* u, const float* km, const float* kpc, const int* glist,
                                  const int* gcount, float* ft, const uint8_t* mask, LP_GRID_ARGS, void* stream) {
-  return launch_explicit_modal(0, out, nullptr, nullptr, nullptr, u, nullptr, nullptr, nullptr, km, kpc, glist, gcount, ft,
+  return launch_explicit_modal(false, 0, out, nullptr, nullptr, nullptr, u, nullptr, nullptr, nullptr, km, kpc, glist, gcount, ft,
                                mask, LP_GRID, 1, LP_ST);
 }
 
@@ -1854,17 +1858,18 @@ int lpb_apply_explicit_modal_cheb_f32(int mode, float* x, float* r, float* d, co
                                       const int* glist, const int* gcount, float* ft, const uint8_t* mask,
                                       LP_GRID_ARGS, void* stream) {
   if (mode < 1) return LP_ERR_ARG;
-  return launch_explicit_modal(mode, nullptr, x, r, d, u, b, dinv, coef, km, kpc, glist, gcount, ft, mask, LP_GRID, 1,
-                               LP_ST);
+  return launch_explicit_modal(false, mode, nullptr, x, r, d, u, b, dinv, coef, km, kpc, glist, gcount, ft, mask, LP_GRID,
+                               1, LP_ST);
 }
 
 // both (mode 0: out = m K u) for cols columns, each field's columns one after the other; ft: 24 * cells
-// scratch per column
+// scratch per column. km, kpc, glist and gcount are loaded before the launch ahead has ended: they must have been
+// complete when that one began (lpb_pack_modal_f32 ends with a launch that sees to it)
 int lpb_apply_explicit_modal_cols_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b,
                                       const float* dinv, const double* coef, const float* km, const float* kpc,
                                       const int* glist, const int* gcount, float* ft, const uint8_t* mask,
                                       LP_GRID_ARGS, int cols, void* stream) {
-  return launch_explicit_modal(mode, out, x, r, d, u, b, dinv, coef, km, kpc, glist, gcount, ft, mask, LP_GRID, cols,
+  return launch_explicit_modal(true, mode, out, x, r, d, u, b, dinv, coef, km, kpc, glist, gcount, ft, mask, LP_GRID, cols,
                                LP_ST);
 }
 

@@ -197,22 +197,29 @@ __host__ __device__ __forceinline__ int cz_(int k) { return (k >> 2) & 1; }
 template <typename T>
 __device__ __forceinline__ T lp_ldg(const T* p) { return __ldg(p); }
 
-// Launches overlap their start with the kernel before them (programmatic dependent launch): every kernel
-// of the library begins with lp_after_launch, which waits until the kernel before it has finished and
-// its writes are visible, then lets the one after it start; lp_launch is the launch that allows
-// it. A kernel's blocks are so already in place (parameters fetched, barriers set up) when their
-// turn comes, which is most of the time of the many launches of a coarse level.
+// Launches overlap their start with the kernel before them (programmatic dependent launch). The rule that
+// keeps it safe: every block of every kernel waits (griddepcontrol.wait: the launch ahead has finished and its
+// writes are visible) before it lets the next launch start, and before it exits, on every path. So when a
+// kernel's blocks begin, all that was complete when the launch ahead passed its wait is complete, and only
+// what the launch ahead itself writes may still be under way. Most kernels begin with lp_after_launch, both
+// halves at once: their blocks are then already in place (parameters fetched, barriers set up) when
+// their turn comes, which is most of the time of the many launches of a coarse level.
 __device__ __forceinline__ void lp_after_launch() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-// The two halves, for a kernel whose launch ahead is always one of the library's own that begins with
-// lp_after_launch: what was complete when that one began may be read before lp_wait_prior, by loads that
-// pass the L1 by (__ldcg): only the wait makes sure that no line there is older.
+// The two halves, in this order, for the kernels that load before the wait: k_patch_nodes, k_explicit_cells,
+// k_explicit_modal_cells, k_explicit_gather_cheb, k_chain_y, k_chain_s and k_chain_x. What they load there must
+// be older than the launch ahead, either because the same function launched that one and it does not write
+// it, or because its producer ends with an empty launch (k_settled, k_chain_settled) whose wait completes
+// it; where a caller's own launch may have written it, the kernel goes out in stream order (lp_launch_as). Such
+// loads pass the L1 by (__ldcg): only the wait makes sure that no line there is older.
 __device__ __forceinline__ void lp_release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void lp_wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// overlap false: in stream order (the launch ahead has ended before this one begins)
 template <typename... P, typename... A>
-static inline void lp_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+static inline void lp_launch_as(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                A&&... args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -222,8 +229,12 @@ static inline void lp_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap ? 1 : 0;
   (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // a failure is left for LP_LAUNCH_CHECK
+}
+template <typename... P, typename... A>
+static inline void lp_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  lp_launch_as(true, kernel, grid, block, smem, st, static_cast<A&&>(args)...);
 }
 
 // four consecutive values (16-byte aligned)

@@ -386,8 +386,9 @@ void apply(Mg& m, Level& lv, void* out, const void* u) {
   } else if (lv.kind == K_WEIGHTS) {
     level1(m, lv, 0, out, u);
   } else if (lv.km) {
-    m.ok(lpb_apply_explicit_modal_f32((float*)out, (const float*)u, (const float*)lv.km, (const float*)lv.kpc,
-                                      lv.glist, lv.gcount, (float*)lv.ft, lv.mask, HG(g), m.st));
+    m.ok(lpb_apply_explicit_modal_cols_f32(0, (float*)out, nullptr, nullptr, nullptr, (const float*)u, nullptr, nullptr,
+                                           nullptr, (const float*)lv.km, (const float*)lv.kpc, lv.glist, lv.gcount,
+                                           (float*)lv.ft, lv.mask, HG(g), 1, m.st));
   } else {
     m.ok(lv.f32 ? lpb_apply_explicit_sym_f32((float*)out, (const float*)u, (const float*)lv.kp, (float*)lv.ft, lv.mask,
                                              HG(g), m.st)
@@ -765,9 +766,9 @@ void smooth(Mg& m, int i, const void* b, void* x, bool from_zero, bool started =
                                              HG(g), m.st));
         return;
       }
-      m.ok(lpb_apply_explicit_modal_cheb_f32(mode, (float*)x, (float*)r, (float*)d, (const float*)u, (const float*)b,
+      m.ok(lpb_apply_explicit_modal_cols_f32(mode, nullptr, (float*)x, (float*)r, (float*)d, (const float*)u, (const float*)b,
                                              (const float*)lv.dinv, coef, (const float*)lv.km, (const float*)lv.kpc,
-                                             lv.glist, lv.gcount, (float*)lv.ft, lv.mask, HG(g), m.st));
+                                             lv.glist, lv.gcount, (float*)lv.ft, lv.mask, HG(g), 1, m.st));
     };
     if (from_zero) {
       fused(1, d);

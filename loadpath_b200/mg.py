@@ -218,9 +218,10 @@ class DevLevel:
                                                         int(mask_in), 1, st)
         else:
             if fine_kernel and not mask_in and self.km is not None:
-                L.lpb_apply_explicit_modal_f32(out.data_ptr(), u.data_ptr(), self.km.data_ptr(), self.kpc.data_ptr(),
-                                               self.glist.data_ptr(), self.gcount.data_ptr(), self.ft.data_ptr(),
-                                               self.mask.data_ptr(), *g.args, st)
+                L.lpb_apply_explicit_modal_cols_f32(0, out.data_ptr(), None, None, None, u.data_ptr(), None, None, None,
+                                                    self.km.data_ptr(), self.kpc.data_ptr(), self.glist.data_ptr(),
+                                                    self.gcount.data_ptr(), self.ft.data_ptr(), self.mask.data_ptr(),
+                                                    *g.args, 1, st)
             elif fine_kernel and not mask_in:
                 getattr(L, f"lpb_apply_explicit_sym_{sfx}")(out.data_ptr(), u.data_ptr(), self.kp.data_ptr(),
                                                              self.ft.data_ptr(), self.mask.data_ptr(), *g.args, st)
@@ -992,10 +993,10 @@ class GridElasticity:
                                                       b.data_ptr(), lv.dinv.data_ptr(), coef, lv.kp.data_ptr(),
                                                       lv.ft.data_ptr(), lv.mask.data_ptr(), *g.args, st)
                     return
-                L.lpb_apply_explicit_modal_cheb_f32(mode, x.data_ptr(), r.data_ptr(), d.data_ptr(), u.data_ptr(),
+                L.lpb_apply_explicit_modal_cols_f32(mode, None, x.data_ptr(), r.data_ptr(), d.data_ptr(), u.data_ptr(),
                                                     b.data_ptr(), lv.dinv.data_ptr(), coef, lv.km.data_ptr(),
                                                     lv.kpc.data_ptr(), lv.glist.data_ptr(), lv.gcount.data_ptr(),
-                                                    lv.ft.data_ptr(), lv.mask.data_ptr(), *g.args, st)
+                                                    lv.ft.data_ptr(), lv.mask.data_ptr(), *g.args, 1, st)
             if from_zero:
                 fused(1, d)
             else:

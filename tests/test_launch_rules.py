@@ -1,0 +1,33 @@
+"""Host-side rules of the library's launches, seen through a recording stand-in for the CUDA runtime (CPU
+only: no kernel runs)."""
+import pytest
+from launch_recorder import record
+
+GRID = "(8, 4, 12, 16, 16)"   # nx, ny, nz, and the pitches of its layout
+
+
+@pytest.mark.parametrize("call", [
+    "L.lpb_apply_explicit_sym_f32(P(), P(), P(), P(), P(), *g, None)",
+    "L.lpb_apply_explicit_sym_f64(P(), P(), P(), P(), P(), *g, None)",
+    "L.lpb_apply_explicit_sym_noalloc_f32(P(), P(), P(), P(), *g, None)",
+    "L.lpb_apply_explicit_modal_f32(P(), P(), P(), P(), P(), P(), P(), P(), *g, None)",
+    "L.lpb_apply_explicit_modal_cheb_f32(2, None, P(), P(), P(), P(), P(), P(), P(), P(), P(), P(), P(), P(), *g, None)",
+])
+def test_explicit_apply_keeps_stream_order(tmp_path, call):
+    """The cell pass of an explicit apply loads its matrices before it waits for the launch ahead, which may
+    be the caller's own that writes them: the entries that promise stream order launch it in that order."""
+    got = record(tmp_path, f"g = {GRID}\n{call}\nout = recorded()")
+    cells = [r for r in got if r["what"] == "launch" and "_cells" in r["kernel"]]
+    assert len(cells) == 1 and cells[0]["overlap"] == 0
+
+
+@pytest.mark.parametrize("call", [
+    "L.lpb_pack_sym_f32(P(), P(), 64, None)", "L.lpb_pack_sym_f64(P(), P(), 64, None)",
+    "L.lpb_pack_modal_f32(P(), P(), P(), P(), P(), 64, 1e-6, None)",
+    "L.lpb_chain_factor(P(), P(), P(), 16, 4, 4, 8, 8, None)",
+])
+def test_producers_of_early_loads_end_settled(tmp_path, call):
+    """What an overlapping launch loads before its wait comes from passes that end with an empty launch,
+    whose wait completes them."""
+    got = [r for r in record(tmp_path, f"{call}\nout = recorded()") if r["what"] == "launch"]
+    assert "settled" in got[-1]["kernel"] and len(got) > 1
