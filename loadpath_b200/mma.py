@@ -108,9 +108,12 @@ class MMA:
 
     # -- the subproblem (loadpath/mma.py:114-214) ---------------------------------------------
     def _loop(self):
-        """The interior-point loops as a graph with one while node (every buffer it names lives as
-        long as this object), captured at the first update."""
-        if self._exec is None:
+        """The interior-point loops as a graph with one while node, captured at the first update and again
+        when a buffer it names was replaced (a caller may restore low and upp)."""
+        bufs = [t.data_ptr() for t in (self.low, self.upp, self._alfa, self._beta, self._p0, self._q0, self._P, self._Q,
+                                       *self._sets[0], *self._sets[1], self._state, self._part)]
+        if self._exec is None or self._exec_bufs != bufs:
+            self._free_loop()
             L = lib()
             c0 = launches()
             with torch.cuda.device(self.device), torch.cuda.stream(torch.cuda.Stream(self.device)):
@@ -118,16 +121,12 @@ class MMA:
                 handle, outer, exec_ = ctypes.c_longlong(), ctypes.c_void_p(), ctypes.c_void_p()
                 L.lpb_while_begin(st, ctypes.byref(handle), ctypes.byref(outer))
                 try:
-                    L.lpb_mma_loop_body(handle.value, self.n, self.m, self.low.data_ptr(), self.upp.data_ptr(),
-                                        self._alfa.data_ptr(), self._beta.data_ptr(), self._p0.data_ptr(),
-                                        self._q0.data_ptr(), self._P.data_ptr(), self._Q.data_ptr(),
-                                        *(t.data_ptr() for s in self._sets for t in s), self._state.data_ptr(),
-                                        self._part.data_ptr(), st)
+                    L.lpb_mma_loop_body(handle.value, self.n, self.m, *bufs, st)
                 finally:
                     L.lpb_while_end(st, outer, ctypes.byref(exec_))
             self._body = launches() - c0
             add_launches(-self._body)      # recorded, not run
-            self._exec = exec_
+            self._exec, self._exec_bufs = exec_, bufs
         return self._exec
 
     def _subsolv(self, f, epsimin=1e-7):
@@ -148,10 +147,19 @@ class MMA:
         self.lam = o[:self.m].copy()
         return self._sets[int(o[9])][0]
 
+    def _free_loop(self):
+        if self._exec is not None:
+            exec_, self._exec = self._exec, None
+            torch.cuda.synchronize(self.device)
+            lib().lpb_graph_free(exec_)
+
+    def __getstate__(self):
+        """Copies and pickles capture a graph of their own."""
+        return dict(self.__dict__, _exec=None)
+
     def __del__(self):
         if getattr(self, "_exec", None) is not None:
             try:
-                torch.cuda.synchronize(self.device)
-                lib().lpb_graph_free(self._exec)
+                self._free_loop()
             except Exception:
                 pass
