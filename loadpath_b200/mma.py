@@ -134,7 +134,10 @@ class MMA:
         L = lib()
         st = stream_handle()
         x0, xsi0, eta0 = self._sets[0]
-        host = [np.ascontiguousarray(v, float) for v in (self.a, self.c, self.d, f)]
+        # (d may be one number for all constraints; a and c have a value each)
+        host = [np.ascontiguousarray(v, float) for v in (self.a, self.c, np.broadcast_to(self.d, (self.m,)), f)]
+        if any(v.shape != (self.m,) for v in host):
+            raise ValueError(f"a and c take {self.m} values each")
         L.lpb_mma_sub_init(self.n, self._alfa.data_ptr(), self._beta.data_ptr(), x0.data_ptr(), xsi0.data_ptr(),
                            eta0.data_ptr(), st)
         L.lpb_mma_loop_begin(self.m, self._state.data_ptr(), self._out.data_ptr(), *(v.ctypes.data for v in host),

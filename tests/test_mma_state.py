@@ -88,3 +88,17 @@ def test_copies_have_a_loop_of_their_own(fake, make):
     n = len(fake.graphs)
     del mma, other
     assert sorted(fake.freed) == sorted(fake.graphs) and n == 2
+
+
+def test_penalty_weights_one_for_all(fake):
+    """d as one number for all constraints; a and c of another length are refused, not read past their end."""
+    mma = fake.mma(m=3)
+    mma.d = 2.0
+    fake.update(mma)
+    a, c, d, f = fake.hosts[-1]
+    assert a.tolist() == [0.0] * 3 and c.tolist() == [1000.0] * 3 and d.tolist() == [2.0] * 3
+    for name in ("a", "c"):
+        short = fake.mma(m=3)
+        setattr(short, name, np.ones(2))
+        with pytest.raises(ValueError):
+            fake.update(short)
