@@ -1071,9 +1071,7 @@ int lpb_band_inverse(double* ainv, const double* t, const double* linv, const do
   if (bd.D <= INV_RING_D) {
     typedef InvRing<INV_RING_CB> IR;
     const size_t smem = IR::smem(bd.D);
-    if (cudaFuncSetAttribute(k_band_inverse_ring<INV_RING_CB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess)
-      return LP_ERR_SIZE;
+    if (!lp_smem_limit((const void*)k_band_inverse_ring<INV_RING_CB>, (int)smem)) return LP_ERR_SIZE;
     lp_launch(k_band_inverse_ring<INV_RING_CB>, (unsigned)(np / INV_RING_CB), 32 * IR::NW, smem, LP_ST, ainv, t, linv, sgn, bd);
     lp_launch(k_sym_lower, dim3(bd.nt, bd.nt), 256, 0, LP_ST, ainv, np);
     LP_LAUNCH_CHECK();
@@ -1084,8 +1082,7 @@ int lpb_band_inverse(double* ainv, const double* t, const double* linv, const do
   if (chunk > bd.D) chunk = bd.D;
   if (chunk < 1) return LP_ERR_SIZE;
   const long long smem = (2LL * chunk + 2) * INV_TILE * sizeof(double);
-  if (cudaFuncSetAttribute(k_band_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return LP_ERR_SIZE;
+  if (!lp_smem_limit((const void*)k_band_inverse, (int)smem)) return LP_ERR_SIZE;
   lp_launch(k_band_inverse, (unsigned)(np / INV_COLS), 512, (size_t)smem, LP_ST, ainv, t, linv, sgn, bd, chunk);
   lp_launch(k_sym_lower, dim3(bd.nt, bd.nt), 256, 0, LP_ST, ainv, np);
   LP_LAUNCH_CHECK();

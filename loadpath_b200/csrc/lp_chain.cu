@@ -760,9 +760,8 @@ int chain_pass(double* ws, const T* fi, T* fo, long long cstride, const Chain& c
   }
   const int gb = (c.P - 1) * ((c.b + SOLVE_ROWS - 1) / SOLVE_ROWS);
   const int s1 = 2 * NC * c.M * 8, s2 = NC * c.MS * 8, s3 = NC * 2 * c.b * 8;
-  if (cudaFuncSetAttribute(k_chain_y<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, s1) != cudaSuccess ||
-      cudaFuncSetAttribute(k_chain_s<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, s2) != cudaSuccess ||
-      cudaFuncSetAttribute(k_chain_x<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, s3) != cudaSuccess)
+  if (!lp_smem_limit((const void*)k_chain_y<T, NC>, s1) || !lp_smem_limit((const void*)k_chain_s<T, NC>, s2) ||
+      !lp_smem_limit((const void*)k_chain_x<T, NC>, s3))
     return LP_ERR_SIZE;
   lp_launch(k_chain_y<T, NC>, pairs + gb, 256, s1, st, ws, fi, cstride, c);
   lp_launch(k_chain_s<T, NC>, (c.nS + SOLVE_ROWS - 1) / SOLVE_ROWS, 256, s2, st, ws, fo, cstride, c);

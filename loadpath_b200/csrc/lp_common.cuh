@@ -77,6 +77,11 @@ static inline bool lp_grid_ok(const LpGrid& g) {
 enum { LP_KNOB_FINE_F32 = 1, LP_KNOB_FINE_F64 = 2, LP_KNOB_L1_F32 = 3, LP_KNOB_L1_F64 = 4, LP_KNOB_MAX = 4 };
 int lp_tune_lookup(int knob, int nx, int ny, int nz);
 
+// Raises a kernel's dynamic shared-memory limit on the current device to at least bytes; false when the
+// device has not that much. The limit belongs to the process: it is never lowered, so a launch that
+// another thread is about to make keeps what it asked for (lp_graph.cu).
+bool lp_smem_limit(const void* kernel, int bytes);
+
 // The degree-2 Chebyshev updates, one definition for the standalone vector kernels and the
 // explicit levels' gather that applies them as it forms A u (the same expression, so the same bits)
 template <typename T>

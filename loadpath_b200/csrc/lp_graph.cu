@@ -2,7 +2,9 @@
 // end+instantiate / launch / free), so the solver records its set-up, CG head and CG tail once
 // and replays each with one launch; capturable asynchronous copies and fills.
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <utility>
 
 #include "lp_common.cuh"
 
@@ -92,6 +94,22 @@ int lp_tune_lookup(int knob, int nx, int ny, int nz) {
     if (g_tune[i].knob == knob && g_tune[i].nx == nx && g_tune[i].ny == ny && g_tune[i].nz == nz)
       return g_tune[i].value;
   return 0;
+}
+
+bool lp_smem_limit(const void* kernel, int bytes) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, int> limits;   // (device, kernel)
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  std::lock_guard<std::mutex> lock(mu);
+  int& limit = limits[{dev, kernel}];
+  if (bytes <= limit) return true;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  limit = bytes;
+  return true;
 }
 
 extern "C" {

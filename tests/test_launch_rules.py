@@ -31,3 +31,34 @@ def test_producers_of_early_loads_end_settled(tmp_path, call):
     whose wait completes them."""
     got = [r for r in record(tmp_path, f"{call}\nout = recorded()") if r["what"] == "launch"]
     assert "settled" in got[-1]["kernel"] and len(got) > 1
+
+
+def _limits_hold(records):
+    """No limit is lowered, and every launch is within its kernel's limit from then on."""
+    limit = {}
+    for r in records:
+        key = r["kernel"], r["device"]
+        if r["what"] == "limit":
+            assert r["bytes"] >= limit.get(key, 0), r
+            limit[key] = r["bytes"]
+        elif r["bytes"] > 48 * 1024:
+            assert r["bytes"] <= limit.get(key, 0), r
+
+
+@pytest.mark.parametrize("call", [
+    "L.lpb_chain_solve_f32(P(), P(), P(), *grid(n), None)", "L.lpb_chain_solve_f64(P(), P(), P(), *grid(n), None)",
+    "L.lpb_chain_solve_cols_f32(P(), P(), 1 << 20, 4, P(), *grid(n), None)",
+    "L.lpb_band_inverse(P(), P(), P(), P(), *grid(n), None)",
+])
+def test_shared_memory_limits_are_never_lowered(tmp_path, call):
+    """A kernel's dynamic shared-memory limit belongs to the process: a solve of a small level must not take it
+    from under the launch of a large one that another thread is making."""
+    body = f"""
+def grid(n):
+    p = (n[2] + 1 + 3) // 4 * 4
+    return (*n, p, p)
+for n in ((40, 10, 8), (6, 2, 2), (30, 10, 6), (40, 10, 8), (8, 3, 3)):
+    assert {call} == 0
+out = recorded()
+"""
+    _limits_hold(record(tmp_path, body))
