@@ -37,7 +37,6 @@
 // (1 - m) u of the masked operator vanish and the kernel writes m * K u.
 #include <cstring>
 #include <initializer_list>
-#include <mutex>
 
 #include "lp_common.cuh"
 #include "lp_modal.cuh"
@@ -533,30 +532,6 @@ __global__ void k_fine_dot_final(const double* __restrict__ part, long long n, d
 
 static bool fine_args_ok(const LpGrid& g) { return lp_grid_ok(g) && g.pz % 4 == 0 && g.cpz == g.pz; }
 
-// resident blocks of a kernel on this device at the given dynamic shared memory (and the
-// attribute that allows it), looked up once per kernel
-static long long resident_blocks(const void* kfn, int smem) {
-  static std::mutex mu;
-  static const void* keys[8];
-  static long long vals[8];
-  static int n = 0;
-  std::lock_guard<std::mutex> lock(mu);
-  for (int i = 0; i < n; ++i)
-    if (keys[i] == kfn) return vals[i];
-  if (cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return 0;
-  int per_sm = 1, dev = 0, nsm = 148;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, TXC * TYC, smem);
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const long long v = (long long)(per_sm > 0 ? per_sm : 1) * nsm;
-  if (n < 8) {
-    keys[n] = kfn;
-    vals[n] = v;
-    ++n;
-  }
-  return v;
-}
-
 // The seven coefficient classes of the cubic-symmetric modal matrix from lpb_modal_ke's 45
 // values: {a - b, b, d, b2, d2, e2, t}. False when an entry strays from its class by more than
 // 1e-9 of the largest, or the exact identities of the isotropic unit brick (the linear shear block
@@ -645,7 +620,7 @@ static int launch_fine(T* out, const T* u, const T* e, const uint8_t* mask, cons
   } else {
     kfn = (const void*)k_apply_fine<double, 0>;
   }
-  const long long slots = resident_blocks(kfn, smem);
+  const long long slots = lp_resident_blocks(kfn, TXC * TYC, smem);
   if (!slots) return LP_ERR_LAUNCH;
   const int gx = (g.NX() + TXC - 2) / (TXC - 1), gy = (g.NY() + TYC - 2) / (TYC - 1);
   const int nchunks = g.pz / (int)zc;

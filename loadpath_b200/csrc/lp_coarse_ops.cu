@@ -1466,17 +1466,11 @@ static int launch_level1(T* out, const T* u, const T* wc, const int* pid, const 
     if (!lp_make_map(&maps.w, wc, 4, wd, wb, sizeof(T), 128)) return LP_ERR_ARG;
   }
   const int smem = (int)sizeof(L1Smem<T>) + 1024;
-  static long long slots = 0;   // resident blocks on the device (queried once per process)
+  const long long slots = lp_resident_blocks((const void*)k_level1<T, MODE>, LCOL, smem);
+  if (slots < 1) return LP_ERR_LAUNCH;
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (!slots) {
-    if (cudaFuncSetAttribute(k_level1<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return LP_ERR_LAUNCH;
-    int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_level1<T, MODE>, LCOL, smem);
-    slots = (long long)(per_sm > 0 ? per_sm : 1) * nsm;
-  }
   const int gx = (g.NX() + LX - 2) / (LX - 1), gy = (g.NY() + LY - 2) / (LY - 1), nchunks = g.pz / 4;
   // persistent blocks: all resident ones (or the tuned number per SM)
   long long nb = slots < L1_MAX_BLOCKS ? slots : L1_MAX_BLOCKS;

@@ -81,6 +81,9 @@ int lp_tune_lookup(int knob, int nx, int ny, int nz);
 // device has not that much. The limit belongs to the process: it is never lowered, so a launch that
 // another thread is about to make keeps what it asked for (lp_graph.cu).
 bool lp_smem_limit(const void* kernel, int bytes);
+// resident blocks of a kernel on the current device at this block size and dynamic shared memory (the limit
+// raised to it), looked up once per device; 0 when the device cannot run it
+long long lp_resident_blocks(const void* kernel, int threads, int smem);
 
 // The degree-2 Chebyshev updates, one definition for the standalone vector kernels and the
 // explicit levels' gather that applies them as it forms A u (the same expression, so the same bits)

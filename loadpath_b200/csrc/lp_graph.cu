@@ -112,6 +112,20 @@ bool lp_smem_limit(const void* kernel, int bytes) {
   return true;
 }
 
+long long lp_resident_blocks(const void* kernel, int threads, int smem) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, long long> blocks;   // (device, kernel)
+  int dev = 0, per_sm = 1, nsm = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  long long& n = blocks[{dev, kernel}];
+  if (n) return n;
+  if (!lp_smem_limit(kernel, smem)) return 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  return n = (long long)(per_sm > 0 ? per_sm : 1) * nsm;
+}
+
 extern "C" {
 
 // Sets (value > 0) or clears (value 0) the tuned launch geometry of a knob for one grid; the

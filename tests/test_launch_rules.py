@@ -62,3 +62,26 @@ for n in ((40, 10, 8), (6, 2, 2), (30, 10, 6), (40, 10, 8), (8, 3, 3)):
 out = recorded()
 """
     _limits_hold(record(tmp_path, body))
+
+
+@pytest.mark.parametrize("call", [
+    *(f"L.lpb_apply_fine_{t}(P(), P(), P(), P(), host, P(), *g, None)" for t in ("f32", "f64")),
+    *(f"L.lpb_apply_level1_{t}({m}, {f}, P(), P(), P(), None, None, None, P(), host, host, P(), *g, None)"
+      for t in ("f32", "f64") for m, f in ((0, "P(), None, None, None, P(), None"), (1, "P(), P(), None, d, d, P()"),
+                                           (2, "P(), d, P(), P(), d, P()"), (3, "P(), P(), P(), d, d, None"))),
+])
+def test_every_device_gets_its_limit(tmp_path, call):
+    """The marches' shared-memory limits are set on each device that they run on."""
+    body = f"""
+from loadpath_b200.fem import hex8_ke
+ke, modal = np.ascontiguousarray(hex8_ke(0.3, "im")), np.zeros(1024)
+L.lpb_modal_ke(ke.ctypes.data, modal.ctypes.data)
+g, d, host = (8, 4, 11, 12, 12), P(), modal.ctypes.data
+for device in (0, 1, 0):
+    on_device(device)
+    assert {call} == 0
+out = recorded()
+"""
+    got = record(tmp_path, body)
+    assert {r["device"] for r in got if r["what"] == "launch"} == {0, 1}
+    _limits_hold(got)
