@@ -44,8 +44,6 @@ constexpr int FT_THREADS = 32 * FT_Y;
 constexpr int FT_XH = 40;        // staged columns per row, from 4 below the tile
 constexpr int FT_BLOCKS = 296;   // two resident blocks on each of 148 SMs (one at reach 3)
 
-constexpr double TRIAL_EXP_BETA = 0.5;   // smallest slope of the projection that a volume trial takes by exp
-
 // The operation on a cell before the taps are applied.
 struct FilterIn {
   const double* v;
@@ -53,10 +51,16 @@ struct FilterIn {
 };
 // OC trial at a multiplier: clip(ts / sl, max(0, x - move), min(1, x + move)), flagged cells held.
 // WRITE: the accepted design, with the expressions of k_oc_stepped and k_project (lp_simp.cu). A trial
-// that only measures the volume forms the step and the projection from products with the inverses
-// and 1 - 2 / (exp(2 t) + 1) for tanh t, each within a rounding or two of those (the divisions and
-// tanh took half of its time). 1 - 2 / (exp(2 t) + 1) is off by a rounding of 1, which the division by
-// den, about beta on a slope below 1, would make large: there tanh stays.
+// that only measures the volume has the same values: its two divisors, sl and den, are the same for all
+// cells, so a quotient is the product with the divisor's inverse corrected by its remainder (trial_quotient),
+// three operations where a division takes over ten (a design update of 192 x 96 x 96 cells, nine trials and
+// the write: 644 us; 626 with the products uncorrected and tanh by way of exp, off by up to a rounding of 1).
+// a / b from y = 1 / b, correctly rounded (Markstein's theorem: one fused correction of a quotient that is off by
+// rounding, with y itself the rounded inverse); a quotient that is infinite, or a NaN, stays
+__device__ __forceinline__ double trial_quotient(double a, double b, double y) {
+  const double q = a * y, r = fma(-q, b, a);
+  return isfinite(q) ? fma(r, y, q) : q;
+}
 template <bool WRITE>
 struct TrialIn {
   const double* ts;      // x sqrt(-dc / dv)
@@ -94,7 +98,7 @@ __device__ __forceinline__ double pre(const TrialIn<WRITE>& f, long long c, doub
   } else {
     // compares and selects; a NaN step goes to the lower bound, as fmax takes it
     const double l = xv - f.move, h = xv + f.move, lo = l > 0.0 ? l : 0.0, hi = h < 1.0 ? h : 1.0;
-    v = ts * f.isl;
+    v = trial_quotient(ts, f.sl, f.isl);
     v = v > lo ? v : lo;
     v = v < hi ? v : hi;
   }
@@ -161,9 +165,8 @@ __device__ __forceinline__ void finish(const TrialOut<WRITE>& o, const TrialIn<W
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     xt[q] = r[q] / h[q];
-    if constexpr (WRITE) xp[q] = (o.tbe + tanh(o.beta * (xt[q] - o.eta))) / o.den;
-    else if (o.beta < TRIAL_EXP_BETA) xp[q] = (o.tbe + tanh(o.beta * (xt[q] - o.eta))) * o.iden;
-    else xp[q] = (o.tbe + (1.0 - 2.0 / (exp(2.0 * o.beta * (xt[q] - o.eta)) + 1.0))) * o.iden;
+    const double num = o.tbe + tanh(o.beta * (xt[q] - o.eta));
+    xp[q] = WRITE ? num / o.den : trial_quotient(num, o.den, o.iden);
     if (q < n) {
       if (o.flags) {
         const uint8_t fl = o.flags[c + q];
