@@ -31,6 +31,7 @@
 #include <algorithm>
 
 #include "lp_common.cuh"
+#include "lp_quotient.cuh"
 #include "lp_tma.cuh"
 
 #define LP_MAX_TAPS 1024
@@ -52,15 +53,9 @@ struct FilterIn {
 // OC trial at a multiplier: clip(ts / sl, max(0, x - move), min(1, x + move)), flagged cells held.
 // WRITE: the accepted design, with the expressions of k_oc_stepped and k_project (lp_simp.cu). A trial
 // that only measures the volume has the same values: its two divisors, sl and den, are the same for all
-// cells, so a quotient is the product with the divisor's inverse corrected by its remainder (trial_quotient),
+// cells, so a quotient is the product with the divisor's inverse corrected by its remainder (lp_quotient),
 // three operations where a division takes over ten (a design update of 192 x 96 x 96 cells, nine trials and
 // the write: 644 us; 626 with the products uncorrected and tanh by way of exp, off by up to a rounding of 1).
-// a / b from y = 1 / b, correctly rounded (Markstein's theorem: one fused correction of a quotient that is off by
-// rounding, with y itself the rounded inverse); a quotient that is infinite, or a NaN, stays
-__device__ __forceinline__ double trial_quotient(double a, double b, double y) {
-  const double q = a * y, r = fma(-q, b, a);
-  return isfinite(q) ? fma(r, y, q) : q;
-}
 template <bool WRITE>
 struct TrialIn {
   const double* ts;      // x sqrt(-dc / dv)
@@ -98,7 +93,7 @@ __device__ __forceinline__ double pre(const TrialIn<WRITE>& f, long long c, doub
   } else {
     // compares and selects; a NaN step goes to the lower bound, as fmax takes it
     const double l = xv - f.move, h = xv + f.move, lo = l > 0.0 ? l : 0.0, hi = h < 1.0 ? h : 1.0;
-    v = trial_quotient(ts, f.sl, f.isl);
+    v = lp_quotient_inf(ts, f.sl, f.isl);
     v = v > lo ? v : lo;
     v = v < hi ? v : hi;
   }
@@ -166,7 +161,7 @@ __device__ __forceinline__ void finish(const TrialOut<WRITE>& o, const TrialIn<W
   for (int q = 0; q < 4; ++q) {
     xt[q] = r[q] / h[q];
     const double num = o.tbe + tanh(o.beta * (xt[q] - o.eta));
-    xp[q] = WRITE ? num / o.den : trial_quotient(num, o.den, o.iden);
+    xp[q] = WRITE ? num / o.den : lp_quotient(num, o.den, o.iden);
     if (q < n) {
       if (o.flags) {
         const uint8_t fl = o.flags[c + q];

@@ -20,6 +20,7 @@
 #include <math.h>
 
 #include "lp_common.cuh"
+#include "lp_mma_var.cuh"
 
 #define LP_MMA_MAXM 8
 #define LP_MMA_BLOCKS 592
@@ -304,9 +305,10 @@ __global__ void __launch_bounds__(LP_MMA_THREADS) k_mma_trial(long long n, int m
 // recomputed from the point and dlam, so a step reads 11 arrays and then reads 11 and writes 3, where
 // newton_a, newton_b and trial move 44. Between the passes one block each (k_mma_steg, k_mma_test) does
 // what the host did: step length, line search, epsi's descent, the (m + 1) system. The passes are bound by
-// memory (14 MB an array at 192 x 96 x 96 variables); quotients that share a divisor share its
-// reciprocal, since with each division of its own the float64 units took as long as the memory. An update
-// there takes 2.73 ms, with the host between the passes it took 9.98 ms (half of it waiting for results).
+// memory (14 MB an array at 192 x 96 x 96 variables) and the float64 units together; quotients that share a
+// divisor share its inverse, corrected (lp_mma_var.cuh). An update there takes 2.97 ms; 2.76 with the products
+// left uncorrected, which are off by up to twice as much as divisions; 9.98 with the host between the passes
+// (half of it waiting for results).
 constexpr int MMA_LOOP_BLOCKS = 296;   // two per SM
 
 struct MmaState {
@@ -350,35 +352,6 @@ __global__ void k_mma_begin(MmaState* __restrict__ st, const double* __restrict_
   }
 }
 
-// One variable: its constants, point and the reciprocals of its distances
-struct MmaVar {
-  double x, s, e, up, lo, al, be;
-  double iux, ixl, ixa, ibx;
-  __device__ __forceinline__ void reciprocals() {
-    iux = 1.0 / (up - x);
-    ixl = 1.0 / (x - lo);
-    ixa = 1.0 / (x - al);
-    ibx = 1.0 / (be - x);
-  }
-  // delx and diagx at p.lam, q.lam
-  __device__ __forceinline__ void newton(double plam, double qlam, double epsi, double& delx, double& diagx) const {
-    const double pu = plam * (iux * iux), ql = qlam * (ixl * ixl);
-    delx = pu - ql - epsi * ixa + epsi * ibx;
-    diagx = 2.0 * (pu * iux + ql * ixl) + s * ixa + e * ibx;
-  }
-};
-
-// the direction of variable j: (dx, dxsi, deta) from dlam
-__device__ __forceinline__ void mma_direction(const MmaVar& v, double plam, double qlam, double gp, double gq, double epsi,
-                                              double& dx, double& ds, double& de) {
-  double delx, diagx;
-  v.newton(plam, qlam, epsi, delx, diagx);
-  const double gtl = gp * (v.iux * v.iux) - gq * (v.ixl * v.ixl);   // (GG^T dlam)_j
-  dx = -(delx + gtl) / diagx;
-  ds = -v.s + epsi * v.ixa - v.s * dx * v.ixa;
-  de = -v.e + epsi * v.ibx + v.e * dx * v.ibx;
-}
-
 __device__ __forceinline__ MmaVar mma_var(const MmaArrays& A, const MmaSets& sets, int which, long long j) {
   MmaVar v;
   v.x = (which ? sets.v[1][0] : sets.v[0][0])[j];
@@ -420,13 +393,13 @@ __global__ void __launch_bounds__(LP_MMA_THREADS, M > 2 ? 1 : 2) k_mma_maxima(lo
         gp += P * dlam[i];
         gq += Q * dlam[i];
       }
-    v.reciprocals();
+    v.distances();
     double dx, ds, de;
-    mma_direction(v, plam, qlam, gp, gq, epsi, dx, ds, de);
+    v.direction(plam, qlam, gp, gq, epsi, dx, ds, de);
     acc[0] = fmax(acc[0], -1.01 * ds / v.s);
     acc[1] = fmax(acc[1], -1.01 * de / v.e);
-    acc[2] = fmax(acc[2], -1.01 * dx * v.ixa);
-    acc[3] = fmax(acc[3], 1.01 * dx * v.ibx);
+    acc[2] = fmax(acc[2], v.over_xa(-1.01 * dx));
+    acc[3] = fmax(acc[3], v.over_bx(1.01 * dx));
   }
   block_reduce<4>(acc, is_max, part);
 }
@@ -541,9 +514,9 @@ __global__ void __launch_bounds__(LP_MMA_THREADS, M > 2 ? 1 : 2) k_mma_move(long
       }
     }
     if (move) {
-      v.reciprocals();
+      v.distances();
       double dx, ds, de;
-      mma_direction(v, plam, qlam, gp, gq, epsi, dx, ds, de);
+      v.direction(plam, qlam, gp, gq, epsi, dx, ds, de);
       v.x += steg * dx;
       v.s += steg * ds;
       v.e += steg * de;
@@ -551,26 +524,24 @@ __global__ void __launch_bounds__(LP_MMA_THREADS, M > 2 ? 1 : 2) k_mma_move(long
       (which ? sets.v[0][1] : sets.v[1][1])[j] = v.s;
       (which ? sets.v[0][2] : sets.v[1][2])[j] = v.e;
     }
-    v.reciprocals();
-    const double iux2 = v.iux * v.iux, ixl2 = v.ixl * v.ixl;
-    const double r1 = pnew * iux2 - qnew * ixl2 - v.s + v.e;
-    const double r5 = v.s * (v.x - v.al) - epsi, r6 = v.e * (v.be - v.x) - epsi;
+    v.distances();
+    const double r1 = v.over_ux2(pnew) - v.over_xl2(qnew) - v.s + v.e;
+    const double r5 = v.s * v.xa - epsi, r6 = v.e * v.bx - epsi;
     acc[0] += r1 * r1 + r5 * r5 + r6 * r6;
     acc[1] = fmax(acc[1], fmax(fabs(r1), fmax(fabs(r5), fabs(r6))));
     double delx, diagx;
     v.newton(pnew, qnew, epsi, delx, diagx);
-    const double idg = 1.0 / diagx, t = delx * idg;
+    const double idg = 1.0 / diagx, t = lp_quotient(delx, diagx, idg);
     int k = 2 + 2 * M;
     double gg[M];
 #pragma unroll
-    for (int i = 0; i < M; ++i) gg[i] = P[i] * iux2 - Q[i] * ixl2;
+    for (int i = 0; i < M; ++i) gg[i] = v.over_ux2(P[i]) - v.over_xl2(Q[i]);
 #pragma unroll
     for (int i = 0; i < M; ++i) {
-      acc[2 + i] += P[i] * v.iux + Q[i] * v.ixl;
+      acc[2 + i] += v.over_ux(P[i]) + v.over_xl(Q[i]);
       acc[2 + M + i] += gg[i] * t;
-      const double h = gg[i] * idg;
 #pragma unroll
-      for (int i2 = i; i2 < M; ++i2) acc[k++] += h * gg[i2];
+      for (int i2 = i; i2 < M; ++i2) acc[k++] += lp_quotient(gg[i] * gg[i2], diagx, idg);
     }
   }
   block_reduce<K>(acc, is_max, part);
