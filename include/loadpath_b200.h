@@ -330,7 +330,8 @@ int lpb_dinv_mask_f64(double* av, const double* dinv, const uint8_t* m, int nx, 
 /* ---- SIMP loop (loadpath/simp.py:1143-1228, :1861, :1901-1904, :2001;
  * loadpath/benchmarks/reference.py:48-110; loadpath/femops.py:51-78, loadpath/mg.py:975-988) */
 int lpb_filter(double* out, const double* v, const int* toff, const double* tw, int ntaps, const double* hs_in, const double* hs_out, double* e_out, double penal, double emin, int nx, int ny, int nz, int pz, int cpz, void* stream);
-/* lpb_filter with the taps' reach (the largest |offset|) named by the caller */
+/* lpb_filter for a cone's taps in order, with their reach (the largest |offset|) named by the caller: up to reach 3
+ * by classes of equal weight, 2 to 14 times faster (any other list comes out right, but slower than lpb_filter's) */
 int lpb_filter_reach(double* out, const double* v, const int* toff, const double* tw, int ntaps, int reach, const double* hs_in, const double* hs_out, double* e_out, double penal, double emin, int nx, int ny, int nz, int pz, int cpz, void* stream);
 int lpb_simp_law(double* e, const double* x, double penal, double emin, int nx, int ny, int nz, int pz, int cpz, void* stream);
 int lpb_element_energy_f64(double* ce, const double* u, const double* v, const double* ke, int nx, int ny, int nz, int pz, int cpz, void* stream);

@@ -26,9 +26,11 @@
 // block per chunk, and 550 us with the next chunk staged through registers and a branch per tap.
 //
 // The staged form takes tap lists without repeats whose weights are those of their class and |dz| and
-// whose classes are whole (every cone's), up to the reach that the caller names; other lists, and
-// fields that do not start on a 16-byte boundary, are gathered from global memory cell by cell.
+// whose classes are whole (every cone's), up to reach 3. Lists that reach further, fields that do not start on a
+// 16-byte boundary and all lists of lpb_filter are taken tap by tap (k_filter_taps). Where the march meets
+// another list (lpb_filter_reach, lpb_oc_trial) it gathers cell by cell from global memory.
 #include <algorithm>
+#include <type_traits>
 
 #include "lp_common.cuh"
 #include "lp_quotient.cuh"
@@ -216,6 +218,44 @@ __device__ __forceinline__ int class_size(int k) {
   return n;
 }
 
+// whether the list is one the staged form takes: within reach R, every (class, |dz|) whole with one
+// weight, no repeats (counting catches one together with a missing tap only where the list is sorted,
+// so sorted lists alone are taken). Fills tp; the whole block calls it.
+template <int R>
+__device__ bool list_staged(FilterTaps& tp, const int* __restrict__ toff, const double* __restrict__ tw, int ntaps,
+                            bool refuse) {
+  constexpr int NK = 2 * R * R + 1;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  int bad = refuse;
+  for (int i = tid; i < NK * (R + 1); i += nt) tp.count[i / (R + 1)][i % (R + 1)] = 0;
+  for (int i = tid; i < ntaps; i += nt) {
+    const int dx = toff[3 * i], dy = toff[3 * i + 1], dz = toff[3 * i + 2];
+    bad |= max(abs(dx), max(abs(dy), abs(dz))) > R;
+    if (i) {
+      const int px = toff[3 * i - 3], py = toff[3 * i - 2], pz = toff[3 * i - 1];
+      bad |= !(px < dx || (px == dx && (py < dy || (py == dy && pz < dz))));
+    }
+  }
+  if (__syncthreads_or(bad)) return false;
+  for (int i = tid; i < ntaps; i += nt) {
+    const int k = toff[3 * i] * toff[3 * i] + toff[3 * i + 1] * toff[3 * i + 1], dz = abs(toff[3 * i + 2]);
+    tp.w[k][dz] = tw[i];
+    atomicAdd(&tp.count[k][dz], 1);
+  }
+  __syncthreads();
+  bad = 0;
+  for (int i = tid; i < ntaps; i += nt) {
+    const int k = toff[3 * i] * toff[3 * i] + toff[3 * i + 1] * toff[3 * i + 1], dz = abs(toff[3 * i + 2]);
+    bad |= !(tp.w[k][dz] == tw[i]) || tp.count[k][dz] != class_size<R>(k) * (dz ? 2 : 1);
+  }
+  if (tid < NK) {
+    unsigned m = 0;
+    for (int dz = 0; dz <= R; ++dz) m |= (tp.count[tid][dz] ? 1u : 0u) << dz;
+    tp.present[tid] = m;
+  }
+  return __syncthreads_or(bad) == 0;
+}
+
 // taps from global memory, cell by cell
 template <class In, class Out>
 __device__ void gather_item(const In& in, const Out& o, const int* __restrict__ toff, const double* __restrict__ tw,
@@ -296,42 +336,10 @@ k_filter_march(const __grid_constant__ FilterMaps maps, const In in, const Out o
   unsigned char* slabs = smem_raw + ((1024u - (raw_off & 1023u)) & 1023u);   // a: stages 0, 1, then b: 0, 1
   __shared__ FilterTaps tp;
   __shared__ alignas(8) uint64_t full[2];
-  constexpr int YH = FT_Y + 2 * R, SLAB = Slab<R>::BYTES, NK = 2 * R * R + 1;
+  constexpr int YH = FT_Y + 2 * R, SLAB = Slab<R>::BYTES;
   constexpr uint32_t BYTES = FT_XH * YH * 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // whether the list is one the staged form takes: within reach R, every (class, |dz|) whole with one
-  // weight, no repeats (counting catches one together with a missing tap only where the list is sorted,
-  // so sorted lists alone are taken)
-  int bad = !tma;
-  for (int i = tid; i < NK * (R + 1); i += FT_THREADS) tp.count[i / (R + 1)][i % (R + 1)] = 0;
-  for (int i = tid; i < ntaps; i += FT_THREADS) {
-    const int dx = toff[3 * i], dy = toff[3 * i + 1], dz = toff[3 * i + 2];
-    bad |= max(abs(dx), max(abs(dy), abs(dz))) > R;
-    if (i) {
-      const int px = toff[3 * i - 3], py = toff[3 * i - 2], pz = toff[3 * i - 1];
-      bad |= !(px < dx || (px == dx && (py < dy || (py == dy && pz < dz))));
-    }
-  }
-  bool staged = __syncthreads_or(bad) == 0;
-  if (staged) {
-    for (int i = tid; i < ntaps; i += FT_THREADS) {
-      const int k = toff[3 * i] * toff[3 * i] + toff[3 * i + 1] * toff[3 * i + 1], dz = abs(toff[3 * i + 2]);
-      tp.w[k][dz] = tw[i];
-      atomicAdd(&tp.count[k][dz], 1);
-    }
-    __syncthreads();
-    bad = 0;
-    for (int i = tid; i < ntaps; i += FT_THREADS) {
-      const int k = toff[3 * i] * toff[3 * i] + toff[3 * i + 1] * toff[3 * i + 1], dz = abs(toff[3 * i + 2]);
-      bad |= !(tp.w[k][dz] == tw[i]) || tp.count[k][dz] != class_size<R>(k) * (dz ? 2 : 1);
-    }
-    if (tid < NK) {
-      unsigned m = 0;
-      for (int dz = 0; dz <= R; ++dz) m |= (tp.count[tid][dz] ? 1u : 0u) << dz;
-      tp.present[tid] = m;
-    }
-    staged = __syncthreads_or(bad) == 0;
-  }
+  bool staged = list_staged<R>(tp, toff, tw, ntaps, tma == 0);
   if (tid == 0) {
     lp_mbar_init(&full[0], 1);
     lp_mbar_init(&full[1], 1);
@@ -433,6 +441,114 @@ k_filter_march(const __grid_constant__ FilterMaps maps, const In in, const Out o
   }
 }
 
+// Taps one after another, for the lists and fields the march does not take:
+//   out = H (v / hs_in) / hs_out, with e_out also the SIMP law on the result.
+// A block takes a tile of 32 x 8 cell columns times one z chunk (4 cells): it stages the tile with its halo of
+// reach R (the largest |offset| of the taps, up to TAPS_R) in shared memory, v / hs_in formed once per staged
+// cell and zeros outside the grid, and each thread sums the taps for the 4 cells of its column in the list's
+// order. Taps that reach further are gathered from global memory, cell by cell, in the same order: bound by
+// the loads' latency, so the blocks are small and many (reach 4, 192 x 96 x 96 cells: 1141 us; in the march's
+// blocks of 512, one per SM, 4690).
+constexpr int TAPS_X = 32, TAPS_Y = 8, TAPS_R = 2;
+__global__ void __launch_bounds__(256) k_filter_taps(double* __restrict__ out, const double* __restrict__ v,
+                                                     const int* __restrict__ toff, const double* __restrict__ tw,
+                                                     int ntaps, const double* __restrict__ hs_in,
+                                                     const double* __restrict__ hs_out, double* __restrict__ e_out,
+                                                     double penal, double emin, LpGrid g) {
+  lp_after_launch();
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ double tile[(4 + 2 * TAPS_R) * (TAPS_Y + 2 * TAPS_R) * (TAPS_X + 2 * TAPS_R)];
+  __shared__ int s_reach;
+  int* so = reinterpret_cast<int*>(smem_raw);
+  double* sw = reinterpret_cast<double*>(smem_raw + ((3 * ntaps * sizeof(int) + 15) & ~15));
+  if (threadIdx.x == 0) s_reach = 0;
+  __syncthreads();
+  int reach = 0;
+  for (int i = threadIdx.x; i < ntaps; i += blockDim.x) {
+    const int dx = toff[3 * i], dy = toff[3 * i + 1], dz = toff[3 * i + 2];
+    so[3 * i] = dx;
+    so[3 * i + 1] = dy;
+    so[3 * i + 2] = dz;
+    sw[i] = tw[i];
+    reach = max(reach, max(abs(dx), max(abs(dy), abs(dz))));
+  }
+  if (reach) atomicMax(&s_reach, reach);
+  __syncthreads();
+  const int R = s_reach;
+  const int nbx = (g.nx + TAPS_X - 1) / TAPS_X, nby = (g.ny + TAPS_Y - 1) / TAPS_Y;
+  const int bx = (int)(blockIdx.x % nbx), rest = (int)(blockIdx.x / nbx);
+  const int by = rest % nby, cz = rest / nby;
+  const int x0 = bx * TAPS_X, y0 = by * TAPS_Y;
+  const int x = x0 + (int)(threadIdx.x & 31), y = y0 + (int)(threadIdx.x >> 5);
+  const bool own = x < g.nx && y < g.ny;
+  if (R > TAPS_R) {
+    if (!own) return;
+    for (int zq = 0; zq < 4; ++zq) {
+      const int z = 4 * cz + zq;
+      if (z >= g.nz) break;
+      double acc = 0.0;
+      for (int i = 0; i < ntaps; ++i) {
+        const int xx = x + so[3 * i], yy = y + so[3 * i + 1], zz = z + so[3 * i + 2];
+        if (xx < 0 || yy < 0 || zz < 0 || xx >= g.nx || yy >= g.ny || zz >= g.nz) continue;
+        const long long c = g.cell(xx, yy, zz);
+        double vi = v[c];
+        if (hs_in) vi = vi / hs_in[c];
+        acc += sw[i] * vi;
+      }
+      const long long c = g.cell(x, y, z);
+      if (hs_out) acc = acc / hs_out[c];
+      out[c] = acc;
+      if (e_out) e_out[c] = emin + pow(acc, penal) * (1.0 - emin);
+    }
+    return;
+  }
+  const int XH = TAPS_X + 2 * R, YH = TAPS_Y + 2 * R, ZH = 4 + 2 * R, P = XH * YH;
+  const int CR = (R + 3) / 4;  // halo chunks on each side
+  // the taps' offsets in the staged tile, written over their first coordinate
+  for (int i = threadIdx.x; i < ntaps; i += blockDim.x) so[3 * i] += (so[3 * i + 2] * YH + so[3 * i + 1]) * XH;
+  // a warp stages a (chunk, y) row at a time: 4 XH doubles contiguous in memory, lanes along it
+  const int rowlen = 4 * XH, nrows = (2 * CR + 1) * YH;
+  const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5), nwarps = (int)(blockDim.x >> 5);
+  for (int row = warp; row < nrows; row += nwarps) {
+    const int cr = row / YH, yl = row - cr * YH;
+    const int gy = y0 - R + yl, zbase = 4 * (cz - CR + cr);
+    const bool yok = gy >= 0 && gy < g.ny;
+    for (int j = lane; j < rowlen; j += 32) {
+      const int xl = j >> 2, gz = zbase + (j & 3);
+      const int zl = gz - (4 * cz - R);
+      if (zl < 0 || zl >= ZH) continue;
+      const int gx = x0 - R + xl;
+      double val = 0.0;
+      if (yok && gx >= 0 && gx < g.nx && gz >= 0 && gz < g.nz) {
+        const long long c = g.cell(gx, gy, gz);
+        val = v[c];
+        if (hs_in) val = val / hs_in[c];
+      }
+      tile[(zl * YH + yl) * XH + xl] = val;
+    }
+  }
+  __syncthreads();
+  if (!own) return;
+  const int ctr = (R * YH + R + (int)(threadIdx.x >> 5)) * XH + R + (int)(threadIdx.x & 31);
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int i = 0; i < ntaps; ++i) {
+    const int o = ctr + so[3 * i];
+    const double w = sw[i];
+#pragma unroll
+    for (int zq = 0; zq < 4; ++zq) acc[zq] += w * tile[o + zq * P];
+  }
+#pragma unroll
+  for (int zq = 0; zq < 4; ++zq) {
+    const int z = 4 * cz + zq;
+    if (z >= g.nz) break;
+    const long long c = g.cell(x, y, z);
+    double r = acc[zq];
+    if (hs_out) r = r / hs_out[c];
+    out[c] = r;
+    if (e_out) e_out[c] = emin + pow(r, penal) * (1.0 - emin);
+  }
+}
+
 // ordered sum of the blocks' volumes
 __global__ void k_filter_volume(const double* __restrict__ part, int n, double* __restrict__ out) {
   lp_after_launch();
@@ -455,6 +571,7 @@ __global__ void k_oc_step_base(double* __restrict__ ts, const double* __restrict
   }
 }
 
+constexpr int NO_TMA = 1;   // nothing launched
 template <int R, class In, class Out>
 int launch_reach(const In& in, const Out& o, const int* toff, const double* tw, int ntaps, LpGrid g, bool vec,
                  double* part, int* nblocks, cudaStream_t st) {
@@ -477,15 +594,16 @@ int launch_reach(const In& in, const Out& o, const int* toff, const double* tw, 
   FilterMaps maps{};
   const uint64_t dims[4] = {4, (uint64_t)g.nx, (uint64_t)g.ny, (uint64_t)(g.cpz / 4)};
   const uint32_t box[4] = {4, FT_XH, FT_Y + 2 * R, 1};
-  // a field that TMA cannot address (not 16-byte aligned) is gathered
+  // a field that TMA cannot address (not 16-byte aligned) is a trial's to gather, a filter's to take by taps
   bool tma = lp_make_map(&maps.a, raw_a(in), 4, dims, box, 8, 32);
   if (tma && raw_b(in)) tma = lp_make_map(&maps.b, raw_b(in), 4, dims, box, 8, 32);
+  if (!tma && std::is_same<In, FilterIn>::value) return NO_TMA;
   const int smem = (raw_b(in) ? 4 : 2) * Slab<R>::BYTES + 1024;
   if (cudaFuncSetAttribute(k_filter_march<R, In, Out>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            4 * Slab<R>::BYTES + 1024) != cudaSuccess)
     return LP_ERR_LAUNCH;
   lp_launch(k_filter_march<R, In, Out>, nb, FT_THREADS, smem, st, maps, in, o, toff, tw, ntaps, g, best, tma ? 1 : 0, vec ? 1 : 0,
-                                                           part);
+            part);
   if (nblocks) *nblocks = nb;
   LP_LAUNCH_CHECK();
   return LP_OK;
@@ -497,6 +615,17 @@ int launch_march(const In& in, const Out& o, const int* toff, const double* tw, 
   if (reach <= 1) return launch_reach<1>(in, o, toff, tw, ntaps, g, vec, part, nblocks, st);
   if (reach == 2) return launch_reach<2>(in, o, toff, tw, ntaps, g, vec, part, nblocks, st);
   return launch_reach<FT_R>(in, o, toff, tw, ntaps, g, vec, part, nblocks, st);
+}
+
+int launch_taps(const FilterIn& in, const FilterOut& o, const int* toff, const double* tw, int ntaps, LpGrid g,
+                cudaStream_t st) {
+  const size_t smem = ((3 * ntaps * sizeof(int) + 15) & ~(size_t)15) + ntaps * sizeof(double);
+  const long long tiles = (long long)((g.nx + TAPS_X - 1) / TAPS_X) * ((g.ny + TAPS_Y - 1) / TAPS_Y) * ((g.nz + 3) / 4);
+  if (tiles > 2147483647LL) return LP_ERR_ARG;
+  lp_launch(k_filter_taps, (unsigned)tiles, 256, smem, st, o.out, in.v, toff, tw, ntaps, in.hs_in, o.hs_out, o.e_out, o.penal,
+            o.emin, g);
+  LP_LAUNCH_CHECK();
+  return LP_OK;
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -511,8 +640,8 @@ extern "C" {
 
 // out[c] = sum_t w_t v[c + d_t] (zeros outside the grid); optional division of v by hs_in before and
 // of the sum by hs_out after; with e_out also the SIMP law e_out = emin + out^p (1 - emin). reach: the
-// largest |offset| of the taps (the staged form is made for it; a list that reaches further is
-// gathered)
+// largest |offset| of the taps. A cone's taps, in order: the march up to reach 3 (other lists that the march
+// is given it gathers, a few times slower than lpb_filter).
 int lpb_filter_reach(double* out, const double* v, const int* toff, const double* tw, int ntaps, int reach,
                      const double* hs_in, const double* hs_out, double* e_out, double penal, double emin, LP_GRID_ARGS,
                      void* stream) {
@@ -522,12 +651,17 @@ int lpb_filter_reach(double* out, const double* v, const int* toff, const double
   const FilterIn in{v, hs_in};
   const FilterOut o{out, hs_out, e_out, penal, emin};
   const bool vec = aligned16(out) && aligned16(hs_out) && aligned16(e_out);
-  return launch_march(in, o, toff, tw, ntaps, reach, g, vec, nullptr, nullptr, LP_ST);
+  const int rc = reach > FT_R ? NO_TMA : launch_march(in, o, toff, tw, ntaps, reach, g, vec, nullptr, nullptr, LP_ST);
+  return rc == NO_TMA ? launch_taps(in, o, toff, tw, ntaps, g, LP_ST) : rc;
 }
 
+// the same for any list, its taps one after another
 int lpb_filter(double* out, const double* v, const int* toff, const double* tw, int ntaps, const double* hs_in,
                const double* hs_out, double* e_out, double penal, double emin, LP_GRID_ARGS, void* stream) {
-  return lpb_filter_reach(out, v, toff, tw, ntaps, FT_R, hs_in, hs_out, e_out, penal, emin, nx, ny, nz, pz, cpz, stream);
+  LpGrid g = LP_GRID;
+  if (!lp_grid_ok(g) || !out || !v || !toff || !tw || ntaps < 1 || ntaps > LP_MAX_TAPS) return LP_ERR_ARG;
+  if (out == v) return LP_ERR_ARG;
+  return launch_taps(FilterIn{v, hs_in}, FilterOut{out, hs_out, e_out, penal, emin}, toff, tw, ntaps, g, LP_ST);
 }
 
 // ts = x sqrt(-dc / dv): the part of the OC step that every trial multiplier shares

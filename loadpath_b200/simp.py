@@ -52,6 +52,7 @@ class DeviceFilter:
         self.reach = max(max(abs(v) for v in d) for d, _ in taps)
         self.toff = torch.tensor([list(d) for d, _ in taps], dtype=torch.int32, device=grid.device).reshape(-1)
         self.tw = torch.tensor([w for _, w in taps], dtype=torch.float64, device=grid.device)
+        self._cone = self.toff, self.tw
         self.full = float(sum(w for _, w in taps))
         ones = grid.set_cells(grid.cell_field(torch.float64), 1.0)
         self.rowsum = self.apply(grid.cell_field(torch.float64), ones)
@@ -64,10 +65,17 @@ class DeviceFilter:
 
     def apply(self, out, v, hs_in=None, hs_out=None, e_out=None, penal=3.0, emin=1e-9):
         """out = H (v / hs_in) / hs_out; with e_out also e_out = emin + out^p (1 - emin)."""
-        lib().lpb_filter_reach(out.data_ptr(), v.data_ptr(), self.toff.data_ptr(), self.tw.data_ptr(), self.ntaps,
-                               self.reach, ptr(hs_in), ptr(hs_out), ptr(e_out), float(penal), float(emin),
-                               *self.grid.args, stream_handle())
+        L = lib()
+        fn, reach = (L.lpb_filter_reach, (self.reach,)) if self.own_taps else (L.lpb_filter, ())
+        fn(out.data_ptr(), v.data_ptr(), self.toff.data_ptr(), self.tw.data_ptr(), self.ntaps, *reach, ptr(hs_in),
+           ptr(hs_out), ptr(e_out), float(penal), float(emin), *self.grid.args, stream_handle())
         return out
+
+    @property
+    def own_taps(self):
+        """Whether the taps are the cone's that this object made (not a list put in their place, which the
+        general entry is faster for)."""
+        return self.toff is self._cone[0] and self.tw is self._cone[1]
 
 
 class _HostFilter:
@@ -344,8 +352,10 @@ class ProjectedDesign:
         # A trial needs only its volume: one pass over ts = x sqrt(-dc / dv) and x forms the step, the
         # filter and the projection as it goes (lpb_oc_trial) and the last trial's design is written
         # once, after the search. Mirror planes average each trial's design before it is filtered,
-        # and taps past the fused pass's staged reach are cheaper through the filter alone.
-        fused = not self.mirror and self.flt.reach <= FUSED_REACH and x.data_ptr() != self.xn.data_ptr()
+        # and taps that the fused pass does not stage, and a field off the 16-byte boundary that its staging
+        # takes, are cheaper through the filter alone.
+        fused = (not self.mirror and self.flt.own_taps and self.flt.reach <= FUSED_REACH
+                 and x.data_ptr() != self.xn.data_ptr() and x.data_ptr() % 16 == 0)
         if fused:
             if self._ts is None:
                 self._ts = g.cell_field(torch.float64)

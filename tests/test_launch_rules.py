@@ -85,3 +85,19 @@ out = recorded()
     got = record(tmp_path, body)
     assert {r["device"] for r in got if r["what"] == "launch"} == {0, 1}
     _limits_hold(got)
+
+
+@pytest.mark.parametrize("reach,off", [(1, 0), (3, 0), (4, 0), (9, 0), (1, 8), (2, 8)])
+def test_filters_past_the_march_go_tap_by_tap(tmp_path, reach, off):
+    """Cones that reach further than the march stages, fields off the 16-byte boundary and all lists of the
+    general entry take the many small blocks of the tap kernel."""
+    args = f"P(), P() + {off}, P(), P(), 7, {{}}None, None, None, 3.0, 1e-9, 40, 20, 10, 12, 12, None"
+    body = f"""
+assert L.lpb_filter_reach({args.format(f"{reach}, ")}) == 0
+a = recorded()
+assert L.lpb_filter({args.format("")}) == 0
+out = [[r["kernel"] for r in x if r["what"] == "launch"] for x in (a, recorded())]
+"""
+    named, general = record(tmp_path, body)
+    assert len(named) == len(general) == 1 and "k_filter_taps" in general[0]
+    assert ("k_filter_taps" if reach > 3 or off else "k_filter_march") in named[0]
