@@ -89,8 +89,9 @@ int lpb_apply_weights_tma_f64(double* out, const double* u, const double* wc, co
 /* The level-1 apply with its patch cells (patch_k, and patch_m: lpb_patch_modal_* of it, the (npatch, 24, 24)
  * matrices in the corner-parity basis): mode 0 out = m K u; modes 1..3 the Chebyshev updates of
  * lpb_apply_fine_cheb_f32 formed where K u is stored (the fields a mode does not name may be NULL).
- * Small grids take the patch cells in a launch of their own behind the march; modes 1..3 do so only
- * with out given, a field of scratch of its own (any content). */
+ * Small grids, and boxes that may hold more than 64 patch cells in a tile's chunk, take the patch cells in a
+ * launch of their own behind the march; modes 1..3 do so only with out given, a field of scratch of its
+ * own (any content). */
 int lpb_patch_modal_f32(float* pm, const float* pk, long long npatch, void* stream);
 int lpb_patch_modal_f64(double* pm, const double* pk, long long npatch, void* stream);
 int lpb_apply_level1_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b, const float* dinv, const double* coef, const float* wc, const int* patch_id, const float* patch_m, const float* patch_k, const uint8_t* mask, const double* g1, const int* pbox, int* err, int nx, int ny, int nz, int pz, int cpz, void* stream);

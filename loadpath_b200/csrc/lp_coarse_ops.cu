@@ -9,13 +9,14 @@
 // neighbours through shared memory) and forms each cell's product in that basis: ~450 flops
 // against the 4608 of the dense sum. Cells touching held dofs ("patch" cells: weights zero,
 // an explicit masked matrix instead) are taken in the same march, a warp's lanes sharing a cell's
-// dense product.
+// dense product, or by a launch behind it.
 //
 // Levels >= 2 ("explicit"): K_c stored per cell, symmetric, as the 300 upper-triangle entries
 // in entry-major order (entry p of consecutive cells contiguous, so a warp's loads coalesce).
 // Two passes: a cell pass forms the 24 corner forces f_c = K_c u_c into a caller-provided
 // (24, cells) buffer, a node pass sums each node's eight cells' rows and applies the mask.
 #include <cstring>
+#include <numeric>
 
 #include "lp_common.cuh"
 #include "lp_modal.cuh"
@@ -477,7 +478,7 @@ struct L1Box {
   int x, hx, y, hy;
 };
 
-// nodes of columns [x, hx) x [y, hy) and chunks [c, hc) whose patch cells' part comes from k_patch_nodes
+// nodes of columns [x, hx) x [y, hy) and chunks [c, hc) whose patch cells' part comes from the launch behind
 struct L1Nodes {
   int x, hx, y, hy, c, hc;
 };
@@ -604,7 +605,8 @@ __device__ __noinline__ void patch_alone(const T* __restrict__ pm, int patch, co
 // warps per scheduler issue them; what can be cut is the waiting and the rest: two blocks of four
 // warps per SM, whose barriers do not meet, instead of one of eight; one barrier per chunk; masks and
 // patch indices loaded a chunk ahead of their use; the patch cells (dense products) shared by a
-// block's threads in the same launch, or in one behind it on small grids; units split evenly over the SMs instead of whole z segments. Sharing a
+// block's threads in the same launch, or in one behind it (launch_level1 says when); units split evenly over the SMs
+// instead of whole z segments. Sharing a
 // cell's rows between two warps (half the registers, twice the warps) ran 1.2x slower: the modes and
 // indices formed twice cost more issue slots than the extra warps filled.
 //
@@ -916,86 +918,234 @@ __global__ void __launch_bounds__(192) k_patch_modal(T* __restrict__ pm, const T
   }
 }
 
-// Patch cells (weights zero, an explicit masked matrix) after a march without them, node by node over the
-// nodes they touch (one warp per node: the lanes split the 8 cells x 24 columns): MODE 0 out += m * sum of
-// their rows times u; modes 1..3 the Chebyshev update from out, which the march left there, and that
-// sum (the vector kernels' expressions). All it reads but out is older than the march, the launch ahead,
-// so the products are formed while that one runs. bz0 and bnz are whole chunks in modes 1..3.
-template <typename T, int MODE>
-__global__ void __launch_bounds__(256)
-k_patch_nodes(T* __restrict__ out, const T* __restrict__ u, const int* __restrict__ pid, const T* __restrict__ pk,
-              const uint8_t* __restrict__ mask, LpGrid g, int bx0, int by0, int bz0, int bnx, int bny, int bnz,
-              L1Cheb<T> ch) {
-  const long long total = (long long)bnx * bny * bnz;
-  const long long cs = g.comp_stride(), co = 3 * cs * blockIdx.y;   // (the column)
-  const int lane = threadIdx.x & 31;
-  const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  if (warp >= total) {
-    lp_after_launch();
-    return;
+// Patch cells (weights zero, an explicit masked matrix) after a march without them, over the nodes of a box of
+// columns and whole chunks: MODE 0 out += m * sum of their rows times u; modes 1..3 the Chebyshev update from
+// out, which the march left there, and that sum (the vector kernels' expressions). All they read but out is
+// older than the march, the launch ahead, so only the finish waits for that one. Two forms, the same bits:
+//   k_patch_quads   a warp per P planes of a quad (a node column's four planes of a chunk): its lanes load the
+//                   patch indices around and split the 8 cells x 24 columns of each solved node that a
+//                   patch cell touches; three lanes finish the components
+//   k_patch_nodes   for boxes of which such cells are a small part (supports on opposite faces, scattered ones):
+//                   a thread per quad looks for them and lists their nodes, the block's warps take the
+//                   listed nodes, and a thread per quad and component finishes
+// Bound by the latency of their loads. A float32 smoothing (two updates) of 192 x 96 x 96 cells, march
+// included, against a warp per node of the box: held on two opposite x faces 74 us (221), at 40 points 65
+// (205), on one z face 53 (61), on one x face 45 (45).
+constexpr int PN_QUADS = 32;     // most quads of a block of k_patch_nodes
+constexpr int PN_THREADS = 128;
+constexpr int PQ_THREADS = 256;
+// quads from which a box takes k_patch_nodes (float32 smoothing, k_patch_quads and k_patch_nodes: two x faces of 128 x
+// 64 x 64 cells, 19305 quads, 43.1 and 42.9 us; of 192 x 96 x 96, 61740 quads, 96.4 and 71.4)
+constexpr long long PN_FROM = 32768;
+
+template <int P, typename T>
+__device__ __forceinline__ void ldcg_planes(const T* p, T (&v)[P]) {
+  if constexpr (P == 1) {
+    v[0] = __ldcg(p);
+  } else if constexpr (sizeof(T) == 4) {
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(p));
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  } else {
+    const double2 a = __ldcg(reinterpret_cast<const double2*>(p)), b = __ldcg(reinterpret_cast<const double2*>(p) + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
   }
-  const int z = bz0 + (int)(warp % bnz);
-  const long long q = warp / bnz;
-  const int y = by0 + (int)(q % bny), x = bx0 + (int)(q / bny);
-  const long long n = g.node(x, y, z);
-  const uint8_t mb = __ldcg(mask + n);
-  // a node with no solved component keeps its output (the held nodes of a support face are
-  // half of a patch box): the whole warp leaves
-  if (MODE == 0 && !(mb & 7)) {
-    lp_after_launch();
-    return;
-  }
-  // lane -> (cell corner kk = lane / 4, column block of 6 = lane % 4)
-  const int kk = lane >> 2, cb = lane & 3;
-  T a[3] = {T(0), T(0), T(0)};
+}
+
+// a warp's part of the sum at node (x, y, z): lane -> (cell corner kk = lane / 4, column block of 6 = lane % 4),
+// p the patch cell at that corner (-1: none); u: the column's field
+template <typename T>
+__device__ __forceinline__ void patch_node_part(T (&a)[3], const T* __restrict__ u, const T* __restrict__ pk, const LpGrid& g,
+                                                int x, int y, int z, int p) {
+  a[0] = a[1] = a[2] = T(0);
+  if (p < 0) return;
+  const int lane = threadIdx.x & 31, kk = lane >> 2, cb = lane & 3;
   const int cx = x - cx_(kk), cy = y - cy_(kk), cz = z - cz_(kk);
-  int p = -1;
-  if (cx >= 0 && cy >= 0 && cz >= 0 && cx < g.nx && cy < g.ny && cz < g.nz) p = __ldcg(pid + g.cell(cx, cy, cz));
-  if (p >= 0) {
-    const T* kp = pk + (long long)p * 576;
+  const T* kp = pk + (long long)p * 576;
 #pragma unroll
-    for (int c6 = 0; c6 < 6; ++c6) {
-      const int col = 6 * cb + c6, q2 = col / 3, c2 = col % 3;
-      const T uv = __ldcg(u + co + c2 * cs + g.node(cx + cx_(q2), cy + cy_(q2), cz + cz_(q2)));
+  for (int c6 = 0; c6 < 6; ++c6) {
+    const int col = 6 * cb + c6, q2 = col / 3, c2 = col % 3;
+    const T uv = __ldcg(u + c2 * g.comp_stride() + g.node(cx + cx_(q2), cy + cy_(q2), cz + cz_(q2)));
 #pragma unroll
-      for (int cc = 0; cc < 3; ++cc) a[cc] += __ldcg(kp + (3 * kk + cc) * 24 + col) * uv;
-    }
+    for (int cc = 0; cc < 3; ++cc) a[cc] += __ldcg(kp + (3 * kk + cc) * 24 + col) * uv;
   }
-  const bool any = __any_sync(0xffffffffu, p >= 0);
+}
+// the warp's sum of component lane (of lane 0..2)
+template <typename T>
+__device__ __forceinline__ T patch_node_sum(T (&a)[3]) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int cc = 0; cc < 3; ++cc)
     for (int o = 16; o > 0; o >>= 1) a[cc] += __shfl_xor_sync(0xffffffffu, a[cc], o);
-  const T av = lane == 0 ? a[0] : lane == 1 ? a[1] : a[2];   // lane cc < 3 finishes component cc
-  const long long at = (lane < 3 ? lane : 0) * cs + n, i = co + at;
-  T dv = T(0), v0 = T(0), v1 = T(0), v2 = T(0), s = T(0), c1 = T(0), c2 = T(0);
-  if constexpr (MODE != 0) {
-    s = (T)__ldcg(ch.coef + 1);
-    c1 = (T)__ldcg(ch.coef + 2);
-    c2 = (T)__ldcg(ch.coef + 3);
-    dv = __ldcg(ch.dinv + at);
-    v0 = __ldcg((MODE == 1 ? ch.d : MODE == 2 ? ch.b : ch.x) + i);
-    if (MODE != 2) v1 = __ldcg((MODE == 1 ? ch.b : ch.d) + i);
-    if (MODE == 3) v2 = __ldcg(ch.r + i);
-  }
-  lp_wait_prior();
-  lp_release_next();
-  if (lane >= 3) return;
-  const bool on = (mb >> lane) & 1;
-  if constexpr (MODE == 0) {
-    if (any && on) out[i] += av;
-  } else {
-    const T raw = out[i], ad = any && on ? raw + av : raw;
-    if constexpr (MODE == 1) {
-      ch.x[i] = lp_cheb2_zero_v(v0, v1, ad, dv, c1, c2);
-    } else if constexpr (MODE == 2) {
-      T ri, di;
-      lp_residual_scaled_v(v0, ad, dv, s, ri, di);
-      ch.r[i] = ri;
-      ch.d[i] = di;
-    } else {
-      ch.x[i] = lp_cheb2_v(v0, v1, v2, ad, dv, c1, c2);
+  return lane == 0 ? a[0] : lane == 1 ? a[1] : a[2];
+}
+
+// what a component's finish of P planes reads beside out, and the finish: ad = out with the sums added
+template <typename T, int MODE, int P>
+struct PatchFinish {
+  T dv[P], v0[P], v1[P], v2[P], s, c1, c2;
+  __device__ __forceinline__ void load(const L1Cheb<T>& ch, long long at, long long i) {
+    if constexpr (MODE != 0) {
+      s = (T)__ldcg(ch.coef + 1);
+      c1 = (T)__ldcg(ch.coef + 2);
+      c2 = (T)__ldcg(ch.coef + 3);
+      ldcg_planes<P>(ch.dinv + at, dv);
+      ldcg_planes<P>((MODE == 1 ? ch.d : MODE == 2 ? ch.b : ch.x) + i, v0);
+      if constexpr (MODE != 2) ldcg_planes<P>((MODE == 1 ? ch.b : ch.d) + i, v1);
+      if constexpr (MODE == 3) ldcg_planes<P>(ch.r + i, v2);
     }
   }
+  static __device__ __forceinline__ void save(T* p, const T (&v)[P]) {
+    if constexpr (P == 1) *p = v[0];
+    else lp_st4(p, v);
+  }
+  __device__ __forceinline__ void store(T* __restrict__ out, const L1Cheb<T>& ch, long long i, const T (&ad)[P]) const {
+    T a[P], b[P];
+#pragma unroll
+    for (int z = 0; z < P; ++z) {
+      if constexpr (MODE == 1) a[z] = lp_cheb2_zero_v(v0[z], v1[z], ad[z], dv[z], c1, c2);
+      else if constexpr (MODE == 2) lp_residual_scaled_v(v0[z], ad[z], dv[z], s, a[z], b[z]);
+      else if constexpr (MODE == 3) a[z] = lp_cheb2_v(v0[z], v1[z], v2[z], ad[z], dv[z], c1, c2);
+    }
+    if constexpr (MODE == 0) {
+      save(out + i, ad);
+    } else if constexpr (MODE == 2) {
+      save(ch.r + i, a);
+      save(ch.d + i, b);
+    } else {
+      save(ch.x + i, a);
+    }
+  }
+};
+
+template <typename T, int MODE, int P>
+__global__ void __launch_bounds__(PQ_THREADS)
+k_patch_quads(T* __restrict__ out, const T* __restrict__ u, const int* __restrict__ pid, const T* __restrict__ pk,
+              const uint8_t* __restrict__ mask, LpGrid g, int bx0, int by0, int bc0, int bnx, int bny, int bnc,
+              L1Cheb<T> ch) {
+  constexpr int H = sizeof(T) == 4 ? P : (P + 1) / 2;   // nodes whose loads are in flight together
+  const int item = (int)((blockIdx.x * (unsigned)PQ_THREADS + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  const int quad = item / (4 / P), zb = (item % (4 / P)) * P;   // the planes zb .. zb + P - 1 of the quad
+  if (quad >= bnx * bny * bnc) {
+    lp_after_launch();
+    return;
+  }
+  const long long cs = g.comp_stride(), co = 3 * cs * blockIdx.y;   // (the column)
+  const int x = bx0 + quad % bnx, y = by0 + (quad / bnx) % bny, c = bc0 + quad / (bnx * bny);
+  const long long n = g.node(x, y, 4 * c);
+  const uint32_t mb = __ldcg(reinterpret_cast<const unsigned*>(mask + n));
+  // lane -> cell of column lane % 4 (x - bit 0, y - bit 1) and plane 4 c - 1 + lane / 4
+  int pc = -1;
+  {
+    const int cx = x - (lane & 1), cy = y - ((lane >> 1) & 1), cz = 4 * c - 1 + (lane >> 2);
+    if (lane < 20 && cx >= 0 && cy >= 0 && cz >= 0 && cx < g.nx && cy < g.ny && cz < g.nz) pc = __ldcg(pid + g.cell(cx, cy, cz));
+  }
+  const unsigned have = __ballot_sync(0xffffffffu, pc >= 0);
+  unsigned todo = 0;   // the planes whose node is solved and touched: by the cells of its plane or of the one below
+#pragma unroll
+  for (int z = 0; z < P; ++z)
+    if (((mb >> (8 * (zb + z))) & 7) && ((have >> (4 * (zb + z))) & 0xff)) todo |= 1u << z;
+  T sum[P] = {};   // lane cc < 3: component cc of each plane
+  if (todo) {
+#pragma unroll
+    for (int z0 = 0; z0 < P; z0 += H) {
+      T a[H][3];
+#pragma unroll
+      for (int h = 0; h < H; ++h) {   // (the cell at corner kk: one column and plane down per set bit)
+        const int kk = lane >> 2, z = zb + z0 + h, p = __shfl_sync(0xffffffffu, pc, (kk & 3) + 4 * (z + 1 - (kk >> 2)));
+        patch_node_part<T>(a[h], u + co, pk, g, x, y, 4 * c + z, (todo >> (z0 + h)) & 1 ? p : -1);
+      }
+#pragma unroll
+      for (int h = 0; h < H; ++h)
+        if ((todo >> (z0 + h)) & 1) sum[z0 + h] = patch_node_sum<T>(a[h]);
+    }
+  }
+  const int cc = lane < 3 ? lane : 0;
+  const long long at = cc * cs + n + zb, i = co + at;
+  PatchFinish<T, MODE, P> fin;
+  fin.load(ch, at, i);
+  lp_wait_prior();
+  lp_release_next();
+  if (lane >= 3 || (MODE == 0 && !todo)) return;
+  T ad[P];
+  if constexpr (P == 1) ad[0] = out[i];
+  else lp_ld4(out + i, ad);
+#pragma unroll
+  for (int z = 0; z < P; ++z)
+    if (((todo >> z) & 1) && ((mb >> (8 * (zb + z) + cc)) & 1)) ad[z] += sum[z];
+  fin.store(out, ch, i, ad);
+}
+
+template <typename T, int MODE>
+__global__ void __launch_bounds__(PN_THREADS)
+k_patch_nodes(T* __restrict__ out, const T* __restrict__ u, const int* __restrict__ pid, const T* __restrict__ pk,
+              const uint8_t* __restrict__ mask, LpGrid g, int bx0, int by0, int bc0, int bnx, int bny, int bnc, int quads,
+              unsigned stride, L1Cheb<T> ch) {
+  __shared__ T sums[4 * PN_QUADS][3];
+  __shared__ int cells[PN_QUADS][20];      // column k (x - bit 0, y - bit 1) and plane 4 c - 1 + z at 5 k + z
+  __shared__ uint8_t touched[PN_QUADS];    // a bit per plane
+  __shared__ uint8_t list[4 * PN_QUADS];   // 4 quad + plane
+  __shared__ int count;
+  const int total = bnx * bny * bnc, tid = threadIdx.x, lane = tid & 31;
+  const long long cs = g.comp_stride(), co = 3 * cs * blockIdx.y;   // (the column)
+  // this thread's quad and component (a component past the third: none)
+  const int first = (int)((unsigned long long)blockIdx.x * stride % gridDim.x) * quads;
+  const int q = tid & (quads - 1), cc = tid / quads, quad = first + q;
+  const bool in = cc < 3 && quad < total;
+  const int x = bx0 + quad % bnx, y = by0 + (quad / bnx) % bny, c = bc0 + quad / (bnx * bny);
+  const long long n = in ? g.node(x, y, 4 * c) : 0, at = cc * cs + n, i = co + at;
+  if (tid == 0) count = 0;
+  __syncthreads();
+  const uint32_t mb = in ? __ldcg(reinterpret_cast<const unsigned*>(mask + n)) : 0;
+  if (cc == 0) {
+    unsigned bits = 0;   // bit z + 1: a patch cell in plane 4 c + z of the columns around
+    int p[4][5];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int cx = x - (k & 1), cy = y - (k >> 1);
+      const bool col = in && cx >= 0 && cy >= 0 && cx < g.nx && cy < g.ny;
+      const int* pc = pid + (col ? g.cell(cx, cy, 4 * c) : 0);
+      p[k][0] = col && c > 0 ? __ldcg(pc - g.cell_zc_stride() + 3) : -1;
+#pragma unroll
+      for (int z = 0; z < 4; ++z) p[k][z + 1] = col && 4 * c + z < g.nz ? __ldcg(pc + z) : -1;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int z = 0; z < 5; ++z) {
+        cells[q][5 * k + z] = p[k][z];
+        bits |= (p[k][z] >= 0 ? 1u : 0u) << z;
+      }
+    bits = (bits | bits >> 1) & 15;   // a node: the cells of its plane and of the one below
+#pragma unroll
+    for (int z = 0; z < 4; ++z) {
+      if (!((mb >> (8 * z)) & 7)) bits &= ~(1u << z);
+      if ((bits >> z) & 1) list[atomicAdd(&count, 1)] = 4 * q + z;   // (their order changes no bit)
+    }
+    touched[q] = bits;
+  }
+  PatchFinish<T, MODE, 4> fin;
+  if (in) fin.load(ch, at, i);
+  __syncthreads();
+  const int listed = count;
+  for (int e = tid >> 5; e < listed; e += PN_THREADS / 32) {
+    const int node = list[e], nq = first + (node >> 2), z = node & 3;
+    const int kk = lane >> 2;
+    T a[3];
+    patch_node_part<T>(a, u + co, pk, g, bx0 + nq % bnx, by0 + (nq / bnx) % bny, 4 * (bc0 + nq / (bnx * bny)) + z,
+                       cells[node >> 2][5 * (kk & 3) + z + 1 - (kk >> 2)]);
+    const T sum = patch_node_sum<T>(a);
+    if (lane < 3) sums[node][lane] = sum;
+  }
+  if (listed) __syncthreads();   // the sums are there
+  lp_wait_prior();
+  lp_release_next();
+  if (!in || (MODE == 0 && !touched[q])) return;
+  T ad[4];
+  lp_ld4(out + i, ad);
+#pragma unroll
+  for (int z = 0; z < 4; ++z)
+    if (((touched[q] >> z) & 1) && ((mb >> (8 * z + cc)) & 1)) ad[z] += sums[4 * q + z][cc];
+  fin.store(out, ch, i, ad);
 }
 
 // ---- explicit levels: packed symmetric matrices, entry-major ---------------------------------
@@ -1445,6 +1595,36 @@ static const int G1_ROWS[279] = {3, 3, 3, 3, 3, 3, 3, 3, 3, 3, 3, 3, 4, 4, 4, 4,
 static const int G1_TS[279] = {0, 0, 0, 1, 1, 2, 2, 3, 4, 4, 5, 6, 0, 0, 1, 2, 4, 4, 5, 6, 0, 0, 1, 2, 2, 3, 4, 6, 0, 0, 1, 2, 4, 4, 5, 6, 0, 0, 0, 1, 1, 2, 2, 3, 4, 4, 5, 6, 0, 0, 1, 1, 2, 3, 4, 5, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 4, 5, 5, 6, 6, 7, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 4, 5, 5, 6, 6, 7, 0, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 4, 5, 6, 0, 0, 1, 2, 2, 3, 4, 6, 0, 0, 1, 1, 2, 3, 4, 5, 0, 0, 0, 1, 1, 2, 2, 3, 4, 4, 5, 6, 0, 0, 1, 1, 1, 2, 3, 3, 4, 4, 4, 5, 5, 6, 6, 7, 0, 0, 0, 1, 1, 1, 2, 3, 4, 4, 4, 5, 5, 6, 0, 0, 1, 1, 1, 2, 3, 3, 4, 4, 4, 5, 5, 6, 6, 7, 0, 0, 0, 1, 2, 2, 2, 3, 4, 4, 4, 5, 6, 6, 0, 0, 1, 2, 2, 2, 3, 3, 4, 4, 4, 5, 5, 6, 6, 7, 0, 0, 1, 2, 2, 2, 3, 3, 4, 4, 4, 5, 5, 6, 6, 7, 0, 1, 1, 1, 2, 2, 3, 3, 3, 4, 4, 5, 5, 5, 6, 6, 6, 7, 7, 0, 1, 1, 2, 2, 2, 3, 3, 3, 4, 4, 5, 5, 5, 6, 6, 6, 7, 7, 0, 1, 1, 2, 2, 3, 3, 3, 4, 4, 4, 5, 5, 5, 6, 6, 6, 7, 7};
 static const int G1_COLS[279] = {3, 7, 14, 10, 17, 9, 20, 23, 15, 19, 22, 21, 4, 6, 9, 10, 16, 18, 21, 22, 5, 12, 15, 11, 18, 21, 17, 23, 4, 6, 9, 10, 16, 18, 21, 22, 3, 7, 14, 10, 17, 9, 20, 23, 15, 19, 22, 21, 8, 13, 11, 16, 19, 22, 20, 23, 9, 20, 4, 6, 23, 3, 7, 14, 10, 17, 21, 16, 18, 15, 19, 22, 10, 17, 3, 7, 14, 4, 6, 23, 9, 20, 22, 15, 19, 16, 18, 21, 11, 16, 18, 8, 13, 21, 5, 12, 22, 15, 19, 23, 20, 17, 5, 12, 15, 11, 18, 21, 17, 23, 8, 13, 11, 16, 19, 22, 20, 23, 3, 7, 14, 10, 17, 9, 20, 23, 15, 19, 22, 21, 15, 19, 5, 12, 22, 21, 11, 18, 3, 7, 14, 10, 17, 9, 20, 23, 11, 16, 18, 8, 13, 21, 22, 19, 4, 6, 23, 9, 20, 10, 10, 17, 3, 7, 14, 23, 9, 20, 5, 12, 22, 15, 19, 11, 18, 21, 11, 16, 18, 21, 5, 12, 22, 15, 4, 6, 23, 9, 10, 17, 15, 19, 22, 8, 13, 21, 11, 16, 3, 7, 14, 10, 17, 9, 20, 23, 9, 20, 23, 3, 7, 14, 10, 17, 8, 13, 21, 11, 16, 15, 19, 22, 21, 11, 16, 18, 15, 19, 5, 12, 22, 9, 20, 4, 6, 23, 3, 7, 14, 10, 17, 22, 15, 19, 11, 16, 18, 8, 13, 21, 10, 17, 3, 7, 14, 4, 6, 23, 9, 20, 23, 9, 20, 10, 17, 3, 7, 14, 11, 16, 18, 8, 13, 21, 5, 12, 22, 15, 19};
 
+// k_patch_nodes over the chunks of pbox (host, 6 ints: the node box of the patch cells). Nothing on fields that
+// it cannot read by four: the march has reported those (*err).
+template <typename T, int MODE>
+static void launch_patch_nodes(T* out, const T* u, const int* pid, const T* pk, const uint8_t* mask, const int* pbox,
+                               const LpGrid& g, const L1Cheb<T>& ch, int cols, cudaStream_t st) {
+  const uintptr_t fields = reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(ch.x) | reinterpret_cast<uintptr_t>(ch.r) |
+                           reinterpret_cast<uintptr_t>(ch.d) | reinterpret_cast<uintptr_t>(ch.b) |
+                           reinterpret_cast<uintptr_t>(ch.dinv);
+  if ((MODE ? fields & 15 : reinterpret_cast<uintptr_t>(out) & 15) || (reinterpret_cast<uintptr_t>(mask) & 3)) return;
+  const int c0 = pbox[2] >> 2, nc = ((pbox[2] + pbox[5] + 3) >> 2) - c0;
+  const long long total = (long long)pbox[3] * pbox[4] * nc;
+  if (total > PN_FROM) {
+    int quads = 4;   // few quads a block while that leaves the GPU short of blocks
+    while (quads < PN_QUADS && total * cols > quads * 148 * 32LL) quads *= 2;
+    // neighbouring blocks, whose quads have the same share of patch cells, go to different SMs
+    const unsigned nb = (unsigned)((total + quads - 1) / quads);
+    unsigned stride = (unsigned)(0.618 * nb) | 1;
+    while (std::gcd(stride, nb) != 1) stride += 2;
+    lp_launch(k_patch_nodes<T, MODE>, dim3(nb, cols), PN_THREADS, 0, st, out, u, pid, pk, mask, g, pbox[0], pbox[1], c0, pbox[3],
+              pbox[4], nc, quads, stride, ch);
+    return;
+  }
+  // on an x or y face most nodes of the box are touched: a warp each while they are few (192 x 96 x 96 cells,
+  // float32 smoothing: x face 45.2 us, a warp per quad 55.8; y face, twice the nodes, 62.5 and 56.1)
+  const bool face = std::min(pbox[3], pbox[4]) <= 3 && total <= 2048;
+  lp_launch(face ? k_patch_quads<T, MODE, 1> : k_patch_quads<T, MODE, 4>,
+            dim3(lp_blocks(32 * total * (face ? 4 : 1), PQ_THREADS), cols), PQ_THREADS, 0, st, out, u, pid, pk, mask, g, pbox[0],
+            pbox[1], c0, pbox[3], pbox[4], nc, ch);
+}
+
 // pbox: the node box of the patch cells (host, 6 ints), which the split weighs
 template <typename T, int MODE>
 static int launch_level1(T* out, const T* u, const T* wc, const int* pid, const T* pm, const T* pk, const uint8_t* mask,
@@ -1481,9 +1661,14 @@ static int launch_level1(T* out, const T* u, const T* wc, const int* pid, const 
   // The patch cells' products are a chunk's latency over again, which a march of a few units a block does not
   // hide: their own launch, overlapping the march, is then the faster form (applies in us, in the march and
   // apart: 64 x 32 x 32 cells 13.8 and 9.7 in float32, 27.2 and 17.0 in float64; 96 x 48 x 48, 2.2
-  // units a block, 21.0 and 19.7, 41.7 and 34.4; 128 x 64 x 64, 5.2 units, 32.7 and 35.8, 69.7 and 71.4)
+  // units a block, 21.0 and 19.7, 41.7 and 34.4; 128 x 64 x 64, 5.2 units, 32.7 and 35.8, 69.7 and 71.4). So it
+  // is where a tile's chunk may hold more cells than the block takes together, which a thread each then takes
+  // alone (in float32, on a grid of 128 x 64 x 64 cells: a z face held 93.4 and 40.7, two z faces 162.7 and
+  // 72.2; two x faces, whose box says the same, 50.6 and 50.2).
   const bool have_patches = pid && pm && pbox && pbox[3] > 0 && pbox[4] > 0 && pbox[5] > 0;
-  const bool apart = have_patches && pk && out && out != u && units <= 3 * nb;
+  const bool crowded = have_patches && (long long)std::min(LX, pbox[3] - 1) * std::min(LY, pbox[4] - 1) *
+                                               std::min(4, pbox[5] - 1) > L1_PATCH;
+  const bool apart = have_patches && pk && out && out != u && (units <= 3 * nb || crowded);
   if (nb > units) nb = units;
   // block b starts where b / nb of the total weight is reached: a chunk weighs 4, 8 in a tile that holds
   // patch cells (measured: with equal weights the support face's blocks ran 1.8x as long as the mean,
@@ -1510,17 +1695,11 @@ static int launch_level1(T* out, const T* u, const T* wc, const int* pid, const 
   }
   for (; b <= nb; ++b) split.u0[b] = (int)units;
   L1Nodes nodes{};
-  int z0 = 0, nz = 0;
-  if (apart) {
-    z0 = MODE ? pbox[2] & ~3 : pbox[2];
-    nz = (MODE ? (pbox[2] + pbox[5] + 3) & ~3 : pbox[2] + pbox[5]) - z0;
-    if (MODE) nodes = L1Nodes{pbox[0], pbox[0] + pbox[3], pbox[1], pbox[1] + pbox[4], z0 >> 2, (z0 + nz) >> 2};
-  }
+  if (apart && MODE)
+    nodes = L1Nodes{pbox[0], pbox[0] + pbox[3], pbox[1], pbox[1] + pbox[4], pbox[2] >> 2, (pbox[2] + pbox[5] + 3) >> 2};
   lp_launch(k_level1<T, MODE>, dim3((unsigned)nb, cols), LCOL, smem, st, maps, split, out, wc, patches ? pid : nullptr, pm, mask,
             gc, g, nchunks, err, ch, box, nodes);
-  if (apart)
-    lp_launch(k_patch_nodes<T, MODE>, dim3(lp_blocks((long long)pbox[3] * pbox[4] * nz * 32, 256), cols), 256, 0, st, out, u,
-              pid, pk, mask, g, pbox[0], pbox[1], z0, pbox[3], pbox[4], nz, ch);
+  if (apart) launch_patch_nodes<T, MODE>(out, u, pid, pk, mask, pbox, g, ch, cols, st);
   LP_LAUNCH_CHECK();
   return LP_OK;
 }
@@ -1533,9 +1712,7 @@ static int apply_weights_tma(T* out, const T* u, const T* wc, const int* pid, co
   const int rc = launch_level1<T, 0>(out, u, wc, nullptr, nullptr, nullptr, mask, g1, nullptr, err, g, st, L1Cheb<T>{});
   if (rc != LP_OK) return rc;
   if (pid && pk && pbox && pbox[3] > 0 && pbox[4] > 0 && pbox[5] > 0) {
-    const long long nb = (long long)pbox[3] * pbox[4] * pbox[5];
-    lp_launch(k_patch_nodes<T, 0>, lp_blocks(nb * 32, 256), 256, 0, st, out, u, pid, pk, mask, g, pbox[0], pbox[1], pbox[2],
-              pbox[3], pbox[4], pbox[5], L1Cheb<T>{});
+    launch_patch_nodes<T, 0>(out, u, pid, pk, mask, pbox, g, L1Cheb<T>{}, 1, st);
     LP_LAUNCH_CHECK();
   }
   return LP_OK;
@@ -1745,7 +1922,7 @@ int lpb_patch_modal_f64(double* pm, const double* pk, long long npatch, void* st
   return LP_OK;
 }
 
-// the level-1 apply with its patch cells (patch_m from lpb_patch_modal_*) in one launch: mode 0 out = m K u;
+// the level-1 apply with its patch cells (patch_m from lpb_patch_modal_*): mode 0 out = m K u;
 // modes 1..3 the Chebyshev updates of lpb_apply_fine_cheb_f32 (out not used; the fields a mode does
 // not name may be NULL)
 int lpb_apply_level1_f32(int mode, float* out, float* x, float* r, float* d, const float* u, const float* b,

@@ -216,8 +216,8 @@ __device__ __forceinline__ void lp_after_launch() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-// The two halves, in this order, for the kernels that load before the wait: k_patch_nodes, k_explicit_cells,
-// k_explicit_modal_cells, k_explicit_gather_cheb, k_chain_y, k_chain_s and k_chain_x. What they load there must
+// The two halves, in this order, for the kernels that load before the wait: k_patch_quads, k_patch_nodes,
+// k_explicit_cells, k_explicit_modal_cells, k_explicit_gather_cheb, k_chain_y, k_chain_s and k_chain_x. What they load there must
 // be older than the launch ahead, either because the same function launched that one and it does not write
 // it, or because its producer ends with an empty launch (k_settled, k_chain_settled) whose wait completes
 // it; where a caller's own launch may have written it, the kernel goes out in stream order (lp_launch_as). Such

@@ -101,3 +101,25 @@ out = [[r["kernel"] for r in x if r["what"] == "launch"] for x in (a, recorded()
     named, general = record(tmp_path, body)
     assert len(named) == len(general) == 1 and "k_filter_taps" in general[0]
     assert ("k_filter_taps" if reach > 3 or off else "k_filter_march") in named[0]
+
+
+@pytest.mark.parametrize("box,kernel", [
+    ("0, 0, 0, 129, 65, 2", "k_patch_quads"),      # a z face: 128 patch cells in a tile's chunk
+    ("0, 0, 0, 129, 65, 65", "k_patch_nodes"),     # supports on opposite faces
+    ("0, 0, 0, 2, 65, 65", None),                  # an x face: 32, in the march
+    ("0, 0, 0, 129, 2, 65", None),                 # a y face: 64
+])
+@pytest.mark.parametrize("mode", [0, 2])
+def test_crowded_patch_cells_leave_the_march(tmp_path, box, kernel, mode):
+    """On a grid of several units a block, patch cells stay in the level-1 march unless a tile's chunk may hold
+    more of them than the block takes together."""
+    fields = "P(), None, None, None, P(), None" if mode == 0 else "P(), d, P(), P(), d, P()"
+    body = f"""
+d, host, box = P(), np.ones(279), np.array([{box}], np.int32)
+assert L.lpb_apply_level1_f32({mode}, {fields}, P(), P(), P(), P(), P(), P(), P(), host.ctypes.data, box.ctypes.data, P(),
+                              128, 64, 64, 68, 68, None) == 0
+out = [r["kernel"] for r in recorded() if r["what"] == "launch"]
+"""
+    got = record(tmp_path, body)
+    assert "k_level1" in got[0] and len(got) == (1 if kernel is None else 2)
+    assert kernel is None or kernel in got[1]
