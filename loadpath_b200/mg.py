@@ -290,7 +290,8 @@ class DevLevel:
 class _CoarseSolve(dict):
     """The coarsest level's direct solve: chain (the workspace of lp_chain.cu's blocks, or None), or the
     band's dense inverse ainv with its scratch v; n dofs on grid. With the chain in use, ainv is
-    formed from the same band when it is first asked for."""
+    formed from the same band when it is first asked for, while this is its owner's hierarchy (a
+    rebuild writes another operator over the band)."""
 
     def __init__(self, ge, **kw):
         super().__init__(**kw)
@@ -300,6 +301,8 @@ class _CoarseSolve(dict):
         if key != "ainv":
             raise KeyError(key)
         ge = self._ge()
+        if ge is None or ge._coarse is not self:
+            raise RuntimeError("the band of this coarse solve is gone: its owner built another hierarchy or was released")
         ge._join_coarse()
         ge._band_buffers(self["v"].numel() // 32)
         ge._band_inverse()
