@@ -447,8 +447,9 @@ int lpb_live_outside(const uint8_t* state, const uint8_t* keep, double* part, do
  * update over n variables and m <= 8 constraints, float64, device arrays; P, Q, df are (m, n)
  * row-major. `part` is scratch of lpb_mma_part_len(m) doubles; each reduction writes its values to
  * `out` / `bsum` (device) with M = m rounded up to 1, 2, 4 or 8 entries per m-sized group.
- * lam / dlam are HOST pointers to m doubles. The host runs the interior-point loops and the
- * (m + 1) x (m + 1) Newton system (loadpath/mma.py:127-214). */
+ * lam / dlam are HOST pointers to m doubles. The interior-point loops and the (m + 1) x (m + 1) Newton
+ * system (loadpath/mma.py:127-214) run on the device (lpb_mma_loop_*), or on the host around
+ * lpb_mma_newton_a, lpb_mma_newton_b and lpb_mma_trial. */
 long long lpb_mma_part_len(int m);
 /* sanitise x, df0, df in place (non-finite values as the reference reads them), move the
  * asymptotes (init: the first two iterations), alfa/beta, p0 q0 P Q; bsum[i] = sum_j P_ij / (upp_j -
@@ -465,7 +466,6 @@ int lpb_mma_newton_b(long long n, int m, const double* low, const double* upp, c
 /* (xs, xsi, eta) = (xs0, xsi0, eta0) + steg (dx, dxsi, deta) (dx NULL: evaluate at xs0 only);
  * out = [sum of squares, largest magnitude of the residual's n-sized rows, gvec (M)] */
 int lpb_mma_trial(long long n, int m, const double* low, const double* upp, const double* alfa, const double* beta, const double* p0, const double* q0, const double* P, const double* Q, const double* xs0, const double* xsi0, const double* eta0, const double* dx, const double* dxsi, const double* deta, double steg, const double* lam, double epsi, double* xs, double* xsi, double* eta, double* part, double* out, void* stream);
-/* xnew = clip(finite(xs) ? xs : x, alfa, beta)   (loadpath/mma.py:104-108) */
 /* the subproblem's loops on the device: lpb_mma_loop_begin writes the starting state (b = bsum - f; a, c,
  * d, f HOST pointers to m doubles), lpb_mma_loop_body records one body (four launches) between
  * lpb_while_begin and lpb_while_end, the sets (x0, xsi0, eta0) from lpb_mma_sub_init and (x1, ...) scratch.
@@ -474,6 +474,7 @@ int lpb_mma_trial(long long n, int m, const double* low, const double* upp, cons
 int lpb_mma_state_len(void);
 int lpb_mma_loop_begin(int m, double* state, const double* bsum, const double* a, const double* c, const double* d, const double* f, double a0, double epsimin, void* stream);
 int lpb_mma_loop_body(long long handle, long long n, int m, const double* low, const double* upp, const double* alfa, const double* beta, const double* p0, const double* q0, const double* P, const double* Q, double* x0, double* xsi0, double* eta0, double* x1, double* xsi1, double* eta1, double* state, double* part, void* stream);
+/* xnew = clip(finite(xs) ? xs : x, alfa, beta)   (loadpath/mma.py:104-108) */
 int lpb_mma_finish(long long n, const double* xs, const double* x, const double* alfa, const double* beta, double* xnew, void* stream);
 
 

@@ -12,7 +12,7 @@
 // Why. The band's factor and inverse are chains over all tile rows (one panel solve, product and pivot
 // factor per 32 dofs, 9-10 us each) and the dense inverse of all n dofs is read whole by every solve:
 // 411 MB at 31 x 11 x 7 nodes, 136 MB at 17 x 9 x 9. Here the segments are inverted side by side, so
-// the chain is one segment's dofs and then the separators', and the stored blocks are 110 and 50 MB.
+// the chain is one segment's dofs and then the separators', and a solve reads 96 and 48 MB.
 //
 // Inverses are symmetric sweeps in place, 32 pivots at a time: with P = A_KK^-1 and Q = A_:K P,
 //   A_KK <- -P,  A_:K <- Q,  A_rc <- A_rc - Q_r A_cK^T,
@@ -50,8 +50,9 @@ struct Chain {
   __host__ __device__ int sep(int k) const { return start[k + 1] - 1; }   // plane of separator k
 };
 
-// Segment lengths: the P that minimizes the sweeps' time, steps in sequence (5 us each) plus their
-// operations (at 12 TFLOP/s); false when the band is the better form (too few planes to cut, or a plane
+// Segment lengths: the P that minimizes the sweeps' steps in sequence, at 5 us each, plus their operations, at 12
+// TFLOP/s (a step alone is 5 us and its tiles the rest of the 12 to 15 us that it takes beside the power
+// iterations); false when the band is the better form (too few planes to cut, or a plane
 // or chain beyond the tables).
 bool chain_plan(int nx, int ny, int nz, Chain& c) {
   c.bd = lp_band(nx + 1, ny + 1, nz + 1);

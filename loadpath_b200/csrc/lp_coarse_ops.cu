@@ -928,14 +928,14 @@ __global__ void __launch_bounds__(192) k_patch_modal(T* __restrict__ pm, const T
 //   k_patch_nodes   for boxes of which such cells are a small part (supports on opposite faces, scattered ones):
 //                   a thread per quad looks for them and lists their nodes, the block's warps take the
 //                   listed nodes, and a thread per quad and component finishes
-// Bound by the latency of their loads. A float32 smoothing (two updates) of 192 x 96 x 96 cells, march
+// Bound by the latency of their loads. A float32 smoothing (two updates) of 96 x 48 x 48 level-1 cells, march
 // included, against a warp per node of the box: held on two opposite x faces 74 us (221), at 40 points 65
 // (205), on one z face 53 (61), on one x face 45 (45).
 constexpr int PN_QUADS = 32;     // most quads of a block of k_patch_nodes
 constexpr int PN_THREADS = 128;
 constexpr int PQ_THREADS = 256;
-// quads from which a box takes k_patch_nodes (float32 smoothing, k_patch_quads and k_patch_nodes: two x faces of 128 x
-// 64 x 64 cells, 19305 quads, 43.1 and 42.9 us; of 192 x 96 x 96, 61740 quads, 96.4 and 71.4)
+// quads from which a box takes k_patch_nodes (float32 smoothing, k_patch_quads and k_patch_nodes: two x faces of 64 x
+// 32 x 32 cells, 19305 quads, 43.1 and 42.9 us; of 96 x 48 x 48, 61789 quads, 96.4 and 71.4)
 constexpr long long PN_FROM = 32768;
 
 template <int P, typename T>
@@ -1595,8 +1595,8 @@ static const int G1_ROWS[279] = {3, 3, 3, 3, 3, 3, 3, 3, 3, 3, 3, 3, 4, 4, 4, 4,
 static const int G1_TS[279] = {0, 0, 0, 1, 1, 2, 2, 3, 4, 4, 5, 6, 0, 0, 1, 2, 4, 4, 5, 6, 0, 0, 1, 2, 2, 3, 4, 6, 0, 0, 1, 2, 4, 4, 5, 6, 0, 0, 0, 1, 1, 2, 2, 3, 4, 4, 5, 6, 0, 0, 1, 1, 2, 3, 4, 5, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 4, 5, 5, 6, 6, 7, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 4, 5, 5, 6, 6, 7, 0, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 4, 5, 6, 0, 0, 1, 2, 2, 3, 4, 6, 0, 0, 1, 1, 2, 3, 4, 5, 0, 0, 0, 1, 1, 2, 2, 3, 4, 4, 5, 6, 0, 0, 1, 1, 1, 2, 3, 3, 4, 4, 4, 5, 5, 6, 6, 7, 0, 0, 0, 1, 1, 1, 2, 3, 4, 4, 4, 5, 5, 6, 0, 0, 1, 1, 1, 2, 3, 3, 4, 4, 4, 5, 5, 6, 6, 7, 0, 0, 0, 1, 2, 2, 2, 3, 4, 4, 4, 5, 6, 6, 0, 0, 1, 2, 2, 2, 3, 3, 4, 4, 4, 5, 5, 6, 6, 7, 0, 0, 1, 2, 2, 2, 3, 3, 4, 4, 4, 5, 5, 6, 6, 7, 0, 1, 1, 1, 2, 2, 3, 3, 3, 4, 4, 5, 5, 5, 6, 6, 6, 7, 7, 0, 1, 1, 2, 2, 2, 3, 3, 3, 4, 4, 5, 5, 5, 6, 6, 6, 7, 7, 0, 1, 1, 2, 2, 3, 3, 3, 4, 4, 4, 5, 5, 5, 6, 6, 6, 7, 7};
 static const int G1_COLS[279] = {3, 7, 14, 10, 17, 9, 20, 23, 15, 19, 22, 21, 4, 6, 9, 10, 16, 18, 21, 22, 5, 12, 15, 11, 18, 21, 17, 23, 4, 6, 9, 10, 16, 18, 21, 22, 3, 7, 14, 10, 17, 9, 20, 23, 15, 19, 22, 21, 8, 13, 11, 16, 19, 22, 20, 23, 9, 20, 4, 6, 23, 3, 7, 14, 10, 17, 21, 16, 18, 15, 19, 22, 10, 17, 3, 7, 14, 4, 6, 23, 9, 20, 22, 15, 19, 16, 18, 21, 11, 16, 18, 8, 13, 21, 5, 12, 22, 15, 19, 23, 20, 17, 5, 12, 15, 11, 18, 21, 17, 23, 8, 13, 11, 16, 19, 22, 20, 23, 3, 7, 14, 10, 17, 9, 20, 23, 15, 19, 22, 21, 15, 19, 5, 12, 22, 21, 11, 18, 3, 7, 14, 10, 17, 9, 20, 23, 11, 16, 18, 8, 13, 21, 22, 19, 4, 6, 23, 9, 20, 10, 10, 17, 3, 7, 14, 23, 9, 20, 5, 12, 22, 15, 19, 11, 18, 21, 11, 16, 18, 21, 5, 12, 22, 15, 4, 6, 23, 9, 10, 17, 15, 19, 22, 8, 13, 21, 11, 16, 3, 7, 14, 10, 17, 9, 20, 23, 9, 20, 23, 3, 7, 14, 10, 17, 8, 13, 21, 11, 16, 15, 19, 22, 21, 11, 16, 18, 15, 19, 5, 12, 22, 9, 20, 4, 6, 23, 3, 7, 14, 10, 17, 22, 15, 19, 11, 16, 18, 8, 13, 21, 10, 17, 3, 7, 14, 4, 6, 23, 9, 20, 23, 9, 20, 10, 17, 3, 7, 14, 11, 16, 18, 8, 13, 21, 5, 12, 22, 15, 19};
 
-// k_patch_nodes over the chunks of pbox (host, 6 ints: the node box of the patch cells). Nothing on fields that
-// it cannot read by four: the march has reported those (*err).
+// The patch cells' launch over the chunks of pbox (host, 6 ints: their node box). Nothing on fields that it cannot
+// read by four: the march has reported those (*err).
 template <typename T, int MODE>
 static void launch_patch_nodes(T* out, const T* u, const int* pid, const T* pk, const uint8_t* mask, const int* pbox,
                                const LpGrid& g, const L1Cheb<T>& ch, int cols, cudaStream_t st) {
@@ -1617,7 +1617,7 @@ static void launch_patch_nodes(T* out, const T* u, const int* pid, const T* pk, 
               pbox[4], nc, quads, stride, ch);
     return;
   }
-  // on an x or y face most nodes of the box are touched: a warp each while they are few (192 x 96 x 96 cells,
+  // on an x or y face most nodes of the box are touched: a warp each while they are few (96 x 48 x 48 cells,
   // float32 smoothing: x face 45.2 us, a warp per quad 55.8; y face, twice the nodes, 62.5 and 56.1)
   const bool face = std::min(pbox[3], pbox[4]) <= 3 && total <= 2048;
   lp_launch(face ? k_patch_quads<T, MODE, 1> : k_patch_quads<T, MODE, 4>,

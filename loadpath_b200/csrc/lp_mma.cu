@@ -14,8 +14,8 @@
 //   lpb_mma_finish    non-finite results back to the old design, clip to [alfa, beta]
 //   lpb_mma_loop_*    the whole subproblem on the device: the loops as a graph's while node, the m-sized
 //                     variables and the (m + 1) system in a state block (below)
-// With newton_a, newton_b and trial the host runs the loops, the m-sized parts of the residual and the
-// (m + 1) x (m + 1) solve.
+// newton_a, newton_b and trial are the same steps for a caller whose host runs the loops, the m-sized parts of the
+// residual and the (m + 1) x (m + 1) solve.
 // Reductions go through fixed per-block partials summed in order (the same bits every run).
 #include <math.h>
 
@@ -882,6 +882,7 @@ int lpb_mma_loop_body(long long handle, long long n, int m, const double* low, c
   return LP_OK;
 }
 
+// xnew = clip(finite(xs) ? xs : x, alfa, beta)
 int lpb_mma_finish(long long n, const double* xs, const double* x, const double* alfa, const double* beta,
                    double* xnew, void* stream) {
   if (n < 1 || !xs || !x || !alfa || !beta || !xnew) return LP_ERR_ARG;

@@ -158,7 +158,7 @@ class DevLevel:
         self.scratch = None      # weights: level1's
         self.mask = None
         self.dinv = None
-        self.coef = None         # device: lmax and the Chebyshev coefficients (lpb_cheb_coef)
+        self.coef = None         # device: lmax and the Chebyshev coefficients (lpb_pw_coef)
         self.n_active = 0
 
     @property
