@@ -66,16 +66,20 @@ class DeviceFilter:
     def apply(self, out, v, hs_in=None, hs_out=None, e_out=None, penal=3.0, emin=1e-9):
         """out = H (v / hs_in) / hs_out; with e_out also e_out = emin + out^p (1 - emin)."""
         L = lib()
-        fn, reach = (L.lpb_filter_reach, (self.reach,)) if self.own_taps else (L.lpb_filter, ())
+        fn, reach = (L.lpb_filter_reach, (self.reach,)) if self._own_taps() else (L.lpb_filter, ())
         fn(out.data_ptr(), v.data_ptr(), self.toff.data_ptr(), self.tw.data_ptr(), self.ntaps, *reach, ptr(hs_in),
            ptr(hs_out), ptr(e_out), float(penal), float(emin), *self.grid.args, stream_handle())
         return out
 
-    @property
-    def own_taps(self):
+    def _own_taps(self):
         """Whether the taps are the cone's that this object made (not a list put in their place, which the
         general entry is faster for)."""
         return self.toff is self._cone[0] and self.tw is self._cone[1]
+
+    @property
+    def cone(self):
+        """Whether apply is this class's, with its own taps: what another pass may take the taps for."""
+        return type(self).apply is DeviceFilter.apply and "apply" not in vars(self) and self._own_taps()
 
 
 class _HostFilter:
@@ -353,8 +357,10 @@ class ProjectedDesign:
         # filter and the projection as it goes (lpb_oc_trial) and the last trial's design is written
         # once, after the search. Mirror planes average each trial's design before it is filtered,
         # and taps that the fused pass does not stage, and a field off the 16-byte boundary that its staging
-        # takes, are cheaper through the filter alone.
-        fused = (not self.mirror and self.flt.own_taps and self.flt.reach <= FUSED_REACH
+        # takes, are cheaper through the filter alone. A filter or a physical density of the caller's own
+        # (apply or physical overridden) is asked for each trial.
+        fused = (not self.mirror and getattr(self.flt, "cone", False) and self.flt.reach <= FUSED_REACH
+                 and type(self).physical is ProjectedDesign.physical and "physical" not in vars(self)
                  and x.data_ptr() != self.xn.data_ptr() and x.data_ptr() % 16 == 0)
         if fused:
             if self._ts is None:
