@@ -1200,7 +1200,10 @@ class GridElasticity:
         nb = 8 * n
         part = self._part_cg
         sfx = "f64" if r32 is None else "f32"
-        starts = self._starts(0)
+        # (a float64 solve asks a preconditioner of the caller's own, precondition_device overridden, each time)
+        other = r32 is None and (type(self).precondition_device is not GridElasticity.precondition_device
+                                 or "precondition_device" in vars(self))
+        starts = self._starts(0) and not other
         src = self._buf("cg_b", g, torch.float64)
         if b.data_ptr() != src.data_ptr():
             L.lpb_memcpy_async(src.data_ptr(), b.data_ptr(), nb, stream_handle())
@@ -1246,9 +1249,9 @@ class GridElasticity:
         def tail():
             # z = V(r); r.z; x += alpha p; p = z + (rz_new / rz) p
             st = stream_handle()
-            z = self._vcycle(0, r if r32 is None else r32, starts)
-            getattr(L, f"lpb_cg_rz_{sfx}")(r.data_ptr(), z.data_ptr(), n, part.data_ptr(), 1, st)
-            getattr(L, f"lpb_cg_p_{sfx}")(p.data_ptr(), x.data_ptr(), z.data_ptr(), n, sc.data_ptr(), part.data_ptr(), 1,
+            zv = self.precondition_device(r, z) if other else self._vcycle(0, r if r32 is None else r32, starts)
+            getattr(L, f"lpb_cg_rz_{sfx}")(r.data_ptr(), zv.data_ptr(), n, part.data_ptr(), 1, st)
+            getattr(L, f"lpb_cg_p_{sfx}")(p.data_ptr(), x.data_ptr(), zv.data_ptr(), n, sc.data_ptr(), part.data_ptr(), 1,
                                           st)
 
         warm = x0 is not None
