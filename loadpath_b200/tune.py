@@ -113,13 +113,16 @@ def save(path):
 
 def load(path):
     """Results saved by save(); they take effect for grids tuned again in this process (which
-    then reuses them without timing)."""
+    then reuses them without timing). Level-1 results timed over other values than blocks per SM (files
+    of the time when that knob was the length of a z segment) are left out, and their grids timed again."""
     if not os.path.exists(path):
         return 0
     with open(path) as fh:
         d = json.load(fh)
     for k, v in d.items():
         name, nx, ny, nz = k.split()
-        _RESULTS[(name, int(nx), int(ny), int(nz))] = {"best": int(v["best"]),
-                                                         "us": {int(z): t for z, t in v["us"].items()}}
+        us = {int(z): t for z, t in v["us"].items()}
+        if name.startswith("level1") and not set(us) <= set(candidates(BLOCKS_PER_SM, 1)):
+            continue
+        _RESULTS[(name, int(nx), int(ny), int(nz))] = {"best": int(v["best"]), "us": us}
     return len(d)
