@@ -1708,7 +1708,7 @@ static int launch_level1(T* out, const T* u, const T* wc, const int* pid, const 
 template <typename T>
 static int apply_weights_tma(T* out, const T* u, const T* wc, const int* pid, const T* pk, const uint8_t* mask,
                              const double* g1, const int* pbox, int* err, LpGrid g, cudaStream_t st) {
-  if (out == u) return LP_ERR_ARG;
+  if (out == u || (reinterpret_cast<uintptr_t>(out) & 15)) return LP_ERR_ARG;
   const int rc = launch_level1<T, 0>(out, u, wc, nullptr, nullptr, nullptr, mask, g1, nullptr, err, g, st, L1Cheb<T>{});
   if (rc != LP_OK) return rc;
   if (pid && pk && pbox && pbox[3] > 0 && pbox[4] > 0 && pbox[5] > 0) {

@@ -123,3 +123,21 @@ out = [r["kernel"] for r in recorded() if r["what"] == "launch"]
     got = record(tmp_path, body)
     assert "k_level1" in got[0] and len(got) == (1 if kernel is None else 2)
     assert kernel is None or kernel in got[1]
+
+
+@pytest.mark.parametrize("fields", ["P() + 8, P()", "P(), P() + 8", "d, d"])
+def test_level1_apply_refuses_what_it_cannot_address(tmp_path, fields):
+    """An output or input off the 16-byte boundary, or the two the same, is refused before anything is launched."""
+    body = f"""
+from loadpath_b200._lib import LpError
+d, host = P(), np.ones(279)
+out = []
+for fn in (L.lpb_apply_weights_tma_f32, L.lpb_apply_weights_tma_f64):
+    try:
+        fn({fields}, P(), None, None, P(), host.ctypes.data, None, P(), 8, 4, 11, 12, 12, None)
+        out.append("taken")
+    except LpError:
+        out.append("refused")
+out.append(sum(r["what"] == "launch" for r in recorded()))
+"""
+    assert record(tmp_path, body) == ["refused", "refused", 0]
