@@ -27,14 +27,15 @@ KNOBS = {"fine_f32": 1, "fine_f64": 2, "level1_f32": 3, "level1_f64": 4}
 _RESULTS = {}        # (knob name, nx, ny, nz) -> {"best": value, "us": {value: time}}
 
 
-def candidates(most, lo):
-    """Knob values to time: a geometric spread from lo up to most (and 0, the launcher's own choice)."""
-    c = {0, most}
+def candidates(nchunks, lo):
+    """Knob values to time: a geometric spread from lo up to nchunks, the most there can be (and 0, the
+    launcher's own choice)."""
+    c = {0, nchunks}
     v = lo
-    while v < most:
+    while v < nchunks:
         c.add(v)
         v = v + 1 if v < 4 else int(v * 1.5)
-    return sorted(x for x in c if x == 0 or lo <= x <= most)
+    return sorted(x for x in c if x == 0 or lo <= x <= nchunks)
 
 
 def _time(fn, reps):
@@ -49,6 +50,7 @@ def _time(fn, reps):
 
 
 BLOCKS_PER_SM = 2        # the most any of the applies keeps resident
+FINE_CANDIDATES = tuple(candidates(BLOCKS_PER_SM, 1))   # persistent blocks per SM (0: all that fit)
 
 
 def _tune_one(name, grid, fn, reps):
@@ -59,7 +61,7 @@ def _tune_one(name, grid, fn, reps):
         L.lpb_tune_set(knob, grid.nx, grid.ny, grid.nz, _RESULTS[key]["best"])
         return _RESULTS[key]
     times = {}
-    for z in candidates(BLOCKS_PER_SM, 1):
+    for z in FINE_CANDIDATES:
         L.lpb_tune_set(knob, grid.nx, grid.ny, grid.nz, z)
         times[z] = _time(fn, reps)
     best = min(times, key=times.get)
@@ -122,7 +124,7 @@ def load(path):
     for k, v in d.items():
         name, nx, ny, nz = k.split()
         us = {int(z): t for z, t in v["us"].items()}
-        if name.startswith("level1") and not set(us) <= set(candidates(BLOCKS_PER_SM, 1)):
+        if name.startswith("level1") and not set(us) <= set(FINE_CANDIDATES):
             continue
         _RESULTS[(name, int(nx), int(ny), int(nz))] = {"best": int(v["best"]), "us": us}
     return len(d)

@@ -20,3 +20,10 @@ def test_files_of_segment_lengths_are_timed_again(tmp_path, monkeypatch):
     want = dict(tune._RESULTS)
     tune._RESULTS.clear()
     assert tune.load(path) == 2 and tune._RESULTS == want
+
+
+def test_candidates_keep_their_interface():
+    from loadpath_b200 import tune
+
+    assert tune.candidates(nchunks=9, lo=2) == [0, 2, 3, 4, 6, 9]
+    assert tune.FINE_CANDIDATES == (0, 1, 2)
