@@ -50,8 +50,8 @@ struct Chain {
   __host__ __device__ int sep(int k) const { return start[k + 1] - 1; }   // plane of separator k
 };
 
-// Segment lengths: the P that minimizes the sweeps' steps in sequence, at 5 us each, plus their operations, at 12
-// TFLOP/s (a step alone is 5 us and its tiles the rest of the 12 to 15 us that it takes beside the power
+// Segment lengths: the P that minimizes the sweeps' steps in sequence, priced at 5 us each, plus their operations,
+// at 12 TFLOP/s (measured, a step with its operations takes 11 us alone and 12 to 15 beside the power
 // iterations); false when the band is the better form (too few planes to cut, or a plane
 // or chain beyond the tables).
 bool chain_plan(int nx, int ny, int nz, Chain& c) {
