@@ -10,6 +10,9 @@ zero. Host arrays are in grid order, (3, NX, NY, NZ) for nodes and (nx, ny, nz) 
 """
 from __future__ import annotations
 
+import contextlib
+import threading
+
 import numpy as np
 import torch
 
@@ -31,6 +34,47 @@ def stream_handle() -> int:
 
 def ptr(t) -> int | None:
     return None if t is None else t.data_ptr()
+
+
+_recording = threading.local()
+_late = []   # (device, free, exec) of objects collected during a capture
+
+
+@contextlib.contextmanager
+def recording():
+    """Around each capture of this package: Python may collect another solver in it (one that an
+    exception's traceback held), and the wait before its graphs are freed would end the capture."""
+    _recording.depth = getattr(_recording, "depth", 0) + 1
+    try:
+        yield
+    finally:
+        _recording.depth -= 1
+        free_late()
+
+
+def capturing() -> bool:
+    """Whether this thread records a graph: one of this package, or its caller's on the current stream."""
+    if getattr(_recording, "depth", 0):
+        return True
+    return torch.cuda.is_initialized() and torch.cuda.is_current_stream_capturing()
+
+
+def free_later(device, free, execs):
+    """Graphs of an object that went during a capture: freed behind it."""
+    _late.extend((device, free, e) for e in execs)
+
+
+def free_late():
+    if not _late or capturing():
+        return
+    items = []
+    with contextlib.suppress(IndexError):      # (each taken by one thread)
+        while True:
+            items.append(_late.pop())
+    for device in {d for d, _, _ in items}:
+        torch.cuda.synchronize(device)
+    for _, free, e in items:
+        free(e)
 
 
 class DevGrid:

@@ -32,7 +32,7 @@ import torch
 
 from . import fem
 from ._lib import LpError, add_launches, launches, lib
-from .grid import DevGrid, ptr, stream_handle, torch_dtype
+from .grid import DevGrid, capturing, free_late, free_later, ptr, recording, stream_handle, torch_dtype
 
 __all__ = ["GridElasticity", "BoxMesh", "LMAX_SAFETY", "STALL", "prolong", "restrict"]
 
@@ -1141,7 +1141,7 @@ class GridElasticity:
             c0 = launches()
             # captured on a side stream (the legacy default stream cannot be captured), launched
             # on the working stream
-            with torch.cuda.stream(self._cap_stream):
+            with torch.cuda.stream(self._cap_stream), recording():
                 st0 = stream_handle()
                 if loop:
                     handle, outer = ctypes.c_longlong(), ctypes.c_void_p()
@@ -1817,7 +1817,11 @@ class GridElasticity:
 
     def __del__(self):
         try:
-            self._free_graphs()
+            if capturing():
+                free_later(self.device, lib().lpb_graph_free, [v[0] for k, v in self._gcache.items() if k != "sig"])
+            else:
+                self._free_graphs()
+                free_late()
         except Exception:
             pass
 

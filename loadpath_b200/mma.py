@@ -25,7 +25,7 @@ import numpy as np
 import torch
 
 from ._lib import add_launches, launches, lib
-from .grid import stream_handle
+from .grid import capturing, free_late, free_later, recording, stream_handle
 
 __all__ = ["MMA"]
 
@@ -116,7 +116,7 @@ class MMA:
             self._free_loop()
             L = lib()
             c0 = launches()
-            with torch.cuda.device(self.device), torch.cuda.stream(torch.cuda.Stream(self.device)):
+            with torch.cuda.device(self.device), torch.cuda.stream(torch.cuda.Stream(self.device)), recording():
                 st = stream_handle()
                 handle, outer, exec_ = ctypes.c_longlong(), ctypes.c_void_p(), ctypes.c_void_p()
                 L.lpb_while_begin(st, ctypes.byref(handle), ctypes.byref(outer))
@@ -163,6 +163,10 @@ class MMA:
     def __del__(self):
         if getattr(self, "_exec", None) is not None:
             try:
-                self._free_loop()
+                if capturing():
+                    free_later(self.device, lib().lpb_graph_free, [self._exec])
+                else:
+                    self._free_loop()
+                    free_late()
             except Exception:
                 pass
